@@ -7,7 +7,10 @@
 // implicit: the internal node splitting at s has local id s - 1, found by a
 // root-to-node descent per node. Optionally the reference's kd-median tree
 // (ModifiedKdBVH.h:207-237) is built on the host and uploaded (bh_tree = 1).
-// Local ids: internal nodes 0..n-2, leaf of object position p = n-1+p.
+// Storage: the two children of a node lie side by side, at an even position
+// of the loop's record arrays (node_place), so that the headers of a pair of
+// siblings share one 128-byte line; the root is at position 1, and position 0
+// is unused. A node's id in the traversal is its position.
 //
 // Moments (compute_link.h:95-114, compute_link.cpp:333-389) are built in
 // FP64 bottom-up: each leaf thread walks to the root; at every parent the
@@ -123,13 +126,13 @@ struct __align__(32) NodeHdr {
   double m[3];      // centre (leaves: segment midpoint)
   double r;         // half the box diagonal
   double rsq;       // its square, 0.25 |diag|^2, for the reference's split rule
-  int32_t left;     // internal: local child ids; leaf: left = -1 - segment
-  int32_t right;
+  int32_t left;     // internal: position of the first child (the second follows it); leaf: -1 - segment
   int32_t lo;       // leaf: its segment; curve-order node: first segment of its range
   int32_t cnt;      // leaves below (curve-order: the range is [lo, lo + cnt))
   float tn;         // |c_M| and ||C_D||_F / sqrt(3) of the node's moments: the
   float dn;         // Eq. 14 weights, formed when a pair is classified far
-};                  // 64 B: two 32-byte loads (load_hdr), never across a 128 B line
+  int32_t pad;
+};                  // 64 B: two 32-byte loads (load_hdr); two siblings fill one 128 B line
 static_assert(sizeof(NodeHdr) == 64, "NodeHdr layout");
 struct __align__(32) NodeMom {
   float t[3];
@@ -227,15 +230,29 @@ struct TreeArgs {
   const int64_t *node_base;  // loop -> first global node
   const int32_t *loops;      // loops that need a tree
   int32_t nloops;
-  int32_t *children;         // 2 per global node (internal nodes only used)
-  int32_t *parent;           // per global node
-  int32_t *leaf_seg;         // per global node: segment of a leaf (kd trees permute)
-  int32_t *arrive;           // per global node: arrival counter
-  BuildNode *bn;              // per internal node: bn[int_start[k] + id] for the k-th listed loop
+  // Curve-order trees: build records by internal node, bn[sum of (n - 1) over
+  // the earlier listed loops + split - 1]; place[the same] = (position of the
+  // node, position of its first child).
+  // kd-median trees: everything by node position (base + position).
+  BuildNode *bn;
+  int2 *place;
+  int32_t *children;         // kd: position of the first child; -1 for a leaf
+  int32_t *parent;           // kd: position of the parent; -1 for the root
+  int32_t *leaf_seg;         // kd: segment of a leaf
+  int32_t *arrive;           // kd: arrival counter
+  int32_t *leaf_pos;         // kd: position of the leaf of each object (by listed loop)
   NodeHdr *hdr;
   NodeMom *mom;
-  const int64_t *int_start;   // listed loop -> first build record (sum of (n - 1) before it)
 };
+
+// Storage position of the first child of a node of a loop's tree: the node
+// covers the leaves [lo, ...) in tree order and its path from the root turns
+// left `lefts` times. A subtree of m leaves takes 2 m - 2 positions below its
+// root; the children of a node come first, then the left child's subtree, then
+// the right child's. So the left child's children lie 2 further, the right
+// child's 2 x (leaves of the left child) further, and over a path that adds up
+// to 2 (lo + lefts). The root, at position 1, has its children at 2.
+__host__ __device__ __forceinline__ int32_t child_place(int64_t lo, int lefts) { return (int32_t)(2 * (lo + lefts) + 2); }
 
 __device__ __forceinline__ int find_loop_of(const int64_t *start, int n, int64_t x) {
   int lo = 0, hi = n;
@@ -281,15 +298,15 @@ __device__ __forceinline__ int32_t add_one_rank(int32_t *count, int32_t key, boo
 }
 
 // Curve-order topology: thread per internal node (local id s - 1 splits at s).
-// seg_start[k] = sum of (n - 1) over the first k listed loops. With height
-// != nullptr it also records the node's height ceil(log2(range size)) (the
-// children of a node are always lower) and counts the nodes per height.
+// seg_start[k] = sum of (n - 1) over the first k listed loops. It also
+// records the node's height ceil(log2(range size)) (the children of a node are
+// always lower) and counts the nodes per height.
 __global__ void curve_tree_topology(TreeArgs A, const int64_t *seg_start, int64_t g0, int64_t total_internal,
                                     uint8_t *height, int32_t *height_count, int2 *range) {
   const int64_t first = g0 + (int64_t)blockIdx.x * blockDim.x, g = first + threadIdx.x;
   const int64_t last = min(first + (int64_t)blockDim.x, total_internal) - 1;
   const int k = block_loop_of(seg_start, A.nloops, first, last, min(g, last));
-  if (height) {  // every lane of the warp takes part in the counting
+  {  // every lane of the warp takes part in the counting
     int32_t h = 0;
     if (g < total_internal) {
       const int l = A.loops[k];
@@ -310,32 +327,27 @@ __global__ void curve_tree_topology(TreeArgs A, const int64_t *seg_start, int64_
   if (g >= total_internal) return;
   const int l = A.loops[k];
   const int64_t n = A.off[l + 1] - A.off[l];
-  const int32_t node = (int32_t)(g - seg_start[k]);  // local internal id
-  const int64_t s = node + 1;                        // split position
-  const int64_t base = A.node_base[l];
+  const int64_t s = g - seg_start[k] + 1;  // split position
   int64_t lo = 0, hi = n, psize = 0;
-  int32_t par = -1;
+  int32_t pos = 1;
+  int lefts = 0;
   for (int depth = 0; depth < 64; ++depth) {
     const int64_t m = lo + (hi - lo) / 2;
     if (m == s) break;
-    par = (int32_t)(m - 1);
+    const int32_t kids = child_place(lo, lefts);
     psize = hi - lo;
-    if (s < m) hi = m;
-    else lo = m;
+    if (s < m) {
+      hi = m;
+      ++lefts;
+      pos = kids;
+    } else {
+      lo = m;
+      pos = kids + 1;
+    }
   }
-  if (range) {  // the node's segment range; bit 31 of .y: its parent is built by build_height
-    const bool need = par >= 0 && psize > (int64_t(1) << kSmallHeight);
-    range[g] = make_int2((int32_t)lo, (int32_t)hi | (need ? INT_MIN : 0));
-  }
-  const int32_t leaf0 = (int32_t)(n - 1);
-  const int32_t left = (s - lo == 1) ? leaf0 + (int32_t)lo : (int32_t)(lo + (s - lo) / 2 - 1);
-  const int32_t right = (hi - s == 1) ? leaf0 + (int32_t)s : (int32_t)(s + (hi - s) / 2 - 1);
-  A.children[2 * (base + node)] = left;
-  A.children[2 * (base + node) + 1] = right;
-  A.parent[base + node] = par;
-  A.parent[base + left] = node;
-  A.parent[base + right] = node;
-  A.arrive[base + node] = 0;
+  // The node's segment range; bit 31 of .y: its parent is built by build_height.
+  range[g] = make_int2((int32_t)lo, (int32_t)hi | (psize > (int64_t(1) << kSmallHeight) ? INT_MIN : 0));
+  A.place[g] = make_int2(pos, child_place(lo, lefts));
 }
 
 // Reads a record written by another thread of this launch: L2 loads (the
@@ -362,16 +374,15 @@ __device__ void accumulate_child(BuildNode &P, const BuildNode &C) {
     }
 }
 
-__device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg, int32_t l,
-                                   int32_t r) {
+__device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg,
+                                   int32_t kids) {
   const double dx = B.hi[0] - B.lo[0], dy = B.hi[1] - B.lo[1], dz = B.hi[2] - B.lo[2];
   H.m[0] = B.mid[0];
   H.m[1] = B.mid[1];
   H.m[2] = B.mid[2];
   H.rsq = 0.25 * (dx * dx + dy * dy + dz * dz);
   H.r = sqrt(H.rsq);
-  H.left = leaf ? -1 - seg : l;
-  H.right = leaf ? -1 : r;
+  H.left = leaf ? -1 - seg : kids;
   H.lo = B.seg_lo;
   H.cnt = B.seg_cnt;
   const double tn = sqrt(B.t[0] * B.t[0] + B.t[1] * B.t[1] + B.t[2] * B.t[2]);
@@ -384,6 +395,7 @@ __device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, b
   for (int a = 0; a < 18; ++a) M.Q[a] = (float)B.Q[a];
   H.tn = (float)tn;
   H.dn = (float)(sqrt(dd) * kInvRt3);
+  H.pad = 0;
   // Leaf: |c|^3 / 36, which is also (1/3) ||C_Q||_F for c c c^T / 12.
   M.qn = (float)(leaf ? tn * tn * tn / 36.0 : sqrt(qq) / 3.0);
   M.pad = 0.f;
@@ -391,10 +403,10 @@ __device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, b
 
 // Traversal records of a node, formed in registers and stored as vectors.
 __device__ __forceinline__ void finish_record(const BuildNode &B, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg,
-                                              int32_t l, int32_t r) {
+                                              int32_t kids) {
   NodeHdr h;
   NodeMom m;
-  finish_record_regs(B, h, m, leaf, seg, l, r);
+  finish_record_regs(B, h, m, leaf, seg, kids);
   put16(&H, h);
   put16(&M, m);
 }
@@ -434,11 +446,24 @@ __global__ void __launch_bounds__(256) build_leaves(TreeArgs A, const int64_t *s
   const int l = A.loops[k];
   const int64_t o = A.off[l], n = A.off[l + 1] - o;
   const int64_t base = A.node_base[l];
-  // Curve order: leaf position p holds segment p (the identity leaf map,
-  // written here for build_height).
+  // The leaf's position, by the descent to its segment.
   const int32_t seg = (int32_t)(g - seg_start2[k]);
-  const int32_t node = (int32_t)(n - 1 + seg);
-  A.leaf_seg[base + node] = seg;
+  int32_t node = 1;
+  {
+    int32_t lo = 0, hi = (int32_t)n;
+    int lefts = 0;
+    while (hi - lo > 1) {
+      const int32_t mid = lo + (hi - lo) / 2;
+      node = child_place(lo, lefts);
+      if (seg < mid) {
+        hi = mid;
+        ++lefts;
+      } else {
+        lo = mid;
+        ++node;
+      }
+    }
+  }
   const int64_t v0 = o + seg, v1 = o + (seg + 1 == n ? 0 : seg + 1);
   double t[3], d[3];
   NodeHdr h;
@@ -452,9 +477,9 @@ __global__ void __launch_bounds__(256) build_leaves(TreeArgs A, const int64_t *s
   h.rsq = 0.25 * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
   h.r = sqrt(h.rsq);
   h.left = -1 - seg;
-  h.right = -1;
   h.lo = seg;
   h.cnt = 1;
+  h.pad = 0;
   const double tn = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
   h.tn = (float)tn;
   h.dn = 0.f;
@@ -475,33 +500,31 @@ __global__ void __launch_bounds__(256) build_leaves(TreeArgs A, const int64_t *s
 // instead of a 320 B record written and read back). The arrival counter is
 // an acquire-release atomic, which orders the first child's record before
 // the second child's reads.
-__global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t total, bool walk_up) {
+__global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t total) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
   const int k = find_loop_of(seg_start2, A.nloops, g);
   const int l = A.loops[k];
   const int64_t o = A.off[l], n = A.off[l + 1] - o;
   const int64_t base = A.node_base[l];
-  int32_t node = (int32_t)(n - 1 + (g - seg_start2[k]));
+  int32_t node = A.leaf_pos[g];
   {
     const int32_t seg = A.leaf_seg[base + node];
     BuildNode B;
     leaf_build(A.xyz, o, n, seg, B);
-    finish_record(B, A.hdr[base + node], A.mom[base + node], true, seg, 0, 0);
+    finish_record(B, A.hdr[base + node], A.mom[base + node], true, seg, 0);
   }
-  const int32_t first_leaf = (int32_t)(n - 1);
-  if (!walk_up) return;
   for (int guard = 0; guard < 128; ++guard) {
     const int32_t par = A.parent[base + node];
     if (par < 0) break;
     cuda::atomic_ref<int32_t, cuda::thread_scope_device> arrive(A.arrive[base + par]);
     if (arrive.fetch_add(1, cuda::memory_order_acq_rel) == 0) break;  // first arrival stops
-    const int32_t cl = A.children[2 * (base + par)], cr = A.children[2 * (base + par) + 1];
+    const int32_t kids = A.children[base + par];
     BuildNode L, R;
-    if (cl >= first_leaf) leaf_build(A.xyz, o, n, A.leaf_seg[base + cl], L);
-    else load_cg(A.bn + A.int_start[k] + cl, L);
-    if (cr >= first_leaf) leaf_build(A.xyz, o, n, A.leaf_seg[base + cr], R);
-    else load_cg(A.bn + A.int_start[k] + cr, R);
+    if (A.children[base + kids] < 0) leaf_build(A.xyz, o, n, A.leaf_seg[base + kids], L);
+    else load_cg(A.bn + base + kids, L);
+    if (A.children[base + kids + 1] < 0) leaf_build(A.xyz, o, n, A.leaf_seg[base + kids + 1], R);
+    else load_cg(A.bn + base + kids + 1, R);
     BuildNode P;
     for (int a = 0; a < 3; ++a) {
       P.lo[a] = fmin(L.lo[a], R.lo[a]);
@@ -515,8 +538,8 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
     accumulate_child(P, R);
     P.seg_lo = L.seg_lo;
     P.seg_cnt = L.seg_cnt + R.seg_cnt;
-    A.bn[A.int_start[k] + par] = P;
-    finish_record(P, A.hdr[base + par], A.mom[base + par], false, 0, cl, cr);
+    A.bn[base + par] = P;
+    finish_record(P, A.hdr[base + par], A.mom[base + par], false, 0, kids);
     node = par;
   }
 }
@@ -552,8 +575,7 @@ __global__ void build_small(TreeArgs A, const int64_t *seg_start, const int32_t 
   const int l = A.loops[k];
   const int64_t o = A.off[l], n = A.off[l + 1] - o;
   const int64_t base = A.node_base[l];
-  const int32_t node = (int32_t)(g - seg_start[k]);
-  const int2 rg = range[g];
+  const int2 rg = range[g], at = A.place[g];
   const int32_t lo = rg.x, hi = rg.y & INT_MAX;
   const bool need = rg.y < 0;
   const double *V = A.xyz + 3 * o;
@@ -597,27 +619,26 @@ __global__ void build_small(TreeArgs A, const int64_t *seg_start, const int32_t 
   P.seg_lo = lo;
   P.seg_cnt = hi - lo;
   if (need) put16(A.bn + g, P);
-  const int32_t cl = A.children[2 * (base + node)], cr = A.children[2 * (base + node) + 1];
-  finish_record(P, A.hdr[base + node], A.mom[base + node], false, 0, cl, cr);
+  finish_record(P, A.hdr[base + at.x], A.mom[base + at.x], false, 0, at.y);
 }
 
-__global__ void build_height(TreeArgs A, const int64_t *seg_start, const int32_t *bucket, int64_t count) {
+__global__ void build_height(TreeArgs A, const int64_t *seg_start, const int32_t *bucket, int64_t count,
+                             const int2 *range) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= count) return;
   const int64_t g = bucket[e];
   if (g < 0 || g >= seg_start[A.nloops]) return;  // only after a height-count mismatch, which the host reports
   const int k = find_loop_of(seg_start, A.nloops, g);
   const int l = A.loops[k];
-  const int64_t o = A.off[l], n = A.off[l + 1] - o;
   const int64_t base = A.node_base[l];
-  const int32_t par = (int32_t)(g - seg_start[k]);
-  const int32_t first_leaf = (int32_t)(n - 1);
-  const int32_t cl = A.children[2 * (base + par)], cr = A.children[2 * (base + par) + 1];
+  // Height > kSmallHeight: both children are internal; their build records
+  // are at their split positions.
+  const int2 rg = range[g], at = A.place[g];
+  const int32_t lo = rg.x, hi = rg.y & INT_MAX, mid = lo + (hi - lo) / 2;
+  const BuildNode *bn = A.bn + seg_start[k] - 1;
   BuildNode L, R;
-  if (cl >= first_leaf) leaf_build(A.xyz, o, n, A.leaf_seg[base + cl], L);
-  else get16(A.bn + seg_start[k] + cl, L);
-  if (cr >= first_leaf) leaf_build(A.xyz, o, n, A.leaf_seg[base + cr], R);
-  else get16(A.bn + seg_start[k] + cr, R);
+  get16(bn + lo + (mid - lo) / 2, L);
+  get16(bn + mid + (hi - mid) / 2, R);
   BuildNode P;
   for (int a = 0; a < 3; ++a) {
     P.lo[a] = fmin(L.lo[a], R.lo[a]);
@@ -632,7 +653,7 @@ __global__ void build_height(TreeArgs A, const int64_t *seg_start, const int32_t
   P.seg_lo = L.seg_lo;
   P.seg_cnt = L.seg_cnt + R.seg_cnt;
   put16(A.bn + g, P);
-  finish_record(P, A.hdr[base + par], A.mom[base + par], false, 0, cl, cr);
+  finish_record(P, A.hdr[base + at.x], A.mom[base + at.x], false, 0, at.y);
 }
 
 // ------------------------------------------------------------------ traversal
@@ -1261,16 +1282,22 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
             const bool split2 = (!leaf1 && !leaf2) ? (h2.rsq > h1.rsq) : !leaf2;
             if (split2) {
               c0 = make_int2(pr.x, h2.left);
-              c1 = make_int2(pr.x, h2.right);
+              c1 = make_int2(pr.x, h2.left + 1);
             } else {
               c0 = make_int2(h1.left, pr.y);
-              c1 = make_int2(h1.right, pr.y);
+              c1 = make_int2(h1.left + 1, pr.y);
             }
           }
         }
         // Recording for training: opened pairs and far pairs near the threshold.
         if (kRecord && act && kind != 1 && sep >= A.rec_smin && sep * sep <= 1.5625f * (float)itolsq) {
-          uint32_t hsh = (uint32_t)slot * 0x9E3779B1u ^ (uint32_t)pr.x * 0x85EBCA77u ^ (uint32_t)pr.y * 0xC2B2AE3Du;
+          // The hash takes the nodes' numbers in tree order (internal: split
+          // position - 1, leaf: n - 1 + segment), which do not depend on
+          // where the records are stored.
+          const NodeHdr h1 = load_hdr(H1 + pr.x), h2 = load_hdr(H2 + pr.y);
+          const uint32_t id1 = h1.left < 0 ? (uint32_t)(A.off[l1 + 1] - A.off[l1] - 1 + h1.lo) : (uint32_t)(h1.lo + h1.cnt / 2 - 1);
+          const uint32_t id2 = h2.left < 0 ? (uint32_t)(A.off[l2 + 1] - A.off[l2] - 1 + h2.lo) : (uint32_t)(h2.lo + h2.cnt / 2 - 1);
+          uint32_t hsh = (uint32_t)slot * 0x9E3779B1u ^ id1 * 0x85EBCA77u ^ id2 * 0xC2B2AE3Du;
           hsh ^= hsh >> 15;
           hsh *= 0x2C1B3C6Du;
           hsh ^= hsh >> 12;
@@ -2009,10 +2036,10 @@ __global__ void __launch_bounds__(32 * kWarps) bh_classify(ClassifyArgs A) {
           const bool split2 = (!leaf1 && !leaf2) ? (h2.rsq > h1.rsq) : !leaf2;
           if (split2) {
             c0 = make_int2(pr.x, h2.left);
-            c1 = make_int2(pr.x, h2.right);
+            c1 = make_int2(pr.x, h2.left + 1);
           } else {
             c0 = make_int2(h1.left, pr.y);
-            c1 = make_int2(h1.right, pr.y);
+            c1 = make_int2(h1.left + 1, pr.y);
           }
         }
       }
@@ -2128,18 +2155,14 @@ __global__ void __launch_bounds__(256) bh_leaf_chunks(EvalArgs A) {
 // Initial batches: the root pair of every slot in `slots`; clears their sums.
 // The root pair of each listed slot as a batch; clears the slot's far,
 // exact and error sums.
-__global__ void root_batches(const int32_t *slots, int64_t n, const int32_t *slot_loops, const int64_t *off,
-                             int32_t tree_kind, Batch *out, unsigned long long *acc_lk,
+__global__ void root_batches(const int32_t *slots, int64_t n, Batch *out, unsigned long long *acc_lk,
                              unsigned long long *acc_err, unsigned long long *acc_exact) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int s = slots[k];
-  const int l1 = slot_loops[2 * s], l2 = slot_loops[2 * s + 1];
-  const int64_t n1 = off[l1 + 1] - off[l1], n2 = off[l2 + 1] - off[l2];
   out[k].slot = s;
   out[k].count = 1;
-  out[k].pairs[0] = tree_kind == 0 ? make_int2((int)(n1 / 2 - 1), (int)(n2 / 2 - 1))
-                                   : make_int2((int)(n1 - 2), (int)(n2 - 2));
+  out[k].pairs[0] = make_int2(1, 1);
   acc_lk[s] = 0;
   acc_err[s] = 0;
   acc_exact[s] = 0;
@@ -2181,7 +2204,6 @@ struct PersistArgs {
   const int32_t *slot_loops;   // 2 per slot
   const int32_t *slot_pair;    // slot -> caller pair
   int32_t nslots;
-  int32_t tree_kind;
   double epssq, beta0, beta_limit, target_error, err_scale, err_limit;
   int32_t escalations;
   double *slot_itolsq;         // per slot, current pass
@@ -2286,12 +2308,9 @@ __device__ void finish_pass(PersistArgs &A, int slot, int lane) {
   atomicAdd(&A.q[kQLeft], 1ULL);
   const unsigned long long t = atomicAdd(&A.q[kQTail], 1ULL);
   Batch &B = A.ring[t & (kRing - 1)];
-  const int l1 = A.slot_loops[2 * slot], l2 = A.slot_loops[2 * slot + 1];
-  const int64_t n1 = A.off[l1 + 1] - A.off[l1], n2 = A.off[l2 + 1] - A.off[l2];
   B.slot = slot;
   B.count = 1;
-  B.pairs[0] = A.tree_kind == 0 ? make_int2((int)(n1 / 2 - 1), (int)(n2 / 2 - 1))
-                                : make_int2((int)(n1 - 2), (int)(n2 - 2));
+  B.pairs[0] = make_int2(1, 1);
   __threadfence();
   atomicExch(&A.ready[t & (kRing - 1)], t + 1);
 }
@@ -2363,8 +2382,7 @@ __global__ void __launch_bounds__(32 * kWarps) bh_persistent(PersistArgs A) {
         stack[lane] = make_int2(__ldcg(&src[lane].x), __ldcg(&src[lane].y));
       }
     } else if (lane == 0) {
-      stack[0] = A.tree_kind == 0 ? make_int2((int)(n1 / 2 - 1), (int)(n2 / 2 - 1))
-                                  : make_int2((int)(n1 - 2), (int)(n2 - 2));
+      stack[0] = make_int2(1, 1);
     }
     int top = cnt0, nspill = 0, nf = 0, nl = 0, steps = 0;
     bool overflow = false;
@@ -2440,10 +2458,10 @@ __global__ void __launch_bounds__(32 * kWarps) bh_persistent(PersistArgs A) {
           const bool split2 = (!leaf1 && !leaf2) ? (h2.rsq > h1.rsq) : !leaf2;
           if (split2) {
             c0 = make_int2(pr.x, h2.left);
-            c1 = make_int2(pr.x, h2.right);
+            c1 = make_int2(pr.x, h2.left + 1);
           } else {
             c0 = make_int2(h1.left, pr.y);
-            c1 = make_int2(h1.right, pr.y);
+            c1 = make_int2(h1.left + 1, pr.y);
           }
         }
       }
@@ -2560,37 +2578,18 @@ __global__ void sample_features(const int64_t *node_base, const NodeHdr *hdr, co
   est_out[k] = (float)log10(e * err_scale + 1e-30);
 }
 
-// Segment range [lo, hi) of local node `node` of the curve-order tree over n
-// segments (the topology of curve_tree_topology).
-__device__ __forceinline__ void node_range(int64_t n, int32_t node, int64_t &lo, int64_t &hi) {
-  if (node >= n - 1) {
-    lo = node - (n - 1);
-    hi = lo + 1;
-    return;
-  }
-  const int64_t s = node + 1;
-  lo = 0;
-  hi = n;
-  for (int d = 0; d < 64; ++d) {
-    const int64_t m = lo + (hi - lo) / 2;
-    if (m == s) return;
-    if (s < m) hi = m;
-    else lo = m;
-  }
-}
-
 // One CTA per sample: the exact FP64 sum over the two nodes' segment ranges
 // (the leaf term seg_term_fp64) and the log10 error of the multipole value.
-__global__ void sample_exact(const double *xyz, const int64_t *off, const int32_t *slot_loops, const int4 *samples,
-                             const double *approx, int64_t n, int64_t max_terms, float *target, int32_t *valid) {
+__global__ void sample_exact(const double *xyz, const int64_t *off, const int64_t *node_base, const NodeHdr *hdr,
+                             const int32_t *slot_loops, const int4 *samples, const double *approx, int64_t n,
+                             int64_t max_terms, float *target, int32_t *valid) {
   const int64_t k = blockIdx.x;
   if (k >= n) return;
   const int4 sm = samples[k];
   const int la = slot_loops[2 * sm.x], lb = slot_loops[2 * sm.x + 1];
   const int64_t oa = off[la], na = off[la + 1] - oa, ob = off[lb], nb = off[lb + 1] - ob;
-  int64_t a0, a1, b0, b1;
-  node_range(na, sm.y, a0, a1);
-  node_range(nb, sm.z, b0, b1);
+  const NodeHdr &ha = hdr[node_base[la] + sm.y], &hb = hdr[node_base[lb] + sm.z];
+  const int64_t a0 = ha.lo, a1 = a0 + ha.cnt, b0 = hb.lo, b1 = b0 + hb.cnt;
   if ((a1 - a0) * (b1 - b0) > max_terms) {
     if (threadIdx.x == 0) valid[k] = 0;
     return;
@@ -2618,9 +2617,12 @@ __global__ void scatter_kernel(const double *src, const int32_t *idx, int64_t n,
   if (k < n) dst[idx[k]] = src[k];
 }
 
-// Host kd-median tree (ModifiedKdBVH.h:101-132, :207-237), for bh_tree = 1:
-// children in local ids, leaf_seg per leaf position.
-void host_kd_tree(const double *xyz, int64_t n, std::vector<int32_t> &children, std::vector<int32_t> &leaf_seg) {
+// Host kd-median tree (ModifiedKdBVH.h:101-132, :207-237), for bh_tree = 1,
+// by node position (2 n positions, see child_place): children (position of
+// the first child, -1 for a leaf), parent (-1 for the root) and leaf_seg;
+// leaf_pos per object.
+void host_kd_tree(const double *xyz, int64_t n, int32_t *children, int32_t *parent, int32_t *leaf_seg,
+                  int32_t *leaf_pos) {
   std::vector<double> lo(3 * n), hi(3 * n), cen(3 * n);
   for (int64_t s = 0; s < n; ++s) {
     const double *p = xyz + 3 * s, *q = xyz + 3 * ((s + 1) % n);
@@ -2632,55 +2634,30 @@ void host_kd_tree(const double *xyz, int64_t n, std::vector<int32_t> &children, 
   }
   std::vector<int32_t> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
-  children.assign(2 * (n - 1), 0);
-  int32_t next = 0;
   struct R {
-    std::vector<int32_t> &idx, &ch;
+    std::vector<int32_t> &idx;
     const std::vector<double> &cen;
-    int32_t &next;
-    int64_t n;
-    int32_t go(int64_t from, int64_t to, int dim) {
+    int32_t *ch, *par, *ls, *lp;
+    void go(int64_t from, int64_t to, int dim, int32_t me, int lefts) {
       auto cmp = [&](int32_t a, int32_t b) { return cen[3 * a + dim] < cen[3 * b + dim]; };
       const int64_t size = to - from;
-      int32_t l, r;
-      if (size == 2) {
-        l = (int32_t)(from + n - 1);
-        r = (int32_t)(from + n);
-      } else if (size == 3) {
-        const int64_t mid = from + 2;
-        std::nth_element(idx.begin() + from, idx.begin() + mid, idx.begin() + to, cmp);
-        l = go(from, mid, (dim + 1) % 3);
-        r = (int32_t)(mid + n - 1);
-      } else {
-        const int64_t mid = from + size / 2;
-        std::nth_element(idx.begin() + from, idx.begin() + mid, idx.begin() + to, cmp);
-        l = go(from, mid, (dim + 1) % 3);
-        r = go(mid, to, (dim + 1) % 3);
+      if (size == 1) {
+        ch[me] = -1;
+        ls[me] = idx[from];
+        lp[from] = me;
+        return;
       }
-      const int32_t me = next++;
-      ch[2 * me] = l;
-      ch[2 * me + 1] = r;
-      return me;
+      const int64_t mid = size == 2 ? from + 1 : size == 3 ? from + 2 : from + size / 2;
+      if (size > 2) std::nth_element(idx.begin() + from, idx.begin() + mid, idx.begin() + to, cmp);
+      const int32_t kids = child_place(from, lefts);
+      ch[me] = kids;
+      par[kids] = par[kids + 1] = me;
+      go(from, mid, (dim + 1) % 3, kids, lefts + 1);
+      go(mid, to, (dim + 1) % 3, kids + 1, lefts);
     }
-  } rec{idx, children, cen, next, n};
-  rec.go(0, n, 0);
-  leaf_seg = idx;
-}
-
-__global__ void parents_from_children(const int32_t *children, const int64_t *node_base, const int64_t *off,
-                                      const int32_t *loops, int32_t nloops, const int64_t *seg_start,
-                                      int64_t total_internal, int32_t *parent, int32_t *arrive) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total_internal) return;
-  const int k = find_loop_of(seg_start, nloops, g);
-  const int l = loops[k];
-  const int64_t base = node_base[l];
-  const int32_t node = (int32_t)(g - seg_start[k]);
-  const int64_t n = off[l + 1] - off[l];
-  parent[base + children[2 * (base + node)]] = node;
-  parent[base + children[2 * (base + node) + 1]] = node;
-  arrive[base + node] = 0;
-  if (node == n - 2) parent[base + node] = -1;
+  } rec{idx, cen, children, parent, leaf_seg, leaf_pos};
+  parent[1] = -1;
+  rec.go(0, n, 0, 1, 0);
 }
 
 }  // namespace
@@ -2709,7 +2686,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     const int64_t n = h_off[l + 1] - h_off[l];
     loops.push_back(l);
     node_base[l] = nodes;
-    nodes += 2 * n - 1;
+    nodes += 2 * n;  // position 0 is unused; even, so that sibling headers share a line
     seg_int.push_back(seg_int.back() + (n - 1));
     seg_all.push_back(seg_all.back() + n);
     int d = 0;
@@ -2723,11 +2700,10 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   int64_t *d_base = ctx.d_bh[1].as<int64_t>(nl_all);
   int64_t *d_segint = ctx.d_bh[2].as<int64_t>(nloops + 1);
   int64_t *d_segall = ctx.d_bh[3].as<int64_t>(nloops + 1);
-  int32_t *d_children = ctx.d_bh[4].as<int32_t>(2 * nodes);
-  int32_t *d_parent = ctx.d_bh[5].as<int32_t>(nodes);
-  int32_t *d_leafseg = ctx.d_bh[6].as<int32_t>(nodes);
-  int32_t *d_arrive = ctx.d_bh[7].as<int32_t>(nodes);
-  BuildNode *d_bn = ctx.d_bh[8].as<BuildNode>(std::max<int64_t>(tot_int, 1));  // internal nodes only
+  const bool kd = prm.bh_tree == 1;
+  int2 *d_place = kd ? nullptr : ctx.d_bh[4].as<int2>(std::max<int64_t>(tot_int, 1));
+  int32_t *d_kd = kd ? ctx.d_bh[5].as<int32_t>(4 * nodes + tot_leaf) : nullptr;  // children, parent, leaf_seg, arrive, leaf_pos
+  BuildNode *d_bn = ctx.d_bh[8].as<BuildNode>(kd ? nodes : std::max<int64_t>(tot_int, 1));
   NodeHdr *d_hdr = ctx.d_bh[9].as<NodeHdr>(nodes);
   NodeMom *d_mom = ctx.d_bh[10].as<NodeMom>(nodes);
   cudaStream_t st = ctx.stream;
@@ -2735,8 +2711,8 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   FLN_CUDA(cudaMemcpyAsync(d_base, node_base.data(), nl_all * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   FLN_CUDA(cudaMemcpyAsync(d_segint, seg_int.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   FLN_CUDA(cudaMemcpyAsync(d_segall, seg_all.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  TreeArgs T{d_xyz, d_off, d_base, d_loops, nloops, d_children, d_parent, d_leafseg, d_arrive, d_bn, d_hdr, d_mom,
-             d_segint};
+  TreeArgs T{d_xyz, d_off, d_base, d_loops, nloops, d_bn, d_place, d_kd, d_kd + nodes, d_kd + 2 * nodes,
+             d_kd + 3 * nodes, d_kd + 4 * nodes, d_hdr, d_mom};
   // Slots: pairs ordered by decreasing estimated work. Host work, done once
   // the tree build is queued (while the GPU runs it, before the host waits
   // for its counts).
@@ -2762,26 +2738,20 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   if (prm.bh_tree == 1) {
     // The reference's kd-median tree, built on the host from a copy of the loops.
     wait_xyz_pieces(ctx);
-    std::vector<int32_t> ch_all(2 * nodes, 0), ls_all(nodes, 0);
+    std::vector<int32_t> kd_all(4 * nodes + tot_leaf, 0);
     std::vector<double> xyz_host(3 * h_off.back());
     FLN_CUDA(cudaMemcpyAsync(xyz_host.data(), d_xyz, xyz_host.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaStreamSynchronize(st));
 #pragma omp parallel for schedule(dynamic)
     for (int k = 0; k < nloops; ++k) {
       const int l = loops[k];
-      const int64_t n = h_off[l + 1] - h_off[l];
-      std::vector<int32_t> ch, ls;
-      host_kd_tree(xyz_host.data() + 3 * h_off[l], n, ch, ls);
-      std::copy(ch.begin(), ch.end(), ch_all.begin() + 2 * node_base[l]);
-      for (int64_t p = 0; p < n; ++p) ls_all[node_base[l] + n - 1 + p] = ls[p];
+      int32_t *t = kd_all.data() + node_base[l];
+      host_kd_tree(xyz_host.data() + 3 * h_off[l], h_off[l + 1] - h_off[l], t, t + nodes, t + 2 * nodes,
+                   kd_all.data() + 4 * nodes + seg_all[k]);
     }
-    FLN_CUDA(cudaMemcpyAsync(d_children, ch_all.data(), ch_all.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    FLN_CUDA(cudaMemcpyAsync(d_leafseg, ls_all.data(), ls_all.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    parents_from_children<<<(int)((tot_int + 255) / 256), 256, 0, st>>>(d_children, d_base, d_off, d_loops, nloops,
-                                                                        d_segint, tot_int, d_parent, d_arrive);
+    FLN_CUDA(cudaMemcpyAsync(d_kd, kd_all.data(), kd_all.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     FLN_CUDA(cudaStreamSynchronize(st));  // host vectors go out of scope
-    ++launches;
-    build_moments<<<(int)((tot_leaf + 127) / 128), 128, 0, st>>>(T, d_segall, tot_leaf, true);
+    build_moments<<<(int)((tot_leaf + 127) / 128), 128, 0, st>>>(T, d_segall, tot_leaf);
     FLN_CUDA(cudaGetLastError());
     ++launches;
   } else {
@@ -2848,7 +2818,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         }
         for (int h = kSmallHeight + 1; h < 64; ++h) {
           if (!hcnt[h]) continue;
-          build_height<<<(hcnt[h] + 127) / 128, 128, 0, st>>>(T, d_segint, d_bucket + hoff[h], hcnt[h]);
+          build_height<<<(hcnt[h] + 127) / 128, 128, 0, st>>>(T, d_segint, d_bucket + hoff[h], hcnt[h], d_range);
           ++launches;
         }
         FLN_CUDA(cudaGetLastError());
@@ -2983,8 +2953,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     FLN_CUDA(cudaMemcpyAsync(d_active, roots.data(), na * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     FLN_CUDA(cudaMemcpyAsync(d_itol, itol_slots.data(), np * sizeof(double), cudaMemcpyHostToDevice, st));
     if (na > 0) {
-      root_batches<<<(int)((na + 255) / 256), 256, 0, st>>>(d_active, na, d_slots, d_off, prm.bh_tree == 1 ? 1 : 0,
-                                                            d_batch[0], d_acc, d_acc_err, d_acc_exact);
+      root_batches<<<(int)((na + 255) / 256), 256, 0, st>>>(d_active, na, d_batch[0], d_acc, d_acc_err, d_acc_exact);
       FLN_CUDA(cudaGetLastError());
       ++launches;
     }
@@ -3178,8 +3147,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     FLN_CUDA(cudaMemcpyAsync(d_q, q0, sizeof q0, cudaMemcpyHostToDevice, st));
     FLN_CUDA(cudaMemsetAsync(d_fl, 0, np * sizeof(int32_t), st));
     FLN_CUDA(cudaMemsetAsync(d_cnt4, 0, 4 * sizeof(double) + sizeof(int32_t), st));
-    PersistArgs P{d_xyz, d_off, d_base, d_hdr, d_mom, d_slots, d_slot_pair, (int32_t)np, prm.bh_tree == 1 ? 1 : 0,
-                  prm.epssq, b0, prm.barnes_hut_beta_limit, prm.target_error, prm.error_est_scale,
+    PersistArgs P{d_xyz, d_off, d_base, d_hdr, d_mom, d_slots, d_slot_pair, (int32_t)np, prm.epssq, b0, prm.barnes_hut_beta_limit, prm.target_error, prm.error_est_scale,
                   prm.bh_err_limit, prm.bh_escalations, d_sitol, d_pass_arr, d_left, d_acc, d_acc_err, d_ring,
                   d_ready, d_q, d_lk_out, d_err_out, d_fl, d_cnt4, d_spill, d_status, spill_cap,
                   prm.bh_wait_polls > 0 ? (long long)prm.bh_wait_polls : kWaitPolls};
@@ -3419,8 +3387,8 @@ void learned_collect(Context &ctx, const double *d_xyz, const int64_t *d_off, co
   FLN_CUDA(cudaGetLastError());
   for (int64_t k0 = 0; k0 < n; k0 += (int64_t)1 << 30) {
     const int64_t m = std::min<int64_t>(n - k0, (int64_t)1 << 30);
-    sample_exact<<<(int)m, 128, 0, st>>>(d_xyz, d_off, d_slots, d_rec + k0, d_approx + k0, m, max_terms, d_T + k0,
-                                         d_valid + k0);
+    sample_exact<<<(int)m, 128, 0, st>>>(d_xyz, d_off, d_base, d_hdr, d_slots, d_rec + k0, d_approx + k0, m, max_terms,
+                                         d_T + k0, d_valid + k0);
     FLN_CUDA(cudaGetLastError());
   }
   std::vector<float> hx(kMlpIn * n), ht(n), hs(n), he(n);
