@@ -79,12 +79,6 @@ constexpr int kWarps = 4;          // warps per traversal CTA
 #endif
 constexpr int kStack = FLN_BH_STACK;
 constexpr int kSpill = 8192;       // global spill entries per warp
-// Curve-order nodes of at most 2^kSmallHeight segments are built straight
-// from their segments (build_small), the rest level by level (build_height).
-#ifndef FLN_BUILD_SMALL_HEIGHT
-#define FLN_BUILD_SMALL_HEIGHT 4
-#endif
-constexpr int kSmallHeight = FLN_BUILD_SMALL_HEIGHT;
 #ifndef FLN_BUCKET_SOFT_LOG2
 #define FLN_BUCKET_SOFT_LOG2 19  // exact-list chunks per round before it stops taking batches
 #endif
@@ -103,22 +97,19 @@ struct __align__(16) BuildNode {
 };
 static_assert(sizeof(BuildNode) == 320, "BuildNode layout");
 
-// Record copies as 16-byte vectors (a thread's record is contiguous; with
-// field-by-field stores every warp instruction would touch 32 lines).
-template <class T>
-__device__ __forceinline__ void put16(T *dst, const T &src) {
-  static_assert(sizeof(T) % 16 == 0 && alignof(T) >= 16, "16-byte record");
-  const int4 *s = reinterpret_cast<const int4 *>(&src);
-  int4 *d = reinterpret_cast<int4 *>(dst);
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(T) / 16); ++i) d[i] = s[i];
+// Record stores as 32-byte vectors (a thread's record is contiguous; with
+// field-by-field stores every warp instruction would touch 32 lines, and
+// narrower vectors would write half sectors).
+__device__ __forceinline__ void store32(void *p, const unsigned long long *w) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(w[0]), "l"(w[1]), "l"(w[2]), "l"(w[3])
+               : "memory");
 }
 template <class T>
-__device__ __forceinline__ void get16(const T *src, T &dst) {
-  const int4 *s = reinterpret_cast<const int4 *>(src);
-  int4 *d = reinterpret_cast<int4 *>(&dst);
+__device__ __forceinline__ void put32(T *dst, const T &src) {
+  static_assert(sizeof(T) % 32 == 0 && alignof(T) >= 32, "32-byte record");
+  const unsigned long long *w = reinterpret_cast<const unsigned long long *>(&src);
 #pragma unroll
-  for (int i = 0; i < (int)(sizeof(T) / 16); ++i) d[i] = s[i];
+  for (int i = 0; i < (int)(sizeof(T) / 32); ++i) store32(reinterpret_cast<char *>(dst) + 32 * i, w + 4 * i);
 }
 
 // Traversal records.
@@ -230,16 +221,16 @@ struct TreeArgs {
   const int64_t *node_base;  // loop -> first global node
   const int32_t *loops;      // loops that need a tree
   int32_t nloops;
-  // Curve-order trees: build records by internal node, bn[sum of (n - 1) over
-  // the earlier listed loops + split - 1]; place[the same] = (position of the
-  // node, position of its first child).
+  // Curve-order trees (build_curve_trees): listed loop k is cut into
+  // blk_start[k + 1] - blk_start[k] = 2^d blocks, the nodes of depth d; bn and
+  // arrive hold its nodes of depth <= d at 2 blk_start[k] + 2^depth + index.
   // kd-median trees: everything by node position (base + position).
+  const int64_t *blk_start;
   BuildNode *bn;
-  int2 *place;
+  int32_t *arrive;           // arrival counters, zero at the start
   int32_t *children;         // kd: position of the first child; -1 for a leaf
   int32_t *parent;           // kd: position of the parent; -1 for the root
   int32_t *leaf_seg;         // kd: segment of a leaf
-  int32_t *arrive;           // kd: arrival counter
   int32_t *leaf_pos;         // kd: position of the leaf of each object (by listed loop)
   NodeHdr *hdr;
   NodeMom *mom;
@@ -262,92 +253,6 @@ __device__ __forceinline__ int find_loop_of(const int64_t *start, int n, int64_t
     else hi = mid;
   }
   return lo;
-}
-
-// The listed loop of index x, for a block whose threads take the consecutive
-// indices [first, last]: two threads search the whole list for the block's
-// first and last index, and every thread then searches only between the two
-// (a block crosses few loop boundaries). Every thread of the block must call
-// it once (it synchronises the block).
-__device__ __forceinline__ int block_loop_of(const int64_t *start, int n, int64_t first, int64_t last, int64_t x) {
-  __shared__ int s_range[2];
-  if (threadIdx.x == 0) s_range[0] = find_loop_of(start, n, first);
-  if (threadIdx.x == (blockDim.x > 1 ? 1 : 0)) s_range[1] = find_loop_of(start, n, last);
-  __syncthreads();
-  int lo = s_range[0], hi = s_range[1] + 1;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (start[mid] <= x) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// count[key] += 1 for the calling lane, one atomic per distinct key of the
-// warp; returns the count before the warp's run plus the lane's rank among
-// the lanes of the warp with its key.
-__device__ __forceinline__ int32_t add_one_rank(int32_t *count, int32_t key, bool active) {
-  const unsigned act = __ballot_sync(0xffffffffu, active);
-  if (!active) return 0;
-  const unsigned peers = __match_any_sync(act, key);
-  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-  int32_t base = 0;
-  if (lane == leader) base = atomicAdd(&count[key], __popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  return base + __popc(peers & ((1u << lane) - 1));
-}
-
-// Curve-order topology: thread per internal node (local id s - 1 splits at s).
-// seg_start[k] = sum of (n - 1) over the first k listed loops. It also
-// records the node's height ceil(log2(range size)) (the children of a node are
-// always lower) and counts the nodes per height.
-__global__ void curve_tree_topology(TreeArgs A, const int64_t *seg_start, int64_t g0, int64_t total_internal,
-                                    uint8_t *height, int32_t *height_count, int2 *range) {
-  const int64_t first = g0 + (int64_t)blockIdx.x * blockDim.x, g = first + threadIdx.x;
-  const int64_t last = min(first + (int64_t)blockDim.x, total_internal) - 1;
-  const int k = block_loop_of(seg_start, A.nloops, first, last, min(g, last));
-  {  // every lane of the warp takes part in the counting
-    int32_t h = 0;
-    if (g < total_internal) {
-      const int l = A.loops[k];
-      const int64_t n = A.off[l + 1] - A.off[l];
-      const int64_t s = g - seg_start[k] + 1;
-      int64_t lo = 0, hi = n;
-      for (int depth = 0; depth < 64; ++depth) {
-        const int64_t mid = lo + (hi - lo) / 2;
-        if (mid == s) break;
-        if (s < mid) hi = mid;
-        else lo = mid;
-      }
-      h = 64 - __clzll((unsigned long long)(hi - lo - 1));
-      height[g] = (uint8_t)h;
-    }
-    add_one_rank(height_count, h, g < total_internal);
-  }
-  if (g >= total_internal) return;
-  const int l = A.loops[k];
-  const int64_t n = A.off[l + 1] - A.off[l];
-  const int64_t s = g - seg_start[k] + 1;  // split position
-  int64_t lo = 0, hi = n, psize = 0;
-  int32_t pos = 1;
-  int lefts = 0;
-  for (int depth = 0; depth < 64; ++depth) {
-    const int64_t m = lo + (hi - lo) / 2;
-    if (m == s) break;
-    const int32_t kids = child_place(lo, lefts);
-    psize = hi - lo;
-    if (s < m) {
-      hi = m;
-      ++lefts;
-      pos = kids;
-    } else {
-      lo = m;
-      pos = kids + 1;
-    }
-  }
-  // The node's segment range; bit 31 of .y: its parent is built by build_height.
-  range[g] = make_int2((int32_t)lo, (int32_t)hi | (psize > (int64_t(1) << kSmallHeight) ? INT_MIN : 0));
-  A.place[g] = make_int2(pos, child_place(lo, lefts));
 }
 
 // Reads a record written by another thread of this launch: L2 loads (the
@@ -407,8 +312,8 @@ __device__ __forceinline__ void finish_record(const BuildNode &B, NodeHdr &H, No
   NodeHdr h;
   NodeMom m;
   finish_record_regs(B, h, m, leaf, seg, kids);
-  put16(&H, h);
-  put16(&M, m);
+  put32(&H, h);
+  put32(&M, m);
 }
 
 // Leaf record of segment `seg` of a loop at vertex offset o with n segments
@@ -431,67 +336,6 @@ __device__ void leaf_build(const double *xyz, int64_t o, int64_t n, int32_t seg,
   const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
   for (int kk = 0; kk < 3; ++kk)
     for (int e = 0; e < 6; ++e) B.Q[6 * kk + e] = ((1.0 / 12.0) * B.t[kk]) * (B.t[ii[e]] * B.t[jj[e]]);
-}
-
-// Leaf records of the curve-order trees (thread per leaf), straight from the
-// segment's two vertices: the values finish_record forms from leaf_build's
-// record (box, midpoint, tangent c, C_D = 0, C_Q,k = c_k c c^T / 12), without
-// an FP64 build record in registers, so the kernel runs at full occupancy.
-__global__ void __launch_bounds__(256) build_leaves(TreeArgs A, const int64_t *seg_start2, int64_t g0,
-                                                    int64_t total) {
-  const int64_t first = g0 + (int64_t)blockIdx.x * blockDim.x, g = first + threadIdx.x;
-  const int64_t last = min(first + (int64_t)blockDim.x, total) - 1;
-  const int k = block_loop_of(seg_start2, A.nloops, first, last, min(g, last));
-  if (g >= total) return;
-  const int l = A.loops[k];
-  const int64_t o = A.off[l], n = A.off[l + 1] - o;
-  const int64_t base = A.node_base[l];
-  // The leaf's position, by the descent to its segment.
-  const int32_t seg = (int32_t)(g - seg_start2[k]);
-  int32_t node = 1;
-  {
-    int32_t lo = 0, hi = (int32_t)n;
-    int lefts = 0;
-    while (hi - lo > 1) {
-      const int32_t mid = lo + (hi - lo) / 2;
-      node = child_place(lo, lefts);
-      if (seg < mid) {
-        hi = mid;
-        ++lefts;
-      } else {
-        lo = mid;
-        ++node;
-      }
-    }
-  }
-  const int64_t v0 = o + seg, v1 = o + (seg + 1 == n ? 0 : seg + 1);
-  double t[3], d[3];
-  NodeHdr h;
-  NodeMom m;
-  for (int a = 0; a < 3; ++a) {
-    const double p0 = A.xyz[3 * v0 + a], p1 = A.xyz[3 * v1 + a];
-    t[a] = p1 - p0;
-    h.m[a] = 0.5 * p0 + 0.5 * p1;
-    d[a] = fmax(p0, p1) - fmin(p0, p1);
-  }
-  h.rsq = 0.25 * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-  h.r = sqrt(h.rsq);
-  h.left = -1 - seg;
-  h.lo = seg;
-  h.cnt = 1;
-  h.pad = 0;
-  const double tn = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
-  h.tn = (float)tn;
-  h.dn = 0.f;
-  for (int a = 0; a < 3; ++a) m.t[a] = (float)t[a];
-  for (int a = 0; a < 9; ++a) m.D[a] = 0.f;
-  const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
-  for (int kk = 0; kk < 3; ++kk)
-    for (int e = 0; e < 6; ++e) m.Q[6 * kk + e] = (float)(((1.0 / 12.0) * t[kk]) * (t[ii[e]] * t[jj[e]]));
-  m.qn = (float)(tn * tn * tn / 36.0);
-  m.pad = 0.f;
-  put16(&A.hdr[base + node], h);
-  put16(&A.mom[base + node], m);
 }
 
 // Thread per leaf: write the leaf's traversal record and walk up; the second
@@ -544,116 +388,310 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
   }
 }
 
-// Level-synchronous build of curve-order trees: the internal nodes of one
-// height, listed in bucket[0, count), each from its two children, which
-// earlier launches finished (leaves: rebuilt from their vertices). Same
-// arithmetic as the walk-up of build_moments, so the same records.
-__global__ void bucket_heights(const uint8_t *height, int64_t g0, int64_t total_internal, const int32_t *height_off,
-                               int32_t *cursor, int32_t *bucket) {
-  const int64_t g = g0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int32_t h = g < total_internal ? height[g] : 0;
-  const int32_t r = add_one_rank(cursor, h, g < total_internal);
-  const int64_t pos = (int64_t)height_off[h] + r;
-  if (g < total_internal && pos < total_internal) bucket[pos] = (int32_t)g;  // a count mismatch is caught on the host
+// Curve-order trees, all loops in one launch. A loop of n segments is cut
+// into the 2^d nodes of the smallest depth d at which none holds more than
+// kBlockLeaves segments (the nodes of one depth differ by at most one
+// segment); a CTA builds one such block and everything below it:
+//  - the block's vertices go to shared memory once (coalesced);
+//  - leaves: a thread each, straight from the two vertices;
+//  - groups (the block's nodes of the first depth with at most 4 segments):
+//    a thread sums a group's leaf moments about the group's centre, other
+//    threads do the two-segment nodes inside the groups. (A leaf has C_D = 0
+//    and C_Q,k = c_k c c^T / 12, so the shift of compute_link.cpp:367-381 adds
+//    c r^T and c_k r r^T with r = leaf midpoint - node centre.);
+//  - the levels above, up to the block's root: four lanes per node. Row k of
+//    C_D, C_Q,k and axis k of the box depend on the children's row k and the
+//    centres only, so lane k forms them from the children's FP64 records in
+//    shared memory.
+// The block's root then goes to global memory, and the warp that finds its
+// sibling there already (an arrival counter) builds the parent, up to the
+// loop's root; children are always added left first, so the result does not
+// depend on who arrives last. FP64 throughout; records are rounded to FP32 at
+// the end.
+//
+// What bounds it: 384 B of records are written per segment; measured 4.7 ms for
+// 28M segments of mixed sizes (2.3 TB/s of records) and 2.75 ms for 14.1M,
+// against 8.6 and 4.66 ms for the build it replaces (topology, leaf,
+// height-bucket, small-node and one launch per height), which read each vertex
+// about 30 times through scattered 8-byte loads and wrote 16-byte pieces. The
+// last levels of a block and the way up keep only one warp busy, so a block is
+// as large as four resident CTAs' shared memory allows: with 512 leaves 4.7 ms,
+// 256 leaves 5.9, 128 leaves 7.3 (same case); three CTAs of 168 registers
+// instead of four of 128: 5.3 ms; leaving the last levels to one warp while the
+// others write the leaves: 6.5 against 5.9 ms (at 256 leaves).
+constexpr int kBuildThreads = 128;
+constexpr int kBlockLeaves = 512;
+constexpr int kGroups = kBlockLeaves / 4;  // most groups of a block
+constexpr int kRecD = 39;            // doubles of a record in shared memory (odd: no bank conflicts):
+// Dynamic shared memory: 32 floats of staging per quad, the vertices, the
+// groups' records (56 KB: four CTAs per SM).
+constexpr int kBuildSmem = (kBuildThreads / 4 * 16 + 3 * (kBlockLeaves + 1) + kGroups * kRecD) * 8;
+constexpr int kRLo = 0, kRHi = 3, kRMid = 6, kRT = 9, kRD = 12, kRQ = 21;
+
+struct NodeAt {        // a node on a descent from the root
+  int32_t lo, hi;      // its segments
+  int32_t pos, lefts;  // storage position; left turns of its path
+};
+__device__ __forceinline__ NodeAt descend(NodeAt v, int code, int steps) {
+  for (int b = steps - 1; b >= 0; --b) {
+    const int32_t mid = v.lo + (v.hi - v.lo) / 2, kids = child_place(v.lo, v.lefts);
+    if ((code >> b) & 1) {
+      v.lo = mid;
+      v.pos = kids + 1;
+    } else {
+      v.hi = mid;
+      v.pos = kids;
+      ++v.lefts;
+    }
+  }
+  return v;
 }
 
-// Nodes of height 1..kSmallHeight (at most 2^kSmallHeight segments), one
-// thread each, built straight from their segments: box = the range's
-// vertices; c_M, C_D and C_Q = the leaves' moments shifted to the node centre
-// (for a leaf, C_D = 0 and C_Q,k = c_k c c^T / 12, so the shift adds c r^T and
-// c_k r r^T with r = leaf midpoint - node centre). Algebraically the pairwise
-// build of build_height; it writes no build record except for nodes whose
-// parent build_height builds. Most internal nodes are this low, so this
-// skips most of the 320-byte build records.
-__global__ void build_small(TreeArgs A, const int64_t *seg_start, const int32_t *bucket, int64_t count,
-                            const int2 *range) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
-  const int64_t g = bucket[e];
-  if (g < 0 || g >= seg_start[A.nloops]) return;  // only after a height-count mismatch, which the host reports
-  const int k = find_loop_of(seg_start, A.nloops, g);
-  const int l = A.loops[k];
-  const int64_t o = A.off[l], n = A.off[l + 1] - o;
-  const int64_t base = A.node_base[l];
-  const int2 rg = range[g], at = A.place[g];
-  const int32_t lo = rg.x, hi = rg.y & INT_MAX;
-  const bool need = rg.y < 0;
-  const double *V = A.xyz + 3 * o;
-  BuildNode P;
+// One node from its two children's records L and R, by the four lanes of a
+// quad (q = lane & 3; lane 3 repeats lane 2 and stores its share of the
+// moments). Writes the traversal records of the node at `v` and its FP64
+// record to `out` (which may be L or R). stage: 32 floats of this quad.
+__device__ __forceinline__ void combine_quad(const double *L, const double *R, double *out, const NodeAt &v,
+                                             NodeHdr *hdr, NodeMom *mom, float *stage, int q, bool write) {
+  const int k = min(q, 2), qb = (threadIdx.x & 31) & ~3;
+  const unsigned mask = 0xfu << qb;  // the quad
+  const double blo = fmin(L[kRLo + k], R[kRLo + k]), bhi = fmax(L[kRHi + k], R[kRHi + k]);
+  const double mk = 0.5 * (bhi + blo), dk = bhi - blo;
+  double mid[3], dg[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    P.lo[a] = V[3 * lo + a];
-    P.hi[a] = P.lo[a];
+    mid[a] = __shfl_sync(mask, mk, qb + a);
+    dg[a] = __shfl_sync(mask, dk, qb + a);
   }
-  for (int32_t v = lo + 1; v <= hi; ++v) {
-    const int64_t w = v == n ? 0 : v;
-    for (int a = 0; a < 3; ++a) {
-      const double x = V[3 * w + a];
-      P.lo[a] = fmin(P.lo[a], x);
-      P.hi[a] = fmax(P.hi[a], x);
+  double t = 0.0, D[3] = {0.0, 0.0, 0.0}, Q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const double *C = c ? R : L;
+    const double r[3] = {C[kRMid] - mid[0], C[kRMid + 1] - mid[1], C[kRMid + 2] - mid[2]};
+    const double ct = C[kRT + k];
+    const double cd[3] = {C[kRD + 3 * k], C[kRD + 3 * k + 1], C[kRD + 3 * k + 2]};
+    t += ct;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) D[b] += cd[b] + ct * r[b];
+    const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+    for (int e = 0; e < 6; ++e)
+      Q[e] += C[kRQ + 6 * k + e] + r[jj[e]] * cd[ii[e]] + r[ii[e]] * cd[jj[e]] + ct * (r[ii[e]] * r[jj[e]]);
+  }
+  double tt = t * t, dd = D[0] * D[0] + D[1] * D[1] + D[2] * D[2], qq = 0.0;
+#pragma unroll
+  for (int e = 0; e < 6; ++e) qq += (e < 3 ? 1.0 : 2.0) * Q[e] * Q[e];
+  auto sum3 = [&](double x) {
+    return (__shfl_sync(mask, x, qb) + __shfl_sync(mask, x, qb + 1)) + __shfl_sync(mask, x, qb + 2);
+  };
+  tt = sum3(tt);
+  dd = sum3(dd);
+  qq = sum3(qq);
+  __syncwarp(mask);  // every lane has read the children's records
+  if (!write) return;
+  if (q < 3) {
+    out[kRLo + k] = blo;
+    out[kRHi + k] = bhi;
+    out[kRMid + k] = mk;
+    out[kRT + k] = t;
+    stage[k] = (float)t;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      out[kRD + 3 * k + b] = D[b];
+      stage[3 + 3 * k + b] = (float)D[b];
     }
-  }
-  for (int a = 0; a < 3; ++a) {
-    P.mid[a] = 0.5 * (P.hi[a] + P.lo[a]);
-    P.t[a] = 0.0;
-  }
-  for (int a = 0; a < 9; ++a) P.D[a] = 0.0;
-  for (int a = 0; a < 18; ++a) P.Q[a] = 0.0;
-  const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
-  for (int32_t sg = lo; sg < hi; ++sg) {
-    const int64_t w0 = sg, w1 = sg + 1 == n ? 0 : sg + 1;
-    double t[3], r[3];
-    for (int a = 0; a < 3; ++a) {
-      const double p0 = V[3 * w0 + a], p1 = V[3 * w1 + a];
-      t[a] = p1 - p0;
-      r[a] = (0.5 * p0 + 0.5 * p1) - P.mid[a];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      out[kRQ + 6 * k + e] = Q[e];
+      stage[12 + 6 * k + e] = (float)Q[e];
     }
-    for (int a = 0; a < 3; ++a) P.t[a] += t[a];
-    for (int a = 0; a < 3; ++a)
-      for (int b = 0; b < 3; ++b) P.D[3 * a + b] += t[a] * r[b];
-    for (int kk = 0; kk < 3; ++kk)
-      for (int q = 0; q < 6; ++q) {
-        const int i = ii[q], j = jj[q];
-        P.Q[6 * kk + q] += ((1.0 / 12.0) * t[kk]) * (t[i] * t[j]) + t[kk] * (r[i] * r[j]);
+  } else {
+    stage[30] = (float)(sqrt(qq) / 3.0);
+    stage[31] = 0.f;
+  }
+  __syncwarp(mask);
+  const double rsq = 0.25 * (dg[0] * dg[0] + dg[1] * dg[1] + dg[2] * dg[2]);
+  unsigned long long w[4];
+  if (q == 0) {
+    for (int a = 0; a < 3; ++a) w[a] = (unsigned long long)__double_as_longlong(mid[a]);
+    w[3] = (unsigned long long)__double_as_longlong(sqrt(rsq));
+    store32(hdr, w);
+  } else if (q == 1) {
+    auto two = [](uint32_t a, uint32_t b) { return (unsigned long long)a | ((unsigned long long)b << 32); };
+    w[0] = (unsigned long long)__double_as_longlong(rsq);
+    w[1] = two((uint32_t)child_place(v.lo, v.lefts), (uint32_t)v.lo);
+    w[2] = two((uint32_t)(v.hi - v.lo), __float_as_uint((float)sqrt(tt)));
+    w[3] = two(__float_as_uint((float)(sqrt(dd) * kInvRt3)), 0u);
+    store32(reinterpret_cast<char *>(hdr) + 32, w);
+  }
+  const unsigned long long *sw = reinterpret_cast<const unsigned long long *>(stage) + 4 * q;
+  for (int a = 0; a < 4; ++a) w[a] = sw[a];
+  store32(reinterpret_cast<char *>(mom) + 32 * q, w);
+}
+
+__global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A, int64_t b0) {
+  extern __shared__ __align__(16) double s_dyn[];
+  float (*s_stage)[32] = reinterpret_cast<float (*)[32]>(s_dyn);
+  double *s_v = s_dyn + kBuildThreads / 4 * 16;
+  double *s_rec = s_v + 3 * (kBlockLeaves + 1);
+  __shared__ int s_k;
+  const int tid = threadIdx.x;
+  const int64_t blk = b0 + blockIdx.x;
+  if (tid == 0) s_k = find_loop_of(A.blk_start, A.nloops, blk);
+  __syncthreads();
+  const int k = s_k, l = A.loops[k];
+  const int64_t o = A.off[l], n = A.off[l + 1] - o, first = A.blk_start[k];
+  const int nblk = (int)(A.blk_start[k + 1] - first), j = (int)(blk - first);
+  const int depth = 31 - __clz(nblk);
+  NodeHdr *hdr = A.hdr + A.node_base[l];
+  NodeMom *mom = A.mom + A.node_base[l];
+  const NodeAt whole{0, (int32_t)n, 1, 0};
+  const NodeAt root = descend(whole, j, depth);
+  const int m = root.hi - root.lo;
+  for (int t = tid; t < 3 * (m + 1); t += kBuildThreads) {
+    int64_t v = 3 * (int64_t)root.lo + t;
+    if (v >= 3 * n) v -= 3 * n;
+    s_v[t] = A.xyz[3 * o + v];
+  }
+  __syncthreads();
+  int levels = 0;  // levels between the block's root and its groups
+  while (((m + (1 << levels) - 1) >> levels) > 4) ++levels;
+  const int groups = 1 << levels;
+  // Groups (the first half of the threads) and the two-segment nodes inside
+  // them (the second half).
+  {
+    constexpr int kHalf = kBuildThreads / 2;
+    const bool inner = tid >= kHalf;
+    for (int g = tid & (kHalf - 1); g < groups; g += kHalf) {
+      const NodeAt grp = descend(root, g, levels);
+      const int size = grp.hi - grp.lo;
+      const int nodes = inner ? max(size - 2, 0) : 1;
+      for (int i = 0; i < nodes; ++i) {
+        // Size 3: [lo] [lo+1, lo+3); size 4: [lo, lo+2) [lo+2, lo+4).
+        const NodeAt v = inner ? descend(grp, size == 3 ? 1 : i, 1) : grp;
+        BuildNode P;
+        const double *V = s_v + 3 * (v.lo - root.lo);
+        const int cnt = v.hi - v.lo;
+        for (int a = 0; a < 3; ++a) P.lo[a] = P.hi[a] = V[a];
+        for (int x = 1; x <= cnt; ++x)
+          for (int a = 0; a < 3; ++a) {
+            const double y = V[3 * x + a];
+            P.lo[a] = fmin(P.lo[a], y);
+            P.hi[a] = fmax(P.hi[a], y);
+          }
+        for (int a = 0; a < 3; ++a) {
+          P.mid[a] = 0.5 * (P.hi[a] + P.lo[a]);
+          P.t[a] = 0.0;
+        }
+        for (int a = 0; a < 9; ++a) P.D[a] = 0.0;
+        for (int a = 0; a < 18; ++a) P.Q[a] = 0.0;
+        const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
+        for (int x = 0; x < cnt; ++x) {
+          double t[3], r[3];
+          for (int a = 0; a < 3; ++a) {
+            const double p0 = V[3 * x + a], p1 = V[3 * x + 3 + a];
+            t[a] = p1 - p0;
+            r[a] = (0.5 * p0 + 0.5 * p1) - P.mid[a];
+          }
+          for (int a = 0; a < 3; ++a) P.t[a] += t[a];
+          for (int a = 0; a < 3; ++a)
+            for (int b = 0; b < 3; ++b) P.D[3 * a + b] += t[a] * r[b];
+          for (int kk = 0; kk < 3; ++kk)
+            for (int e = 0; e < 6; ++e)
+              P.Q[6 * kk + e] += ((1.0 / 12.0) * t[kk]) * (t[ii[e]] * t[jj[e]]) + t[kk] * (r[ii[e]] * r[jj[e]]);
+        }
+        P.seg_lo = v.lo;
+        P.seg_cnt = cnt;
+        finish_record(P, hdr[v.pos], mom[v.pos], false, 0, child_place(v.lo, v.lefts));
+        if (!inner) {
+          double *rec = s_rec + g * kRecD;
+          for (int a = 0; a < 3; ++a) {
+            rec[kRLo + a] = P.lo[a];
+            rec[kRHi + a] = P.hi[a];
+            rec[kRMid + a] = P.mid[a];
+            rec[kRT + a] = P.t[a];
+          }
+          for (int a = 0; a < 9; ++a) rec[kRD + a] = P.D[a];
+          for (int a = 0; a < 18; ++a) rec[kRQ + a] = P.Q[a];
+        }
       }
+    }
   }
-  P.seg_lo = lo;
-  P.seg_cnt = hi - lo;
-  if (need) put16(A.bn + g, P);
-  finish_record(P, A.hdr[base + at.x], A.mom[base + at.x], false, 0, at.y);
-}
-
-__global__ void build_height(TreeArgs A, const int64_t *seg_start, const int32_t *bucket, int64_t count,
-                             const int2 *range) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
-  const int64_t g = bucket[e];
-  if (g < 0 || g >= seg_start[A.nloops]) return;  // only after a height-count mismatch, which the host reports
-  const int k = find_loop_of(seg_start, A.nloops, g);
-  const int l = A.loops[k];
-  const int64_t base = A.node_base[l];
-  // Height > kSmallHeight: both children are internal; their build records
-  // are at their split positions.
-  const int2 rg = range[g], at = A.place[g];
-  const int32_t lo = rg.x, hi = rg.y & INT_MAX, mid = lo + (hi - lo) / 2;
-  const BuildNode *bn = A.bn + seg_start[k] - 1;
-  BuildNode L, R;
-  get16(bn + lo + (mid - lo) / 2, L);
-  get16(bn + mid + (hi - mid) / 2, R);
-  BuildNode P;
-  for (int a = 0; a < 3; ++a) {
-    P.lo[a] = fmin(L.lo[a], R.lo[a]);
-    P.hi[a] = fmax(L.hi[a], R.hi[a]);
-    P.mid[a] = 0.5 * (P.hi[a] + P.lo[a]);
-    P.t[a] = 0.0;
+  // Leaves: box, midpoint, tangent c, C_D = 0, C_Q,k = c_k c c^T / 12.
+  for (int i = tid; i < m; i += kBuildThreads) {
+    const int32_t seg = root.lo + i;
+    NodeAt v = root;
+    while (v.hi - v.lo > 1) v = descend(v, seg >= v.lo + (v.hi - v.lo) / 2 ? 1 : 0, 1);
+    double t[3], d[3];
+    NodeHdr h;
+    NodeMom f;
+    for (int a = 0; a < 3; ++a) {
+      const double p0 = s_v[3 * i + a], p1 = s_v[3 * i + 3 + a];
+      t[a] = p1 - p0;
+      h.m[a] = 0.5 * p0 + 0.5 * p1;
+      d[a] = fmax(p0, p1) - fmin(p0, p1);
+    }
+    h.rsq = 0.25 * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    h.r = sqrt(h.rsq);
+    h.left = -1 - seg;
+    h.lo = seg;
+    h.cnt = 1;
+    h.pad = 0;
+    const double tn = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    h.tn = (float)tn;
+    h.dn = 0.f;
+    for (int a = 0; a < 3; ++a) f.t[a] = (float)t[a];
+    for (int a = 0; a < 9; ++a) f.D[a] = 0.f;
+    const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
+    for (int kk = 0; kk < 3; ++kk)
+      for (int e = 0; e < 6; ++e) f.Q[6 * kk + e] = (float)(((1.0 / 12.0) * t[kk]) * (t[ii[e]] * t[jj[e]]));
+    f.qn = (float)(tn * tn * tn / 36.0);
+    f.pad = 0.f;
+    put32(&hdr[v.pos], h);
+    put32(&mom[v.pos], f);
   }
-  for (int a = 0; a < 9; ++a) P.D[a] = 0.0;
-  for (int a = 0; a < 18; ++a) P.Q[a] = 0.0;
-  accumulate_child(P, L);
-  accumulate_child(P, R);
-  P.seg_lo = L.seg_lo;
-  P.seg_cnt = L.seg_cnt + R.seg_cnt;
-  put16(A.bn + g, P);
-  finish_record(P, A.hdr[base + at.x], A.mom[base + at.x], false, 0, at.y);
+  // The levels above the groups: node i of a level with 2^e nodes keeps its
+  // record in its first group's slot.
+  const int q = tid & 3, quad = tid >> 2;
+  for (int e = levels - 1; e >= 0; --e) {
+    __syncthreads();
+    const int step = 1 << (levels - e);
+    for (int i = quad; i < (1 << e); i += kBuildThreads / 4) {
+      const NodeAt v = descend(root, i, e);
+      double *L = s_rec + i * step * kRecD;
+      combine_quad(L, L + (step / 2) * kRecD, L, v, hdr + v.pos, mom + v.pos, s_stage[quad], q, true);
+    }
+  }
+  __syncthreads();
+  // Up from the block's root: one warp; the second of two siblings goes on.
+  if (depth == 0 || tid >= 32) return;
+  BuildNode *up = A.bn + 2 * first;
+  int32_t *arrive = A.arrive + 2 * first;
+  double *own = s_rec, *sib = s_rec + kRecD, *res = s_rec + 2 * kRecD;
+  for (int e = depth, x = j; e > 0; --e, x >>= 1) {
+    double *rec = reinterpret_cast<double *>(up + (1 << e) + x);
+    for (int a = tid; a < kRecD; a += 32) rec[a] = own[a];
+    __threadfence();
+    __syncwarp();
+    int before = 0;
+    if (tid == 0) {
+      cuda::atomic_ref<int32_t, cuda::thread_scope_device> c(arrive[(1 << (e - 1)) + (x >> 1)]);
+      before = c.fetch_add(1, cuda::memory_order_acq_rel);
+    }
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before == 0) return;  // the sibling's warp goes on
+    __threadfence();
+    const double *other = reinterpret_cast<const double *>(up + (1 << e) + (x ^ 1));
+    for (int a = tid; a < kRecD; a += 32) sib[a] = __ldcg(other + a);
+    __syncwarp();
+    const NodeAt v = descend(whole, x >> 1, e - 1);
+    // Every quad of the warp forms the node; the first one stores it.
+    combine_quad((x & 1) ? sib : own, (x & 1) ? own : sib, res, v, hdr + v.pos, mom + v.pos, s_stage[quad], q, quad == 0);
+    __syncwarp();
+    double *t = own;
+    own = res;
+    res = t;
+  }
 }
 
 // ------------------------------------------------------------------ traversal
@@ -1843,35 +1881,6 @@ FLN_TRAVERSE_KERNELS(5)
 FLN_TRAVERSE_KERNELS(6)
 FLN_TRAVERSE_KERNELS(7)
 
-// Internal nodes per height of the curve-order tree of an n-segment loop,
-// added to hcnt[64]: the split of curve_tree_topology ([lo, hi) -> [lo, mid),
-// [mid, hi), mid = lo + (hi - lo) / 2; a node of m >= 2 segments has height
-// ceil(log2 m)). The ranges of one depth have at most two sizes, so this takes
-// O(log n) steps. The host sizes the height launches from it without reading
-// the device's counts back first; the device's counts are checked against it
-// after the build.
-void curve_height_counts(int64_t n, int64_t *hcnt) {
-  std::vector<std::pair<int64_t, int64_t>> cur{{n, 1}}, next;
-  while (!cur.empty()) {
-    next.clear();
-    for (const auto &mc : cur) {
-      const int64_t m = mc.first, c = mc.second;
-      if (m < 2) continue;
-      hcnt[64 - __builtin_clzll((unsigned long long)(m - 1))] += c;
-      for (const int64_t sz : {m / 2, m - m / 2}) {
-        bool merged = false;
-        for (auto &x : next)
-          if (x.first == sz) {
-            x.second += c;
-            merged = true;
-          }
-        if (!merged) next.push_back({sz, c});
-      }
-    }
-    cur.swap(next);
-  }
-}
-
 // Steps a warp spends on a batch in a round of `work` batches on `warps`
 // warps: at most `budget`. While there are fewer batches than warps (the first
 // rounds of a small call, the last heavy loop pairs of a large one) a step
@@ -2691,7 +2700,8 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   std::vector<char> need(nl_all, 0);
   for (int32_t l : h_pairs) need[l] = 1;
   std::vector<int32_t> loops;
-  std::vector<int64_t> node_base(nl_all, 0), seg_int(1, 0), seg_all(1, 0);
+  // blk_start: blocks of the curve-order build (build_curve_trees) before each loop.
+  std::vector<int64_t> node_base(nl_all, 0), seg_all(1, 0), blk_start(1, 0);
   int64_t nodes = 0;
   int maxdepth = 0;
   for (int l = 0; l < nl_all; ++l) {
@@ -2700,32 +2710,34 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     loops.push_back(l);
     node_base[l] = nodes;
     nodes += 2 * n;  // position 0 is unused; even, so that sibling headers share a line
-    seg_int.push_back(seg_int.back() + (n - 1));
     seg_all.push_back(seg_all.back() + n);
+    int64_t nblk = 1;
+    while ((n + nblk - 1) / nblk > kBlockLeaves) nblk *= 2;
+    blk_start.push_back(blk_start.back() + nblk);
     int d = 0;
     while ((int64_t(1) << d) < n) ++d;
     maxdepth = std::max(maxdepth, d);
   }
   const int32_t nloops = (int32_t)loops.size();
-  const int64_t tot_int = seg_int.back(), tot_leaf = seg_all.back();
+  const int64_t tot_leaf = seg_all.back(), tot_blk = blk_start.back();
   // Device buffers (grow-only).
   int32_t *d_loops = ctx.d_bh[0].as<int32_t>(nloops);
   int64_t *d_base = ctx.d_bh[1].as<int64_t>(nl_all);
-  int64_t *d_segint = ctx.d_bh[2].as<int64_t>(nloops + 1);
-  int64_t *d_segall = ctx.d_bh[3].as<int64_t>(nloops + 1);
+  int64_t *d_start = ctx.d_bh[2].as<int64_t>(nloops + 1);  // curve-order: blk_start; kd: seg_all
   const bool kd = prm.bh_tree == 1;
-  int2 *d_place = kd ? nullptr : ctx.d_bh[4].as<int2>(std::max<int64_t>(tot_int, 1));
-  int32_t *d_kd = kd ? ctx.d_bh[5].as<int32_t>(4 * nodes + tot_leaf) : nullptr;  // children, parent, leaf_seg, arrive, leaf_pos
-  BuildNode *d_bn = ctx.d_bh[8].as<BuildNode>(kd ? nodes : std::max<int64_t>(tot_int, 1));
+  int32_t *d_arrive = ctx.d_bh[4].as<int32_t>(kd ? nodes : 2 * tot_blk);
+  int32_t *d_kd = kd ? ctx.d_bh[5].as<int32_t>(3 * nodes + tot_leaf) : nullptr;  // children, parent, leaf_seg, leaf_pos
+  BuildNode *d_bn = ctx.d_bh[8].as<BuildNode>(kd ? nodes : 2 * tot_blk);
   NodeHdr *d_hdr = ctx.d_bh[9].as<NodeHdr>(nodes);
   NodeMom *d_mom = ctx.d_bh[10].as<NodeMom>(nodes);
   cudaStream_t st = ctx.stream;
   FLN_CUDA(cudaMemcpyAsync(d_loops, loops.data(), nloops * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   FLN_CUDA(cudaMemcpyAsync(d_base, node_base.data(), nl_all * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  FLN_CUDA(cudaMemcpyAsync(d_segint, seg_int.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  FLN_CUDA(cudaMemcpyAsync(d_segall, seg_all.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  TreeArgs T{d_xyz, d_off, d_base, d_loops, nloops, d_bn, d_place, d_kd, d_kd + nodes, d_kd + 2 * nodes,
-             d_kd + 3 * nodes, d_kd + 4 * nodes, d_hdr, d_mom};
+  FLN_CUDA(cudaMemcpyAsync(d_start, (kd ? seg_all : blk_start).data(), (nloops + 1) * sizeof(int64_t),
+                           cudaMemcpyHostToDevice, st));
+  FLN_CUDA(cudaMemsetAsync(d_arrive, 0, (kd ? nodes : 2 * tot_blk) * sizeof(int32_t), st));
+  TreeArgs T{d_xyz, d_off, d_base, d_loops, nloops, d_start, d_bn, d_arrive, d_kd, d_kd ? d_kd + nodes : nullptr,
+             d_kd ? d_kd + 2 * nodes : nullptr, d_kd ? d_kd + 3 * nodes : nullptr, d_hdr, d_mom};
   // Slots: pairs ordered by decreasing estimated work. Host work, done once
   // the tree build is queued (while the GPU runs it, before the host waits
   // for its counts).
@@ -2751,7 +2763,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   if (prm.bh_tree == 1) {
     // The reference's kd-median tree, built on the host from a copy of the loops.
     wait_xyz_pieces(ctx);
-    std::vector<int32_t> kd_all(4 * nodes + tot_leaf, 0);
+    std::vector<int32_t> kd_all(3 * nodes + tot_leaf, 0);
     std::vector<double> xyz_host(3 * h_off.back());
     FLN_CUDA(cudaMemcpyAsync(xyz_host.data(), d_xyz, xyz_host.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaStreamSynchronize(st));
@@ -2760,93 +2772,38 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
       const int l = loops[k];
       int32_t *t = kd_all.data() + node_base[l];
       host_kd_tree(xyz_host.data() + 3 * h_off[l], h_off[l + 1] - h_off[l], t, t + nodes, t + 2 * nodes,
-                   kd_all.data() + 4 * nodes + seg_all[k]);
+                   kd_all.data() + 3 * nodes + seg_all[k]);
     }
     FLN_CUDA(cudaMemcpyAsync(d_kd, kd_all.data(), kd_all.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     FLN_CUDA(cudaStreamSynchronize(st));  // host vectors go out of scope
-    build_moments<<<(int)((tot_leaf + 127) / 128), 128, 0, st>>>(T, d_segall, tot_leaf);
+    build_moments<<<(int)((tot_leaf + 127) / 128), 128, 0, st>>>(T, d_start, tot_leaf);
     FLN_CUDA(cudaGetLastError());
     ++launches;
   } else {
-    // Curve-order trees: topology with node heights, leaf records, then one
-    // launch per height (no arrival counters, no serial walk-up chains).
-    uint8_t *d_height = ctx.d_bh[20].as<uint8_t>(std::max<int64_t>(tot_int, 1));
-    // Per group: the device's height counts (checked after the build), then
-    // the height offsets and cursors of bucket_heights.
-    const int max_groups = std::max(ctx.xyz_pieces, 1);
-    int32_t *d_hcnt = ctx.d_bh[18].as<int32_t>((size_t)64 * max_groups + 128);
-    int32_t *d_hoff = d_hcnt + 64 * max_groups, *d_hcur = d_hoff + 64;
-    int32_t *d_bucket = ctx.d_bh[19].as<int32_t>(std::max<int64_t>(tot_int, 1));
-    int2 *d_range = ctx.d_bh[22].as<int2>(std::max<int64_t>(tot_int, 1));
-    // The loops in groups: one per piece of the vertices still arriving from
-    // the host (each group's build waits only for its piece), else one.
-    std::vector<int32_t> group_end;  // loop index (into `loops`) where each group ends
-    std::vector<int> group_piece;
-    if (ctx.xyz_pieces > 0) {
-      int32_t k = 0;
-      for (int i = 0; i < ctx.xyz_pieces; ++i) {
-        while (k < nloops && h_off[loops[k] + 1] <= ctx.xyz_piece_end[i]) ++k;
-        group_end.push_back(k);
-        group_piece.push_back(i);
-      }
-      group_end.back() = nloops;
-    } else {
-      group_end.push_back(nloops);
-      group_piece.push_back(-1);
+    // Curve-order trees: one launch, or one per piece of the vertices still
+    // arriving from the host (each waits only for its piece).
+    if (!ctx.bh_build_smem) {
+      FLN_CUDA(cudaFuncSetAttribute(build_curve_trees, cudaFuncAttributeMaxDynamicSharedMemorySize, kBuildSmem));
+      ctx.bh_build_smem = true;
     }
-    FLN_CUDA(cudaMemsetAsync(d_hcnt, 0, (size_t)64 * max_groups * sizeof(int32_t), st));
-    std::vector<int64_t> host_counts((size_t)64 * group_end.size(), 0);
-    std::vector<int32_t> hoff_all((size_t)64 * group_end.size(), 0);  // lives until the stream has read it
     int32_t k0 = 0;
-    for (size_t gi = 0; gi < group_end.size(); ++gi) {
-      const int32_t k1 = group_end[gi];
-      if (group_piece[gi] >= 0) FLN_CUDA(cudaStreamWaitEvent(st, ctx.ev_piece[group_piece[gi]], 0));
-      if (k1 <= k0) continue;
-      const int64_t i0 = seg_int[k0], i1 = seg_int[k1], f0 = seg_all[k0], f1 = seg_all[k1];
-      int64_t *hc = host_counts.data() + 64 * gi;
-      for (int32_t k = k0; k < k1; ++k) curve_height_counts(h_off[loops[k] + 1] - h_off[loops[k]], hc);
-      if (i1 > i0)
-        curve_tree_topology<<<(int)((i1 - i0 + 255) / 256), 256, 0, st>>>(T, d_segint, i0, i1, d_height,
-                                                                          d_hcnt + 64 * gi, d_range);
-      build_leaves<<<(int)((f1 - f0 + 255) / 256), 256, 0, st>>>(T, d_segall, f0, f1);
-      FLN_CUDA(cudaGetLastError());
-      launches += 2;
-      int32_t hcnt[64];
-      int32_t *hoff = hoff_all.data() + 64 * gi;
-      int64_t acc = i0;  // this group's nodes fill bucket[i0, i1)
-      for (int h = 0; h < 64; ++h) {
-        hcnt[h] = (int32_t)hc[h];
-        hoff[h] = (int32_t)acc;
-        acc += hc[h];
+    for (int i = 0; i < std::max(ctx.xyz_pieces, 1); ++i) {
+      int32_t k1 = k0;
+      if (ctx.xyz_pieces > 0) {
+        FLN_CUDA(cudaStreamWaitEvent(st, ctx.ev_piece[i], 0));
+        while (k1 < nloops && h_off[loops[k1] + 1] <= ctx.xyz_piece_end[i]) ++k1;
+        if (i + 1 == ctx.xyz_pieces) k1 = nloops;
+      } else {
+        k1 = nloops;
       }
-      if (i1 > i0) {
-        FLN_CUDA(cudaMemsetAsync(d_hcur, 0, 64 * sizeof(int32_t), st));
-        FLN_CUDA(cudaMemcpyAsync(d_hoff, hoff, 64 * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-        bucket_heights<<<(int)((i1 - i0 + 255) / 256), 256, 0, st>>>(d_height, i0, i1, d_hoff, d_hcur, d_bucket);
+      for (int64_t b = blk_start[k0]; b < blk_start[k1]; b += INT_MAX) {
+        build_curve_trees<<<(int)std::min<int64_t>(blk_start[k1] - b, INT_MAX), kBuildThreads, kBuildSmem, st>>>(T, b);
         ++launches;
-        const int64_t nsmall = (int64_t)hoff[kSmallHeight + 1] - hoff[1];  // heights 1..kSmallHeight
-        if (nsmall > 0) {
-          build_small<<<(int)((nsmall + 127) / 128), 128, 0, st>>>(T, d_segint, d_bucket + hoff[1], nsmall, d_range);
-          ++launches;
-        }
-        for (int h = kSmallHeight + 1; h < 64; ++h) {
-          if (!hcnt[h]) continue;
-          build_height<<<(hcnt[h] + 127) / 128, 128, 0, st>>>(T, d_segint, d_bucket + hoff[h], hcnt[h], d_range);
-          ++launches;
-        }
-        FLN_CUDA(cudaGetLastError());
       }
+      FLN_CUDA(cudaGetLastError());
       k0 = k1;
     }
     order_slots();
-    // The device's height counts against the host's, which sized the launches.
-    std::vector<int32_t> dev_counts((size_t)64 * group_end.size());
-    FLN_CUDA(cudaMemcpyAsync(dev_counts.data(), d_hcnt, dev_counts.size() * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                             st));
-    FLN_CUDA(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < dev_counts.size(); ++i)
-      if (dev_counts[i] != host_counts[i])
-        throw Error(FLN_ERR_INTERNAL, "curve-order tree: node heights disagree with their count");
   }
   wait_xyz_pieces(ctx);  // the traversal reads every loop's vertices
   FLN_CUDA(cudaEventRecord(ctx.ev3, st));

@@ -114,6 +114,7 @@ struct Context {
   // traversal and of bh_classify; 0 until first queried.
   int bh_per_sm[3] = {0, 0, 0};
   int bh_per_sm_learned = 0, bh_per_sm_classify = 0;
+  bool bh_build_smem = false;  // the tree build's shared memory size is set
   HostBuf h_in, h_out;  // pinned staging of copy_h2d / copy_d2h
   cudaEvent_t ev_stage[2] = {nullptr, nullptr};
   // The exact-list launches of the fused Barnes–Hut rounds run on their own
