@@ -110,21 +110,75 @@ __device__ __noinline__ double term_fp64(double3 p0, double3 p1, double3 q0, dou
 }
 
 // Rescales (x, y) by the power of two that brings max(|x|, |y|) into [1, 2).
+// The exponent is found on the integer pipe.
 __device__ __forceinline__ void renorm(double &x, double &y) {
-  const double m = fmax(fabs(x), fabs(y));
-  int e = (__double2hiint(m) >> 20) & 0x7ff;
+  int e = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >> 20;
   e = min(max(e, 1), 2045);
   const double s = __hiloint2double((2046 - e) << 20, 0);
   x *= s;
   y *= s;
 }
 
+// sqrt(x) for x > 0, within an ulp: the hardware's approximate reciprocal
+// root y (relative error below 2^-19) and one Householder step of third order
+// on h = x y with e = 1 - h y: sqrt(x) = h (1 + e/2 + 3/8 e^2 + O(e^3)). Five
+// FP64 operations and no branch.
+__device__ __forceinline__ double root(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = x * y;
+  const double e = fma(-h, y, 1.0);
+  return fma(fma(0.375, e, 0.5), e * h, h);
+}
+
+__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+
+// A sum of angles as a complex product (x, y), kept near length 1, and a count
+// of full turns (the arctangent addition of compute_link.cpp:245-269). upper:
+// the product lies above the real axis or on its negative half.
+struct AngleSum {
+  double x = 1.0, y = 0.0;
+  int turns = 0;
+  bool upper = false;
+  // Adds arg(px + i py). The sign tests run on the integer pipe.
+  __device__ __forceinline__ void add(double px, double py) {
+    double ny = x * py + px * y;
+    double nx = x * px - y * py;
+    renorm(nx, ny);
+    const bool up = is_zero(ny) ? is_neg(nx) : !is_neg(ny);
+    // Crossed the negative real axis: the product changed sides while the
+    // added angle has the sign of the old side (or is zero).
+    if (up != upper && (is_zero(py) || is_neg(py) != upper)) turns += upper ? 1 : -1;
+    x = nx;
+    y = ny;
+    upper = up;
+  }
+};
+
 // ------------------------------------------------------------------ FP64
-// Tile shape: kB threads per CTA (= curve-1 segments per item), kT curve-2
+// Tile shape: kB threads per CTA, kB curve-1 segments per item, kT curve-2
 // vertices per shared-memory tile.
+//
+// A thread owns two neighbouring curve-1 segments (p0 p1, p1 p2), so that the
+// CTA's threads are two or more groups; the groups take a share of each
+// tile's steps each. Short loops (fewer than kB segments) make more groups,
+// so that the CTA stays full. With v_j = q_k - p_j, w_j = q_{k+1} - p_j and
+// f = q_{k+1} - q_k, a step of the segment p_j p_{j+1} needs
+//   det = e_j . (v_1 x f)  (e_j = p_{j+1} - p_j; one cross product for both
+//         segments, with the relative accuracy of the segment vectors),
+//   the norms of w, v_j . w_j, w_{j+1} . v_j and w_j . w_{j+1}
+// of which the two segments share p1's. That is 102 FP64 operations per two
+// segment pairs, where one segment per thread with library square roots and
+// FP64 sign tests took about 80 per pair.
+//
+// Bound: the FP64 pipe (16 lanes per scheduler and cycle: 204 cycles per
+// warp step of 64 segment pairs, 365 G segment pairs/s at 1,965 MHz).
 template <int kB, int kT>
-__global__ void __launch_bounds__(kB) direct_fp64_kernel(DirectArgs A) {
-  __shared__ double sx[kT + 1], sy[kT + 1], sz[kT + 1];
+__global__ void __launch_bounds__(kB, 512 / kB) direct_fp64_kernel(DirectArgs A) {
+  __shared__ double sq[kT + 1][3], sf[kT][3];  // tile vertices and their differences
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
   for (;;) {
@@ -138,62 +192,93 @@ __global__ void __launch_bounds__(kB) direct_fp64_kernel(DirectArgs A) {
     const int l1 = A.loops[2 * slot], l2 = A.loops[2 * slot + 1];
     const int64_t o1 = A.off[l1], n1 = A.off[l1 + 1] - o1;
     const int64_t o2 = A.off[l2], n2 = A.off[l2 + 1] - o2;
-    const int64_t i = blk * kB + threadIdx.x;
-    const bool active = i < n1;
-    double3 p0 = make_double3(0, 0, 0), p1 = p0;
+    // Threads: `width` segment pairs x `groups` shares of every tile.
+    const int segs = (int)min((int64_t)kB, n1 - blk * kB);
+    const int width = (segs + 1) / 2, groups = kB / width;
+    const int grp = threadIdx.x / width, at = 2 * (threadIdx.x - grp * width);
+    const bool active = grp < groups, second = at + 1 < segs;
+    double3 p0 = make_double3(0, 0, 0), p1 = p0, p2 = p0;
     if (active) {
+      const int64_t i = blk * kB + at;
       p0 = load_v(A.xyz, o1 + i);
       p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
+      p2 = second ? load_v(A.xyz, o1 + (i + 2 == n1 ? 0 : i + 2)) : p1;
     }
-    double xs = 1.0, ys = 0.0, S = -1.0, turns = 0.0;
+    const double e0x = p1.x - p0.x, e0y = p1.y - p0.y, e0z = p1.z - p0.z;
+    const double e1x = p2.x - p1.x, e1y = p2.y - p1.y, e1z = p2.z - p1.z;
+    AngleSum s0, s1;
     for (int64_t k0 = 0; k0 < n2; k0 += kT) {
       const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
       __syncthreads();
       for (int t = threadIdx.x; t <= kt; t += kB) {
         const int64_t kk = k0 + t;
         const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
-        sx[t] = v.x;
-        sy[t] = v.y;
-        sz[t] = v.z;
+        sq[t][0] = v.x;
+        sq[t][1] = v.y;
+        sq[t][2] = v.z;
       }
       __syncthreads();
+      for (int t = threadIdx.x; t < 3 * kt; t += kB) (&sf[0][0])[t] = (&sq[1][0])[t] - (&sq[0][0])[t];
+      __syncthreads();
       if (!active) continue;
-      double ax = sx[0] - p0.x, ay = sy[0] - p0.y, az = sz[0] - p0.z;
-      double bx = sx[0] - p1.x, by = sy[0] - p1.y, bz = sz[0] - p1.z;
-      double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz);
-      double ab = ax * bx + ay * by + az * bz;
-      for (int k = 0; k < kt; ++k) {
-        const double qx = sx[k + 1], qy = sy[k + 1], qz = sz[k + 1];
-        const double cx = qx - p1.x, cy = qy - p1.y, cz = qz - p1.z;
-        const double dx = qx - p0.x, dy = qy - p0.y, dz = qz - p0.z;
-        const double lc = sqrt(cx * cx + cy * cy + cz * cz), ld = sqrt(dx * dx + dy * dy + dz * dz);
-        const double ca = cx * ax + cy * ay + cz * az;
-        const double cb = cx * bx + cy * by + cz * bz;
-        const double ad = ax * dx + ay * dy + az * dz;
-        const double cd = cx * dx + cy * dy + cz * dz;
-        const double det = ax * (by * cz - bz * cy) + az * (bx * cy - by * cx) + ay * (bz * cx - bx * cz);
-        const double t = la * lc;
-        const double div1 = t * lb + ab * lc + ca * lb + cb * la;
-        const double div2 = t * ld + ad * lc + ca * ld + cd * la;
-        const double xp = div1 * div2 - det * det;
-        const double yp = det * (div1 + div2);
-        // Arctangent addition: (xs + i ys) *= (xp + i yp), tracking crossings
-        // of the negative real axis (compute_link.cpp:245-269).
-        double ny = xs * yp + xp * ys;
-        double nx = xs * xp - ys * yp;
-        renorm(nx, ny);
-        if (yp * det < 0) turns += (det > 0) ? 1.0 : -1.0;
-        const double s3 = (ny > 0.0 || (ny == 0.0 && nx < 0.0)) ? 1.0 : -1.0;
-        if (s3 * S < 0 && yp * S >= 0) turns += S;
-        xs = nx;
-        ys = ny;
-        S = s3;
-        ax = dx; ay = dy; az = dz;
-        bx = cx; by = cy; bz = cz;
-        la = ld; lb = lc; ab = cd;
+      const int ka = kt * grp / groups, kb = kt * (grp + 1) / groups;
+      constexpr double kTiny = 1e-300;  // keeps root() away from 0 when two vertices coincide
+      double v0x = sq[ka][0] - p0.x, v0y = sq[ka][1] - p0.y, v0z = sq[ka][2] - p0.z;
+      double v1x = sq[ka][0] - p1.x, v1y = sq[ka][1] - p1.y, v1z = sq[ka][2] - p1.z;
+      double v2x = sq[ka][0] - p2.x, v2y = sq[ka][1] - p2.y, v2z = sq[ka][2] - p2.z;
+      double L0 = root(fma(v0x, v0x, fma(v0y, v0y, fma(v0z, v0z, kTiny))));
+      double L1 = root(fma(v1x, v1x, fma(v1y, v1y, fma(v1z, v1z, kTiny))));
+      double L2 = root(fma(v2x, v2x, fma(v2y, v2y, fma(v2z, v2z, kTiny))));
+      double ab0 = v0x * v1x + v0y * v1y + v0z * v1z, ab1 = v1x * v2x + v1y * v2y + v1z * v2z;
+      for (int k = ka; k < kb; ++k) {
+        const double qx = sq[k + 1][0], qy = sq[k + 1][1], qz = sq[k + 1][2];
+        const double fx = sf[k][0], fy = sf[k][1], fz = sf[k][2];
+        const double w0x = qx - p0.x, w0y = qy - p0.y, w0z = qz - p0.z;
+        const double w1x = qx - p1.x, w1y = qy - p1.y, w1z = qz - p1.z;
+        const double w2x = qx - p2.x, w2y = qy - p2.y, w2z = qz - p2.z;
+        const double M0 = root(fma(w0x, w0x, fma(w0y, w0y, fma(w0z, w0z, kTiny))));
+        const double M1 = root(fma(w1x, w1x, fma(w1y, w1y, fma(w1z, w1z, kTiny))));
+        const double M2 = root(fma(w2x, w2x, fma(w2y, w2y, fma(w2z, w2z, kTiny))));
+        const double cx = v1y * fz - v1z * fy, cy = v1z * fx - v1x * fz, cz = v1x * fy - v1y * fx;
+        const double g0 = v0x * w0x + v0y * w0y + v0z * w0z;
+        const double g1 = v1x * w1x + v1y * w1y + v1z * w1z;
+        const double g2 = v2x * w2x + v2y * w2y + v2z * w2z;
+        {
+          const double det = e0x * cx + e0y * cy + e0z * cz;
+          const double cd = w1x * w0x + w1y * w0y + w1z * w0z;
+          const double u = L0 * M1 + (w1x * v0x + w1y * v0y + w1z * v0z);
+          const double div1 = L1 * u + (ab0 * M1 + g1 * L0);
+          const double div2 = M0 * u + (g0 * M1 + cd * L0);
+          const double sum = div1 + div2;
+          if (is_neg(sum) && !is_zero(det)) s0.turns += is_neg(det) ? -1 : 1;
+          s0.add(div1 * div2 - det * det, det * sum);
+          ab0 = cd;
+        }
+        {
+          const double det = e1x * cx + e1y * cy + e1z * cz;
+          const double cd = w2x * w1x + w2y * w1y + w2z * w1z;
+          const double u = L1 * M2 + (w2x * v1x + w2y * v1y + w2z * v1z);
+          const double div1 = L2 * u + (ab1 * M2 + g2 * L1);
+          const double div2 = M1 * u + (g1 * M2 + cd * L1);
+          const double sum = div1 + div2;
+          if (is_neg(sum) && !is_zero(det)) s1.turns += is_neg(det) ? -1 : 1;
+          s1.add(div1 * div2 - det * det, det * sum);
+          ab1 = cd;
+        }
+        v0x = w0x; v0y = w0y; v0z = w0z;
+        v1x = w1x; v1y = w1y; v1z = w1z;
+        v2x = w2x; v2y = w2y; v2z = w2z;
+        L0 = M0; L1 = M1; L2 = M2;
       }
     }
-    const double v = active ? atan2(ys, xs) * kInvTwoPi + turns : 0.0;
+    double v = 0.0;
+    if (active) {
+      if (second) {
+        s0.add(s1.x, s1.y);
+        s0.turns += s1.turns;
+      }
+      v = atan2(s0.y, s0.x) * kInvTwoPi + (double)s0.turns;
+    }
     const double s = block_sum<kB>(v, s_red);
     if (threadIdx.x == 0) A.partial[item] = s;
   }
