@@ -109,12 +109,11 @@ __device__ __noinline__ double term_fp64(double3 p0, double3 p1, double3 q0, dou
   return r;
 }
 
-// Rescales (x, y) by the power of two that brings max(|x|, |y|) into [1, 2).
-// The exponent is found on the integer pipe.
+// Rescales (x, y) by the power of two that brings max(|x|, |y|) into [1, 2),
+// with the exponent from the integer pipe.
 __device__ __forceinline__ void renorm(double &x, double &y) {
-  int e = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >> 20;
-  e = min(max(e, 1), 2045);
-  const double s = __hiloint2double((2046 - e) << 20, 0);
+  const int e = max(__double2hiint(x) & 0x7ff00000, __double2hiint(y) & 0x7ff00000);
+  const double s = __hiloint2double(0x7fe00000 - min(e, 0x7fd00000), 0);
   x *= s;
   y *= s;
 }
@@ -131,32 +130,85 @@ __device__ __forceinline__ double root(double x) {
   return fma(fma(0.375, e, 0.5), e * h, h);
 }
 
-__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }
-__device__ __forceinline__ bool is_zero(double x) {
-  return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
-}
-
-// A sum of angles as a complex product (x, y), kept near length 1, and a count
-// of full turns (the arctangent addition of compute_link.cpp:245-269). upper:
-// the product lies above the real axis or on its negative half.
+// A sum of angles as a complex product (x, y) and a count of full turns (the
+// arctangent addition of compute_link.cpp:245-269).
 struct AngleSum {
   double x = 1.0, y = 0.0;
   int turns = 0;
-  bool upper = false;
-  // Adds arg(px + i py). The sign tests run on the integer pipe.
-  __device__ __forceinline__ void add(double px, double py) {
-    double ny = x * py + px * y;
-    double nx = x * px - y * py;
-    renorm(nx, ny);
-    const bool up = is_zero(ny) ? is_neg(nx) : !is_neg(ny);
-    // Crossed the negative real axis: the product changed sides while the
-    // added angle has the sign of the old side (or is zero).
-    if (up != upper && (is_zero(py) || is_neg(py) != upper)) turns += upper ? 1 : -1;
+  // Above the real axis or on its negative half.
+  static __device__ __forceinline__ bool upper(double x, double y) { return y > 0.0 || (y == 0.0 && x < 0.0); }
+  // Adds the angle of the segment-pair term (px + i py), where py = det x sum:
+  // its arctangent's principal value, a turn more or less when sum < 0.
+  // The product crosses the negative real axis when it changes sides while the
+  // added angle has the sign of the old side (or is zero); since that angle is
+  // at most half a turn, the old or the new product then lies left of the
+  // imaginary axis, which is rare, so the crossing test sits in a branch.
+  __device__ __forceinline__ void add(double px, double py, double det, double sum) {
+    const double ny = x * py + px * y;
+    const double nx = x * px - y * py;
+    if (__builtin_expect((__double2hiint(x) | __double2hiint(nx) | __double2hiint(sum)) < 0, 0)) {
+      if (sum < 0.0 && det != 0.0) turns += det > 0.0 ? 1 : -1;
+      const bool was = upper(x, y);
+      if (upper(nx, ny) != was && (was ? py >= 0.0 : py <= 0.0)) turns += was ? 1 : -1;
+    }
     x = nx;
     y = ny;
-    upper = up;
   }
 };
+
+// The walk of two neighbouring segments p0 p1, p1 p2 along curve 2, at q_k:
+// v_j = q_k - p_j, their norms, and the dot products of neighbours.
+struct Walk2 {
+  double v0x, v0y, v0z, v1x, v1y, v1z, v2x, v2y, v2z;
+  double L0, L1, L2, ab0, ab1;
+};
+struct __align__(16) TileVertex {  // a curve-2 vertex q and f = next vertex - q: three 16-byte loads
+  double2 q01, q2f0, f12;
+};
+struct Segs2 {
+  double3 p0, p1, p2, e0, e1;  // e_j = p_{j+1} - p_j
+};
+
+constexpr double kTiny = 1e-300;  // keeps root() away from 0 when two vertices coincide
+__device__ __forceinline__ void walk_to(const Segs2 &S, const TileVertex &t, Walk2 &w) {
+  const double qx = t.q01.x, qy = t.q01.y, qz = t.q2f0.x;
+  w.v0x = qx - S.p0.x; w.v0y = qy - S.p0.y; w.v0z = qz - S.p0.z;
+  w.v1x = qx - S.p1.x; w.v1y = qy - S.p1.y; w.v1z = qz - S.p1.z;
+  w.v2x = qx - S.p2.x; w.v2y = qy - S.p2.y; w.v2z = qz - S.p2.z;
+  w.L0 = root(fma(w.v0x, w.v0x, fma(w.v0y, w.v0y, fma(w.v0z, w.v0z, kTiny))));
+  w.L1 = root(fma(w.v1x, w.v1x, fma(w.v1y, w.v1y, fma(w.v1z, w.v1z, kTiny))));
+  w.L2 = root(fma(w.v2x, w.v2x, fma(w.v2y, w.v2y, fma(w.v2z, w.v2z, kTiny))));
+  w.ab0 = w.v0x * w.v1x + w.v0y * w.v1y + w.v0z * w.v1z;
+  w.ab1 = w.v1x * w.v2x + w.v1y * w.v2y + w.v1z * w.v2z;
+}
+
+// One step q_k -> q_{k+1} (f = q_{k+1} - q_k): the walk goes from a to w, and
+// the two segments' terms are added to s0 and s1.
+__device__ __forceinline__ void walk_step(const Segs2 &S, const Walk2 &a, Walk2 &w, const TileVertex &at,
+                                          const TileVertex &to, AngleSum &s0, AngleSum &s1) {
+  walk_to(S, to, w);
+  const double fx = at.q2f0.y, fy = at.f12.x, fz = at.f12.y;
+  const double cx = a.v1y * fz - a.v1z * fy, cy = a.v1z * fx - a.v1x * fz, cz = a.v1x * fy - a.v1y * fx;
+  const double g0 = a.v0x * w.v0x + a.v0y * w.v0y + a.v0z * w.v0z;
+  const double g1 = a.v1x * w.v1x + a.v1y * w.v1y + a.v1z * w.v1z;
+  const double g2 = a.v2x * w.v2x + a.v2y * w.v2y + a.v2z * w.v2z;
+  {
+    const double det = S.e0.x * cx + S.e0.y * cy + S.e0.z * cz;
+    const double u = a.L0 * w.L1 + (w.v1x * a.v0x + w.v1y * a.v0y + w.v1z * a.v0z);
+    const double div1 = a.L1 * u + (a.ab0 * w.L1 + g1 * a.L0);
+    const double div2 = w.L0 * u + (g0 * w.L1 + w.ab0 * a.L0);
+    const double sum = div1 + div2;
+    s0.add(div1 * div2 - det * det, det * sum, det, sum);
+  }
+  {
+    const double det = S.e1.x * cx + S.e1.y * cy + S.e1.z * cz;
+    const double u = a.L1 * w.L2 + (w.v2x * a.v1x + w.v2y * a.v1y + w.v2z * a.v1z);
+    const double div1 = a.L2 * u + (a.ab1 * w.L2 + g2 * a.L1);
+    const double div2 = w.L1 * u + (g1 * w.L2 + w.ab1 * a.L1);
+    const double sum = div1 + div2;
+    s1.add(div1 * div2 - det * det, det * sum, det, sum);
+  }
+}
 
 // ------------------------------------------------------------------ FP64
 // Tile shape: kB threads per CTA, kB curve-1 segments per item, kT curve-2
@@ -170,15 +222,21 @@ struct AngleSum {
 //   det = e_j . (v_1 x f)  (e_j = p_{j+1} - p_j; one cross product for both
 //         segments, with the relative accuracy of the segment vectors),
 //   the norms of w, v_j . w_j, w_{j+1} . v_j and w_j . w_{j+1}
-// of which the two segments share p1's. That is 102 FP64 operations per two
-// segment pairs, where one segment per thread with library square roots and
-// FP64 sign tests took about 80 per pair.
+// of which the two segments share p1's: 50 FP64 operations per segment pair,
+// where one segment per thread with library square roots and FP64 sign tests
+// took about 80.
 //
-// Bound: the FP64 pipe (16 lanes per scheduler and cycle: 204 cycles per
-// warp step of 64 segment pairs, 365 G segment pairs/s at 1,965 MHz).
+// Bound: the schedulers. An FP64 instruction holds a scheduler's issue port
+// for two cycles (16 lanes), so a step of 64 segment pairs costs 200 cycles
+// plus one for every other instruction; hence the sign tests in a rare branch,
+// the tile in 16-byte loads, the rescaling once per two steps and the
+// two-state walk. 12 walks of 4,001 steps (1.84e9 segment pairs), B200: 12.6 ms
+// with one segment per thread, 8.0 with two, 7.6 with the two-state walk, 6.9
+// with the rest (267 G segment pairs/s; 372 G at 200 cycles a step). Twelve
+// warps of 144 registers per SM; sixteen of 128 took 7.1 ms.
 template <int kB, int kT>
-__global__ void __launch_bounds__(kB, 512 / kB) direct_fp64_kernel(DirectArgs A) {
-  __shared__ double sq[kT + 1][3], sf[kT][3];  // tile vertices and their differences
+__global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_kernel(DirectArgs A) {
+  __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
   for (;;) {
@@ -197,15 +255,16 @@ __global__ void __launch_bounds__(kB, 512 / kB) direct_fp64_kernel(DirectArgs A)
     const int width = (segs + 1) / 2, groups = kB / width;
     const int grp = threadIdx.x / width, at = 2 * (threadIdx.x - grp * width);
     const bool active = grp < groups, second = at + 1 < segs;
-    double3 p0 = make_double3(0, 0, 0), p1 = p0, p2 = p0;
+    Segs2 S;
+    S.p0 = S.p1 = S.p2 = make_double3(0, 0, 0);
     if (active) {
       const int64_t i = blk * kB + at;
-      p0 = load_v(A.xyz, o1 + i);
-      p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
-      p2 = second ? load_v(A.xyz, o1 + (i + 2 == n1 ? 0 : i + 2)) : p1;
+      S.p0 = load_v(A.xyz, o1 + i);
+      S.p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
+      S.p2 = second ? load_v(A.xyz, o1 + (i + 2 == n1 ? 0 : i + 2)) : S.p1;
     }
-    const double e0x = p1.x - p0.x, e0y = p1.y - p0.y, e0z = p1.z - p0.z;
-    const double e1x = p2.x - p1.x, e1y = p2.y - p1.y, e1z = p2.z - p1.z;
+    S.e0 = make_double3(S.p1.x - S.p0.x, S.p1.y - S.p0.y, S.p1.z - S.p0.z);
+    S.e1 = make_double3(S.p2.x - S.p1.x, S.p2.y - S.p1.y, S.p2.z - S.p1.z);
     AngleSum s0, s1;
     for (int64_t k0 = 0; k0 < n2; k0 += kT) {
       const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
@@ -213,68 +272,37 @@ __global__ void __launch_bounds__(kB, 512 / kB) direct_fp64_kernel(DirectArgs A)
       for (int t = threadIdx.x; t <= kt; t += kB) {
         const int64_t kk = k0 + t;
         const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
-        sq[t][0] = v.x;
-        sq[t][1] = v.y;
-        sq[t][2] = v.z;
+        tile[t].q01 = make_double2(v.x, v.y);
+        tile[t].q2f0.x = v.z;
       }
       __syncthreads();
-      for (int t = threadIdx.x; t < 3 * kt; t += kB) (&sf[0][0])[t] = (&sq[1][0])[t] - (&sq[0][0])[t];
+      for (int t = threadIdx.x; t < kt; t += kB) {
+        tile[t].q2f0.y = tile[t + 1].q01.x - tile[t].q01.x;
+        tile[t].f12 = make_double2(tile[t + 1].q01.y - tile[t].q01.y, tile[t + 1].q2f0.x - tile[t].q2f0.x);
+      }
       __syncthreads();
       if (!active) continue;
       const int ka = kt * grp / groups, kb = kt * (grp + 1) / groups;
-      constexpr double kTiny = 1e-300;  // keeps root() away from 0 when two vertices coincide
-      double v0x = sq[ka][0] - p0.x, v0y = sq[ka][1] - p0.y, v0z = sq[ka][2] - p0.z;
-      double v1x = sq[ka][0] - p1.x, v1y = sq[ka][1] - p1.y, v1z = sq[ka][2] - p1.z;
-      double v2x = sq[ka][0] - p2.x, v2y = sq[ka][1] - p2.y, v2z = sq[ka][2] - p2.z;
-      double L0 = root(fma(v0x, v0x, fma(v0y, v0y, fma(v0z, v0z, kTiny))));
-      double L1 = root(fma(v1x, v1x, fma(v1y, v1y, fma(v1z, v1z, kTiny))));
-      double L2 = root(fma(v2x, v2x, fma(v2y, v2y, fma(v2z, v2z, kTiny))));
-      double ab0 = v0x * v1x + v0y * v1y + v0z * v1z, ab1 = v1x * v2x + v1y * v2y + v1z * v2z;
-      for (int k = ka; k < kb; ++k) {
-        const double qx = sq[k + 1][0], qy = sq[k + 1][1], qz = sq[k + 1][2];
-        const double fx = sf[k][0], fy = sf[k][1], fz = sf[k][2];
-        const double w0x = qx - p0.x, w0y = qy - p0.y, w0z = qz - p0.z;
-        const double w1x = qx - p1.x, w1y = qy - p1.y, w1z = qz - p1.z;
-        const double w2x = qx - p2.x, w2y = qy - p2.y, w2z = qz - p2.z;
-        const double M0 = root(fma(w0x, w0x, fma(w0y, w0y, fma(w0z, w0z, kTiny))));
-        const double M1 = root(fma(w1x, w1x, fma(w1y, w1y, fma(w1z, w1z, kTiny))));
-        const double M2 = root(fma(w2x, w2x, fma(w2y, w2y, fma(w2z, w2z, kTiny))));
-        const double cx = v1y * fz - v1z * fy, cy = v1z * fx - v1x * fz, cz = v1x * fy - v1y * fx;
-        const double g0 = v0x * w0x + v0y * w0y + v0z * w0z;
-        const double g1 = v1x * w1x + v1y * w1y + v1z * w1z;
-        const double g2 = v2x * w2x + v2y * w2y + v2z * w2z;
-        {
-          const double det = e0x * cx + e0y * cy + e0z * cz;
-          const double cd = w1x * w0x + w1y * w0y + w1z * w0z;
-          const double u = L0 * M1 + (w1x * v0x + w1y * v0y + w1z * v0z);
-          const double div1 = L1 * u + (ab0 * M1 + g1 * L0);
-          const double div2 = M0 * u + (g0 * M1 + cd * L0);
-          const double sum = div1 + div2;
-          if (is_neg(sum) && !is_zero(det)) s0.turns += is_neg(det) ? -1 : 1;
-          s0.add(div1 * div2 - det * det, det * sum);
-          ab0 = cd;
-        }
-        {
-          const double det = e1x * cx + e1y * cy + e1z * cz;
-          const double cd = w2x * w1x + w2y * w1y + w2z * w1z;
-          const double u = L1 * M2 + (w2x * v1x + w2y * v1y + w2z * v1z);
-          const double div1 = L2 * u + (ab1 * M2 + g2 * L1);
-          const double div2 = M1 * u + (g1 * M2 + cd * L1);
-          const double sum = div1 + div2;
-          if (is_neg(sum) && !is_zero(det)) s1.turns += is_neg(det) ? -1 : 1;
-          s1.add(div1 * div2 - det * det, det * sum);
-          ab1 = cd;
-        }
-        v0x = w0x; v0y = w0y; v0z = w0z;
-        v1x = w1x; v1y = w1y; v1z = w1z;
-        v2x = w2x; v2y = w2y; v2z = w2z;
-        L0 = M0; L1 = M1; L2 = M2;
+      // Two steps per pass, the walk going a -> b -> a (no copies of its state).
+      Walk2 a, b;
+      walk_to(S, tile[ka], a);
+      int k = ka;
+      for (; k + 2 <= kb; k += 2) {
+        walk_step(S, a, b, tile[k], tile[k + 1], s0, s1);
+        walk_step(S, b, a, tile[k + 1], tile[k + 2], s0, s1);
+        renorm(s0.x, s0.y);  // a term is at most 64 |q - p|^6: no overflow in two steps below 1e24
+        renorm(s1.x, s1.y);
+      }
+      if (k < kb) {
+        walk_step(S, a, b, tile[k], tile[k + 1], s0, s1);
+        renorm(s0.x, s0.y);
+        renorm(s1.x, s1.y);
       }
     }
     double v = 0.0;
     if (active) {
       if (second) {
-        s0.add(s1.x, s1.y);
+        s0.add(s1.x, s1.y, 0.0, 0.0);
         s0.turns += s1.turns;
       }
       v = atan2(s0.y, s0.x) * kInvTwoPi + (double)s0.turns;
