@@ -39,7 +39,7 @@ Context::~Context() {
   if (exact_stream) cudaStreamSynchronize(exact_stream);
   if (copy_stream) cudaStreamSynchronize(copy_stream);
   for (DevBuf *b : {&d_xyz, &d_off, &d_pairs, &d_loops, &d_items, &d_partial, &d_counter, &d_lk, &d_err, &d_flags,
-                    &d_near})
+                    &d_near, &d_redo})
     b->release();
   for (auto &b : d_bh) b.release();
   d_mlp.release();
@@ -136,14 +136,7 @@ void copy_d2h(Context &ctx, void *h_dst, const void *d_src, size_t bytes) {
 // Scatters src[k] into dst[idx[k]] for the FP64 recompute (defined in bh.cu).
 void scatter_doubles(Context &ctx, const double *src, const int32_t *idx, int64_t n, double *dst);
 
-// Runs the requested method over device-resident loops and pairs, then the
-// margin check and FP64 direct-sum recompute of the pairs that fail it.
-static int run_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                     const std::vector<int32_t> &h_pairs, fln_method method, const fln_params &prm,
-                     double *d_lk, double *d_err, int32_t *d_flags) {
-  const int64_t np = (int64_t)h_pairs.size() / 2;
-  int launches = 0;
-  double near_terms = 0;
+static void clear_stats(Context &ctx) {
   ctx.stats.ms_main_kernel = 0;
   ctx.stats.ms_tree_build = 0;
   ctx.stats.bh_far_evals = ctx.stats.bh_leaf_evals = 0;
@@ -154,30 +147,49 @@ static int run_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, co
   ctx.stats.bh_far_reused = ctx.stats.bh_far_subtracted = 0;
   ctx.stats.beta_retried = 0;
   ctx.stats.bh_escalated = 0;
-  if (!d_err) d_err = ctx.d_err.as<double>(std::max<int64_t>(np, 1));  // Barnes–Hut needs one
-  if (method == FLN_METHOD_DIRECTSUM) {
-    launches += direct_sum_device(ctx, d_xyz, d_off, h_off, h_pairs, prm.precision, prm.near_factor, d_lk,
-                                  prm.precision == FLN_PREC_MIXED ? &near_terms : nullptr, prm.direct_tile);
-    if (d_err) FLN_CUDA(cudaMemsetAsync(d_err, 0, np * sizeof(double), ctx.stream));
-    if (d_flags) FLN_CUDA(cudaMemsetAsync(d_flags, 0, np * sizeof(int32_t), ctx.stream));
-  } else {
-    launches += barnes_hut_device(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags);
-  }
-  ctx.stats.near_fp64_terms = near_terms;
-  const bool checked = !(method == FLN_METHOD_DIRECTSUM && prm.precision == FLN_PREC_FP64);
+  ctx.stats.near_fp64_terms = 0;
   ctx.stats.fp64_recomputed = 0;
-  if (checked && np > 0) {
+}
+
+// Direct sum over device-resident loops and pairs, with the margin check and
+// FP64 recompute of the mixed precision.
+static int run_direct(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops, const int32_t *d_pairs,
+                      int64_t np, const fln_params &prm, double *d_lk, double *d_err, int32_t *d_flags) {
+  clear_stats(ctx);
+  const bool checked = prm.precision != FLN_PREC_FP64;
+  // A margin is in [0, 0.5]: at most 0 recomputes only what is not finite, and
+  // what no margin reaches (NaN too) recomputes every pair.
+  const double margin = prm.fp64_margin <= 0 ? 0.0 : prm.fp64_margin <= 0.5 ? prm.fp64_margin : 1.0;
+  const DirectResult r = direct_sum_device(ctx, d_xyz, d_off, nloops, d_pairs, np, prm.precision, prm.near_factor,
+                                           checked ? margin : -1.0, d_lk, d_err, d_flags, prm.direct_tile);
+  ctx.stats.near_fp64_terms = checked ? r.near_terms : 0.0;
+  ctx.stats.fp64_recomputed = r.redone;
+  ctx.stats.segment_pairs = r.work;
+  ctx.stats.pairs = np;
+  return r.launches;
+}
+
+// Barnes–Hut over device-resident loops and pairs, then the margin check and
+// FP64 direct-sum recompute of the pairs that fail it.
+static int run_barnes_hut(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
+                          const std::vector<int32_t> &h_pairs, const fln_params &prm, double *d_lk, double *d_err,
+                          int32_t *d_flags) {
+  const int64_t np = (int64_t)h_pairs.size() / 2;
+  clear_stats(ctx);
+  if (!d_err) d_err = ctx.d_err.as<double>(std::max<int64_t>(np, 1));
+  int launches = barnes_hut_device(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags);
+  if (np > 0) {
     std::vector<double> lk(np), err(np, 0.0);
     FLN_CUDA(cudaMemcpyAsync(lk.data(), d_lk, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-    if (d_err) FLN_CUDA(cudaMemcpyAsync(err.data(), d_err, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+    FLN_CUDA(cudaMemcpyAsync(err.data(), d_err, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
     FLN_CUDA(cudaStreamSynchronize(ctx.stream));
     std::vector<int32_t> redo_idx, redo_pairs;
     for (int64_t p = 0; p < np; ++p) {
       const double r = std::round(lk[p]);
       const double margin = 0.5 - std::fabs(lk[p] - r);
-      // Low margin, non-finite, or a Barnes–Hut error estimate that could
-      // reach the rounding boundary: recompute in FP64 direct sum.
-      if (!(margin >= prm.fp64_margin) || (method == FLN_METHOD_BARNESHUT && !(err[p] <= prm.bh_err_limit))) {
+      // Low margin, non-finite, or an error estimate that could reach the
+      // rounding boundary: recompute in FP64 direct sum.
+      if (!(margin >= prm.fp64_margin) || !(err[p] <= prm.bh_err_limit)) {
         redo_idx.push_back((int32_t)p);
         redo_pairs.push_back(h_pairs[2 * p]);
         redo_pairs.push_back(h_pairs[2 * p + 1]);
@@ -185,9 +197,12 @@ static int run_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, co
     }
     if (!redo_idx.empty()) {
       const int64_t nr = (int64_t)redo_idx.size();
-      double *d_tmp = ctx.d_near.as<double>(nr + nr / 2 + 2);
-      int32_t *d_idx = reinterpret_cast<int32_t *>(d_tmp + nr);
-      launches += direct_sum_device(ctx, d_xyz, d_off, h_off, redo_pairs, FLN_PREC_FP64, 0.0, d_tmp, nullptr);
+      double *d_tmp = ctx.d_redo.as<double>(nr + nr / 2 + 2 + nr);
+      int32_t *d_idx = reinterpret_cast<int32_t *>(d_tmp + nr), *d_pr = d_idx + nr + (nr & 1);
+      FLN_CUDA(cudaMemcpyAsync(d_pr, redo_pairs.data(), 2 * nr * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
+      launches += direct_sum_device(ctx, d_xyz, d_off, (int32_t)h_off.size() - 1, d_pr, nr, FLN_PREC_FP64, 0.0, -1.0,
+                                    d_tmp, nullptr, nullptr)
+                      .launches;
       FLN_CUDA(cudaMemcpyAsync(d_idx, redo_idx.data(), nr * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
       scatter_doubles(ctx, d_tmp, d_idx, nr, d_lk);
       ++launches;
@@ -349,30 +364,69 @@ void compute_pairs_host(Context &ctx, const double *xyz, const int64_t *loop_off
   std::vector<int32_t> h_pairs(pairs, pairs + 2 * npairs);
   check_inputs(h_off, nloops, h_pairs);
   const int64_t nv = h_off[nloops];
-  double *d_xyz = ctx.d_xyz.as<double>(3 * std::max<int64_t>(nv, 1));
-  int64_t *d_off = ctx.d_off.as<int64_t>(nloops + 1);
-  double *d_lk = ctx.d_lk.as<double>(std::max<int64_t>(npairs, 1));
-  double *d_err = ctx.d_err.as<double>(std::max<int64_t>(npairs, 1));
-  int32_t *d_flags = ctx.d_flags.as<int32_t>(std::max<int64_t>(npairs, 1));
+  const size_t bx = 3 * nv * sizeof(double), bo = (nloops + 1) * sizeof(int64_t), bp = 2 * npairs * sizeof(int32_t);
+  const int64_t np1 = std::max<int64_t>(npairs, 1);
+  // Results in one buffer: sums, estimates, flags.
+  double *d_lk = ctx.d_lk.as<double>(2 * np1 + (np1 + 1) / 2), *d_err = d_lk + np1;
+  int32_t *d_flags = reinterpret_cast<int32_t *>(d_err + np1);
+  const size_t br = npairs * (2 * sizeof(double) + sizeof(int32_t));
+  const bool bh = method == FLN_METHOD_BARNESHUT;
+  // A small call's inputs go up in one copy from pinned memory, and its
+  // results come back in one: the call is a handful of launches, and each
+  // pageable copy would cost as much as one of them.
+  constexpr size_t kSmallCall = size_t(1) << 20;
+  const bool small = bx + bo + bp <= kSmallCall && br <= kSmallCall;
+  double *d_xyz;
+  int64_t *d_off;
+  int32_t *d_pairs;
   FLN_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
   ctx.xyz_pieces = 0;
-  if (!(method == FLN_METHOD_BARNESHUT && prm.bh_tree == 0 && copy_xyz_pieces(ctx, d_xyz, xyz, h_off)))
-    copy_h2d(ctx, d_xyz, xyz, 3 * nv * sizeof(double));
-  FLN_CUDA(cudaMemcpyAsync(d_off, h_off.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx.stream));
+  if (small) {
+    char *h = static_cast<char *>(ctx.h_call.need(2 * kSmallCall));
+    char *d = static_cast<char *>(ctx.d_xyz.need(std::max<size_t>(bx + bo + bp, 16)));
+    std::memcpy(h, h_off.data(), bo);
+    if (bp) std::memcpy(h + bo, h_pairs.data(), bp);
+    if (bx) std::memcpy(h + bo + bp, xyz, bx);
+    FLN_CUDA(cudaMemcpyAsync(d, h, bx + bo + bp, cudaMemcpyHostToDevice, ctx.stream));
+    d_off = reinterpret_cast<int64_t *>(d);
+    d_pairs = reinterpret_cast<int32_t *>(d + bo);
+    d_xyz = reinterpret_cast<double *>(d + bo + bp);
+  } else {
+    d_xyz = ctx.d_xyz.as<double>(3 * std::max<int64_t>(nv, 1));
+    d_off = ctx.d_off.as<int64_t>(nloops + 1);
+    d_pairs = nullptr;
+    if (!(bh && prm.bh_tree == 0 && copy_xyz_pieces(ctx, d_xyz, xyz, h_off))) copy_h2d(ctx, d_xyz, xyz, bx);
+    FLN_CUDA(cudaMemcpyAsync(d_off, h_off.data(), bo, cudaMemcpyHostToDevice, ctx.stream));
+    if (!bh) {
+      d_pairs = ctx.d_pairs.as<int32_t>(2 * np1);
+      FLN_CUDA(cudaMemcpyAsync(d_pairs, h_pairs.data(), bp, cudaMemcpyHostToDevice, ctx.stream));
+    }
+  }
   int launches = 0;
   try {
-    launches = run_pairs(ctx, d_xyz, d_off, h_off, h_pairs, method, prm, d_lk, d_err, d_flags);
+    launches = bh ? run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags)
+                  : run_direct(ctx, d_xyz, d_off, nloops, d_pairs, npairs, prm, d_lk, d_err, d_flags);
   } catch (...) {
     wait_xyz_pieces(ctx);
     throw;
   }
   wait_xyz_pieces(ctx);
   FLN_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
-  FLN_CUDA(cudaMemcpyAsync(lk_out, d_lk, npairs * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-  if (err_out) FLN_CUDA(cudaMemcpyAsync(err_out, d_err, npairs * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-  if (flags_out)
-    FLN_CUDA(cudaMemcpyAsync(flags_out, d_flags, npairs * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx.stream));
-  FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+  if (small && npairs > 0) {
+    char *h = static_cast<char *>(ctx.h_call.need(2 * kSmallCall)) + kSmallCall;
+    FLN_CUDA(cudaMemcpyAsync(h, d_lk, 2 * np1 * sizeof(double) + np1 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                             ctx.stream));
+    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+    std::memcpy(lk_out, h, npairs * sizeof(double));
+    if (err_out) std::memcpy(err_out, h + np1 * sizeof(double), npairs * sizeof(double));
+    if (flags_out) std::memcpy(flags_out, h + 2 * np1 * sizeof(double), npairs * sizeof(int32_t));
+  } else {
+    FLN_CUDA(cudaMemcpyAsync(lk_out, d_lk, npairs * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+    if (err_out) FLN_CUDA(cudaMemcpyAsync(err_out, d_err, npairs * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+    if (flags_out)
+      FLN_CUDA(cudaMemcpyAsync(flags_out, d_flags, npairs * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx.stream));
+    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+  }
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1);
   ctx.stats.ms_kernels = ms;
@@ -513,18 +567,25 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz, const i
     Context &c = *ctx->c;
     const double t0 = now_ms();
     FLN_CUDA(cudaSetDevice(c.device));
-    std::vector<int64_t> h_off(nloops + 1);
-    std::vector<int32_t> h_pairs(2 * npairs);
     FLN_CUDA(cudaEventRecord(c.ev0, c.stream));
-    FLN_CUDA(cudaMemcpyAsync(h_off.data(), d_loop_offsets, (nloops + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
-                             c.stream));
-    if (npairs)
-      FLN_CUDA(cudaMemcpyAsync(h_pairs.data(), d_pairs, 2 * npairs * sizeof(int32_t), cudaMemcpyDeviceToHost,
+    int launches;
+    if (method == FLN_METHOD_DIRECTSUM && npairs > 0) {
+      // Planned and checked on the device: nothing comes to the host first.
+      launches = run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, npairs, prm, d_lk_out, d_err_out, d_flags_out);
+    } else {
+      std::vector<int64_t> h_off(nloops + 1);
+      std::vector<int32_t> h_pairs(2 * npairs);
+      FLN_CUDA(cudaMemcpyAsync(h_off.data(), d_loop_offsets, (nloops + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                                c.stream));
-    FLN_CUDA(cudaStreamSynchronize(c.stream));
-    check_inputs(h_off, nloops, h_pairs);
-    const int launches = run_pairs(c, d_xyz, d_loop_offsets, h_off, h_pairs, method, prm, d_lk_out, d_err_out,
-                                   d_flags_out);
+      if (npairs)
+        FLN_CUDA(cudaMemcpyAsync(h_pairs.data(), d_pairs, 2 * npairs * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                 c.stream));
+      FLN_CUDA(cudaStreamSynchronize(c.stream));
+      check_inputs(h_off, nloops, h_pairs);
+      launches = method == FLN_METHOD_DIRECTSUM
+                     ? run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, 0, prm, d_lk_out, d_err_out, d_flags_out)
+                     : run_barnes_hut(c, d_xyz, d_loop_offsets, h_off, h_pairs, prm, d_lk_out, d_err_out, d_flags_out);
+    }
     FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
     FLN_CUDA(cudaStreamSynchronize(c.stream));
     float ms = 0;
@@ -776,11 +837,13 @@ fln_status fln_autotune_direct(fln_ctx *ctx, const double *xyz, const int64_t *l
     const int64_t np = (int64_t)h_pairs.size() / 2;
     double *d_lk = c.d_lk.as<double>(np), *d_err = c.d_err.as<double>(np);
     int32_t *d_fl = c.d_flags.as<int32_t>(np);
+    int32_t *d_pr = c.d_pairs.as<int32_t>(2 * np);
+    FLN_CUDA(cudaMemcpyAsync(d_pr, h_pairs.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, c.stream));
     auto time_of = [&](const fln_params &p) {
       double best = 1e300;
       for (int rep = 0; rep < 3; ++rep) {
         FLN_CUDA(cudaEventRecord(c.ev0, c.stream));
-        run_pairs(c, d_xyz, d_off, h_off, h_pairs, FLN_METHOD_DIRECTSUM, p, d_lk, d_err, d_fl);
+        run_direct(c, d_xyz, d_off, nloops, d_pr, np, p, d_lk, d_err, d_fl);
         FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
         best = std::min(best, (double)c.elapsed(c.ev0, c.ev1));
       }
@@ -834,7 +897,7 @@ fln_status fln_autotune(fln_ctx *ctx, const double *xyz, const int64_t *loop_off
       double best = 1e300;
       for (int rep = 0; rep < 3; ++rep) {
         FLN_CUDA(cudaEventRecord(c.ev0, c.stream));
-        run_pairs(c, d_xyz, d_off, h_off, h_pairs, FLN_METHOD_BARNESHUT, p, d_lk, d_err, d_fl);
+        run_barnes_hut(c, d_xyz, d_off, h_off, h_pairs, p, d_lk, d_err, d_fl);
         FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
         best = std::min(best, (double)c.elapsed(c.ev0, c.ev1));
       }

@@ -1,12 +1,13 @@
 // Direct summation of the Gauss linking integral on B200 (sm_100a).
 //
-// Work: every potential loop pair (i, j) is split into items of kBlockSegs
-// consecutive segments of its longer loop ("curve 1"); one CTA of kBlockSegs
-// threads takes items from a device work queue (an atomic counter) until it
-// runs dry, so all pairs — 16-segment rings to 2^18-segment loops — run in
-// one persistent launch. Each thread owns one curve-1 segment and walks all
-// curve-2 segments, which the CTA stages tile by tile in shared memory
-// (coalesced loads, broadcast reads). Per segment pair it evaluates the
+// Work: every potential loop pair (i, j) is split into items: kBlockSegs
+// consecutive segments of its longer loop ("curve 1") against a span of the
+// other; one CTA of kBlockSegs threads takes items from a device work queue
+// (an atomic counter) until it runs dry, so all pairs — 16-segment rings to
+// 2^18-segment loops — run in one persistent launch. The items are planned on
+// the device (plan_items), so that a call has one host wait. Each thread owns
+// one or two curve-1 segments and walks curve-2 segments, which the CTA stages
+// tile by tile in shared memory (coalesced loads, broadcast reads). Per segment pair it evaluates the
 // closed-form solid-angle term of Arai 2013 as the reference does
 // (src/compute_link.cpp:126-178, :200-280): with a = q_k - p_i,
 // b = q_k - p_{i+1}, c = q_{k+1} - p_{i+1}, d = q_{k+1} - p_i,
@@ -51,16 +52,51 @@ constexpr int kBlockSegs = 128;  // default: threads per CTA = curve-1 segments 
 constexpr int kTile = 256;       // default: curve-2 vertices per shared-memory tile
 constexpr double kInvTwoPi = 0.15915494309189533576888376337251436;
 
+// What a call's plan and its kernels tell each other and the host.
+struct PlanHead {
+  unsigned long long queue;  // work queue head
+  unsigned long long near;   // mixed: segment pairs evaluated in FP64
+  unsigned long long items;
+  unsigned long long redo;   // pairs that failed the margin check
+  double work;               // sum over pairs of n_i n_j
+  int32_t status;            // kBad* bits
+  int32_t pad;
+};
+constexpr int kBadStart = 1, kBadOrder = 2, kBadPair = 4, kBadSize = 8, kBadSame = 16;
+
 struct DirectArgs {
   const double *xyz;          // 3 doubles per vertex
   const int64_t *off;         // loop offsets
-  const int32_t *loops;       // per slot: (curve-1 loop, curve-2 loop)
-  const int64_t *item_start;  // per slot: first item; nslots + 1 entries
-  int32_t nslots;
-  int64_t items;
-  double *partial;                   // per item
-  unsigned long long *counter;       // [0] work queue head, [1] near-term count
+  const int32_t *pairs;       // (i, j) per pair
+  int64_t *start;             // per pair: its first item
+  int32_t *item_pair;         // per item: its pair; null: searched in start (npairs + 1 entries)
+  int32_t npairs;
+  int64_t cap;                // room for items
+  int64_t target;             // items a call should have at least (plan_span); 0: one span
+  PlanHead *head;
+  double *partial;            // per item
   float near_factor;
+};
+
+// Curve-2 segments per item. A call whose pairs give few items of kBlockSegs
+// segments is cut along curve 2 as well, so that it fills the chip and ends
+// evenly: `target` items (eight per resident CTA) of about the same work, down
+// to 32 segments, below which a CTA's start costs more than its terms. 12
+// walks of 4,001 steps: 5.85 ms without, SPANMS with (B200, whole call); four
+// pairs of 300 x 211 segments: PAIRUS.
+__device__ __forceinline__ int64_t plan_span(double work, int block, int64_t target) {
+  if (target == 0) return int64_t(1) << 62;
+  const double want = work / ((double)block * (double)target);
+  int64_t span = 32;
+  while ((double)span < want) span *= 2;
+  return span;
+}
+
+// The pair of an item, its longer loop first, and the item's share of it.
+struct Item {
+  int64_t o1, n1, o2, n2;  // vertex offsets and segment counts
+  int64_t first;           // first curve-1 segment
+  int64_t k0, k1;          // curve-2 segments
 };
 
 __device__ __forceinline__ int find_slot(const int64_t *start, int n, int64_t item) {
@@ -71,6 +107,34 @@ __device__ __forceinline__ int find_slot(const int64_t *start, int n, int64_t it
     else hi = mid;
   }
   return lo;
+}
+
+__device__ __forceinline__ Item item_of(const DirectArgs &A, int64_t item, int block, int64_t span) {
+  const int p = A.item_pair ? A.item_pair[item] : find_slot(A.start, A.npairs, item);
+  int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
+  Item it;
+  it.o1 = A.off[a];
+  it.n1 = A.off[a + 1] - it.o1;
+  it.o2 = A.off[b];
+  it.n2 = A.off[b + 1] - it.o2;
+  if (it.n2 > it.n1) {
+    const int64_t o = it.o1, n = it.n1;
+    it.o1 = it.o2;
+    it.n1 = it.n2;
+    it.o2 = o;
+    it.n2 = n;
+  }
+  const int64_t x = item - A.start[p], spans = (it.n2 + span - 1) / span;
+  it.first = x / spans * block;
+  it.k0 = x % spans * span;
+  it.k1 = min(it.n2, it.k0 + span);
+  return it;
+}
+
+// The items of a valid plan that fits; 0 otherwise.
+__device__ __forceinline__ int64_t plan_ready(const DirectArgs &A) {
+  const int64_t n = (int64_t)A.head->items;
+  return A.head->status == 0 && n <= A.cap ? n : 0;
 }
 
 __device__ __forceinline__ double3 load_v(const double *xyz, int64_t v) {
@@ -239,26 +303,24 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
+  const int64_t items = plan_ready(A), span = plan_span(A.head->work, kB, A.target);
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(A.counter, 1ULL);
+    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
     __syncthreads();
     const int64_t item = s_item;
-    if (item >= A.items) break;
-    const int slot = find_slot(A.item_start, A.nslots, item);
-    const int64_t blk = item - A.item_start[slot];
-    const int l1 = A.loops[2 * slot], l2 = A.loops[2 * slot + 1];
-    const int64_t o1 = A.off[l1], n1 = A.off[l1 + 1] - o1;
-    const int64_t o2 = A.off[l2], n2 = A.off[l2 + 1] - o2;
+    if (item >= items) break;
+    const Item it = item_of(A, item, kB, span);
+    const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
     // Threads: `width` segment pairs x `groups` shares of every tile.
-    const int segs = (int)min((int64_t)kB, n1 - blk * kB);
+    const int segs = (int)min((int64_t)kB, n1 - it.first);
     const int width = (segs + 1) / 2, groups = kB / width;
     const int grp = threadIdx.x / width, at = 2 * (threadIdx.x - grp * width);
     const bool active = grp < groups, second = at + 1 < segs;
     Segs2 S;
     S.p0 = S.p1 = S.p2 = make_double3(0, 0, 0);
     if (active) {
-      const int64_t i = blk * kB + at;
+      const int64_t i = it.first + at;
       S.p0 = load_v(A.xyz, o1 + i);
       S.p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
       S.p2 = second ? load_v(A.xyz, o1 + (i + 2 == n1 ? 0 : i + 2)) : S.p1;
@@ -266,8 +328,8 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
     S.e0 = make_double3(S.p1.x - S.p0.x, S.p1.y - S.p0.y, S.p1.z - S.p0.z);
     S.e1 = make_double3(S.p2.x - S.p1.x, S.p2.y - S.p1.y, S.p2.z - S.p1.z);
     AngleSum s0, s1;
-    for (int64_t k0 = 0; k0 < n2; k0 += kT) {
-      const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
+    for (int64_t k0 = it.k0; k0 < it.k1; k0 += kT) {
+      const int kt = (int)min(it.k1 - k0, (int64_t)kT);
       __syncthreads();
       for (int t = threadIdx.x; t <= kt; t += kB) {
         const int64_t kk = k0 + t;
@@ -362,18 +424,16 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
   __shared__ float s_box[kB / 32][14];
   __shared__ long long s_item;
   const float INF = __int_as_float(0x7f800000);
+  const int64_t items = plan_ready(A), span = plan_span(A.head->work, kB, A.target);
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(A.counter, 1ULL);
+    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
     __syncthreads();
     const int64_t item = s_item;
-    if (item >= A.items) break;
-    const int slot = find_slot(A.item_start, A.nslots, item);
-    const int64_t blk = item - A.item_start[slot];
-    const int l1 = A.loops[2 * slot], l2 = A.loops[2 * slot + 1];
-    const int64_t o1 = A.off[l1], n1 = A.off[l1 + 1] - o1;
-    const int64_t o2 = A.off[l2], n2 = A.off[l2 + 1] - o2;
-    const int64_t i = blk * kB + threadIdx.x;
+    if (item >= items) break;
+    const Item it = item_of(A, item, kB, span);
+    const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
+    const int64_t i = it.first + threadIdx.x;
     const bool active = i < n1;
     double3 p0 = make_double3(0, 0, 0), p1 = p0;
     if (active) {
@@ -385,9 +445,15 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
     double acc = 0.0, near_turns = 0.0;
     int turns = 0;
     unsigned near_count = 0;
-    for (int64_t k0 = 0; k0 < n2; k0 += kT) {
-      const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
-      const double3 O = load_v(A.xyz, o2 + k0);
+    // Tiles of kT vertices from the loop's start (an item may begin or end
+    // inside one): the origin of a tile's FP32 coordinates and the runs of its
+    // sums do not depend on the span.
+    for (int64_t k0 = it.k0, next; k0 < it.k1; k0 = next) {
+      const int64_t base = k0 / kT * kT;
+      next = min(it.k1, base + kT);
+      const int kt = (int)(next - k0);
+      const bool inside = k0 > base;
+      const double3 O = load_v(A.xyz, o2 + base);
       __syncthreads();
       for (int t = threadIdx.x; t <= kt; t += kB) {
         const int64_t kk = k0 + t;
@@ -434,7 +500,9 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
       float4 q = sq[0];
       float ax = q.x - r0x, ay = q.y - r0y, az = q.z - r0z;
       float bx_ = q.x - r1x, by = q.y - r1y, bz = q.z - r1z;
-      float la = sqrtf(ax * ax + ay * ay + az * az), lb = sqrtf(bx_ * bx_ + by * by + bz * bz);
+      // A walk that begins inside a tile takes the norms as its steps form them.
+      const float aa = ax * ax + ay * ay + az * az, bb = bx_ * bx_ + by * by + bz * bz;
+      float la = inside ? aa * rsqrtf(aa) : sqrtf(aa), lb = inside ? bb * rsqrtf(bb) : sqrtf(bb);
       float ab = ax * bx_ + ay * by + az * bz;
       float accf = 0.f;
 #if FLN_MIXED_ACC == 1
@@ -507,19 +575,137 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
     const double v = active ? acc * kInvTwoPi + (double)turns + near_turns : 0.0;
     const double s = block_sum<kB>(v, s_red);
     if (threadIdx.x == 0) A.partial[item] = s;
-    if (near_count) atomicAdd(A.counter + 1, (unsigned long long)near_count);
+    if (near_count) atomicAdd(&A.head->near, (unsigned long long)near_count);
   }
 }
 
-// Sums the item partials of each slot in item order and scatters the result
-// to the caller's pair index.
-__global__ void reduce_items_kernel(const double *partial, const int64_t *item_start, const int32_t *order,
-                                    int32_t nslots, double *lk_out) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslots) return;
+// Sums the item partials of each pair, a warp per pair, in a fixed order, and
+// checks the sum's margin to the rounding boundary (margin < 0: no check):
+// pairs that fail it, or are not finite, go to the list `redo`. The estimate
+// and the flags of a direct sum are 0.
+__global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, int block, double margin, double *lk,
+                                                           double *err, int32_t *flags, int32_t *redo) {
+  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (p >= A.npairs || (plan_ready(A) == 0)) return;
+  const int64_t span = plan_span(A.head->work, block, A.target);
+  const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
+  const int64_t na = A.off[a + 1] - A.off[a], nb = A.off[b + 1] - A.off[b];
+  const int64_t n = (max(na, nb) + block - 1) / block * ((min(na, nb) + span - 1) / span), s = A.start[p];
   double acc = 0.0;
-  for (int64_t it = item_start[s]; it < item_start[s + 1]; ++it) acc += partial[it];
-  lk_out[order[s]] = acc;
+  for (int64_t x = lane; x < n; x += 32) acc += A.partial[s + x];
+  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane) return;
+  lk[p] = acc;
+  if (err) err[p] = 0.0;
+  if (flags) flags[p] = 0;
+  if (margin >= 0.0 && !(0.5 - fabs(acc - round(acc)) >= margin)) redo[atomicAdd(&A.head->redo, 1ULL)] = (int32_t)p;
+}
+
+// Checks the offsets and pairs and sums n_i n_j (a whole number: exact in any
+// order below 2^53), for the thread's share of them.
+__device__ __forceinline__ void plan_check(const int64_t *off, int32_t nloops, const int32_t *pairs, int64_t npairs,
+                                           int64_t t, int64_t nt, int &status, double &work) {
+  if (t == 0 && off[0] != 0) status |= kBadStart;
+  for (int64_t l = t; l < nloops; l += nt)
+    if (off[l + 1] < off[l]) status |= kBadOrder;
+  for (int64_t p = t; p < npairs; p += nt) {
+    const int a = pairs[2 * p], b = pairs[2 * p + 1];
+    if (a < 0 || a >= nloops || b < 0 || b >= nloops) {
+      status |= kBadPair;
+      continue;
+    }
+    const int64_t na = off[a + 1] - off[a], nb = off[b + 1] - off[b];
+    if (na < 2 || nb < 2) status |= kBadSize;
+    if (a == b) status |= kBadSame;
+    work += (double)na * (double)nb;
+  }
+}
+
+// Items of the pairs [p0 + 32 w, ...) of a warp: reserved with one atomic,
+// pairs in order, and written to the item list.
+__device__ __forceinline__ void plan_warp(const DirectArgs &A, int block, int64_t p, int64_t span, int lane) {
+  int64_t n = 0;
+  if (p < A.npairs) {
+    const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
+    const int64_t na = A.off[a + 1] - A.off[a], nb = A.off[b + 1] - A.off[b];
+    n = (max(na, nb) + block - 1) / block * ((min(na, nb) + span - 1) / span);
+  }
+  int64_t incl = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int64_t at = 0;
+  if (lane == 31) at = (int64_t)atomicAdd(&A.head->items, (unsigned long long)incl);
+  at = __shfl_sync(0xffffffffu, at, 31);
+  const int64_t total = __shfl_sync(0xffffffffu, incl, 31), mine = at + incl - n;
+  if (p < A.npairs) A.start[p] = mine;
+  if (at + total > A.cap) return;  // the host makes room and plans again
+  for (int j = 0; j < 32; ++j) {
+    const int64_t s = __shfl_sync(0xffffffffu, mine, j), c = __shfl_sync(0xffffffffu, n, j);
+    for (int64_t x = lane; x < c; x += 32) A.item_pair[s + x] = (int32_t)(p - lane + j);
+  }
+}
+
+__global__ void __launch_bounds__(256) plan_work(DirectArgs A, int32_t nloops) {
+  int status = 0;
+  double work = 0.0;
+  plan_check(A.off, nloops, A.pairs, A.npairs, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+             (int64_t)gridDim.x * blockDim.x, status, work);
+  status = __reduce_or_sync(0xffffffffu, status);
+  for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
+  if ((threadIdx.x & 31) == 0) {
+    if (status) atomicOr(&A.head->status, status);
+    if (work > 0) atomicAdd(&A.head->work, work);
+  }
+}
+
+__global__ void __launch_bounds__(256) plan_items(DirectArgs A, int block) {
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (A.head->status || p - (threadIdx.x & 31) >= A.npairs) return;
+  plan_warp(A, block, p, plan_span(A.head->work, block, A.target), threadIdx.x & 31);
+}
+
+// Both in one CTA, for calls of few pairs; it also clears the head.
+constexpr int64_t kPlanSmall = 2048;
+__global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops, int block) {
+  __shared__ int s_status;
+  __shared__ double s_work[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_status = 0;
+  __syncthreads();
+  int status = 0;
+  double work = 0.0;
+  plan_check(A.off, nloops, A.pairs, A.npairs, threadIdx.x, 1024, status, work);
+  status = __reduce_or_sync(0xffffffffu, status);
+  for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
+  if (lane == 0) {
+    s_work[w] = work;
+    if (status) atomicOr(&s_status, status);
+  }
+  __syncthreads();
+  work = 0.0;
+  for (int x = 0; x < 32; ++x) work += s_work[x];
+  if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, work, s_status, 0};
+  __syncthreads();
+  if (s_status) return;
+  const int64_t span = plan_span(work, block, A.target);
+  for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, block, p, span, lane);
+}
+
+// The pairs of the redo list, and back: sums and flags of recomputed pairs.
+__global__ void gather_pairs(const int32_t *list, int64_t n, const int32_t *pairs, int32_t *out) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  out[2 * k] = pairs[2 * (int64_t)list[k]];
+  out[2 * k + 1] = pairs[2 * (int64_t)list[k] + 1];
+}
+__global__ void scatter_redo(const int32_t *list, int64_t n, const double *src, double *lk, int32_t *flags) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  lk[list[k]] = src[k];
+  if (flags) flags[list[k]] |= FLN_PAIR_FP64_RECOMPUTED;
 }
 
 // The tile shapes the direct sum can run with (fln_params.direct_tile), the
@@ -533,83 +719,99 @@ constexpr TileShape kShapes[kDirectTileShapes] = {{128, 256}, {128, 128}, {128, 
 static_assert(kShapes[0].block == kBlockSegs && kShapes[0].tile == kTile, "the default shape comes first");
 
 template <int kB, int kT>
-void launch_direct_t(cudaStream_t st, int sms, int precision, const DirectArgs &A) {
-  if (precision == FLN_PREC_FP64) {
-    const int per_sm = occupancy_of((const void *)direct_fp64_kernel<kB, kT>, kB);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(A.items, (int64_t)sms * per_sm));
-    direct_fp64_kernel<kB, kT><<<grid, kB, 0, st>>>(A);
-  } else {
-    const int per_sm = occupancy_of((const void *)direct_mixed_kernel<kB, kT>, kB);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(A.items, (int64_t)sms * per_sm));
-    direct_mixed_kernel<kB, kT><<<grid, kB, 0, st>>>(A);
-  }
+void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
+  auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
+  const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, kB);
+  kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), kB, 0, st>>>(A);
 }
 
-void launch_direct(int shape, cudaStream_t st, int sms, int precision, const DirectArgs &A) {
+void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
   switch (shape) {
-    case 1: launch_direct_t<128, 128>(st, sms, precision, A); break;
-    case 2: launch_direct_t<128, 512>(st, sms, precision, A); break;
-    case 3: launch_direct_t<256, 256>(st, sms, precision, A); break;
-    case 4: launch_direct_t<256, 512>(st, sms, precision, A); break;
-    case 5: launch_direct_t<64, 256>(st, sms, precision, A); break;
-    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, A); break;
+    case 1: launch_direct_t<128, 128>(st, sms, precision, most, A); break;
+    case 2: launch_direct_t<128, 512>(st, sms, precision, most, A); break;
+    case 3: launch_direct_t<256, 256>(st, sms, precision, most, A); break;
+    case 4: launch_direct_t<256, 512>(st, sms, precision, most, A); break;
+    case 5: launch_direct_t<64, 256>(st, sms, precision, most, A); break;
+    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, A); break;
   }
 }
 
 }  // namespace
 
-int direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                      const std::vector<int32_t> &h_pairs, int precision, double near_factor, double *d_lk_out,
-                      double *near_terms_out, int tile_shape) {
+DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
+                               const int32_t *d_pairs, int64_t np, int precision, double near_factor, double margin,
+                               double *d_lk, double *d_err, int32_t *d_flags, int tile_shape) {
   if (tile_shape < 0 || tile_shape >= kDirectTileShapes)
     throw Error(FLN_ERR_INVALID_ARGUMENT, "direct_tile in [0, " + std::to_string(kDirectTileShapes - 1) + "]");
+  DirectResult R;
+  if (np == 0) return R;
+  if (np > INT32_MAX) throw Error(FLN_ERR_INVALID_ARGUMENT, "more than 2^31 - 1 pairs");
   const int kB = kShapes[tile_shape].block;
-  const int64_t np = (int64_t)h_pairs.size() / 2;
-  if (np == 0) return 0;
-  // Plan: orient each pair so its longer loop is curve 1, and order slots by
-  // decreasing work so the queue hands out the largest pairs first.
-  std::vector<int32_t> order(np);
-  std::iota(order.begin(), order.end(), 0);
-  auto nseg = [&](int l) { return h_off[l + 1] - h_off[l]; };
-  std::vector<double> cost(np);
-  for (int64_t p = 0; p < np; ++p) cost[p] = (double)nseg(h_pairs[2 * p]) * (double)nseg(h_pairs[2 * p + 1]);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-  std::vector<int32_t> loops(2 * np);
-  std::vector<int64_t> start(np + 1);
-  start[0] = 0;
-  for (int64_t s = 0; s < np; ++s) {
-    int a = h_pairs[2 * order[s]], b = h_pairs[2 * order[s] + 1];
-    if (nseg(b) > nseg(a)) std::swap(a, b);
-    loops[2 * s] = a;
-    loops[2 * s + 1] = b;
-    start[s + 1] = start[s] + (nseg(a) + kB - 1) / kB;
+  cudaStream_t st = ctx.stream;
+  PlanHead *d_head = ctx.d_counter.as<PlanHead>(1);
+  int64_t *d_start = ctx.d_items.as<int64_t>(np);
+  int32_t *d_redo = margin >= 0 ? ctx.d_near.as<int32_t>(np) : nullptr;
+  PlanHead &head = *static_cast<PlanHead *>(ctx.h_head.need(sizeof(PlanHead)));
+  const int64_t target = (int64_t)ctx.num_sms * 8 * (512 / kB);
+  // Room for the items: of the largest call so far, or a guess; a plan that
+  // does not fit runs no kernel and is made again with room.
+  ctx.direct_items = std::max<int64_t>(ctx.direct_items, std::max<int64_t>(4 * target, 2 * np));
+  for (int attempt = 0;; ++attempt) {
+    const int64_t cap = ctx.direct_items;
+    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, d_head,
+                 ctx.d_partial.as<double>(cap), (float)near_factor};
+    if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
+      plan_small<<<1, 1024, 0, st>>>(A, nloops, kB);
+    } else {
+      FLN_CUDA(cudaMemsetAsync(d_head, 0, sizeof(PlanHead), st));
+      const int64_t most = std::max<int64_t>(np, nloops);
+      plan_work<<<(int)std::min<int64_t>((most + 255) / 256, 8 * ctx.num_sms), 256, 0, st>>>(A, nloops);
+      plan_items<<<(int)((np + 255) / 256), 256, 0, st>>>(A, kB);
+      ++R.launches;
+    }
+    FLN_CUDA(cudaGetLastError());
+    FLN_CUDA(cudaEventRecord(ctx.ev2, st));
+    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, A);
+    FLN_CUDA(cudaGetLastError());
+    FLN_CUDA(cudaEventRecord(ctx.ev3, st));
+    reduce_items_kernel<<<(int)((np + 7) / 8), 256, 0, st>>>(A, kB, margin, d_lk, d_err, d_flags, d_redo);
+    FLN_CUDA(cudaGetLastError());
+    R.launches += 3;
+    FLN_CUDA(cudaMemcpyAsync(&head, d_head, sizeof head, cudaMemcpyDeviceToHost, st));
+    FLN_CUDA(cudaStreamSynchronize(st));
+    if (head.status) {
+      throw Error(FLN_ERR_INVALID_ARGUMENT,
+                  head.status & kBadStart ? "loop_offsets must start at 0 and hold nloops + 1 entries."
+                  : head.status & kBadOrder ? "loop_offsets must be non-decreasing."
+                  : head.status & kBadPair ? "pair index out of range."
+                  : head.status & kBadSize ? "every loop in a pair needs at least two vertices."
+                                           : "a pair must name two different loops.");
+    }
+    if ((int64_t)head.items <= cap) break;
+    if (attempt > 0) throw Error(FLN_ERR_INTERNAL, "direct sum: the plan does not fit its own count");
+    ctx.direct_items = (int64_t)head.items;
   }
-  const int64_t items = start[np];
-  int32_t *d_loops = ctx.d_loops.as<int32_t>(2 * np + np);
-  int32_t *d_order = d_loops + 2 * np;
-  int64_t *d_start = ctx.d_items.as<int64_t>(np + 1);
-  double *d_partial = ctx.d_partial.as<double>(items);
-  unsigned long long *d_counter = ctx.d_counter.as<unsigned long long>(2);
-  FLN_CUDA(cudaMemcpyAsync(d_loops, loops.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
-  FLN_CUDA(cudaMemcpyAsync(d_order, order.data(), np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
-  FLN_CUDA(cudaMemcpyAsync(d_start, start.data(), (np + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx.stream));
-  FLN_CUDA(cudaMemsetAsync(d_counter, 0, 2 * sizeof(unsigned long long), ctx.stream));
-  DirectArgs A{d_xyz, d_off, d_loops, d_start, (int32_t)np, items, d_partial, d_counter, (float)near_factor};
-  FLN_CUDA(cudaEventRecord(ctx.ev2, ctx.stream));
-  launch_direct(tile_shape, ctx.stream, ctx.num_sms, precision, A);
-  FLN_CUDA(cudaGetLastError());
-  FLN_CUDA(cudaEventRecord(ctx.ev3, ctx.stream));
-  reduce_items_kernel<<<(int)((np + 255) / 256), 256, 0, ctx.stream>>>(d_partial, d_start, d_order, (int32_t)np,
-                                                                      d_lk_out);
-  FLN_CUDA(cudaGetLastError());
-  if (near_terms_out) {
-    unsigned long long h = 0;
-    FLN_CUDA(cudaMemcpyAsync(&h, d_counter + 1, sizeof h, cudaMemcpyDeviceToHost, ctx.stream));
-    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
-    *near_terms_out = (double)h;
+  float ms = 0;
+  FLN_CUDA(cudaEventElapsedTime(&ms, ctx.ev2, ctx.ev3));
+  ctx.stats.ms_main_kernel += ms;
+  R.near_terms = (double)head.near;
+  R.work = head.work;
+  R.redone = (int64_t)head.redo;
+  if (R.redone > 0) {
+    const int64_t nr = R.redone;
+    int32_t *list = ctx.d_redo.as<int32_t>(3 * nr + (nr & 1) + 2 * nr);  // list, pairs, sums
+    FLN_CUDA(cudaMemcpyAsync(list, d_redo, nr * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+    int32_t *pairs = list + nr;
+    double *sums = reinterpret_cast<double *>(list + 3 * nr + (nr & 1));
+    const int grid = (int)((nr + 255) / 256);
+    gather_pairs<<<grid, 256, 0, st>>>(list, nr, d_pairs, pairs);
+    FLN_CUDA(cudaGetLastError());
+    R.launches += 2 + direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, nr, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr,
+                                        nullptr, 0).launches;
+    scatter_redo<<<grid, 256, 0, st>>>(list, nr, sums, d_lk, d_flags);
+    FLN_CUDA(cudaGetLastError());
   }
-  ctx.stats.ms_main_kernel += ctx.elapsed(ctx.ev2, ctx.ev3);
-  return 2;
+  return R;
 }
 
 }  // namespace fln
@@ -624,7 +826,7 @@ int direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
 // paths where an allocation failure cannot be handled. For them the direct
 // sum runs entirely in the caller's input and output buffers plus one
 // file-scope device array, g_noalloc_scratch, of kNoAllocScratchBytes
-// (about 9.3 MB). Every GPU that loads libfln.so holds that array until the
+// (about 8.9 MB). Every GPU that loads libfln.so holds that array until the
 // process exits. Limits: at most kNoAllocMaxPairs loop pairs per call and
 // kNoAllocMaxItems work items (one item = 128 segments of the longer loop of
 // a pair, summed over the pairs); larger calls are rejected with
@@ -649,29 +851,22 @@ namespace {
 
 constexpr int64_t kNoAllocMaxPairs = 65536;
 constexpr int64_t kNoAllocMaxItems = int64_t(1) << 20;
-constexpr size_t kNaHeader = 256;  // counters[2], total items, status
-constexpr size_t kNaLoops = kNaHeader;                                       // int32 x 2 per pair
-constexpr size_t kNaOrder = kNaLoops + 2 * kNoAllocMaxPairs * 4;             // int32 per pair
-constexpr size_t kNaStart = kNaOrder + kNoAllocMaxPairs * 4;                 // int64 per pair + 1
+constexpr size_t kNaHeader = 256;  // PlanHead
+constexpr size_t kNaStart = kNaHeader;                                       // int64 per pair + 1
 constexpr size_t kNaPartial = (kNaStart + (kNoAllocMaxPairs + 1) * 8 + 255) / 256 * 256;  // double per item
 constexpr size_t kNoAllocScratchBytes = kNaPartial + kNoAllocMaxItems * 8;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
-struct NaHeader {
-  unsigned long long counter[2];  // work queue head, near-singular term count
-  long long total_items;
-  int status;                     // bit 0: bad pair index, bit 1: loop with < 2 vertices
-};
+static_assert(sizeof(PlanHead) <= kNaHeader, "the header's room");
+// status of the plan: bit 0: bad pair index, bit 1: loop with < 2 vertices
 
-// One CTA plans the call inside the scratch array: orients each pair (longer
-// loop first), counts its items, scans them into item_start and clears the
-// counters the direct-sum kernels start from.
+// One CTA plans the call inside the scratch array: counts each pair's items
+// (kBlockSegs segments of its longer loop against the whole other one), scans
+// them into start and clears the counters the direct-sum kernels start from.
 __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t nloops, const int32_t *pairs,
                                                      int64_t npairs, unsigned char *scratch) {
-  NaHeader *h = reinterpret_cast<NaHeader *>(scratch);
-  int32_t *loops = reinterpret_cast<int32_t *>(scratch + kNaLoops);
-  int32_t *order = reinterpret_cast<int32_t *>(scratch + kNaOrder);
+  PlanHead *h = reinterpret_cast<PlanHead *>(scratch);
   int64_t *start = reinterpret_cast<int64_t *>(scratch + kNaStart);
   __shared__ long long s_warp[32];
   __shared__ long long s_carry;
@@ -686,28 +881,17 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
     const int64_t p = base + threadIdx.x;
     long long items = 0;
     if (p < npairs) {
-      int a = pairs[2 * p], b = pairs[2 * p + 1];
+      const int a = pairs[2 * p], b = pairs[2 * p + 1];
       if (a < 0 || a >= nloops || b < 0 || b >= nloops || a == b) {
         atomicOr(&s_status, 1);
       } else {
-        int64_t na = off[a + 1] - off[a], nb = off[b + 1] - off[b];
+        const int64_t na = off[a + 1] - off[a], nb = off[b + 1] - off[b];
         if (na < 2 || nb < 2) {
           atomicOr(&s_status, 2);
         } else {
-          if (nb > na) {
-            const int t = a;
-            a = b;
-            b = t;
-            const int64_t tn = na;
-            na = nb;
-            nb = tn;
-          }
-          items = (na + kBlockSegs - 1) / kBlockSegs;
+          items = (max(na, nb) + kBlockSegs - 1) / kBlockSegs;
         }
       }
-      loops[2 * p] = a;
-      loops[2 * p + 1] = b;
-      order[p] = (int32_t)p;
     }
     // Exclusive block scan of `items`.
     long long incl = items;
@@ -734,10 +918,7 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
   }
   if (threadIdx.x == 0) {
     start[npairs] = s_carry;
-    h->counter[0] = 0;
-    h->counter[1] = 0;
-    h->total_items = s_carry;
-    h->status = s_status;
+    *h = PlanHead{0, 0, (unsigned long long)s_carry, 0, 0.0, s_status, 0};
   }
 }
 
@@ -795,37 +976,26 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   if (!scratch) return fail(st, msg);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   noalloc_plan<<<1, 1024, 0, s>>>(d_loop_offsets, nloops, d_pairs, npairs, scratch);
-  NaHeader h;
+  PlanHead h;
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h, scratch, sizeof h, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(FLN_ERR_CUDA, std::string("fln_linking_numbers_direct_noalloc: ") + cudaGetErrorString(e));
   if (h.status & 1) return fail(FLN_ERR_INVALID_ARGUMENT, "fln_linking_numbers_direct_noalloc: pair index out of range or a pair names one loop twice");
   if (h.status & 2) return fail(FLN_ERR_INVALID_ARGUMENT, "fln_linking_numbers_direct_noalloc: every loop in a pair needs at least two vertices");
-  if (h.total_items > kNoAllocMaxItems)
-    return fail(FLN_ERR_INVALID_ARGUMENT, "fln_linking_numbers_direct_noalloc: " + std::to_string(h.total_items) +
+  if ((int64_t)h.items > kNoAllocMaxItems)
+    return fail(FLN_ERR_INVALID_ARGUMENT, "fln_linking_numbers_direct_noalloc: " + std::to_string((int64_t)h.items) +
                                               " work items exceed the limit of " + std::to_string(kNoAllocMaxItems) +
                                               " (one item = 128 segments of the longer loop of a pair)");
-  int dev = 0, sms = 0, per_sm = 0;
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The default tile shape (the planning kernel cuts items of kBlockSegs).
-  DirectArgs A{d_xyz, d_loop_offsets, reinterpret_cast<const int32_t *>(scratch + kNaLoops),
-               reinterpret_cast<const int64_t *>(scratch + kNaStart), (int32_t)npairs, h.total_items,
-               reinterpret_cast<double *>(scratch + kNaPartial), reinterpret_cast<unsigned long long *>(scratch),
-               (float)kDefaultNearFactor};
-  if (precision == FLN_PREC_FP64) {
-    per_sm = occupancy_of((const void *)direct_fp64_kernel<kBlockSegs, kTile>, kBlockSegs);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h.total_items, (int64_t)sms * std::max(per_sm, 1)));
-    direct_fp64_kernel<kBlockSegs, kTile><<<grid, kBlockSegs, 0, s>>>(A);
-  } else {
-    per_sm = occupancy_of((const void *)direct_mixed_kernel<kBlockSegs, kTile>, kBlockSegs);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h.total_items, (int64_t)sms * std::max(per_sm, 1)));
-    direct_mixed_kernel<kBlockSegs, kTile><<<grid, kBlockSegs, 0, s>>>(A);
-  }
-  reduce_items_kernel<<<(int)((npairs + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<const double *>(scratch + kNaPartial), reinterpret_cast<const int64_t *>(scratch + kNaStart),
-      reinterpret_cast<const int32_t *>(scratch + kNaOrder), (int32_t)npairs, d_lk_out);
+  const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
+                     (int32_t)npairs, (int64_t)h.items, 0, reinterpret_cast<PlanHead *>(scratch),
+                     reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
+  launch_direct(0, s, sms, precision, (int64_t)h.items, A);
+  reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, kBlockSegs, -1.0, d_lk_out, nullptr, nullptr, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FLN_ERR_CUDA, std::string("fln_linking_numbers_direct_noalloc: ") + cudaGetErrorString(e));
   return FLN_OK;

@@ -68,16 +68,6 @@ struct HostBuf {
   }
 };
 
-// Direct-sum schedule: the pair list oriented and ordered for the kernel,
-// and the work items (pair, block of kBlockSegs curve-1 segments).
-struct DirectPlan {
-  std::vector<int32_t> order;       // kernel slot -> caller pair index
-  std::vector<int32_t> loops;       // 2 per slot: (curve-1 loop, curve-2 loop)
-  std::vector<int64_t> item_start;  // slot -> first item; size nslots + 1
-  int64_t items = 0;
-  double segment_pairs = 0;
-};
-
 // Learned opening criterion of the Barnes–Hut traversal (learned.cuh has the
 // weight layout; frag == nullptr: off).
 struct MlpFrag;
@@ -107,7 +97,7 @@ struct Context {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
   fln_stats stats{};
   // Device buffers.
-  DevBuf d_xyz, d_off, d_pairs, d_loops, d_items, d_partial, d_counter, d_lk, d_err, d_flags, d_near;
+  DevBuf d_xyz, d_off, d_pairs, d_loops, d_items, d_partial, d_counter, d_lk, d_err, d_flags, d_near, d_redo;
   DevBuf d_bh[28];
   int64_t bh_front_hint = 0;  // frontier records of the largest Barnes–Hut first pass so far
   // CTAs per SM of the traversal kernels (per occupancy set), of the learned
@@ -116,6 +106,8 @@ struct Context {
   int bh_per_sm_learned = 0, bh_per_sm_classify = 0;
   bool bh_build_smem = false;  // the tree build's shared memory size is set
   HostBuf h_in, h_out;  // pinned staging of copy_h2d / copy_d2h
+  HostBuf h_call, h_head;  // pinned: a small call's inputs and results; the head of a direct sum's plan
+  int64_t direct_items = 0;  // room for a direct sum's items (the largest call so far)
   cudaEvent_t ev_stage[2] = {nullptr, nullptr};
   // The exact-list launches of the fused Barnes–Hut rounds run on their own
   // stream, beside the next round's traversal; ev_round holds an event pair
@@ -185,15 +177,24 @@ constexpr double kDefaultNearFactor = 4.0;
 // list, 128 ran the traversal in 48.0 ms against 49.6 ms at 256.
 constexpr int kDefaultBhBudget = 128;
 
-// Plans and runs the direct sum over `npairs` pairs of the loops in device
-// memory. d_xyz/d_off describe the loops; h_off is the host copy of the
-// offsets; h_pairs the host copy of the pairs. Writes lk (per caller pair) to
-// d_lk_out. Returns the number of kernel launches.
-// tile_shape: index into the direct sum's tile shapes (fln_params.direct_tile).
+// Plans (on the device) and runs the direct sum over `npairs` pairs of the
+// loops in device memory; everything but the returned counts stays there.
+// Checks the offsets and pairs; throws FLN_ERR_INVALID_ARGUMENT before any sum
+// is written when they are bad. margin >= 0: pairs whose distance to the
+// rounding boundary is below it, or which are not finite, are recomputed in
+// FP64 (FLN_PAIR_FP64_RECOMPUTED). d_err and d_flags may be null; they get 0
+// otherwise. tile_shape: index into the direct sum's tile shapes
+// (fln_params.direct_tile).
+struct DirectResult {
+  int launches = 0;
+  double near_terms = 0;  // mixed: segment pairs evaluated in FP64
+  double work = 0;        // sum over pairs of n_i n_j
+  int64_t redone = 0;     // pairs recomputed in FP64
+};
 constexpr int kDirectTileShapes = 6;
-int direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                      const std::vector<int32_t> &h_pairs, int precision, double near_factor, double *d_lk_out,
-                      double *near_terms_out, int tile_shape = 0);
+DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
+                               const int32_t *d_pairs, int64_t npairs, int precision, double near_factor,
+                               double margin, double *d_lk, double *d_err, int32_t *d_flags, int tile_shape = 0);
 
 // Barnes–Hut over the same inputs; err per pair after ERROR_EST_SCALE and the
 // reference's beta retry; flags gets FLN_PAIR_BETA_RETRIED. Returns launches.
