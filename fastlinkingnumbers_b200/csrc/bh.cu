@@ -394,11 +394,11 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
 // segment); a CTA builds one such block and everything below it:
 //  - the block's vertices go to shared memory once (coalesced);
 //  - leaves: a thread each, straight from the two vertices;
-//  - groups (the block's nodes of the first depth with at most 4 segments):
-//    a thread sums a group's leaf moments about the group's centre, other
-//    threads do the two-segment nodes inside the groups. (A leaf has C_D = 0
-//    and C_Q,k = c_k c c^T / 12, so the shift of compute_link.cpp:367-381 adds
-//    c r^T and c_k r r^T with r = leaf midpoint - node centre.);
+//  - nodes of at most 16 segments: a thread sums the leaf moments of its
+//    segments about the node's centre. (A leaf has C_D = 0 and C_Q,k =
+//    c_k c c^T / 12, so the shift of compute_link.cpp:367-381 adds c r^T and
+//    c_k r r^T with r = leaf midpoint - node centre.) The largest of them, the
+//    groups, also keep their FP64 record in shared memory;
 //  - the levels above, up to the block's root: four lanes per node. Row k of
 //    C_D, C_Q,k and axis k of the box depend on the children's row k and the
 //    centres only, so lane k forms them from the children's FP64 records in
@@ -409,22 +409,24 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
 // depend on who arrives last. FP64 throughout; records are rounded to FP32 at
 // the end.
 //
-// What bounds it: 384 B of records are written per segment; measured 4.7 ms for
-// 28M segments of mixed sizes (2.3 TB/s of records) and 2.75 ms for 14.1M,
+// What bounds it: 384 B of records are written per segment; measured 4.0 ms for
+// 28M segments of mixed sizes (2.7 TB/s of records) and 2.4 ms for 14.1M,
 // against 8.6 and 4.66 ms for the build it replaces (topology, leaf,
 // height-bucket, small-node and one launch per height), which read each vertex
-// about 30 times through scattered 8-byte loads and wrote 16-byte pieces. The
+// about 30 times through scattered 8-byte loads and wrote 16-byte pieces. It
+// sums in that build's order, so the records are the same bit for bit. The
 // last levels of a block and the way up keep only one warp busy, so a block is
-// as large as four resident CTAs' shared memory allows: with 512 leaves 4.7 ms,
-// 256 leaves 5.9, 128 leaves 7.3 (same case); three CTAs of 168 registers
-// instead of four of 128: 5.3 ms; leaving the last levels to one warp while the
-// others write the leaves: 6.5 against 5.9 ms (at 256 leaves).
+// as large as four resident CTAs' shared memory allows: 1,024 leaves 4.0 ms,
+// 512 leaves 4.8, 256 leaves 5.9 (same case); five CTAs of 96 registers 5.6
+// instead of 4.8 (at 512); leaving the last levels to one warp while the
+// others write the leaves 6.5 instead of 5.9 (at 256, an earlier form).
 constexpr int kBuildThreads = 128;
-constexpr int kBlockLeaves = 512;
-constexpr int kGroups = kBlockLeaves / 4;  // most groups of a block
+constexpr int kBlockLeaves = 1024;
+constexpr int kGroupLeaves = 16, kGroupDepth = 4;  // levels of a group with internal nodes
+constexpr int kGroups = kBlockLeaves / kGroupLeaves;  // most groups of a block
 constexpr int kRecD = 39;            // doubles of a record in shared memory (odd: no bank conflicts):
 // Dynamic shared memory: 32 floats of staging per quad, the vertices, the
-// groups' records (56 KB: four CTAs per SM).
+// groups' records (47 KB: four CTAs per SM).
 constexpr int kBuildSmem = (kBuildThreads / 4 * 16 + 3 * (kBlockLeaves + 1) + kGroups * kRecD) * 8;
 constexpr int kRLo = 0, kRHi = 3, kRMid = 6, kRT = 9, kRD = 12, kRQ = 21;
 
@@ -478,15 +480,20 @@ __device__ __forceinline__ void combine_quad(const double *L, const double *R, d
     for (int e = 0; e < 6; ++e)
       Q[e] += C[kRQ + 6 * k + e] + r[jj[e]] * cd[ii[e]] + r[ii[e]] * cd[jj[e]] + ct * (r[ii[e]] * r[jj[e]]);
   }
-  double tt = t * t, dd = D[0] * D[0] + D[1] * D[1] + D[2] * D[2], qq = 0.0;
+  // The norms' squares, summed in the order of finish_record_regs.
+  const double t0 = __shfl_sync(mask, t, qb), t1 = __shfl_sync(mask, t, qb + 1), t2 = __shfl_sync(mask, t, qb + 2);
+  const double tt = t0 * t0 + t1 * t1 + t2 * t2;
+  double dd = 0.0, qq = 0.0;
 #pragma unroll
-  for (int e = 0; e < 6; ++e) qq += (e < 3 ? 1.0 : 2.0) * Q[e] * Q[e];
-  auto sum3 = [&](double x) {
-    return (__shfl_sync(mask, x, qb) + __shfl_sync(mask, x, qb + 1)) + __shfl_sync(mask, x, qb + 2);
-  };
-  tt = sum3(tt);
-  dd = sum3(dd);
-  qq = sum3(qq);
+  for (int a = 0; a < 3; ++a) {
+    double x = dd, y = qq;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) x += D[b] * D[b];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) y += (e < 3 ? 1.0 : 2.0) * Q[e] * Q[e];
+    dd = __shfl_sync(mask, x, qb + a);
+    qq = __shfl_sync(mask, y, qb + a);
+  }
   __syncwarp(mask);  // every lane has read the children's records
   if (!write) return;
   if (q < 3) {
@@ -534,10 +541,13 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
   float (*s_stage)[32] = reinterpret_cast<float (*)[32]>(s_dyn);
   double *s_v = s_dyn + kBuildThreads / 4 * 16;
   double *s_rec = s_v + 3 * (kBlockLeaves + 1);
-  __shared__ int s_k;
+  __shared__ int s_k, s_chunk;
   const int tid = threadIdx.x;
   const int64_t blk = b0 + blockIdx.x;
-  if (tid == 0) s_k = find_loop_of(A.blk_start, A.nloops, blk);
+  if (tid == 0) {
+    s_k = find_loop_of(A.blk_start, A.nloops, blk);
+    s_chunk = 0;
+  }
   __syncthreads();
   const int k = s_k, l = A.loops[k];
   const int64_t o = A.off[l], n = A.off[l + 1] - o, first = A.blk_start[k];
@@ -555,27 +565,46 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
   }
   __syncthreads();
   int levels = 0;  // levels between the block's root and its groups
-  while (((m + (1 << levels) - 1) >> levels) > 4) ++levels;
+  while (((m + (1 << levels) - 1) >> levels) > kGroupLeaves) ++levels;
   const int groups = 1 << levels;
-  // Groups (the first half of the threads) and the two-segment nodes inside
-  // them (the second half).
+  // The groups and the nodes inside them, the largest first: level d of a
+  // group has up to 2^d nodes. (Just above the groups, nodes of 16 segments
+  // can lie beside nodes of 17; those of 16 are summed here too, as level -1.)
+  // A warp takes 32 nodes of one level at a time.
+  const bool over = levels > 0 && (m >> (levels - 1)) == kGroupLeaves;
+  auto parent_is_summed = [&](int g) {
+    const NodeAt v = descend(root, g >> 1, levels - 1);
+    return v.hi - v.lo == kGroupLeaves;
+  };
   {
-    constexpr int kHalf = kBuildThreads / 2;
-    const bool inner = tid >= kHalf;
-    for (int g = tid & (kHalf - 1); g < groups; g += kHalf) {
-      const NodeAt grp = descend(root, g, levels);
-      const int size = grp.hi - grp.lo;
-      const int nodes = inner ? max(size - 2, 0) : 1;
-      for (int i = 0; i < nodes; ++i) {
-        // Size 3: [lo] [lo+1, lo+3); size 4: [lo, lo+2) [lo+2, lo+4).
-        const NodeAt v = inner ? descend(grp, size == 3 ? 1 : i, 1) : grp;
+    const int lane = tid & 31;
+    for (;;) {
+      int chunk = 0;
+      if (lane == 0) chunk = atomicAdd(&s_chunk, 1);
+      chunk = __shfl_sync(0xffffffffu, chunk, 0);
+      int d = over ? -1 : 0;
+      auto nodes_at = [&](int level) { return level < 0 ? groups >> 1 : groups << level; };
+      for (; d < kGroupDepth; ++d) {  // the level of this chunk
+        const int c = (nodes_at(d) + 31) / 32;
+        if (chunk < c) break;
+        chunk -= c;
+      }
+      if (d == kGroupDepth) break;
+      const int x = 32 * chunk + lane;
+      NodeAt v{0, 0, 0, 0};
+      if (x < nodes_at(d)) {
+        v = descend(root, d < 0 ? x : x >> d, d < 0 ? levels - 1 : levels);
+        for (int b = d - 1; b >= 0 && v.hi - v.lo > 1; --b) v = descend(v, (x >> b) & 1, 1);
+        if (d < 0 && v.hi - v.lo > kGroupLeaves) v.hi = v.lo;
+      }
+      if (v.hi - v.lo > 1) {
         BuildNode P;
         const double *V = s_v + 3 * (v.lo - root.lo);
         const int cnt = v.hi - v.lo;
         for (int a = 0; a < 3; ++a) P.lo[a] = P.hi[a] = V[a];
-        for (int x = 1; x <= cnt; ++x)
+        for (int u = 1; u <= cnt; ++u)
           for (int a = 0; a < 3; ++a) {
-            const double y = V[3 * x + a];
+            const double y = V[3 * u + a];
             P.lo[a] = fmin(P.lo[a], y);
             P.hi[a] = fmax(P.hi[a], y);
           }
@@ -586,10 +615,10 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
         for (int a = 0; a < 9; ++a) P.D[a] = 0.0;
         for (int a = 0; a < 18; ++a) P.Q[a] = 0.0;
         const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
-        for (int x = 0; x < cnt; ++x) {
+        for (int u = 0; u < cnt; ++u) {
           double t[3], r[3];
           for (int a = 0; a < 3; ++a) {
-            const double p0 = V[3 * x + a], p1 = V[3 * x + 3 + a];
+            const double p0 = V[3 * u + a], p1 = V[3 * u + 3 + a];
             t[a] = p1 - p0;
             r[a] = (0.5 * p0 + 0.5 * p1) - P.mid[a];
           }
@@ -603,8 +632,8 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
         P.seg_lo = v.lo;
         P.seg_cnt = cnt;
         finish_record(P, hdr[v.pos], mom[v.pos], false, 0, child_place(v.lo, v.lefts));
-        if (!inner) {
-          double *rec = s_rec + g * kRecD;
+        if (d < 0 || (d == 0 && !(over && parent_is_summed(x)))) {
+          double *rec = s_rec + (d < 0 ? 2 * x : x) * kRecD;
           for (int a = 0; a < 3; ++a) {
             rec[kRLo + a] = P.lo[a];
             rec[kRHi + a] = P.hi[a];
@@ -658,6 +687,7 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
     const int step = 1 << (levels - e);
     for (int i = quad; i < (1 << e); i += kBuildThreads / 4) {
       const NodeAt v = descend(root, i, e);
+      if (v.hi - v.lo <= kGroupLeaves) continue;
       double *L = s_rec + i * step * kRecD;
       combine_quad(L, L + (step / 2) * kRecD, L, v, hdr + v.pos, mom + v.pos, s_stage[quad], q, true);
     }
@@ -1890,7 +1920,13 @@ FLN_TRAVERSE_KERNELS(7)
 // 2,000 steps 2.05 ms at 128 and 1.46 at 16; mixed sizes (28M segments) 25.8 ms
 // at 128, 23.8 at 16, 23.4 at 32; 200 walks of 50,000 steps 121.9 ms at 128,
 // 124.6 at 32 and 135 at 16. By this rule: 1.45, 23.2 and 120.4 ms.
-int round_budget(int budget, int64_t work, int64_t warps) {
+// Calls of fewer than kShortRounds segments keep the full budget: they end
+// after a round or two either way, and the sums of unlinked loops, which are
+// nothing but errors of 1e-3 and less, show in their ninth digit how the
+// partial sums were grouped when each is rounded to 2^-40.
+constexpr int64_t kShortRounds = int64_t(1) << 17;
+int round_budget(int budget, int64_t segments, int64_t work, int64_t warps) {
+  if (segments < kShortRounds) return budget;
   return std::min(budget, work <= warps ? 16 : work <= 4 * warps ? 32 : budget);
 }
 
@@ -3016,7 +3052,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         }
         const int gmax = (A.learned.frag && !A.rec) ? grid_l : (front ? grid_f : grid);
         const int64_t work = nin + (nstream - pos);
-        A.budget = round_budget(budget, work, (int64_t)gmax * kWarps);
+        A.budget = round_budget(budget, tot_leaf, work, (int64_t)gmax * kWarps);
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>((work + kWarps - 1) / kWarps, gmax));
         FLN_CUDA(cudaEventRecord(event_at(4 * nev + 3), st));
         if (A.rec)

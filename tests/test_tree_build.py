@@ -1,15 +1,17 @@
 """Curve-order tree build at the edges of its blocks and groups: loops of a
-few segments, around the 512-segment block, and of several blocks, against the
-oracle's FP64 restatement of the same trees and traversal."""
+few segments, around the 16-segment groups and the 1,024-segment block, and of
+several blocks, against the oracle's FP64 restatement of the same trees and
+traversal."""
 import numpy as np
 import pytest
 
 from fastlinkingnumbers_b200 import Engine
 from oracle import pyoracle
 
-# 2..9: one group and its shapes; 31..33: levels of a small block; 511..513:
-# one block or two; 1023..1025 and 2049: four blocks; 5,000 and 20,011: many.
-SIZES = [2, 3, 4, 5, 6, 7, 8, 9, 31, 32, 33, 255, 257, 511, 512, 513, 1023, 1024, 1025, 2049, 5000, 20011]
+# 2..17: one group and its shapes, or two; 33, 65, 130: nodes of 16 segments
+# beside nodes of 17; 1023..1025: one block or two; the rest: several.
+SIZES = [2, 3, 4, 5, 6, 7, 8, 9, 15, 16, 17, 31, 32, 33, 34, 65, 130, 257, 511, 513, 1023, 1024, 1025, 2047, 2049, 5000,
+         20011]
 
 
 @pytest.mark.gpu
