@@ -72,7 +72,8 @@ struct DirectArgs {
   int32_t *item_pair;         // per item: its pair; null: searched in start (npairs + 1 entries)
   int32_t npairs;
   int64_t cap;                // room for items
-  int64_t target;             // items a call should have at least (plan_span); 0: one span
+  int64_t target;             // items a call should have at least (plan_span)
+  double least;               // calls of less work (PlanHead::work) take the whole of curve 2 per item
   PlanHead *head;
   double *partial;            // per item
   float near_factor;
@@ -81,12 +82,14 @@ struct DirectArgs {
 // Curve-2 segments per item. A call whose pairs give few items of kBlockSegs
 // segments is cut along curve 2 as well, so that it fills the chip and ends
 // evenly: `target` items (eight per resident CTA) of about the same work, down
-// to 32 segments, below which a CTA's start costs more than its terms. 12
-// walks of 4,001 steps: 5.85 ms without, SPANMS with (B200, whole call); four
-// pairs of 300 x 211 segments: PAIRUS.
-__device__ __forceinline__ int64_t plan_span(double work, int block, int64_t target) {
-  if (target == 0) return int64_t(1) << 62;
-  const double want = work / ((double)block * (double)target);
+// to 32 segments, below which a CTA's start costs more than its terms. The
+// mixed precision does so only from kMixedSpans segment pairs: cutting a walk
+// regroups its FP64 sum, and below that the sums stay bit for bit those of one
+// walk per segment (all there is to see when no loops are linked).
+constexpr double kMixedSpans = 1 << 30;
+__device__ __forceinline__ int64_t plan_span(const DirectArgs &A, double work, int block) {
+  if (work < A.least) return int64_t(1) << 62;
+  const double want = work / ((double)block * (double)A.target);
   int64_t span = 32;
   while ((double)span < want) span *= 2;
   return span;
@@ -171,6 +174,12 @@ __device__ __noinline__ double term_fp64(double3 p0, double3 p1, double3 q0, dou
   double r = atan2(yp, xp) * kInvTwoPi;
   if (yp * det < 0) r += (det > 0) ? 1.0 : -1.0;
   return r;
+}
+
+// The term of segment q.x of curve 1 and q.y of curve 2.
+__device__ __forceinline__ double near_term(const double *xyz, int64_t o1, int64_t n1, int64_t o2, int64_t n2, int2 q) {
+  return term_fp64(load_v(xyz, o1 + q.x), load_v(xyz, o1 + (q.x + 1 == n1 ? 0 : q.x + 1)), load_v(xyz, o2 + q.y),
+                   load_v(xyz, o2 + (q.y + 1 == n2 ? 0 : q.y + 1)));
 }
 
 // Rescales (x, y) by the power of two that brings max(|x|, |y|) into [1, 2),
@@ -303,7 +312,7 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
-  const int64_t items = plan_ready(A), span = plan_span(A.head->work, kB, A.target);
+  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work, kB);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
@@ -374,21 +383,154 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   }
 }
 
+// A lone pair: one curve-1 segment per thread, library square roots, each
+// segment's whole walk in one thread. The sum of one unlinked pair is nothing
+// but the rounding of its terms, so the per-pair functions (fln_direct_pair)
+// keep this order and these operations, bit for bit.
+__global__ void __launch_bounds__(kBlockSegs) direct_fp64_lone_kernel(DirectArgs A) {
+  constexpr int kB = kBlockSegs, kT = kTile;
+  __shared__ double sx[kT + 1], sy[kT + 1], sz[kT + 1];
+  __shared__ double s_red[kB / 32];
+  __shared__ long long s_item;
+  const int64_t items = plan_ready(A);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
+    __syncthreads();
+    const int64_t item = s_item;
+    if (item >= items) break;
+    const Item it = item_of(A, item, kB, int64_t(1) << 62);
+    const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
+    const int64_t i = it.first + threadIdx.x;
+    const bool active = i < n1;
+    double3 p0 = make_double3(0, 0, 0), p1 = p0;
+    if (active) {
+      p0 = load_v(A.xyz, o1 + i);
+      p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
+    }
+    double xs = 1.0, ys = 0.0, S = -1.0, turns = 0.0;
+    for (int64_t k0 = 0; k0 < n2; k0 += kT) {
+      const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
+      __syncthreads();
+      for (int t = threadIdx.x; t <= kt; t += kB) {
+        const int64_t kk = k0 + t;
+        const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
+        sx[t] = v.x;
+        sy[t] = v.y;
+        sz[t] = v.z;
+      }
+      __syncthreads();
+      if (!active) continue;
+      double ax = sx[0] - p0.x, ay = sy[0] - p0.y, az = sz[0] - p0.z;
+      double bx = sx[0] - p1.x, by = sy[0] - p1.y, bz = sz[0] - p1.z;
+      double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz);
+      double ab = ax * bx + ay * by + az * bz;
+      for (int k = 0; k < kt; ++k) {
+        const double qx = sx[k + 1], qy = sy[k + 1], qz = sz[k + 1];
+        const double cx = qx - p1.x, cy = qy - p1.y, cz = qz - p1.z;
+        const double dx = qx - p0.x, dy = qy - p0.y, dz = qz - p0.z;
+        const double lc = sqrt(cx * cx + cy * cy + cz * cz), ld = sqrt(dx * dx + dy * dy + dz * dz);
+        const double ca = cx * ax + cy * ay + cz * az;
+        const double cb = cx * bx + cy * by + cz * bz;
+        const double ad = ax * dx + ay * dy + az * dz;
+        const double cd = cx * dx + cy * dy + cz * dz;
+        const double det = ax * (by * cz - bz * cy) + az * (bx * cy - by * cx) + ay * (bz * cx - bx * cz);
+        const double t = la * lc;
+        const double div1 = t * lb + ab * lc + ca * lb + cb * la;
+        const double div2 = t * ld + ad * lc + ca * ld + cd * la;
+        const double xp = div1 * div2 - det * det;
+        const double yp = det * (div1 + div2);
+        // Arctangent addition: (xs + i ys) *= (xp + i yp), tracking crossings
+        // of the negative real axis (compute_link.cpp:245-269).
+        double ny = xs * yp + xp * ys;
+        double nx = xs * xp - ys * yp;
+        renorm(nx, ny);
+        if (yp * det < 0) turns += (det > 0) ? 1.0 : -1.0;
+        const double s3 = (ny > 0.0 || (ny == 0.0 && nx < 0.0)) ? 1.0 : -1.0;
+        if (s3 * S < 0 && yp * S >= 0) turns += S;
+        xs = nx;
+        ys = ny;
+        S = s3;
+        ax = dx; ay = dy; az = dz;
+        bx = cx; by = cy; bz = cz;
+        la = ld; lb = lc; ab = cd;
+      }
+    }
+    const double v = active ? atan2(ys, xs) * kInvTwoPi + turns : 0.0;
+    const double s = block_sum<kB>(v, s_red);
+    if (threadIdx.x == 0) A.partial[item] = s;
+  }
+}
+
 // ------------------------------------------------------------------ mixed
+// Two FP32 values in a 64-bit register pair: one instruction does two adds,
+// multiplies or fused multiply-adds (add/mul/fma.rn.f32x2), each rounded as
+// the scalar one. They take the FMA pipe as long as two scalar instructions,
+// but one issue slot.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float lo2(F2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(F2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ F2 neg2(F2 v) { return v ^ 0x8000000080000000ull; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// 1 / sqrt(x) and y / x by the hardware's approximations, as rsqrtf and
+// __fdividef but for subnormal x (treated as 0): a subnormal squared distance
+// is far below any segment length, so its pair is a near one, and a
+// subnormal x of a term (64 |q - p|^6, coordinates of 1e-7 and less) has lost
+// the term's digits already.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float div_normal(float y, float x) {
+  float r;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(y), "f"(x));
+  return r;
+}
+struct F2x3 {
+  F2 x, y, z;
+};
+__device__ __forceinline__ F2 dot2(const F2x3 &a, const F2x3 &b) {
+  return fma2(a.z, b.z, fma2(a.x, b.x, mul2(a.y, b.y)));
+}
+__device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, float by, float bz) {
+  return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
+}
+
 // arctan(t) for |t| <= 1/4 from its Maclaurin series t - t^3/3 + t^5/5 - t^7/7
 // + t^9/9; the first omitted term is below 2.2e-8 |t|, under FP32 rounding.
-__device__ __forceinline__ float atan_small(float t) {
-  const float u = t * t;
-  float p = fmaf(u, 1.0f / 9.0f, -1.0f / 7.0f);
-  p = fmaf(p, u, 1.0f / 5.0f);
-  p = fmaf(p, u, -1.0f / 3.0f);
-  p = fmaf(p, u, 1.0f);
-  return p * t;
+__device__ __forceinline__ F2 atan_small2(F2 t) {
+  auto c = [](float v) { return pack2(v, v); };
+  const F2 u = mul2(t, t);
+  F2 p = fma2(u, c(1.0f / 9.0f), c(-1.0f / 7.0f));
+  p = fma2(p, u, c(1.0f / 5.0f));
+  p = fma2(p, u, c(-1.0f / 3.0f));
+  p = fma2(p, u, c(1.0f));
+  return mul2(p, t);
 }
 
 // Minimum and maximum over the CTA of 7 values each (a box and a length);
 // the result is in out[0..6] (min) and out[7..13] (max) for every thread.
-template <int kB>
+template <int kThreads>
 __device__ __forceinline__ void block_minmax7(float *lo, float *hi, float (*s_box)[14], float *out) {
   for (int o = 16; o; o >>= 1)
     for (int v = 0; v < 7; ++v) {
@@ -404,27 +546,141 @@ __device__ __forceinline__ void block_minmax7(float *lo, float *hi, float (*s_bo
   __syncthreads();
   for (int v = 0; v < 14; ++v) {
     float r = s_box[0][v];
-    for (int w = 1; w < kB / 32; ++w) r = v < 7 ? fminf(r, s_box[w][v]) : fmaxf(r, s_box[w][v]);
+    for (int w = 1; w < kThreads / 32; ++w) r = v < 7 ? fminf(r, s_box[w][v]) : fmaxf(r, s_box[w][v]);
     out[v] = r;
   }
 }
 
-// Accumulation of a thread's terms over a tile: 0 = FP32 over the tile
-// (up to kT terms), 1 = FP32 with Kahan compensation, 2 = FP64 per term,
-// 3 = FP32 runs of 32 terms folded into FP64 (the rounding error of a run is
-// bounded by 32 terms instead of kT, for one FP64 add per 32 terms).
-#ifndef FLN_MIXED_ACC
-#define FLN_MIXED_ACC 3
-#endif
+// A tile vertex: q relative to the tile's origin and the segment f to the next
+// vertex, every value twice (the two halves of a packed operand), and
+// near_factor x the segment's length.
+struct __align__(16) MixVertex {
+  float4 qxy, qzw, fxy, fz;
+};
 
+// The packed state of the walks of two neighbouring segments (p0 p1) and
+// (p1 p2): low halves the first segment's, high halves the second's.
+struct MixWalk {
+  F2x3 a, b;  // q - p_j, q - p_{j+1}
+  F2 la, lb;  // their norms
+  F2 ab;      // a . b
+  float m0, m1;  // min(la, lb) of each
+};
+struct MixSegs {
+  F2x3 ra, rb;  // p_j, p_{j+1} relative to the tile's origin
+  F2x3 e, ne;   // e = p_{j+1} - p_j and -e
+  float near0, near1;  // near_factor x their lengths
+};
+
+// Vectors and norms of the walk at vertex v. The products of the shared
+// vertex p1 are formed once (the second segment's a is the first one's b).
+__device__ __forceinline__ void mix_at(const MixSegs &S, const MixVertex &v, MixWalk &w, F2 &aa, float &cc) {
+  const F2 qx = pack2(v.qxy.x, v.qxy.y), qy = pack2(v.qxy.z, v.qxy.w), qz = pack2(v.qzw.x, v.qzw.y);
+  w.a = F2x3{add2(qx, S.ra.x), add2(qy, S.ra.y), add2(qz, S.ra.z)};  // ra, rb hold -p
+  w.b = F2x3{add2(qx, S.rb.x), add2(qy, S.rb.y), add2(qz, S.rb.z)};
+  aa = dot2(w.a, w.a);
+  const float x = hi2(w.b.x), y = hi2(w.b.y), z = hi2(w.b.z);
+  cc = dot_f(x, y, z, x, y, z);
+  w.ab = dot2(w.b, w.a);
+}
+
+// Terms of one step that are not both on the fast path: near pairs get 0 and
+// their bit, the others the full arctangent with the branch turn.
+__device__ __forceinline__ void mix_slow(F2 xp, F2 yp, F2 sdiv, F2 det, bool near0, bool near1, bool fast0, bool fast1,
+                                         unsigned bit, float &t0, float &t1, unsigned &mask0, unsigned &mask1,
+                                         int &turns0, int &turns1) {
+  if (near0) {
+    t0 = 0.f;
+    mask0 |= bit;
+  } else if (!fast0) {
+    t0 = atan2f(lo2(yp), lo2(xp));
+    if (lo2(sdiv) < 0.f && lo2(det) != 0.f) turns0 += lo2(det) > 0.f ? 1 : -1;
+  }
+  if (near1) {
+    t1 = 0.f;
+    mask1 |= bit;
+  } else if (!fast1) {
+    t1 = atan2f(hi2(yp), hi2(xp));
+    if (hi2(sdiv) < 0.f && hi2(det) != 0.f) turns1 += hi2(det) > 0.f ? 1 : -1;
+  }
+}
+
+// One step q_k -> q_{k+1} (step j of its run): the walk goes from a to w; the
+// two terms are added to sum0 and sum1. A near pair adds 0 and sets bit j of its mask.
+__device__ __forceinline__ void mix_step(const MixSegs &S, const MixWalk &a, MixWalk &w, const MixVertex &at,
+                                         const MixVertex &to, bool far_tile, int j, float &sum0, float &sum1, unsigned &mask0,
+                                         unsigned &mask1, int &turns0, int &turns1) {
+  F2 dd;
+  float cc;
+  mix_at(S, to, w, dd, cc);
+  w.la = mul2(dd, pack2(rsqrt_normal(lo2(dd)), rsqrt_normal(hi2(dd))));
+  w.lb = pack2(hi2(w.la), cc * rsqrt_normal(cc));
+  w.m0 = fminf(lo2(w.la), hi2(w.la));
+  w.m1 = fminf(lo2(w.lb), hi2(w.lb));
+  const F2 fx = pack2(at.fxy.x, at.fxy.y), fy = pack2(at.fxy.z, at.fxy.w), fz = pack2(at.fz.x, at.fz.y);
+  const F2 ca = dot2(w.b, a.a), cb = dot2(w.b, a.b);
+  const F2 ad = dot2(a.a, w.a);
+  const F2 cx = fma2(fy, S.e.z, mul2(fz, S.ne.y)), cy = fma2(fz, S.e.x, mul2(fx, S.ne.z)),
+           cz = fma2(fx, S.e.y, mul2(fy, S.ne.x));
+  const F2 det = fma2(a.a.z, cz, fma2(a.a.x, cx, mul2(a.a.y, cy)));
+  const F2 t = mul2(a.la, w.lb);
+  const F2 div1 = fma2(cb, a.la, fma2(ca, a.lb, fma2(a.ab, w.lb, mul2(t, a.lb))));
+  const F2 div2 = fma2(w.ab, a.la, fma2(ca, w.la, fma2(ad, w.lb, mul2(t, w.la))));
+  const F2 sdiv = add2(div1, div2);
+  const F2 xp = fma2(div1, div2, mul2(det, neg2(det)));
+  const F2 yp = mul2(det, sdiv);
+  const F2 quarter = mul2(xp, pack2(0.25f, 0.25f));
+  const bool fast0 = lo2(sdiv) > 0.f && fabsf(lo2(yp)) < lo2(quarter);
+  const bool fast1 = hi2(sdiv) > 0.f && fabsf(hi2(yp)) < hi2(quarter);
+  // (fz.z: near_factor x the length of this curve-2 segment)
+  const bool near0 = !far_tile && fminf(a.m0, w.m0) < fmaxf(S.near0, at.fz.z);
+  const bool near1 = !far_tile && fminf(a.m1, w.m1) < fmaxf(S.near1, at.fz.z);
+  // The principal branch, |angle| < 0.245.
+  const F2 small = atan_small2(pack2(div_normal(lo2(yp), lo2(xp)), div_normal(hi2(yp), hi2(xp))));
+  float t0 = lo2(small), t1 = hi2(small);
+  if (__builtin_expect(!(fast0 && fast1) || near0 || near1, 0))
+    mix_slow(xp, yp, sdiv, det, near0, near1, fast0, fast1, 1u << j, t0, t1, mask0, mask1, turns0, turns1);
+  sum0 += t0;
+  sum1 += t1;
+}
+
+// The mixed direct sum: kB curve-1 segments per item, two neighbouring ones
+// per thread (kB / 2 threads), their FP32 arithmetic packed. A segment pair's
+// term, the runs of 32 steps in which terms are summed in FP32 and the order of
+// the FP64 sums are those of one thread per segment: the mixed sum of unlinked
+// loops is the rounding of its terms, and it stays what it was bit for bit. So
+// an item takes the whole of curve 2 (but for large calls, kMixedSpans), and
+// only loops of at most kB / 2 segments make several groups of threads, a run
+// of 32 steps each.
+// Near pairs are noted in a bit mask per run, queued per warp, evaluated 32 at
+// a time in FP64 and added to their segment's sum in order.
+//
+// Bound: issue and the FMA pipe together. A step of 64 segment pairs needs 50
+// packed and 8 scalar FMA-pipe operations (108 cycles of a scheduler's pipe, 709
+// G segment pairs/s) and issues about 120 instructions; the pipe is 60 % and
+// the issue slots 59 % busy. 16 walks of 5,003 steps (4.99e9 segment pairs),
+// B200, whole call: 22.6 ms with one scalar segment per thread and near pairs
+// as a divergent call; 16.7 packed with the near queue; 14.7 with the near and
+// slow terms in one branch, subnormals flushed in the reciprocal and root, and
+// cuts along curve 2. 10,000 linked rings: 1.49 -> 0.87 ms of kernel. Sixteen
+// warps of 128 registers per SM: 12 of 162 take 14.9 ms, 20 of 96 16.0.
 template <int kB, int kT>
-__global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
-  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = length of segment t
+__global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectArgs A) {
+  constexpr int kThreads = kB / 2;
+  __shared__ MixVertex tile[kT + 1];
+  __shared__ int2 s_near[kThreads / 32][64];  // (curve-1 segment of the item x 32 + lane, curve-2 segment) left to FP64
+  __shared__ double s_term[kThreads / 32][32];
   __shared__ double s_red[kB / 32];
-  __shared__ float s_box[kB / 32][14];
+  __shared__ double s_seg[kB];  // per segment of the item
+  __shared__ float s_box[kThreads / 32][14];
   __shared__ long long s_item;
   const float INF = __int_as_float(0x7f800000);
-  const int64_t items = plan_ready(A), span = plan_span(A.head->work, kB, A.target);
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1;
+  int2 *queue = s_near[threadIdx.x >> 5];
+  double *term = s_term[threadIdx.x >> 5];
+  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work, kB);
+  unsigned long long near_count = 0;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
@@ -433,61 +689,104 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
     if (item >= items) break;
     const Item it = item_of(A, item, kB, span);
     const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
-    const int64_t i = it.first + threadIdx.x;
-    const bool active = i < n1;
-    double3 p0 = make_double3(0, 0, 0), p1 = p0;
-    if (active) {
-      p0 = load_v(A.xyz, o1 + i);
-      p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
+    const int segs = (int)min((int64_t)kB, n1 - it.first);
+    // Groups: of at most as many as there are runs (more only for short loops).
+    const int width = (segs + 1) / 2, groups = n1 > kB / 2 ? 1 : (int)min((int64_t)(kThreads / width), (n2 + 31) / 32);
+    const int grp = threadIdx.x / width, at = 2 * (threadIdx.x - grp * width);
+    const bool active = grp < groups, second = active && at + 1 < segs;
+    const int64_t i0 = it.first + (active ? at : 0);
+    const int64_t i1 = i0 + 1 == n1 ? 0 : i0 + 1, i2 = second ? (i1 + 1 == n1 ? 0 : i1 + 1) : i1;
+    MixSegs S;
+    float len0, len1;
+    {
+      const double3 p0 = load_v(A.xyz, o1 + i0), p1 = load_v(A.xyz, o1 + i1), p2 = load_v(A.xyz, o1 + i2);
+      const float x0 = (float)(p1.x - p0.x), y0 = (float)(p1.y - p0.y), z0 = (float)(p1.z - p0.z);
+      const float x1 = (float)(p2.x - p1.x), y1 = (float)(p2.y - p1.y), z1 = (float)(p2.z - p1.z);
+      S.e = F2x3{pack2(x0, x1), pack2(y0, y1), pack2(z0, z1)};
+      S.ne = F2x3{neg2(S.e.x), neg2(S.e.y), neg2(S.e.z)};
+      len0 = sqrtf(dot_f(x0, y0, z0, x0, y0, z0));
+      len1 = sqrtf(dot_f(x1, y1, z1, x1, y1, z1));
+      S.near0 = A.near_factor * len0;
+      S.near1 = A.near_factor * len1;
     }
-    const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
-    const float len1 = sqrtf(ex * ex + ey * ey + ez * ez);
-    double acc = 0.0, near_turns = 0.0;
-    int turns = 0;
-    unsigned near_count = 0;
-    // Tiles of kT vertices from the loop's start (an item may begin or end
-    // inside one): the origin of a tile's FP32 coordinates and the runs of its
-    // sums do not depend on the span.
-    for (int64_t k0 = it.k0, next; k0 < it.k1; k0 = next) {
-      const int64_t base = k0 / kT * kT;
-      next = min(it.k1, base + kT);
-      const int kt = (int)(next - k0);
-      const bool inside = k0 > base;
-      const double3 O = load_v(A.xyz, o2 + base);
+    double acc0 = 0.0, acc1 = 0.0, near0 = 0.0, near1 = 0.0;
+    int turns0 = 0, turns1 = 0, queued = 0;
+    // Evaluates the oldest n queued pairs (n <= 32); every lane adds those of
+    // its segments, oldest first.
+    auto flush = [&](int n) {
+      int2 q = make_int2(0, 0);
+      if (lane < n) {
+        q = queue[lane];
+        int64_t seg = it.first + (q.x >> 5);
+        if (seg >= n1) seg -= n1;
+        term[lane] = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)seg, q.y));
+      }
+      __syncwarp();
+      for (int x = 0; x < n; ++x) {
+        const int who = queue[x].x;
+        const double v = term[x];
+        if ((who & 31) == lane) {
+          if (who >> 5 == at) near0 += v;
+          else near1 += v;
+        }
+      }
+      __syncwarp();
+      q = queue[32 + lane];
+      __syncwarp();
+      queue[lane] = q;
+      __syncwarp();
+    };
+    for (int64_t k0 = it.k0; k0 < it.k1; k0 += kT) {  // a span is a multiple of kT (kMixedSpans)
+      const int kt = (int)min(it.k1 - k0, (int64_t)kT);
+      const double3 O = load_v(A.xyz, o2 + k0);
       __syncthreads();
-      for (int t = threadIdx.x; t <= kt; t += kB) {
+      for (int t = threadIdx.x; t <= kt; t += kThreads) {
         const int64_t kk = k0 + t;
         const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
-        sq[t] = make_float4((float)(v.x - O.x), (float)(v.y - O.y), (float)(v.z - O.z), 0.f);
+        const float x = (float)(v.x - O.x), y = (float)(v.y - O.y), z = (float)(v.z - O.z);
+        tile[t].qxy = make_float4(x, x, y, y);
+        tile[t].qzw.x = z;
+        tile[t].qzw.y = z;
       }
       __syncthreads();
-      const float r0x = (float)(p0.x - O.x), r0y = (float)(p0.y - O.y), r0z = (float)(p0.z - O.z);
-      const float r1x = (float)(p1.x - O.x), r1y = (float)(p1.y - O.y), r1z = (float)(p1.z - O.z);
-      // Boxes of this thread's curve-1 segment (slots 0-2, length 3) and of
-      // its curve-2 tile vertices (slots 4-6, length 3 of the max).
+      // Boxes of this thread's curve-1 segments (slots 0-2) and of its
+      // curve-2 tile vertices (slots 4-6), the longest segment (slot 3).
       float lo[7], hi[7];
       for (int v = 0; v < 7; ++v) {
         lo[v] = INF;
         hi[v] = -INF;
       }
-      if (active) {
-        lo[0] = fminf(r0x, r1x); hi[0] = fmaxf(r0x, r1x);
-        lo[1] = fminf(r0y, r1y); hi[1] = fmaxf(r0y, r1y);
-        lo[2] = fminf(r0z, r1z); hi[2] = fmaxf(r0z, r1z);
-        hi[3] = len1;
+      {
+        const double3 p[3] = {load_v(A.xyz, o1 + i0), load_v(A.xyz, o1 + i1), load_v(A.xyz, o1 + i2)};
+        float x[3], y[3], z[3];
+        for (int v = 0; v < 3; ++v) {
+          x[v] = (float)(p[v].x - O.x);
+          y[v] = (float)(p[v].y - O.y);
+          z[v] = (float)(p[v].z - O.z);
+        }
+        S.ra = F2x3{pack2(-x[0], -x[1]), pack2(-y[0], -y[1]), pack2(-z[0], -z[1])};
+        S.rb = F2x3{pack2(-x[1], -x[2]), pack2(-y[1], -y[2]), pack2(-z[1], -z[2])};
+        if (active) {
+          lo[0] = fminf(x[0], fminf(x[1], x[2])); hi[0] = fmaxf(x[0], fmaxf(x[1], x[2]));
+          lo[1] = fminf(y[0], fminf(y[1], y[2])); hi[1] = fmaxf(y[0], fmaxf(y[1], y[2]));
+          lo[2] = fminf(z[0], fminf(z[1], z[2])); hi[2] = fmaxf(z[0], fmaxf(z[1], z[2]));
+          hi[3] = fmaxf(len0, len1);
+        }
       }
-      for (int t = threadIdx.x; t < kt; t += kB) {
-        const float4 a = sq[t], b = sq[t + 1];
-        const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
-        const float len = sqrtf(fx * fx + fy * fy + fz * fz);
-        sq[t].w = len;
-        lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
-        lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
-        lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
+      for (int t = threadIdx.x; t < kt; t += kThreads) {
+        const float4 axy = tile[t].qxy, bxy = tile[t + 1].qxy;
+        const float az = tile[t].qzw.x, bz = tile[t + 1].qzw.x;
+        const float fx = bxy.x - axy.x, fy = bxy.z - axy.z, fz = bz - az;
+        const float len = sqrtf(dot_f(fx, fy, fz, fx, fy, fz));
+        tile[t].fxy = make_float4(fx, fx, fy, fy);
+        tile[t].fz = make_float4(fz, fz, A.near_factor * len, 0.f);
+        lo[4] = fminf(lo[4], fminf(axy.x, bxy.x)); hi[4] = fmaxf(hi[4], fmaxf(axy.x, bxy.x));
+        lo[5] = fminf(lo[5], fminf(axy.z, bxy.z)); hi[5] = fmaxf(hi[5], fmaxf(axy.z, bxy.z));
+        lo[6] = fminf(lo[6], fminf(az, bz)); hi[6] = fmaxf(hi[6], fmaxf(az, bz));
         hi[3] = fmaxf(hi[3], len);
       }
       float bx[14];
-      block_minmax7<kB>(lo, hi, s_box, bx);
+      block_minmax7<kThreads>(lo, hi, s_box, bx);
       __syncthreads();
       // Box gap between the CTA's curve-1 segments and this tile: no segment
       // pair can be near-singular when it exceeds near_factor x (longest segment).
@@ -496,90 +795,90 @@ __global__ void __launch_bounds__(kB) direct_mixed_kernel(DirectArgs A) {
       const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
       const float lim = A.near_factor * bx[10];
       const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
-      if (!active) continue;
-      float4 q = sq[0];
-      float ax = q.x - r0x, ay = q.y - r0y, az = q.z - r0z;
-      float bx_ = q.x - r1x, by = q.y - r1y, bz = q.z - r1z;
-      // A walk that begins inside a tile takes the norms as its steps form them.
-      const float aa = ax * ax + ay * ay + az * az, bb = bx_ * bx_ + by * by + bz * bz;
-      float la = inside ? aa * rsqrtf(aa) : sqrtf(aa), lb = inside ? bb * rsqrtf(bb) : sqrtf(bb);
-      float ab = ax * bx_ + ay * by + az * bz;
-      float accf = 0.f;
-#if FLN_MIXED_ACC == 1
-      float comp = 0.f;  // Kahan compensation of accf
-#elif FLN_MIXED_ACC == 2
-      double accd = 0.0;
-#endif
-      for (int k = 0; k < kt; ++k) {
-        const float4 qn = sq[k + 1];
-        const float cx = qn.x - r1x, cy = qn.y - r1y, cz = qn.z - r1z;
-        const float dx = qn.x - r0x, dy = qn.y - r0y, dz = qn.z - r0z;
-        const float cc = cx * cx + cy * cy + cz * cz, dd = dx * dx + dy * dy + dz * dz;
-        const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
-        const float cd = cx * dx + cy * dy + cz * dz;
-        bool near = false;
-        if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
-        if (near) {
-          const int64_t kk = k0 + k, kn = kk + 1;
-          near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
-          ++near_count;
-        } else {
-          const float ca = cx * ax + cy * ay + cz * az;
-          const float cb = cx * bx_ + cy * by + cz * bz;
-          const float ad = ax * dx + ay * dy + az * dz;
-          const float fx = qn.x - q.x, fy = qn.y - q.y, fz = qn.z - q.z;
-          const float det = ax * (fy * ez - fz * ey) + ay * (fz * ex - fx * ez) + az * (fx * ey - fy * ex);
-          const float t = la * lc;
-          const float div1 = t * lb + ab * lc + ca * lb + cb * la;
-          const float div2 = t * ld + ad * lc + ca * ld + cd * la;
-          const float sdiv = div1 + div2;
-          const float xp = div1 * div2 - det * det;
-          const float yp = det * sdiv;
-          float term;
-          if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
-            term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
-          } else {
-            term = atan2f(yp, xp);
-            if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;
+      // The runs of 32 steps of this thread's group.
+      const int runs = (kt + 31) / 32, ra = runs * grp / groups, rb = runs * (grp + 1) / groups;
+      const int rounds = (runs + groups - 1) / groups;  // no group has more
+      MixWalk wa, wb;
+      for (int r = 0; r < rounds; ++r) {
+        unsigned near_mask0 = 0, near_mask1 = 0;
+        const int run = ra + r, j0 = 32 * run, steps = active && run < rb ? min(32, kt - j0) : 0;
+        if (steps > 0) {
+          if (r == 0) {
+            F2 aa;
+            float cc;
+            mix_at(S, tile[j0], wa, aa, cc);
+            // Norms at the start of a tile by the square root, inside one as
+            // the steps form them.
+            const bool inside = j0 > 0;
+            const float a0 = lo2(aa), a1 = hi2(aa);
+            const float l0 = inside ? a0 * rsqrt_normal(a0) : sqrtf(a0), l1 = inside ? a1 * rsqrt_normal(a1) : sqrtf(a1);
+            const float l2 = inside ? cc * rsqrt_normal(cc) : sqrtf(cc);
+            wa.la = pack2(l0, l1);
+            wa.lb = pack2(l1, l2);
+            wa.m0 = fminf(l0, l1);
+            wa.m1 = fminf(l1, l2);
           }
-#if FLN_MIXED_ACC == 1
-          const float y_ = term - comp;
-          const float t_ = accf + y_;
-          comp = (t_ - accf) - y_;
-          accf = t_;
-#elif FLN_MIXED_ACC == 2
-          accd += (double)term;
-#else
-          accf += term;
-#endif
+          float sum0 = 0.f, sum1 = 0.f;
+          int j = 0;
+          const MixVertex *at_j = tile + j0;
+          for (; j + 2 <= steps; j += 2, at_j += 2) {
+            mix_step(S, wa, wb, at_j[0], at_j[1], far_tile, j, sum0, sum1, near_mask0, near_mask1, turns0, turns1);
+            mix_step(S, wb, wa, at_j[1], at_j[2], far_tile, j + 1, sum0, sum1, near_mask0, near_mask1, turns0, turns1);
+          }
+          if (j < steps)
+            mix_step(S, wa, wb, at_j[0], at_j[1], far_tile, j, sum0, sum1, near_mask0, near_mask1, turns0, turns1);
+          acc0 += (double)sum0;
+          acc1 += (double)sum1;
+          if (!second) near_mask1 = 0;
         }
-#if FLN_MIXED_ACC == 3
-        if ((k & 31) == 31) {
-          acc += (double)accf;
-          accf = 0.f;
+        // Queue this run's near pairs, one per lane at a time; evaluate 32 at a time.
+        while (__any_sync(0xffffffffu, (near_mask0 | near_mask1) != 0)) {
+          const bool has = (near_mask0 | near_mask1) != 0;
+          const unsigned m = __ballot_sync(0xffffffffu, has);
+          if (has) {
+            const bool first = near_mask0 != 0;
+            const int k = __ffs(first ? near_mask0 : near_mask1) - 1;
+            if (first) near_mask0 &= near_mask0 - 1;
+            else near_mask1 &= near_mask1 - 1;
+            queue[queued + __popc(m & below)] = make_int2((first ? at : at + 1) << 5 | lane, (int)(k0 + j0 + k));
+          }
+          queued += __popc(m);
+          near_count += lane == 0 ? __popc(m) : 0;
+          __syncwarp();
+          if (queued >= 32) {
+            flush(32);
+            queued -= 32;
+          }
         }
-#endif
-        q = qn;
-        ax = dx; ay = dy; az = dz;
-        bx_ = cx; by = cy; bz = cz;
-        la = ld; lb = lc; ab = cd;
       }
-#if FLN_MIXED_ACC == 1
-      acc += (double)accf - (double)comp;
-#elif FLN_MIXED_ACC == 2
-      acc += accd;
-#else
-      acc += (double)accf;
-#endif
     }
-    const double v = active ? acc * kInvTwoPi + (double)turns + near_turns : 0.0;
-    const double s = block_sum<kB>(v, s_red);
-    if (threadIdx.x == 0) A.partial[item] = s;
-    if (near_count) atomicAdd(&A.head->near, (unsigned long long)near_count);
+    if (queued > 0) flush(queued);
+    // The item's sum: 32 segments at a time by a butterfly, those sums in order.
+    for (int g = 0; g < groups; ++g) {
+      if (grp == g) {
+        const double v0 = acc0 * kInvTwoPi + (double)turns0 + near0;
+        const double v1 = second ? acc1 * kInvTwoPi + (double)turns1 + near1 : 0.0;
+        s_seg[at] = g ? s_seg[at] + v0 : v0;
+        s_seg[at + 1] = g ? s_seg[at + 1] + v1 : v1;
+      }
+      __syncthreads();
+    }
+    double r = 0.0;
+    for (int g = threadIdx.x >> 5; g < kB / 32; g += kThreads / 32) {
+      double v = 32 * g + lane < segs ? s_seg[32 * g + lane] : 0.0;
+      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) s_red[g] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int g = 0; g < kB / 32; ++g) r += s_red[g];
+      A.partial[item] = r;
+    }
   }
+  if (near_count) atomicAdd(&A.head->near, near_count);
 }
 
-// Sums the item partials of each pair, a warp per pair, in a fixed order, and
+// Sums the item partials of each pair, a warp per pair, in item order, and
 // checks the sum's margin to the rounding boundary (margin < 0: no check):
 // pairs that fail it, or are not finite, go to the list `redo`. The estimate
 // and the flags of a direct sum are 0.
@@ -588,13 +887,16 @@ __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, int blo
   const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (p >= A.npairs || (plan_ready(A) == 0)) return;
-  const int64_t span = plan_span(A.head->work, block, A.target);
+  const int64_t span = plan_span(A, A.head->work, block);
   const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
   const int64_t na = A.off[a + 1] - A.off[a], nb = A.off[b + 1] - A.off[b];
   const int64_t n = (max(na, nb) + block - 1) / block * ((min(na, nb) + span - 1) / span), s = A.start[p];
   double acc = 0.0;
-  for (int64_t x = lane; x < n; x += 32) acc += A.partial[s + x];
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  for (int64_t x0 = 0; x0 < n; x0 += 32) {  // 32 loads at once, added one after another
+    const double v = x0 + lane < n ? A.partial[s + x0 + lane] : 0.0;
+    const int m = (int)min(n - x0, (int64_t)32);
+    for (int j = 0; j < m; ++j) acc += __shfl_sync(0xffffffffu, v, j);
+  }
   if (lane) return;
   lk[p] = acc;
   if (err) err[p] = 0.0;
@@ -664,7 +966,7 @@ __global__ void __launch_bounds__(256) plan_work(DirectArgs A, int32_t nloops) {
 __global__ void __launch_bounds__(256) plan_items(DirectArgs A, int block) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (A.head->status || p - (threadIdx.x & 31) >= A.npairs) return;
-  plan_warp(A, block, p, plan_span(A.head->work, block, A.target), threadIdx.x & 31);
+  plan_warp(A, block, p, plan_span(A, A.head->work, block), threadIdx.x & 31);
 }
 
 // Both in one CTA, for calls of few pairs; it also clears the head.
@@ -690,7 +992,7 @@ __global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops,
   if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, work, s_status, 0};
   __syncthreads();
   if (s_status) return;
-  const int64_t span = plan_span(work, block, A.target);
+  const int64_t span = plan_span(A, work, block);
   for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, block, p, span, lane);
 }
 
@@ -718,11 +1020,18 @@ constexpr TileShape kShapes[kDirectTileShapes] = {{128, 256}, {128, 128}, {128, 
                                                   {256, 256}, {256, 512}, {64, 256}};
 static_assert(kShapes[0].block == kBlockSegs && kShapes[0].tile == kTile, "the default shape comes first");
 
+// Calls of one pair in FP64, at the default tile shape (direct_fp64_lone_kernel).
+bool lone_pair(int block, int tile, int precision, int64_t npairs) {
+  return precision == FLN_PREC_FP64 && npairs == 1 && block == kBlockSegs && tile == kTile;
+}
+
 template <int kB, int kT>
 void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
   auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
-  const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, kB);
-  kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), kB, 0, st>>>(A);
+  const int threads = precision == FLN_PREC_FP64 ? kB : kB / 2;
+  if (lone_pair(kB, kT, precision, A.npairs)) kernel = direct_fp64_lone_kernel;
+  const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, threads);
+  kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), threads, 0, st>>>(A);
 }
 
 void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
@@ -753,12 +1062,16 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   int32_t *d_redo = margin >= 0 ? ctx.d_near.as<int32_t>(np) : nullptr;
   PlanHead &head = *static_cast<PlanHead *>(ctx.h_head.need(sizeof(PlanHead)));
   const int64_t target = (int64_t)ctx.num_sms * 8 * (512 / kB);
+  // FP64 sums of several pairs and large mixed ones are cut along curve 2.
+  const double least = precision == FLN_PREC_MIXED                                        ? kMixedSpans
+                       : lone_pair(kB, kShapes[tile_shape].tile, precision, np) ? 1e300
+                                                                                : 0.0;
   // Room for the items: of the largest call so far, or a guess; a plan that
   // does not fit runs no kernel and is made again with room.
   ctx.direct_items = std::max<int64_t>(ctx.direct_items, std::max<int64_t>(4 * target, 2 * np));
   for (int attempt = 0;; ++attempt) {
     const int64_t cap = ctx.direct_items;
-    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, d_head,
+    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, d_head,
                  ctx.d_partial.as<double>(cap), (float)near_factor};
     if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
       plan_small<<<1, 1024, 0, st>>>(A, nloops, kB);
@@ -992,7 +1305,7 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The default tile shape (the planning kernel cuts items of kBlockSegs).
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 0, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
   launch_direct(0, s, sms, precision, (int64_t)h.items, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, kBlockSegs, -1.0, d_lk_out, nullptr, nullptr, nullptr);
