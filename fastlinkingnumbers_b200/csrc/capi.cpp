@@ -154,14 +154,16 @@ static void clear_stats(Context &ctx) {
 // Direct sum over device-resident loops and pairs, with the margin check and
 // FP64 recompute of the mixed precision.
 static int run_direct(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops, const int32_t *d_pairs,
-                      int64_t np, const fln_params &prm, double *d_lk, double *d_err, int32_t *d_flags) {
+                      int64_t np, const fln_params &prm, double *d_lk, double *d_err, int32_t *d_flags,
+                      const DirectTail *tail = nullptr, bool *complete = nullptr) {
   clear_stats(ctx);
   const bool checked = prm.precision != FLN_PREC_FP64;
   // A margin is in [0, 0.5]: at most 0 recomputes only what is not finite, and
   // what no margin reaches (NaN too) recomputes every pair.
   const double margin = prm.fp64_margin <= 0 ? 0.0 : prm.fp64_margin <= 0.5 ? prm.fp64_margin : 1.0;
   const DirectResult r = direct_sum_device(ctx, d_xyz, d_off, nloops, d_pairs, np, prm.precision, prm.near_factor,
-                                           checked ? margin : -1.0, d_lk, d_err, d_flags, prm.direct_tile);
+                                           checked ? margin : -1.0, d_lk, d_err, d_flags, prm.direct_tile, tail);
+  if (complete) *complete = r.complete;
   ctx.stats.near_fp64_terms = checked ? r.near_terms : 0.0;
   ctx.stats.fp64_recomputed = r.redone;
   ctx.stats.segment_pairs = r.work;
@@ -403,20 +405,30 @@ void compute_pairs_host(Context &ctx, const double *xyz, const int64_t *loop_off
     }
   }
   int launches = 0;
+  bool complete = false;  // ev1 is recorded and a small call's results are on the host
+  DirectTail tail{ctx.ev1};
+  if (small && npairs > 0) {
+    tail.h_dst = static_cast<char *>(ctx.h_call.ptr) + kSmallCall;
+    tail.d_src = d_lk;
+    tail.bytes = 2 * np1 * sizeof(double) + np1 * sizeof(int32_t);
+  }
+  if (npairs == 1) tail.known_work = (double)(h_off[h_pairs[0] + 1] - h_off[h_pairs[0]]) *
+                                     (double)(h_off[h_pairs[1] + 1] - h_off[h_pairs[1]]);
   try {
     launches = bh ? run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags)
-                  : run_direct(ctx, d_xyz, d_off, nloops, d_pairs, npairs, prm, d_lk, d_err, d_flags);
+                  : run_direct(ctx, d_xyz, d_off, nloops, d_pairs, npairs, prm, d_lk, d_err, d_flags, &tail, &complete);
   } catch (...) {
     wait_xyz_pieces(ctx);
     throw;
   }
   wait_xyz_pieces(ctx);
-  FLN_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
+  if (!complete) FLN_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
   if (small && npairs > 0) {
-    char *h = static_cast<char *>(ctx.h_call.need(2 * kSmallCall)) + kSmallCall;
-    FLN_CUDA(cudaMemcpyAsync(h, d_lk, 2 * np1 * sizeof(double) + np1 * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                             ctx.stream));
-    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+    const char *h = static_cast<const char *>(tail.h_dst);
+    if (!complete) {
+      FLN_CUDA(cudaMemcpyAsync(tail.h_dst, tail.d_src, tail.bytes, cudaMemcpyDeviceToHost, ctx.stream));
+      FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+    }
     std::memcpy(lk_out, h, npairs * sizeof(double));
     if (err_out) std::memcpy(err_out, h + np1 * sizeof(double), npairs * sizeof(double));
     if (flags_out) std::memcpy(flags_out, h + 2 * np1 * sizeof(double), npairs * sizeof(int32_t));
@@ -569,9 +581,12 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz, const i
     FLN_CUDA(cudaSetDevice(c.device));
     FLN_CUDA(cudaEventRecord(c.ev0, c.stream));
     int launches;
+    bool complete = false;  // everything is done and ev1 recorded
     if (method == FLN_METHOD_DIRECTSUM && npairs > 0) {
       // Planned and checked on the device: nothing comes to the host first.
-      launches = run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, npairs, prm, d_lk_out, d_err_out, d_flags_out);
+      const DirectTail tail{c.ev1};
+      launches = run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, npairs, prm, d_lk_out, d_err_out, d_flags_out,
+                            &tail, &complete);
     } else {
       std::vector<int64_t> h_off(nloops + 1);
       std::vector<int32_t> h_pairs(2 * npairs);
@@ -586,8 +601,10 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz, const i
                      ? run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, 0, prm, d_lk_out, d_err_out, d_flags_out)
                      : run_barnes_hut(c, d_xyz, d_loop_offsets, h_off, h_pairs, prm, d_lk_out, d_err_out, d_flags_out);
     }
-    FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
-    FLN_CUDA(cudaStreamSynchronize(c.stream));
+    if (!complete) {
+      FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
+      FLN_CUDA(cudaStreamSynchronize(c.stream));
+    }
     float ms = 0;
     cudaEventElapsedTime(&ms, c.ev0, c.ev1);
     c.stats.ms_kernels = ms;

@@ -74,6 +74,8 @@ struct DirectArgs {
   int64_t cap;                // room for items
   int64_t target;             // items a call should have at least (plan_span)
   double least;               // calls of less work (PlanHead::work) take the whole of curve 2 per item
+  int block;                  // curve-1 segments per item
+  bool lone;                  // one pair in FP64: direct_fp64_lone_kernel below kLoneWork
   PlanHead *head;
   double *partial;            // per item
   float near_factor;
@@ -87,9 +89,17 @@ struct DirectArgs {
 // regroups its FP64 sum, and below that the sums stay bit for bit those of one
 // walk per segment (all there is to see when no loops are linked).
 constexpr double kMixedSpans = 1 << 30;
-__device__ __forceinline__ int64_t plan_span(const DirectArgs &A, double work, int block) {
-  if (work < A.least) return int64_t(1) << 62;
-  const double want = work / ((double)block * (double)A.target);
+// A lone pair of less work than this goes to direct_fp64_lone_kernel, 32
+// curve-1 segments an item.
+constexpr double kLoneWork = 1 << 30;
+constexpr int kLoneSegs = 32;
+__device__ __forceinline__ bool plan_lone(const DirectArgs &A, double work) { return A.lone && work < kLoneWork; }
+__device__ __forceinline__ int plan_block(const DirectArgs &A, double work) {
+  return plan_lone(A, work) ? kLoneSegs : A.block;
+}
+__device__ __forceinline__ int64_t plan_span(const DirectArgs &A, double work) {
+  if (work < A.least || plan_lone(A, work)) return int64_t(1) << 62;
+  const double want = work / ((double)A.block * (double)A.target);
   int64_t span = 32;
   while ((double)span < want) span *= 2;
   return span;
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
-  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work, kB);
+  const int64_t items = plan_lone(A, A.head->work) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
@@ -383,25 +393,29 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   }
 }
 
-// A lone pair: one curve-1 segment per thread, library square roots, each
-// segment's whole walk in one thread. The sum of one unlinked pair is nothing
-// but the rounding of its terms, so the per-pair functions (fln_direct_pair)
-// keep this order and these operations, bit for bit.
-__global__ void __launch_bounds__(kBlockSegs) direct_fp64_lone_kernel(DirectArgs A) {
-  constexpr int kB = kBlockSegs, kT = kTile;
-  __shared__ double sx[kT + 1], sy[kT + 1], sz[kT + 1];
-  __shared__ double s_red[kB / 32];
-  __shared__ long long s_item;
-  const int64_t items = plan_ready(A);
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
-    __syncthreads();
-    const int64_t item = s_item;
-    if (item >= items) break;
-    const Item it = item_of(A, item, kB, int64_t(1) << 62);
+// A lone pair. The sum of one unlinked pair is nothing but the rounding of its
+// terms, so the per-pair functions (fln_direct_pair) keep the operations and
+// the order of one thread per segment, bit for bit: a segment's terms are
+// multiplied in order, 32 segments summed by a butterfly, four such sums in
+// order, then the next four. But a walk of n steps is n times the latency of
+// a whole term, and a small pair has few segments; so an item is 32 segments,
+// seven warps form the terms of 42 steps (lanes = segments, six steps each)
+// while the eighth multiplies those of the 42 before, a chain of two FP64
+// operations per step. The terms are stored scaled by a power of two, which
+// changes no digit of their product. 300 x 211 segments, one call: 131 us with
+// one thread per segment, 75 us now (with the launches and copies around it).
+constexpr int kLoneSteps = 6, kLoneTile = 7 * kLoneSteps, kLoneChunk = 4 * kLoneTile;
+__global__ void __launch_bounds__(256) direct_fp64_lone_kernel(DirectArgs A) {
+  __shared__ double2 s_z[2][kLoneTile][32];
+  __shared__ double s_q[3 * (kLoneChunk + 1)];
+  __shared__ int s_turns[7][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double work = A.head->work;
+  const int64_t items = plan_lone(A, work) ? plan_ready(A) : 0;
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const Item it = item_of(A, item, kLoneSegs, plan_span(A, work));
     const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
-    const int64_t i = it.first + threadIdx.x;
+    const int64_t i = it.first + lane;
     const bool active = i < n1;
     double3 p0 = make_double3(0, 0, 0), p1 = p0;
     if (active) {
@@ -409,56 +423,79 @@ __global__ void __launch_bounds__(kBlockSegs) direct_fp64_lone_kernel(DirectArgs
       p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
     }
     double xs = 1.0, ys = 0.0, S = -1.0, turns = 0.0;
-    for (int64_t k0 = 0; k0 < n2; k0 += kT) {
-      const int kt = (int)(n2 - k0 < kT ? n2 - k0 : kT);
-      __syncthreads();
-      for (int t = threadIdx.x; t <= kt; t += kB) {
-        const int64_t kk = k0 + t;
-        const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
-        sx[t] = v.x;
-        sy[t] = v.y;
-        sz[t] = v.z;
+    int whole = 0;  // turns of the terms themselves
+    const int64_t tiles = (n2 + kLoneTile - 1) / kLoneTile;
+    for (int64_t t = 0; t <= tiles; ++t) {
+      const int64_t k0 = t * kLoneTile;
+      if (t < tiles && t % 4 == 0) {
+        for (int x = threadIdx.x; x < 3 * (kLoneChunk + 1); x += 256) {
+          int64_t v = 3 * k0 + x;
+          if (v >= 3 * n2) v -= 3 * n2;
+          if (v < 3 * n2) s_q[x] = __ldg(A.xyz + 3 * o2 + v);
+        }
+        __syncthreads();
       }
-      __syncthreads();
-      if (!active) continue;
-      double ax = sx[0] - p0.x, ay = sy[0] - p0.y, az = sz[0] - p0.z;
-      double bx = sx[0] - p1.x, by = sy[0] - p1.y, bz = sz[0] - p1.z;
-      double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz);
-      double ab = ax * bx + ay * by + az * bz;
-      for (int k = 0; k < kt; ++k) {
-        const double qx = sx[k + 1], qy = sy[k + 1], qz = sz[k + 1];
-        const double cx = qx - p1.x, cy = qy - p1.y, cz = qz - p1.z;
-        const double dx = qx - p0.x, dy = qy - p0.y, dz = qz - p0.z;
-        const double lc = sqrt(cx * cx + cy * cy + cz * cz), ld = sqrt(dx * dx + dy * dy + dz * dz);
-        const double ca = cx * ax + cy * ay + cz * az;
-        const double cb = cx * bx + cy * by + cz * bz;
-        const double ad = ax * dx + ay * dy + az * dz;
-        const double cd = cx * dx + cy * dy + cz * dz;
-        const double det = ax * (by * cz - bz * cy) + az * (bx * cy - by * cx) + ay * (bz * cx - bx * cz);
-        const double t = la * lc;
-        const double div1 = t * lb + ab * lc + ca * lb + cb * la;
-        const double div2 = t * ld + ad * lc + ca * ld + cd * la;
-        const double xp = div1 * div2 - det * det;
-        const double yp = det * (div1 + div2);
+      if (warp < 7) {
+        const int j0 = warp * kLoneSteps;
+        const int steps = (int)min((int64_t)kLoneSteps, n2 - k0 - j0);
+        if (t < tiles && steps > 0 && active) {
+          const double *q = s_q + 3 * ((int)(t % 4) * kLoneTile + j0);
+          double ax = q[0] - p0.x, ay = q[1] - p0.y, az = q[2] - p0.z;
+          double bx = q[0] - p1.x, by = q[1] - p1.y, bz = q[2] - p1.z;
+          double la = sqrt(ax * ax + ay * ay + az * az), lb = sqrt(bx * bx + by * by + bz * bz);
+          double ab = ax * bx + ay * by + az * bz;
+          for (int j = 0; j < steps; ++j) {
+            const double qx = q[3 * j + 3], qy = q[3 * j + 4], qz = q[3 * j + 5];
+            const double cx = qx - p1.x, cy = qy - p1.y, cz = qz - p1.z;
+            const double dx = qx - p0.x, dy = qy - p0.y, dz = qz - p0.z;
+            const double lc = sqrt(cx * cx + cy * cy + cz * cz), ld = sqrt(dx * dx + dy * dy + dz * dz);
+            const double ca = cx * ax + cy * ay + cz * az;
+            const double cb = cx * bx + cy * by + cz * bz;
+            const double ad = ax * dx + ay * dy + az * dz;
+            const double cd = cx * dx + cy * dy + cz * dz;
+            const double det = ax * (by * cz - bz * cy) + az * (bx * cy - by * cx) + ay * (bz * cx - bx * cz);
+            const double tt = la * lc;
+            const double div1 = tt * lb + ab * lc + ca * lb + cb * la;
+            const double div2 = tt * ld + ad * lc + ca * ld + cd * la;
+            double xp = __fma_rn(div1, div2, -__dmul_rn(det, det));
+            double yp = det * (div1 + div2);
+            if (yp * det < 0) whole += det > 0 ? 1 : -1;
+            renorm(xp, yp);
+            s_z[t & 1][j0 + j][lane] = make_double2(xp, yp);
+            ax = dx; ay = dy; az = dz;
+            bx = cx; by = cy; bz = cz;
+            la = ld; lb = lc; ab = cd;
+          }
+        }
+      } else if (t > 0) {
         // Arctangent addition: (xs + i ys) *= (xp + i yp), tracking crossings
         // of the negative real axis (compute_link.cpp:245-269).
-        double ny = xs * yp + xp * ys;
-        double nx = xs * xp - ys * yp;
-        renorm(nx, ny);
-        if (yp * det < 0) turns += (det > 0) ? 1.0 : -1.0;
-        const double s3 = (ny > 0.0 || (ny == 0.0 && nx < 0.0)) ? 1.0 : -1.0;
-        if (s3 * S < 0 && yp * S >= 0) turns += S;
-        xs = nx;
-        ys = ny;
-        S = s3;
-        ax = dx; ay = dy; az = dz;
-        bx = cx; by = cy; bz = cz;
-        la = ld; lb = lc; ab = cd;
+        const int n = (int)min((int64_t)kLoneTile, n2 - (k0 - kLoneTile));
+        for (int j = 0; j < n; ++j) {
+          const double2 z = s_z[(t - 1) & 1][j][lane];
+          const double xp = z.x, yp = z.y;
+          // (Fused as the compiler fuses the two sums in one loop.)
+          const double ny = __fma_rn(xs, yp, __dmul_rn(xp, ys));
+          const double nx = __fma_rn(xs, xp, -__dmul_rn(ys, yp));
+          const double s3 = (ny > 0.0 || (ny == 0.0 && nx < 0.0)) ? 1.0 : -1.0;
+          if (s3 * S < 0 && yp * S >= 0) turns += S;
+          xs = nx;
+          ys = ny;
+          S = s3;
+        }
+        renorm(xs, ys);
       }
+      __syncthreads();
     }
-    const double v = active ? atan2(ys, xs) * kInvTwoPi + turns : 0.0;
-    const double s = block_sum<kB>(v, s_red);
-    if (threadIdx.x == 0) A.partial[item] = s;
+    if (warp < 7) s_turns[warp][lane] = whole;
+    __syncthreads();
+    if (warp == 7) {
+      for (int w = 0; w < 7; ++w) turns += (double)s_turns[w][lane];
+      double v = active ? atan2(ys, xs) * kInvTwoPi + turns : 0.0;
+      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) A.partial[item] = v;
+    }
+    __syncthreads();
   }
 }
 
@@ -679,7 +716,7 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   const unsigned below = (1u << lane) - 1;
   int2 *queue = s_near[threadIdx.x >> 5];
   double *term = s_term[threadIdx.x >> 5];
-  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work, kB);
+  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work);
   unsigned long long near_count = 0;
   for (;;) {
     __syncthreads();
@@ -882,20 +919,27 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
 // checks the sum's margin to the rounding boundary (margin < 0: no check):
 // pairs that fail it, or are not finite, go to the list `redo`. The estimate
 // and the flags of a direct sum are 0.
-__global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, int block, double margin, double *lk,
-                                                           double *err, int32_t *flags, int32_t *redo) {
+__global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double margin, double *lk, double *err, int32_t *flags, int32_t *redo) {
   const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (p >= A.npairs || (plan_ready(A) == 0)) return;
-  const int64_t span = plan_span(A, A.head->work, block);
+  const double work = A.head->work;
+  const int64_t span = plan_span(A, work), block = plan_block(A, work);
+  const int per = plan_lone(A, work) ? kBlockSegs / kLoneSegs : 1;  // a lone pair's items count in fours
   const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
   const int64_t na = A.off[a + 1] - A.off[a], nb = A.off[b + 1] - A.off[b];
   const int64_t n = (max(na, nb) + block - 1) / block * ((min(na, nb) + span - 1) / span), s = A.start[p];
-  double acc = 0.0;
+  double acc = 0.0, part = 0.0;
   for (int64_t x0 = 0; x0 < n; x0 += 32) {  // 32 loads at once, added one after another
     const double v = x0 + lane < n ? A.partial[s + x0 + lane] : 0.0;
     const int m = (int)min(n - x0, (int64_t)32);
-    for (int j = 0; j < m; ++j) acc += __shfl_sync(0xffffffffu, v, j);
+    for (int j = 0; j < m; ++j) {
+      part += __shfl_sync(0xffffffffu, v, j);
+      if ((j + 1) % per == 0 || j + 1 == m) {
+        acc += part;
+        part = 0.0;
+      }
+    }
   }
   if (lane) return;
   lk[p] = acc;
@@ -926,7 +970,8 @@ __device__ __forceinline__ void plan_check(const int64_t *off, int32_t nloops, c
 
 // Items of the pairs [p0 + 32 w, ...) of a warp: reserved with one atomic,
 // pairs in order, and written to the item list.
-__device__ __forceinline__ void plan_warp(const DirectArgs &A, int block, int64_t p, int64_t span, int lane) {
+__device__ __forceinline__ void plan_warp(const DirectArgs &A, int64_t p, double work, int lane) {
+  const int64_t span = plan_span(A, work), block = plan_block(A, work);
   int64_t n = 0;
   if (p < A.npairs) {
     const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
@@ -963,15 +1008,15 @@ __global__ void __launch_bounds__(256) plan_work(DirectArgs A, int32_t nloops) {
   }
 }
 
-__global__ void __launch_bounds__(256) plan_items(DirectArgs A, int block) {
+__global__ void __launch_bounds__(256) plan_items(DirectArgs A) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (A.head->status || p - (threadIdx.x & 31) >= A.npairs) return;
-  plan_warp(A, block, p, plan_span(A, A.head->work, block), threadIdx.x & 31);
+  plan_warp(A, p, A.head->work, threadIdx.x & 31);
 }
 
 // Both in one CTA, for calls of few pairs; it also clears the head.
 constexpr int64_t kPlanSmall = 2048;
-__global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops, int block) {
+__global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops) {
   __shared__ int s_status;
   __shared__ double s_work[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -992,8 +1037,7 @@ __global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops,
   if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, work, s_status, 0};
   __syncthreads();
   if (s_status) return;
-  const int64_t span = plan_span(A, work, block);
-  for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, block, p, span, lane);
+  for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, p, work, lane);
 }
 
 // The pairs of the redo list, and back: sums and flags of recomputed pairs.
@@ -1020,28 +1064,28 @@ constexpr TileShape kShapes[kDirectTileShapes] = {{128, 256}, {128, 128}, {128, 
                                                   {256, 256}, {256, 512}, {64, 256}};
 static_assert(kShapes[0].block == kBlockSegs && kShapes[0].tile == kTile, "the default shape comes first");
 
-// Calls of one pair in FP64, at the default tile shape (direct_fp64_lone_kernel).
-bool lone_pair(int block, int tile, int precision, int64_t npairs) {
-  return precision == FLN_PREC_FP64 && npairs == 1 && block == kBlockSegs && tile == kTile;
-}
-
 template <int kB, int kT>
-void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
+void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, double known_work, const DirectArgs &A) {
   auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
   const int threads = precision == FLN_PREC_FP64 ? kB : kB / 2;
-  if (lone_pair(kB, kT, precision, A.npairs)) kernel = direct_fp64_lone_kernel;
+  if (A.lone) {
+    // Where the host does not know the work, the plan fits one of the two.
+    direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
+    if (known_work >= 0 && known_work < kLoneWork) return;
+  }
   const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, threads);
   kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), threads, 0, st>>>(A);
 }
 
-void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, const DirectArgs &A) {
+void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, double known_work,
+                   const DirectArgs &A) {
   switch (shape) {
-    case 1: launch_direct_t<128, 128>(st, sms, precision, most, A); break;
-    case 2: launch_direct_t<128, 512>(st, sms, precision, most, A); break;
-    case 3: launch_direct_t<256, 256>(st, sms, precision, most, A); break;
-    case 4: launch_direct_t<256, 512>(st, sms, precision, most, A); break;
-    case 5: launch_direct_t<64, 256>(st, sms, precision, most, A); break;
-    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, A); break;
+    case 1: launch_direct_t<128, 128>(st, sms, precision, most, known_work, A); break;
+    case 2: launch_direct_t<128, 512>(st, sms, precision, most, known_work, A); break;
+    case 3: launch_direct_t<256, 256>(st, sms, precision, most, known_work, A); break;
+    case 4: launch_direct_t<256, 512>(st, sms, precision, most, known_work, A); break;
+    case 5: launch_direct_t<64, 256>(st, sms, precision, most, known_work, A); break;
+    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, known_work, A); break;
   }
 }
 
@@ -1049,7 +1093,7 @@ void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t m
 
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
                                const int32_t *d_pairs, int64_t np, int precision, double near_factor, double margin,
-                               double *d_lk, double *d_err, int32_t *d_flags, int tile_shape) {
+                               double *d_lk, double *d_err, int32_t *d_flags, int tile_shape, const DirectTail *tail) {
   if (tile_shape < 0 || tile_shape >= kDirectTileShapes)
     throw Error(FLN_ERR_INVALID_ARGUMENT, "direct_tile in [0, " + std::to_string(kDirectTileShapes - 1) + "]");
   DirectResult R;
@@ -1062,34 +1106,36 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   int32_t *d_redo = margin >= 0 ? ctx.d_near.as<int32_t>(np) : nullptr;
   PlanHead &head = *static_cast<PlanHead *>(ctx.h_head.need(sizeof(PlanHead)));
   const int64_t target = (int64_t)ctx.num_sms * 8 * (512 / kB);
-  // FP64 sums of several pairs and large mixed ones are cut along curve 2.
-  const double least = precision == FLN_PREC_MIXED                                        ? kMixedSpans
-                       : lone_pair(kB, kShapes[tile_shape].tile, precision, np) ? 1e300
-                                                                                : 0.0;
+  // FP64 sums and large mixed ones are cut along curve 2; a lone FP64 pair has
+  // a kernel of its own.
+  const double least = precision == FLN_PREC_MIXED ? kMixedSpans : 0.0;
+  const bool lone = precision == FLN_PREC_FP64 && np == 1 && tile_shape == 0;
   // Room for the items: of the largest call so far, or a guess; a plan that
   // does not fit runs no kernel and is made again with room.
   ctx.direct_items = std::max<int64_t>(ctx.direct_items, std::max<int64_t>(4 * target, 2 * np));
   for (int attempt = 0;; ++attempt) {
     const int64_t cap = ctx.direct_items;
-    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, d_head,
-                 ctx.d_partial.as<double>(cap), (float)near_factor};
+    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, kB, lone,
+                 d_head, ctx.d_partial.as<double>(cap), (float)near_factor};
     if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
-      plan_small<<<1, 1024, 0, st>>>(A, nloops, kB);
+      plan_small<<<1, 1024, 0, st>>>(A, nloops);
     } else {
       FLN_CUDA(cudaMemsetAsync(d_head, 0, sizeof(PlanHead), st));
       const int64_t most = std::max<int64_t>(np, nloops);
       plan_work<<<(int)std::min<int64_t>((most + 255) / 256, 8 * ctx.num_sms), 256, 0, st>>>(A, nloops);
-      plan_items<<<(int)((np + 255) / 256), 256, 0, st>>>(A, kB);
+      plan_items<<<(int)((np + 255) / 256), 256, 0, st>>>(A);
       ++R.launches;
     }
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, A);
+    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, tail ? tail->known_work : -1.0, A);
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev3, st));
-    reduce_items_kernel<<<(int)((np + 7) / 8), 256, 0, st>>>(A, kB, margin, d_lk, d_err, d_flags, d_redo);
+    reduce_items_kernel<<<(int)((np + 7) / 8), 256, 0, st>>>(A, margin, d_lk, d_err, d_flags, d_redo);
     FLN_CUDA(cudaGetLastError());
     R.launches += 3;
+    if (tail) FLN_CUDA(cudaEventRecord(tail->end, st));
+    if (tail && tail->bytes) FLN_CUDA(cudaMemcpyAsync(tail->h_dst, tail->d_src, tail->bytes, cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaMemcpyAsync(&head, d_head, sizeof head, cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaStreamSynchronize(st));
     if (head.status) {
@@ -1110,6 +1156,7 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   R.near_terms = (double)head.near;
   R.work = head.work;
   R.redone = (int64_t)head.redo;
+  R.complete = tail && R.redone == 0;
   if (R.redone > 0) {
     const int64_t nr = R.redone;
     int32_t *list = ctx.d_redo.as<int32_t>(3 * nr + (nr & 1) + 2 * nr);  // list, pairs, sums
@@ -1120,7 +1167,8 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
     gather_pairs<<<grid, 256, 0, st>>>(list, nr, d_pairs, pairs);
     FLN_CUDA(cudaGetLastError());
     R.launches += 2 + direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, nr, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr,
-                                        nullptr, 0).launches;
+                                        nullptr)
+                      .launches;
     scatter_redo<<<grid, 256, 0, st>>>(list, nr, sums, d_lk, d_flags);
     FLN_CUDA(cudaGetLastError());
   }
@@ -1305,10 +1353,10 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The default tile shape (the planning kernel cuts items of kBlockSegs).
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, false, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
-  launch_direct(0, s, sms, precision, (int64_t)h.items, A);
-  reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, kBlockSegs, -1.0, d_lk_out, nullptr, nullptr, nullptr);
+  launch_direct(0, s, sms, precision, (int64_t)h.items, -1.0, A);
+  reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FLN_ERR_CUDA, std::string("fln_linking_numbers_direct_noalloc: ") + cudaGetErrorString(e));
   return FLN_OK;

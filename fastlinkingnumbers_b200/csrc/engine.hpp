@@ -190,11 +190,22 @@ struct DirectResult {
   double near_terms = 0;  // mixed: segment pairs evaluated in FP64
   double work = 0;        // sum over pairs of n_i n_j
   int64_t redone = 0;     // pairs recomputed in FP64
+  bool complete = false;  // the tail's event and copy are done (no pair was recomputed)
+};
+// What a caller wants at the end of a call without recomputed pairs, before
+// the call's one host wait: an event, and the results copied to the host.
+struct DirectTail {
+  cudaEvent_t end;
+  void *h_dst = nullptr;  // pinned
+  const void *d_src = nullptr;
+  size_t bytes = 0;
+  double known_work = -1.0;  // sum of n_i n_j where the host knows it
 };
 constexpr int kDirectTileShapes = 6;
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
                                const int32_t *d_pairs, int64_t npairs, int precision, double near_factor,
-                               double margin, double *d_lk, double *d_err, int32_t *d_flags, int tile_shape = 0);
+                               double margin, double *d_lk, double *d_err, int32_t *d_flags, int tile_shape = 0,
+                               const DirectTail *tail = nullptr);
 
 // Barnes–Hut over the same inputs; err per pair after ERROR_EST_SCALE and the
 // reference's beta retry; flags gets FLN_PAIR_BETA_RETRIED. Returns launches.

@@ -34,6 +34,11 @@ CASES = {
     "edges": ([2, 3, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 513, 1000], None),
     "long against short": ([20011, 3, 40, 300], None),
     "long pair": ([7001, 6007], [(1, 0)]),
+    # A lone pair's tiles of 42 steps (four to a staged stretch) and items of 32 segments.
+    "lone 2 x 2": ([2, 2], [(0, 1)]),
+    "lone 43 x 42": ([43, 42], [(0, 1)]),
+    "lone 129 x 41": ([41, 129], [(0, 1)]),
+    "lone 337 x 169": ([337, 169], [(0, 1)]),
     "more items than room": ([20000] + [3] * 130, [(k + 1, 0) for k in range(130)]),
     "many pairs": (list(range(2, 72)), None),
 }
