@@ -3,12 +3,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <numeric>
 #include <random>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "engine.hpp"
@@ -89,10 +92,12 @@ static void stage_setup(Context &ctx) {
     if (!e) FLN_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
 }
 
-void copy_h2d(Context &ctx, void *d_dst, const void *h_src, size_t bytes) {
+void fill_h2d(Context &ctx, void *d_dst, size_t bytes, const std::function<void(char *, size_t, size_t)> &fill) {
   if (bytes == 0) return;
-  if (bytes <= kStage / 4 || is_pinned(h_src)) {
-    FLN_CUDA(cudaMemcpyAsync(d_dst, h_src, bytes, cudaMemcpyHostToDevice, ctx.stream));
+  if (bytes <= kStage / 4) {  // not worth the staging buffers
+    std::vector<char> all(bytes);
+    fill(all.data(), 0, bytes);
+    FLN_CUDA(cudaMemcpyAsync(d_dst, all.data(), bytes, cudaMemcpyHostToDevice, ctx.stream));
     FLN_CUDA(cudaStreamSynchronize(ctx.stream));
     return;
   }
@@ -101,18 +106,30 @@ void copy_h2d(Context &ctx, void *d_dst, const void *h_src, size_t bytes) {
   for (size_t o = 0, k = 0; o < bytes; o += kStage, ++k) {
     const size_t len = std::min(kStage, bytes - o);
     FLN_CUDA(cudaEventSynchronize(ctx.ev_stage[k & 1]));  // the copy that last used this buffer is done
-    parallel_memcpy(stage[k & 1], static_cast<const char *>(h_src) + o, len);
+    fill(static_cast<char *>(stage[k & 1]), o, len);
     FLN_CUDA(cudaMemcpyAsync(static_cast<char *>(d_dst) + o, stage[k & 1], len, cudaMemcpyHostToDevice, ctx.stream));
     FLN_CUDA(cudaEventRecord(ctx.ev_stage[k & 1], ctx.stream));
   }
   FLN_CUDA(cudaStreamSynchronize(ctx.stream));
 }
 
-void copy_d2h(Context &ctx, void *h_dst, const void *d_src, size_t bytes) {
+void copy_h2d(Context &ctx, void *d_dst, const void *h_src, size_t bytes) {
+  if (bytes == 0) return;
+  if (bytes <= kStage / 4 || is_pinned(h_src)) {
+    FLN_CUDA(cudaMemcpyAsync(d_dst, h_src, bytes, cudaMemcpyHostToDevice, ctx.stream));
+    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+    return;
+  }
+  fill_h2d(ctx, d_dst, bytes, [&](char *dst, size_t o, size_t len) {
+    parallel_memcpy(dst, static_cast<const char *>(h_src) + o, len);
+  });
+}
+
+void copy_d2h(Context &ctx, cudaStream_t stream, void *h_dst, const void *d_src, size_t bytes, bool all_threads) {
   if (bytes == 0) return;
   if (bytes <= kStage / 4 || is_pinned(h_dst)) {
-    FLN_CUDA(cudaMemcpyAsync(h_dst, d_src, bytes, cudaMemcpyDeviceToHost, ctx.stream));
-    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+    FLN_CUDA(cudaMemcpyAsync(h_dst, d_src, bytes, cudaMemcpyDeviceToHost, stream));
+    FLN_CUDA(cudaStreamSynchronize(stream));
     return;
   }
   stage_setup(ctx);
@@ -122,13 +139,14 @@ void copy_d2h(Context &ctx, void *h_dst, const void *d_src, size_t bytes) {
     if (k < nchunks) {
       const size_t o = k * kStage, len = std::min(kStage, bytes - o);
       FLN_CUDA(cudaMemcpyAsync(stage[k & 1], static_cast<const char *>(d_src) + o, len, cudaMemcpyDeviceToHost,
-                               ctx.stream));
-      FLN_CUDA(cudaEventRecord(ctx.ev_stage[k & 1], ctx.stream));
+                               stream));
+      FLN_CUDA(cudaEventRecord(ctx.ev_stage[k & 1], stream));
     }
     if (k > 0) {
       const size_t j = k - 1, o = j * kStage, len = std::min(kStage, bytes - o);
       FLN_CUDA(cudaEventSynchronize(ctx.ev_stage[j & 1]));
-      parallel_memcpy(static_cast<char *>(h_dst) + o, stage[j & 1], len);
+      if (all_threads) parallel_memcpy(static_cast<char *>(h_dst) + o, stage[j & 1], len);
+      else std::memcpy(static_cast<char *>(h_dst) + o, stage[j & 1], len);
     }
   }
 }
@@ -288,19 +306,28 @@ struct fln_learned {
 namespace fln {
 void set_last_error(const std::string &msg);
 
-// prepare() with Discretize and both potential-link searches on the GPU.
-static void prepare_device(Context &ctx, Model &m, bool discretize_on) {
+// prepare() with Discretize and both potential-link searches on the GPU. The
+// polylines are left on the device (`on_device`) when the caller asks for
+// that, and copied to the model otherwise.
+static void prepare_device(Context &ctx, Model &m, bool discretize_on, DiscretizedOnDevice *on_device = nullptr) {
   if (!discretize_on) {
     prepare(m, false);
     return;
   }
-  discretize_device(ctx, m.curves, m.bcc_xyz.empty() ? nullptr : m.bcc_xyz.data(), m.poly_offsets, m.poly_xyz,
-                    m.pairs, m.rounds);
+  m.prepared = false;
+  const DiscretizedOnDevice d = discretize_device(ctx, m.curves, m.bcc_xyz.empty() ? nullptr : m.bcc_xyz.data(),
+                                                  m.poly_offsets, m.pairs, m.rounds);
   // An open curve that reaches the linking-number stage is an error there
   // (Curve::GetStartPoints, curve.cpp:126-128); one without pairs is not.
   for (size_t p = 0; p < m.pairs.size(); ++p)
     if (!m.curves[m.pairs[p]].closed)
       throw Error(FLN_ERR_UNLOOPED, "Curve::GetStartPoints() does not support unlooped curves.");
+  if (on_device) {
+    *on_device = d;
+    return;
+  }
+  copy_polylines(ctx, ctx.stream, d.d_xyz, 3 * (size_t)m.poly_offsets.back(), m.poly_xyz, true);
+  release_discretized(ctx);
   m.prepared = true;
 }
 }  // namespace fln
@@ -355,6 +382,40 @@ bool copy_xyz_pieces(Context &ctx, double *d_xyz, const double *xyz, const std::
   }
   ctx.xyz_pieces = Context::kXyzPieces;
   return true;
+}
+
+// Sums for loops and pairs that are resident (d_xyz, d_off) and known to the
+// host: the linking-number stage of a certificate whose Discretize just ran.
+void compute_pairs_resident(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
+                            const std::vector<int32_t> &h_pairs, fln_method method, const fln_params &prm,
+                            double *lk_out, double *err_out, int32_t *flags_out) {
+  const double t0 = now_ms();
+  const int32_t nloops = (int32_t)h_off.size() - 1;
+  const int64_t np = (int64_t)h_pairs.size() / 2;
+  FLN_CUDA(cudaSetDevice(ctx.device));
+  check_inputs(h_off, nloops, h_pairs);
+  double *d_lk = ctx.d_lk.as<double>(2 * np + (np + 1) / 2), *d_err = d_lk + np;
+  int32_t *d_flags = reinterpret_cast<int32_t *>(d_err + np);
+  FLN_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
+  ctx.xyz_pieces = 0;
+  int launches;
+  if (method == FLN_METHOD_BARNESHUT) {
+    launches = run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags);
+  } else {
+    int32_t *d_pairs = ctx.d_pairs.as<int32_t>(2 * np);
+    FLN_CUDA(cudaMemcpyAsync(d_pairs, h_pairs.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
+    launches = run_direct(ctx, d_xyz, d_off, nloops, d_pairs, np, prm, d_lk, d_err, d_flags);
+  }
+  FLN_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
+  FLN_CUDA(cudaMemcpyAsync(lk_out, d_lk, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+  FLN_CUDA(cudaMemcpyAsync(err_out, d_err, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+  FLN_CUDA(cudaMemcpyAsync(flags_out, d_flags, np * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx.stream));
+  FLN_CUDA(cudaStreamSynchronize(ctx.stream));
+  float ms = 0;
+  cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1);
+  ctx.stats.ms_kernels = ms;
+  ctx.stats.kernel_launches = launches;
+  ctx.stats.ms_total = now_ms() - t0;
 }
 
 void compute_pairs_host(Context &ctx, const double *xyz, const int64_t *loop_offsets, int32_t nloops,
@@ -479,6 +540,49 @@ void upload_loops(Context &ctx, const double *xyz, const int64_t *loop_offsets, 
   FLN_CUDA(cudaMemcpyAsync(*d_xyz, xyz, 3 * nv * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
   FLN_CUDA(cudaMemcpyAsync(*d_off, h_off.data(), (nloops + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx.stream));
 }
+
+// The polylines of a Discretize on their way to the model, on the context's
+// copy stream from a thread of its own (started only when they are on the
+// device). finish() waits for them and passes their failure on; the destructor
+// waits too, so that nothing outlives a call that throws.
+class PolylineCopy {
+ public:
+  PolylineCopy(Context &ctx, Model &m, const DiscretizedOnDevice &d) : ctx_(ctx), m_(m), d_(d) {
+    if (!d_.d_xyz) return;
+    if (!ctx_.copy_stream) FLN_CUDA(cudaStreamCreateWithFlags(&ctx_.copy_stream, cudaStreamNonBlocking));
+    thread_ = std::thread([this] {
+      try {
+        FLN_CUDA(cudaSetDevice(ctx_.device));
+        // (A team of host threads is worth starting here for large copies only.)
+        const size_t n = 3 * (size_t)m_.poly_offsets.back();
+        copy_polylines(ctx_, ctx_.copy_stream, d_.d_xyz, n, m_.poly_xyz, n > (size_t(1) << 20));
+      } catch (...) {
+        failure_ = std::current_exception();
+      }
+    });
+  }
+  PolylineCopy(const PolylineCopy &) = delete;
+  PolylineCopy &operator=(const PolylineCopy &) = delete;
+  ~PolylineCopy() {
+    if (!thread_.joinable()) return;
+    thread_.join();
+    release_discretized(ctx_);
+  }
+  void finish() {
+    if (!thread_.joinable()) return;
+    thread_.join();
+    if (failure_) std::rethrow_exception(failure_);
+    m_.prepared = true;
+    release_discretized(ctx_);
+  }
+
+ private:
+  Context &ctx_;
+  Model &m_;
+  DiscretizedOnDevice d_;
+  std::thread thread_;
+  std::exception_ptr failure_;
+};
 
 double pinball(float y, float t, double q) {
   const double e = (double)t - (double)y;
@@ -1026,15 +1130,26 @@ fln_status fln_model_set_curves(fln_model *m, fln_seg_type type, int32_t ncurves
     if (!m || ncurves < 0 || (ncurves && !counts)) throw Error(FLN_ERR_INVALID_ARGUMENT, "NULL argument");
     if ((int)type < 0 || (int)type > 3) throw Error(FLN_ERR_INVALID_ARGUMENT, "unknown segment type");
     std::vector<CurveData> cs(ncurves);
-    int64_t at = 0;
+    std::vector<int64_t> at(ncurves + 1, 0);
     for (int32_t i = 0; i < ncurves; ++i) {
       const int64_t n = counts[i] < 0 ? -(int64_t)counts[i] : counts[i];
+      at[i + 1] = at[i] + n;
       cs[i].kind = (SegKind)type;
       cs[i].closed = counts[i] < 0;
-      cs[i].q.resize(n);
       if (n && !xyz) throw Error(FLN_ERR_INVALID_ARGUMENT, "xyz is NULL");
-      for (int64_t k = 0; k < n; ++k, ++at) cs[i].q[k] = {xyz[3 * at], xyz[3 * at + 1], xyz[3 * at + 2]};
     }
+    // Large models by all threads (no exception may leave the parallel loop).
+    std::atomic<bool> no_memory{false};
+#pragma omp parallel for schedule(dynamic, 1) if (at[ncurves] > 100000)
+    for (int32_t i = 0; i < ncurves; ++i) {
+      try {
+        const auto *p = reinterpret_cast<const Vec3 *>(xyz) + at[i];
+        cs[i].q.assign(p, p + (at[i + 1] - at[i]));
+      } catch (...) {
+        no_memory = true;
+      }
+    }
+    if (no_memory) throw std::bad_alloc();
     m->m.curves.swap(cs);
     m->m.bcc_xyz.clear();
     m->m.bcc_xyz.shrink_to_fit();
@@ -1117,13 +1232,17 @@ fln_status fln_certificate_compute(fln_ctx *ctx, const fln_model *model, int for
     const fln_params prm = resolved(params);
     auto *mm = const_cast<fln_model *>(model);  // the prepared polylines are a cache
     const double t0 = now_ms();
+    DiscretizedOnDevice on_device;
     if (!mm->m.prepared || mm->prepared_disc != (discretize != 0)) {
       FLN_CUDA(cudaSetDevice(ctx->c->device));
       if (prm.host_prepare) prepare(mm->m, discretize != 0);
-      else prepare_device(*ctx->c, mm->m, discretize != 0);
+      else prepare_device(*ctx->c, mm->m, discretize != 0, &on_device);
       mm->prepared_disc = discretize != 0;
     }
     const double t1 = now_ms();
+    // Polylines that are still on the device: the sums read them there, while
+    // another thread copies them to the model for its later calls.
+    PolylineCopy copy(*ctx->c, mm->m, on_device);
     const Model &m = mm->m;
     const int32_t nc = (int32_t)m.curves.size();
     const int64_t np = (int64_t)m.pairs.size() / 2;
@@ -1133,12 +1252,16 @@ fln_status fln_certificate_compute(fln_ctx *ctx, const fln_model *model, int for
     cert->c.err.assign(np, 0.0);
     cert->c.flags.assign(np, 0);
     Context &c = *ctx->c;
-    if (np)
+    const fln_method method = force_direct_sum ? FLN_METHOD_DIRECTSUM : FLN_METHOD_BARNESHUT;
+    if (np && on_device.d_xyz)
+      compute_pairs_resident(c, on_device.d_xyz, on_device.d_off, m.poly_offsets, m.pairs, method, prm,
+                             cert->c.lk.data(), cert->c.err.data(), cert->c.flags.data());
+    else if (np)
       compute_pairs_host(c, m.poly_xyz.data(), m.poly_offsets.data(), nc, m.pairs.data(), np,
-                         force_direct_sum ? FLN_METHOD_DIRECTSUM : FLN_METHOD_BARNESHUT, prm, cert->c.lk.data(),
-                         cert->c.err.data(), cert->c.flags.data());
+                         method, prm, cert->c.lk.data(), cert->c.err.data(), cert->c.flags.data());
     else
       c.stats = fln_stats{};
+    copy.finish();
     fill_certificate(cert->c, nc, m.pairs, cert->c.lk);
     c.stats.ms_discretize = t1 - t0;
     c.stats.discretize_rounds = m.rounds;

@@ -31,6 +31,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <limits>
 #include <numeric>
 #include <vector>
@@ -549,6 +550,8 @@ __global__ void __launch_bounds__(kJoinTile) box_join(const double *box, int nc,
 // all-pairs test costs more than the host sweep, which then runs instead.
 constexpr int kJoinMaxCurves = 1 << 17;
 constexpr int kJoinBufs = 34;  // d_disc[34], [35]: the join's own; [36] the float32 upload (0..33: Discretize)
+constexpr int kDiscBufs = 37, kDiscXyz = 33, kDiscOff = 20;  // all; the polylines and their offsets
+constexpr size_t kDiscKeep = size_t(4) << 30;  // device memory kept between calls
 std::vector<Box3> boxes_to_host(Context &ctx, const double *d_box, int nc);
 std::vector<std::pair<int, int>> device_box_pairs(Context &ctx, const double *d_box, int nc) {
   if (nc > kJoinMaxCurves) return box_pairs(boxes_to_host(ctx, d_box, nc));
@@ -598,9 +601,9 @@ std::vector<Box3> boxes_to_host(Context &ctx, const double *d_box, int nc) {
 
 }  // namespace
 
-void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const float *bcc_f32,
-                       std::vector<int64_t> &offsets, DoubleArray &xyz, std::vector<int32_t> &pairs_out,
-                       int32_t &rounds) {
+DiscretizedOnDevice discretize_device(Context &ctx, const std::vector<CurveData> &curves, const float *bcc_f32,
+                                      std::vector<int64_t> &offsets, std::vector<int32_t> &pairs_out,
+                                      int32_t &rounds) {
   const int nc = (int)curves.size();
   cudaStream_t st = ctx.stream;
   DevBuf *B = ctx.d_disc;
@@ -612,26 +615,26 @@ void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const
     seg_off[c + 1] = seg_off[c] + std::max(curves[c].segments(), 0);
     kind[c] = curves[c].kind;
   }
-  // The packed FP64 control points, unless the float32 ones of the BCC file
-  // are uploaded and widened on the device.
-  DoubleArray cp(bcc_f32 ? 0 : 3 * (size_t)std::max<int64_t>(cp_off[nc], 1));
   const int64_t nseg = seg_off[nc];
+  // Input sanity (discretize.cpp:126-160): mean |control point| over the
+  // segment-indexed points, summed in the host's order (a serial sum, by a
+  // thread beside the upload).
   DoubleArray norms((size_t)std::max<int64_t>(nseg, 1));
-#pragma omp parallel for schedule(dynamic, 16)
-  for (int c = 0; c < nc; ++c) {
-    if (!bcc_f32 && !curves[c].q.empty())
-      std::memcpy(&cp[3 * cp_off[c]], &curves[c].q[0].x, curves[c].q.size() * sizeof(Vec3));
+#pragma omp parallel for schedule(dynamic, 4) if (nseg > 50000)
+  for (int c = 0; c < nc; ++c)
     for (int s = 0; s < curves[c].segments(); ++s) {
       const Vec3 &p = curves[c].q[s];
       norms[seg_off[c] + s] = std::sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
     }
-  }
-  // Input sanity (discretize.cpp:126-160): mean |control point| over the
-  // segment-indexed points, summed in the host's order.
-  double norm_sum = 0;
-  for (int64_t k = 0; k < nseg; ++k) norm_sum += norms[k];
-  const double avg = norm_sum / ((double)nseg * 1.73205080757);
-  const double thresh = std::numeric_limits<double>::epsilon() * avg;
+  auto sum_norms = [&norms, nseg]() {
+    double sum = 0;
+    for (int64_t k = 0; k < nseg; ++k) sum += norms[k];
+    const double avg = sum / ((double)nseg * 1.73205080757);
+    return std::numeric_limits<double>::epsilon() * avg;
+  };
+  std::future<double> thresh_later =
+      std::async(nseg > 50000 ? std::launch::async : std::launch::deferred, sum_norms);
+  double thresh = 0;
   if (nseg > INT32_MAX) throw Error(FLN_ERR_OUT_OF_MEMORY, "Discretize: more than 2^31 segments");
 
   double *d_cp = buf<double>(B[0], 3 * std::max<int64_t>(cp_off[nc], 1));
@@ -645,7 +648,18 @@ void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const
     if (nf > 0) widen_f32<<<(int)std::min<int64_t>((nf + 255) / 256, 1 << 20), 256, 0, st>>>(d_f, nf, d_cp);
     FLN_CUDA(cudaGetLastError());
   } else {
-    copy_h2d(ctx, d_cp, cp.data(), 3 * cp_off[nc] * sizeof(double));
+    // The control points are packed straight into the pinned staging buffers.
+    fill_h2d(ctx, d_cp, 3 * (size_t)cp_off[nc] * sizeof(double), [&](char *dst, size_t o, size_t len) {
+      const int64_t b0 = (int64_t)o, b1 = (int64_t)(o + len), unit = sizeof(Vec3);
+      const int c0 = (int)(std::upper_bound(cp_off.begin(), cp_off.end(), b0 / unit) - cp_off.begin()) - 1;
+#pragma omp parallel for schedule(dynamic, 4) if (len > (1 << 20))
+      for (int c = c0; c < nc; ++c) {
+        const int64_t lo = std::max(b0, cp_off[c] * unit), hi = std::min(b1, cp_off[c + 1] * unit);
+        if (lo < hi)
+          std::memcpy(dst + (lo - b0), reinterpret_cast<const char *>(curves[c].q.data()) + (lo - cp_off[c] * unit),
+                      (size_t)(hi - lo));
+      }
+    });
   }
   FLN_CUDA(cudaMemcpyAsync(d_cpoff, cp_off.data(), (nc + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   FLN_CUDA(cudaMemcpyAsync(d_kind, kind.data(), std::max(nc, 1) * sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -739,6 +753,7 @@ void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const
   for (int it = 0; it < kMaxRounds; ++it) {
     ++rounds;
     const double md = build_live();
+    if (it == 0) thresh = thresh_later.get();
     if (it == 0 && !(md >= thresh))
       throw Error(FLN_ERR_SEGMENT_TOO_SMALL,
                   "Discretize: Smallest input segment is smaller than eps * avg coordinate. Consider combining.");
@@ -866,8 +881,6 @@ void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const
   }
   FLN_CUDA(cudaGetLastError());
   FLN_CUDA(cudaStreamSynchronize(st));
-  xyz.resize(3 * nv);
-  copy_d2h(ctx, xyz.data(), d_xyz, 3 * nv * sizeof(double));
   // Potential pairs of the polylines.
   double *d_box = buf<double>(B[27], 6 * (int64_t)nc);
   if (nc > 0) polyline_boxes<<<nc, 256, 0, st>>>(d_xyz, d_out, d_box);
@@ -879,10 +892,29 @@ void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const
     pairs_out[2 * k] = pl[k].first;
     pairs_out[2 * k + 1] = pl[k].second;
   }
-  // The working buffers (tens of GB for 10^8 segments) are not kept for the
-  // linking-number stage that follows.
+  // Working buffers of a large model (tens of GB for 10^8 segments) are not
+  // kept for the linking-number stage that follows; smaller ones stay, because
+  // freeing and allocating 37 buffers takes milliseconds per call.
   FLN_CUDA(cudaStreamSynchronize(st));
-  for (int k = 0; k < 37; ++k) B[k].release();
+  size_t held = 0;
+  for (int k = 0; k < kDiscBufs; ++k) held += B[k].bytes;
+  if (held > kDiscKeep)
+    for (int k = 0; k < kDiscBufs; ++k)
+      if (k != kDiscXyz && k != kDiscOff) B[k].release();
+  return DiscretizedOnDevice{d_xyz, d_out};
+}
+
+void copy_polylines(Context &ctx, cudaStream_t stream, const double *d_xyz, size_t n, DoubleArray &xyz,
+                    bool all_threads) {
+  xyz.resize(n);
+  copy_d2h(ctx, stream, xyz.data(), d_xyz, n * sizeof(double), all_threads);
+}
+
+void release_discretized(Context &ctx) {
+  size_t held = 0;
+  for (int k = 0; k < kDiscBufs; ++k) held += ctx.d_disc[k].bytes;
+  if (held > kDiscKeep)
+    for (int k = 0; k < kDiscBufs; ++k) ctx.d_disc[k].release();
 }
 
 }  // namespace fln

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -24,7 +25,9 @@ namespace fln {
                          std::string(#call) + ": " + cudaGetErrorString(e_));              \
   } while (0)
 
-// Grow-only device buffer.
+// Grow-only device buffer. It grows with some room to spare (an eighth, at
+// most 256 MB, where there is memory for it), so that calls of about the same
+// size do not each free and allocate it again.
 struct DevBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
@@ -33,8 +36,14 @@ struct DevBuf {
       if (ptr) cudaFree(ptr);
       ptr = nullptr;
       bytes = 0;
-      FLN_CUDA(cudaMalloc(&ptr, n));
-      bytes = n;
+      size_t want = n + std::min(n / 8, size_t(256) << 20);
+      if (cudaMalloc(&ptr, want) != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+        want = n;
+        FLN_CUDA(cudaMalloc(&ptr, want));
+      }
+      bytes = want;
     }
     return ptr;
   }
@@ -253,15 +262,30 @@ double learned_gradients(Context &ctx, const float *params, const float *X, cons
 // bcc_f32: the same control points as float32 (curves in order, 3 per
 // point), or nullptr; when given they are uploaded as such and widened on the
 // device (the same doubles, half the copy).
-void discretize_device(Context &ctx, const std::vector<CurveData> &curves, const float *bcc_f32,
-                       std::vector<int64_t> &offsets, DoubleArray &xyz, std::vector<int32_t> &pairs, int32_t &rounds);
+//
+// The polylines stay on the device (DiscretizedOnDevice) until the next call
+// or release_discretized; copy_polylines brings them to the host.
+struct DiscretizedOnDevice {
+  const double *d_xyz = nullptr;
+  const int64_t *d_off = nullptr;
+};
+DiscretizedOnDevice discretize_device(Context &ctx, const std::vector<CurveData> &curves, const float *bcc_f32,
+                                      std::vector<int64_t> &offsets, std::vector<int32_t> &pairs, int32_t &rounds);
+// Copies n doubles to `xyz` on `stream` (see copy_d2h).
+void copy_polylines(Context &ctx, cudaStream_t stream, const double *d_xyz, size_t n, DoubleArray &xyz,
+                    bool all_threads);
+// Gives the polylines' buffers back when they are large.
+void release_discretized(Context &ctx);
 
 // Host<->device copies on ctx.stream that return when the data has arrived.
 // Pinned host memory is copied directly; pageable memory goes in 64 MB
 // chunks through two pinned buffers, the host side by all threads (a single
 // pageable DMA copy runs at a few GB/s, slower still into fresh pages).
 void copy_h2d(Context &ctx, void *d_dst, const void *h_src, size_t bytes);
-void copy_d2h(Context &ctx, void *h_dst, const void *d_src, size_t bytes);
+void copy_d2h(Context &ctx, cudaStream_t stream, void *h_dst, const void *d_src, size_t bytes, bool all_threads);
+// The same for data that is formed on the way: fill(dst, offset, len) writes
+// bytes [offset, offset + len) of it.
+void fill_h2d(Context &ctx, void *d_dst, size_t bytes, const std::function<void(char *, size_t, size_t)> &fill);
 // memcpy by all host threads.
 void parallel_memcpy(void *dst, const void *src, size_t bytes);
 

@@ -2,7 +2,11 @@
 // Discretize, certificates. Internal C++ API behind the C ABI of fln.h.
 #pragma once
 
+#include <sys/mman.h>
+
+#include <cstddef>
 #include <cstdint>
+#include <cstdlib>
 #include <memory>
 #include <new>
 #include <stdexcept>
@@ -37,6 +41,23 @@ struct NoInitAlloc : std::allocator<T> {
   template <class U>
   void construct(U *p) noexcept {
     ::new (static_cast<void *>(p)) U;
+  }
+  // Large arrays on 2 MB pages where the system has them: first touches of
+  // fresh 4 KB pages cost more than the copy that fills them.
+  static constexpr std::size_t kHuge = std::size_t(1) << 21;
+  static constexpr std::size_t kLarge = std::size_t(1) << 23;
+  T *allocate(std::size_t n) {
+    if (n > SIZE_MAX / sizeof(T) - kHuge) throw std::bad_alloc();
+    if (n * sizeof(T) < kLarge) return std::allocator<T>::allocate(n);
+    const std::size_t bytes = (n * sizeof(T) + kHuge - 1) / kHuge * kHuge;
+    void *p = std::aligned_alloc(kHuge, bytes);
+    if (!p) throw std::bad_alloc();
+    madvise(p, bytes, MADV_HUGEPAGE);
+    return static_cast<T *>(p);
+  }
+  void deallocate(T *p, std::size_t n) noexcept {
+    if (n * sizeof(T) < kLarge) std::allocator<T>::deallocate(p, n);
+    else std::free(p);
   }
   template <class U, class... A>
   void construct(U *p, A &&...a) {
