@@ -1930,6 +1930,10 @@ int round_budget(int budget, int64_t segments, int64_t work, int64_t warps) {
   return std::min(budget, work <= warps ? 16 : work <= 4 * warps ? 32 : budget);
 }
 
+// Counter sets of the rounds (32 bytes each), cleared when a pass begins and
+// whenever it has used them all.
+constexpr int kCtrWords = 4, kCtrRounds = 64;
+
 struct TraverseSet {
   void (*plain)(TravArgs), (*front)(TravArgs), (*cont)(TravArgs);
   int ctas;       // CTAs per SM the set is built for
@@ -2210,31 +2214,115 @@ __global__ void __launch_bounds__(256) bh_leaf_chunks(EvalArgs A) {
   }
 }
 
-// Initial batches: the root pair of every slot in `slots`; clears their sums.
-// The root pair of each listed slot as a batch; clears the slot's far,
-// exact and error sums.
-__global__ void root_batches(const int32_t *slots, int64_t n, Batch *out, unsigned long long *acc_lk,
-                             unsigned long long *acc_err, unsigned long long *acc_exact) {
+// What a call counts on the device; the host reads it once per decision.
+struct BhBlock {
+  double counts[8];          // [0] far, [1] segment pairs summed exactly, [2] status (int), [5] exact node pairs,
+                             // [6], [7] frontier pairs kept and opened
+  unsigned long long front;  // frontier records
+  int32_t retry, roots;      // slots the beta retry runs, and of them those that start from the roots
+  int32_t escalate;          // slots whose estimate is still above the limit and whose beta may grow
+  int32_t redo;              // slots that fail the margin check or the limit
+};
+
+// The root pair of each listed slot (null: every slot) as a batch; clears the
+// slot's far, exact and error sums. itol0 > 0: its beta^2 too.
+__global__ void root_batches(const int32_t *slots, int64_t n, double itol0, double *itol, Batch *out,
+                             unsigned long long *acc_lk, unsigned long long *acc_err, unsigned long long *acc_exact) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const int s = slots[k];
+  const int s = slots ? slots[k] : (int)k;
   out[k].slot = s;
   out[k].count = 1;
   out[k].pairs[0] = make_int2(1, 1);
+  if (itol0 > 0) itol[s] = itol0;
   acc_lk[s] = 0;
   acc_err[s] = 0;
   acc_exact[s] = 0;
 }
 
-// Fixed-point sums (far-field + exact) -> per caller pair doubles.
-__global__ void finish_sums(const unsigned long long *acc_lk, const unsigned long long *acc_err,
-                            const unsigned long long *acc_exact, const int32_t *slot_pair, int64_t nslots,
-                            double *lk, double *err) {
+struct FinishArgs {
+  const unsigned long long *acc_lk, *acc_err, *acc_exact;  // per slot, fixed point
+  int64_t n;
+  double *lk, *err;
+  int32_t *flags;
+  double *itol;           // beta^2 per slot
+  const uint8_t *lost;    // frontier not kept (null: no frontier)
+  uint8_t *skip;          // 0: continued from its frontier by the retry
+  int32_t *roots, *redo;  // lists
+  BhBlock *block;
+  double err_scale, target, beta0, beta_limit, err_limit, margin;
+  int32_t escalations;
+};
+__device__ __forceinline__ bool may_escalate(const FinishArgs &A, double err, double beta) {
+  return A.escalations > 0 && !(err <= A.err_limit) && beta < 4.0 * A.beta_limit;
+}
+// Low margin, non-finite, or an error estimate that could reach the rounding
+// boundary: recomputed in FP64 direct sum.
+__device__ __forceinline__ void check_slot(const FinishArgs &A, int64_t s, double lk, double err) {
+  if (!(0.5 - fabs(lk - round(lk)) >= A.margin) || !(err <= A.err_limit))
+    A.redo[atomicAdd(&A.block->redo, 1)] = (int32_t)s;
+}
+
+// Sums and scaled estimates of the first pass, and what each slot needs next:
+// the beta retry (lnc.cpp:165-184), an escalation, a recompute. (The last two
+// stand only if no slot is retried; the host asks again otherwise.)
+__global__ void finish_first(FinishArgs A) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslots) return;
-  const int p = slot_pair[s];
-  lk[p] = (double)(long long)(acc_lk[s] + acc_exact[s]) / kFix;
-  err[p] = (double)(long long)acc_err[s] / kFix;
+  if (s >= A.n) return;
+  const double lk = (double)(long long)(A.acc_lk[s] + A.acc_exact[s]) / kFix;
+  const double e = (double)(long long)A.acc_err[s] / kFix * A.err_scale;
+  A.lk[s] = lk;
+  A.err[s] = e;
+  bool retry = false;
+  // With a positive target, beta* > beta0 needs e > target: below it
+  // (e / target)^(1/4) <= 1, and NaN compares false either way.
+  if (!(A.target > 0) || e > A.target) {
+    const double t = pow(e / A.target, 0.25) * A.beta0, tb = A.beta_limit < t ? A.beta_limit : t;
+    if (tb > A.beta0) {
+      retry = true;
+      A.itol[s] = tb * tb;
+    }
+  }
+  A.flags[s] = retry ? FLN_PAIR_BETA_RETRIED : 0;
+  if (retry) {
+    atomicAdd(&A.block->retry, 1);
+    const bool cont = A.lost && !A.lost[s];
+    if (!cont) A.roots[atomicAdd(&A.block->roots, 1)] = (int32_t)s;
+    if (A.lost) A.skip[s] = cont ? 0 : 1;
+  } else {
+    if (A.lost) A.skip[s] = 1;
+    if (may_escalate(A, e, A.beta0)) atomicAdd(&A.block->escalate, 1);
+    check_slot(A, s, lk, e);
+  }
+}
+
+// Sums and estimates of the slots whose flags have `flag` set (the retried
+// slots) or, with a list, of the listed ones (escalated).
+__global__ void finish_again(FinishArgs A, const int32_t *list, int64_t n, int32_t flag) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int64_t s = list ? list[k] : k;
+  if (!list && !(A.flags[s] & flag)) return;
+  A.lk[s] = (double)(long long)(A.acc_lk[s] + A.acc_exact[s]) / kFix;
+  A.err[s] = (double)(long long)A.acc_err[s] / kFix * A.err_scale;
+}
+
+// Escalation (beyond the reference): a slot whose estimate still exceeds the
+// limit gets twice its beta (at most 4 x beta_limit) and goes on the list.
+__global__ void escalate_slots(FinishArgs A, int32_t *list) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= A.n) return;
+  const double beta = sqrt(A.itol[s]);
+  if (!may_escalate(A, A.err[s], beta)) return;
+  const double nb = fmin(2.0 * beta, 4.0 * A.beta_limit);
+  A.itol[s] = nb * nb;
+  A.flags[s] |= FLN_PAIR_BETA_ESCALATED;
+  list[atomicAdd(&A.block->escalate, 1)] = (int32_t)s;
+}
+
+__global__ void check_slots(FinishArgs A) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < A.n) check_slot(A, s, A.lk[s], A.err[s]);
 }
 
 // ------------------------------------------------------------------ persistent traversal
@@ -2260,7 +2348,6 @@ struct PersistArgs {
   const NodeHdr *hdr;
   const NodeMom *mom;
   const int32_t *slot_loops;   // 2 per slot
-  const int32_t *slot_pair;    // slot -> caller pair
   int32_t nslots;
   double epssq, beta0, beta_limit, target_error, err_scale, err_limit;
   int32_t escalations;
@@ -2335,7 +2422,7 @@ __device__ void finish_pass(PersistArgs &A, int slot, int lane) {
   const double e = (double)(long long)atomicAdd(&A.acc_err[slot], 0ULL) / kFix * A.err_scale;
   const int pass = A.slot_pass[slot];
   const double beta = sqrt(A.slot_itolsq[slot]);
-  const int p = A.slot_pair[slot];
+  const int p = slot;  // slots are the caller's pairs
   const int escalated = pass - ((A.flags[p] & FLN_PAIR_BETA_RETRIED) ? 1 : 0);
   double next = 0.0;
   int flag = 0;
@@ -2670,11 +2757,6 @@ __global__ void sample_exact(const double *xyz, const int64_t *off, const int64_
   }
 }
 
-__global__ void scatter_kernel(const double *src, const int32_t *idx, int64_t n, double *dst) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) dst[idx[k]] = src[k];
-}
-
 // Host kd-median tree (ModifiedKdBVH.h:101-132, :207-237), for bh_tree = 1,
 // by node position (2 n positions, see child_place): children (position of
 // the first child, -1 for a leaf), parent (-1 for the root) and leaf_seg;
@@ -2720,15 +2802,9 @@ void host_kd_tree(const double *xyz, int64_t n, int32_t *children, int32_t *pare
 
 }  // namespace
 
-void scatter_doubles(Context &ctx, const double *src, const int32_t *idx, int64_t n, double *dst) {
-  if (n <= 0) return;
-  scatter_kernel<<<(int)((n + 255) / 256), 256, 0, ctx.stream>>>(src, idx, n, dst);
-  FLN_CUDA(cudaGetLastError());
-}
-
 int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                      const std::vector<int32_t> &h_pairs, const fln_params &prm, double *d_lk_out,
-                      double *d_err_out, int32_t *d_flags_out) {
+                      const std::vector<int32_t> &h_pairs, const int32_t *d_pairs, const fln_params &prm,
+                      double *d_lk_out, double *d_err_out, int32_t *d_flags_out) {
   const int64_t np = (int64_t)h_pairs.size() / 2;
   if (np == 0) return 0;
   const int nl_all = (int)h_off.size() - 1;
@@ -2774,28 +2850,31 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   FLN_CUDA(cudaMemsetAsync(d_arrive, 0, (kd ? nodes : 2 * tot_blk) * sizeof(int32_t), st));
   TreeArgs T{d_xyz, d_off, d_base, d_loops, nloops, d_start, d_bn, d_arrive, d_kd, d_kd ? d_kd + nodes : nullptr,
              d_kd ? d_kd + 2 * nodes : nullptr, d_kd ? d_kd + 3 * nodes : nullptr, d_hdr, d_mom};
-  // Slots: pairs ordered by decreasing estimated work. Host work, done once
-  // the tree build is queued (while the GPU runs it, before the host waits
-  // for its counts).
-  std::vector<int32_t> order(np), slot_loops(2 * np);
-  bool slots_ordered = false;
-  auto order_slots = [&]() {
-    std::iota(order.begin(), order.end(), 0);
-    std::vector<double> cost(np);
-    for (int64_t p = 0; p < np; ++p) {
-      const double a = (double)(h_off[h_pairs[2 * p] + 1] - h_off[h_pairs[2 * p]]);
-      const double b = (double)(h_off[h_pairs[2 * p + 1] + 1] - h_off[h_pairs[2 * p + 1]]);
-      cost[p] = (a + b) * std::log2(a + b + 2.0);
+  // Device times are read at the end of the call, when nothing waits for the
+  // host any more: (start, end, what) of the tree build, of each pass and of
+  // its launches, by event.
+  enum { kTimeTree, kTimeFirst, kTimeRetry, kTimeTraverse, kTimeExact };
+  struct Span {
+    cudaEvent_t a, b;
+    int what;
+  };
+  std::vector<Span> spans;
+  size_t events = 0;
+  auto new_event = [&]() {
+    if (events == ctx.ev_round.size()) {
+      cudaEvent_t e = nullptr;
+      FLN_CUDA(cudaEventCreate(&e));
+      ctx.ev_round.push_back(e);
     }
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-    for (int64_t s = 0; s < np; ++s) {
-      slot_loops[2 * s] = h_pairs[2 * order[s]];
-      slot_loops[2 * s + 1] = h_pairs[2 * order[s] + 1];
-    }
-    slots_ordered = true;
+    return ctx.ev_round[events++];
+  };
+  auto mark = [&](cudaStream_t on) {
+    const cudaEvent_t e = new_event();
+    FLN_CUDA(cudaEventRecord(e, on));
+    return e;
   };
   int launches = 0;
-  FLN_CUDA(cudaEventRecord(ctx.ev2, st));
+  const cudaEvent_t tree0 = mark(st);
   if (prm.bh_tree == 1) {
     // The reference's kd-median tree, built on the host from a copy of the loops.
     wait_xyz_pieces(ctx);
@@ -2839,27 +2918,28 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
       FLN_CUDA(cudaGetLastError());
       k0 = k1;
     }
-    order_slots();
   }
   wait_xyz_pieces(ctx);  // the traversal reads every loop's vertices
-  FLN_CUDA(cudaEventRecord(ctx.ev3, st));
-  ctx.stats.ms_tree_build = ctx.elapsed(ctx.ev2, ctx.ev3);
+  spans.push_back({tree0, mark(st), kTimeTree});
 
-  if (!slots_ordered) order_slots();
-  int32_t *d_slots = ctx.d_bh[11].as<int32_t>(4 * np);
-  int32_t *d_slot_pair = d_slots + 2 * np;
-  int32_t *d_active = d_slots + 3 * np;
+  // Slots are the caller's pairs. (Batches are short, so the order in which
+  // pairs are begun does not matter: see round_budget.)
+  const int32_t *d_slots = d_pairs;
+  int32_t *d_lists = ctx.d_bh[11].as<int32_t>(2 * np);  // slots from the roots (or escalated); slots to recompute
   double *d_itol = ctx.d_bh[12].as<double>(np);
-  double *d_counts = ctx.d_bh[13].as<double>(8);  // far, leaf, retried, escalated, status words
+  BhBlock *d_block = ctx.d_bh[13].as<BhBlock>(1);
+  BhBlock &block = *static_cast<BhBlock *>(ctx.h_head.need(sizeof(BhBlock) + 128));
+  volatile unsigned long long *const h_ctr =  // a round's counters
+      reinterpret_cast<unsigned long long *>(static_cast<char *>(ctx.h_head.ptr) + sizeof(BhBlock));
+  double *d_counts = d_block->counts;
   int32_t *d_status = reinterpret_cast<int32_t *>(d_counts + 2);
   // Per slot, fixed point: far-field sum, error estimate, exact sum.
-  unsigned long long *d_acc = ctx.d_bh[15].as<unsigned long long>(3 * np + 16);
+  unsigned long long *d_acc = ctx.d_bh[15].as<unsigned long long>(3 * np + kCtrWords * kCtrRounds);
   unsigned long long *d_acc_err = d_acc + np;
   unsigned long long *d_acc_exact = d_acc + 2 * np;
-  // [0] queue, [1] next-round count, [2] exact (or far) chunks, [3] leaf chunks, [4] frontier records;
-  // [8, 12) the copy of [0, 4) for the odd rounds of the fused schedule.
+  // Counters of a round: [0] queue, [1] next-round count, [2] exact (or far)
+  // chunks, [3] leaf chunks; a set per round, cleared kCtrRounds at a time.
   unsigned long long *d_ctr = d_acc + 3 * np;
-  unsigned long long *const d_ctrs[2] = {d_ctr, d_ctr + 8};
   const TraverseSet &TS = kTraverseSets[prm.bh_occupancy == 6 ? 1 : prm.bh_occupancy == 7 ? 2 : 0];
   static const bool round_log = std::getenv("FLN_BH_ROUND_LOG") != nullptr;
   // Carveouts and occupancies are set and queried once per context: driver
@@ -2895,10 +2975,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   const int64_t cap = std::max<int64_t>(np, nwarps * ((kStack + kSpill) / 32 + 1));
   Batch *d_batch[2] = {reinterpret_cast<Batch *>(ctx.d_partial.need(2 * cap * sizeof(Batch))), nullptr};
   d_batch[1] = d_batch[0] + cap;
-  FLN_CUDA(cudaMemcpyAsync(d_slots, slot_loops.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  FLN_CUDA(cudaMemcpyAsync(d_slot_pair, order.data(), np * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  FLN_CUDA(cudaMemsetAsync(d_counts, 0, 2 * sizeof(double) + sizeof(int32_t), st));
-  FLN_CUDA(cudaMemsetAsync(d_counts + 5, 0, 3 * sizeof(double), st));  // exact entries, reused, subtracted
+  FLN_CUDA(cudaMemsetAsync(d_block, 0, sizeof(BhBlock), st));
   const double b0 = prm.barnes_hut_init_beta;
   const int budget = prm.bh_budget > 0 ? prm.bh_budget : FLN_BH_BUDGET;
   // Buckets need contiguous segment ranges: curve-order trees only.
@@ -2946,68 +3023,55 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     d_front = reinterpret_cast<FrontRec *>(ctx.d_bh[23].need((size_t)front_cap * sizeof(FrontRec)));
     d_lost = ctx.d_bh[25].as<uint8_t>(2 * np);
     d_skip = d_lost + np;
-    FLN_CUDA(cudaMemsetAsync(d_lost, 0, np, st));
   }
   int64_t front_n = 0;  // records the first pass wrote (<= front_cap)
-  // One Barnes–Hut pass with per-slot beta^2: the root pairs of the slots in
-  // `roots`, then (the retry's continuation) the frontier records of the
-  // slots whose skip byte is 0. `front` records this pass's frontier.
-  auto pass = [&](const std::vector<int32_t> &roots, const std::vector<double> &itol_slots, bool record, bool front,
-                  int64_t nstream) {
+  int passes = 0;
+  // One Barnes–Hut pass with per-slot beta^2: the root pairs of the `na` slots
+  // in d_roots (null: of all slots, at beta0), then (the retry's continuation)
+  // the frontier records of the slots whose skip byte is 0. `front` records
+  // this pass's frontier.
+  auto pass = [&](const int32_t *d_roots, int64_t na, bool record, bool front, int64_t nstream) {
     const bool cont = nstream > 0;  // the retry continued from the frontier
-    const int64_t na = (int64_t)roots.size();
-    FLN_CUDA(cudaMemcpyAsync(d_active, roots.data(), na * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    FLN_CUDA(cudaMemcpyAsync(d_itol, itol_slots.data(), np * sizeof(double), cudaMemcpyHostToDevice, st));
+    const cudaEvent_t pass0 = mark(st);
     if (na > 0) {
-      root_batches<<<(int)((na + 255) / 256), 256, 0, st>>>(d_active, na, d_batch[0], d_acc, d_acc_err, d_acc_exact);
+      root_batches<<<(int)((na + 255) / 256), 256, 0, st>>>(d_roots, na, d_roots ? 0.0 : b0 * b0, d_itol, d_batch[0],
+                                                            d_acc, d_acc_err, d_acc_exact);
       FLN_CUDA(cudaGetLastError());
       ++launches;
     }
-    if (front) FLN_CUDA(cudaMemsetAsync(d_ctr + 4, 0, sizeof(unsigned long long), st));
     int64_t nin = na, pos = 0;
     int cur = 0;
     // Fused rounds: round r's exact-list kernel runs on the exact stream
-    // beside round r + 1's traversal. Round r fills list and counters r & 1;
-    // before it clears them it waits for the exact-list kernel of round r - 2
-    // (which read them). Per round four events: the traversal's end (on st),
-    // the exact-list kernel's start and end (on the exact stream), the
-    // traversal's start (on st).
-    bool pend[2] = {false, false};
+    // beside round r + 1's traversal. Round r fills list r & 1; before that it
+    // waits for the exact-list kernel of round r - 2 (which read it).
     cudaEvent_t done[2] = {nullptr, nullptr};
-    int nev = 0;
-    auto event_at = [&](int x) {
-      while ((int)ctx.ev_round.size() <= x) {
-        cudaEvent_t e = nullptr;
-        FLN_CUDA(cudaEventCreate(&e));
-        ctx.ev_round.push_back(e);
-      }
-      return ctx.ev_round[x];
-    };
     // The context's stream waits for every exact-list launch of the pass
     // (also when the pass throws, so that later work stays ordered).
     auto join = [&]() {
-      if (nev == 0) return;
-      cudaEvent_t e = event_at(4 * nev);
-      FLN_CUDA(cudaEventRecord(e, ctx.exact_stream));
-      FLN_CUDA(cudaStreamWaitEvent(st, e, 0));
+      if (done[0] || done[1]) FLN_CUDA(cudaStreamWaitEvent(st, mark(ctx.exact_stream), 0));
     };
     if (prm.bh_schedule != 2 && !ctx.exact_stream)
       FLN_CUDA(cudaStreamCreateWithFlags(&ctx.exact_stream, cudaStreamNonBlocking));
     try {
       for (int round = 0; (nin > 0 || pos < nstream) && round < 65536; ++round) {
         const int par = round & 1;
-        if (prm.bh_schedule != 2 && pend[par]) FLN_CUDA(cudaStreamWaitEvent(st, done[par], 0));
-        FLN_CUDA(cudaMemsetAsync(prm.bh_schedule == 2 ? d_ctr : d_ctrs[par], 0, 4 * sizeof(unsigned long long), st));
+        if (prm.bh_schedule != 2 && done[par]) FLN_CUDA(cudaStreamWaitEvent(st, done[par], 0));
+        if (round % kCtrRounds == 0) {
+          // (The last exact list still reads its round's set.)
+          if (round > 0 && prm.bh_schedule != 2) FLN_CUDA(cudaStreamWaitEvent(st, done[1 - par], 0));
+          FLN_CUDA(cudaMemsetAsync(d_ctr, 0, kCtrRounds * kCtrWords * sizeof(unsigned long long), st));
+        }
+        unsigned long long *const c = d_ctr + kCtrWords * (round % kCtrRounds);
         if (prm.bh_schedule == 2) {
           // Classify, then evaluate this round's chunks.
           ClassifyArgs C{d_off, d_base, d_hdr, d_slots, d_itol, prm.epssq, d_batch[cur], nin, d_batch[1 - cur], cap,
-                         d_ctr + 1, budget, d_far, d_leaf, d_ctr + 2, d_ctr + 3, chunk_soft, chunk_cap, d_spill,
-                         d_ctr, d_status};
+                         c + 1, budget, d_far, d_leaf, c + 2, c + 3, chunk_soft, chunk_cap, d_spill,
+                         c, d_status};
           const int g = (int)std::max<int64_t>(1, std::min<int64_t>((nin + kWarps - 1) / kWarps, grid_c));
           bh_classify<<<g, 32 * kWarps, 0, st>>>(C);
           FLN_CUDA(cudaGetLastError());
           unsigned long long c4[4];
-          FLN_CUDA(cudaMemcpyAsync(c4, d_ctr, sizeof c4, cudaMemcpyDeviceToHost, st));
+          FLN_CUDA(cudaMemcpyAsync(c4, c, sizeof c4, cudaMemcpyDeviceToHost, st));
           FLN_CUDA(cudaStreamSynchronize(st));
           const int64_t nfar = (int64_t)std::min<unsigned long long>(c4[2], (unsigned long long)chunk_cap);
           const int64_t nleaf = (int64_t)std::min<unsigned long long>(c4[3], (unsigned long long)chunk_cap);
@@ -3035,13 +3099,12 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
           continue;
         }
         if (!d_bkt) throw Error(FLN_ERR_INTERNAL, "Barnes-Hut rounds without an exact list");
-        unsigned long long *const c = d_ctrs[par];
         BucketChunk *const bl = d_bkt + par * bkt_cap;
         TravArgs A{d_xyz, d_off, d_base, d_hdr, d_mom, d_slots, d_itol, prm.epssq, d_batch[cur], nin,
                    d_batch[1 - cur], cap, c + 1, budget, bucket, bl, c + 2, bkt_soft, bkt_cap, d_acc,
                    d_acc_err, d_counts, d_spill, c, d_status,
                    d_front + pos, nstream - pos, d_skip,
-                   front ? d_front : nullptr, d_ctr + 4, front_cap, d_lost, spill_cap,
+                   front ? d_front : nullptr, &d_block->front, front_cap, d_lost, spill_cap,
                    ctx.learned, b0, nullptr, nullptr, 0, 0.f, 0u};
         if (record) {
           A.rec = ctx.recording.rec;
@@ -3054,7 +3117,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         const int64_t work = nin + (nstream - pos);
         A.budget = round_budget(budget, tot_leaf, work, (int64_t)gmax * kWarps);
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>((work + kWarps - 1) / kWarps, gmax));
-        FLN_CUDA(cudaEventRecord(event_at(4 * nev + 3), st));
+        const cudaEvent_t trav0 = mark(st);
         if (A.rec)
           bh_traverse_record<<<g, 32 * kWarps, 0, st>>>(A);
         else if (A.learned.frag)
@@ -3067,22 +3130,21 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         {
           // bh_exact_serial: on the context's stream, after its traversal.
           cudaStream_t xs = prm.bh_exact_serial ? st : ctx.exact_stream;
-          cudaEvent_t et = event_at(4 * nev), e0 = event_at(4 * nev + 1), e1 = event_at(4 * nev + 2);
-          FLN_CUDA(cudaEventRecord(et, st));
+          const cudaEvent_t et = mark(st);
+          spans.push_back({trav0, et, kTimeTraverse});
           FLN_CUDA(cudaStreamWaitEvent(xs, et, 0));
-          FLN_CUDA(cudaEventRecord(e0, xs));
+          const cudaEvent_t e0 = mark(xs);
           bh_buckets<<<ctx.num_sms * 2 * FLN_BUCKET_MIN_CTAS, 32 * kBkWarps, 0, xs>>>(BA);
           FLN_CUDA(cudaGetLastError());
-          FLN_CUDA(cudaEventRecord(e1, xs));
-          done[par] = e1;
-          pend[par] = true;
-          ++nev;
+          done[par] = mark(xs);
+          spans.push_back({e0, done[par], kTimeExact});
         }
         launches += 2;
         ++ctx.stats.bh_rounds;
-        unsigned long long c2[2];
-        FLN_CUDA(cudaMemcpyAsync(c2, c, sizeof c2, cudaMemcpyDeviceToHost, st));
+        FLN_CUDA(cudaMemcpyAsync(const_cast<unsigned long long *>(h_ctr), c, 2 * sizeof(unsigned long long),
+                                 cudaMemcpyDeviceToHost, st));
         FLN_CUDA(cudaStreamSynchronize(st));
+        const unsigned long long c2[2] = {h_ctr[0], h_ctr[1]};
         if (round_log) {  // FLN_BH_ROUND_LOG: cumulative counts after each round, for profiling
           FLN_CUDA(cudaStreamSynchronize(ctx.exact_stream));
           double cnt[8];
@@ -3114,19 +3176,36 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
       throw;
     }
     join();
-    for (int x = 0; x < nev; ++x) {
-      ctx.stats.ms_exact += ctx.elapsed(ctx.ev_round[4 * x + 1], ctx.ev_round[4 * x + 2]);
-      ctx.stats.ms_traverse += ctx.elapsed(ctx.ev_round[4 * x + 3], ctx.ev_round[4 * x]);
-    }
+    spans.push_back({pass0, mark(st), passes++ ? kTimeRetry : kTimeFirst});
     if (nin > 0 || pos < nstream) throw Error(FLN_ERR_INTERNAL, "Barnes-Hut pass did not finish in 65536 rounds");
-    if (front) {
-      unsigned long long nrec = 0;
-      FLN_CUDA(cudaMemcpyAsync(&nrec, d_ctr + 4, sizeof nrec, cudaMemcpyDeviceToHost, st));
-      FLN_CUDA(cudaStreamSynchronize(st));
-      front_n = (int64_t)std::min<unsigned long long>(nrec, (unsigned long long)front_cap);
-      ctx.bh_front_hint = std::max<int64_t>(ctx.bh_front_hint, (int64_t)nrec);
-      ctx.stats.bh_front_records = (int64_t)nrec;
+  };
+  // The call's end: device times, and the FP64 recompute of the listed slots.
+  auto finish_call = [&](int32_t redo) {
+    double ms_of[5] = {0, 0, 0, 0, 0};
+    for (const Span &x : spans) {
+      float ms = 0.f;
+      FLN_CUDA(cudaEventElapsedTime(&ms, x.a, x.b));
+      ms_of[x.what] += ms;
     }
+    ctx.stats.ms_tree_build = ms_of[kTimeTree];
+    ctx.stats.ms_main_kernel += ms_of[kTimeFirst] + ms_of[kTimeRetry];
+    ctx.stats.ms_retry = ms_of[kTimeRetry];
+    ctx.stats.ms_traverse = ms_of[kTimeTraverse];
+    ctx.stats.ms_exact = ms_of[kTimeExact];
+    const double main_ms = ctx.stats.ms_main_kernel;
+    launches += recompute_pairs(ctx, d_xyz, d_off, nl_all, d_pairs, d_lists + np, redo, d_lk_out, d_flags_out);
+    ctx.stats.ms_main_kernel = main_ms;
+    ctx.stats.fp64_recomputed = redo;
+  };
+  int32_t *const d_flags =
+      d_flags_out ? d_flags_out : static_cast<int32_t *>(ctx.d_flags.need(np * sizeof(int32_t)));
+  FinishArgs FA{d_acc, d_acc_err, d_acc_exact, np, d_lk_out, d_err_out, d_flags, d_itol, use_front ? d_lost : nullptr,
+                d_skip, d_lists, d_lists + np, d_block, prm.error_est_scale, prm.target_error, b0,
+                prm.barnes_hut_beta_limit, prm.bh_err_limit, prm.fp64_margin, prm.bh_escalations};
+  const int np_grid = (int)((np + 255) / 256);
+  auto read_block = [&]() {
+    FLN_CUDA(cudaMemcpyAsync(&block, d_block, sizeof block, cudaMemcpyDeviceToHost, st));
+    FLN_CUDA(cudaStreamSynchronize(st));
   };
   // bh_schedule = 1: one persistent launch (retry and escalation on the
   // device). The budgeted rounds below are the default and the fallback when
@@ -3139,7 +3218,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         ctx.d_items.need((size_t)(kRing + kQWords) * sizeof(unsigned long long)));
     unsigned long long *d_q = d_ready + kRing;
     Batch *d_ring = reinterpret_cast<Batch *>(ctx.d_partial.need((size_t)kRing * sizeof(Batch)));
-    int32_t *d_fl = d_flags_out ? d_flags_out : reinterpret_cast<int32_t *>(ctx.d_flags.need(np * sizeof(int32_t)));
+    int32_t *d_fl = d_flags;
     double *d_cnt4 = d_counts;  // [0] far [1] leaf [2] retried [3] escalated [4] status
     d_status = reinterpret_cast<int32_t *>(d_cnt4 + 4);
     std::vector<double> itol0(np, b0 * b0);
@@ -3154,15 +3233,15 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     FLN_CUDA(cudaMemcpyAsync(d_q, q0, sizeof q0, cudaMemcpyHostToDevice, st));
     FLN_CUDA(cudaMemsetAsync(d_fl, 0, np * sizeof(int32_t), st));
     FLN_CUDA(cudaMemsetAsync(d_cnt4, 0, 4 * sizeof(double) + sizeof(int32_t), st));
-    PersistArgs P{d_xyz, d_off, d_base, d_hdr, d_mom, d_slots, d_slot_pair, (int32_t)np, prm.epssq, b0, prm.barnes_hut_beta_limit, prm.target_error, prm.error_est_scale,
+    PersistArgs P{d_xyz, d_off, d_base, d_hdr, d_mom, d_slots, (int32_t)np, prm.epssq, b0, prm.barnes_hut_beta_limit, prm.target_error, prm.error_est_scale,
                   prm.bh_err_limit, prm.bh_escalations, d_sitol, d_pass_arr, d_left, d_acc, d_acc_err, d_ring,
                   d_ready, d_q, d_lk_out, d_err_out, d_fl, d_cnt4, d_spill, d_status, spill_cap,
                   prm.bh_wait_polls > 0 ? (long long)prm.bh_wait_polls : kWaitPolls};
     const int gp = std::min(grid, ctx.num_sms * occupancy_of((const void *)bh_persistent, 32 * kWarps));
-    FLN_CUDA(cudaEventRecord(ctx.ev2, st));
+    const cudaEvent_t run0 = mark(st);
     bh_persistent<<<gp, 32 * kWarps, 0, st>>>(P);
     FLN_CUDA(cudaGetLastError());
-    FLN_CUDA(cudaEventRecord(ctx.ev3, st));
+    spans.push_back({run0, mark(st), kTimeFirst});
     ++launches;
     ctx.stats.bh_rounds = 1;
     double cnt[4];
@@ -3170,7 +3249,6 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     FLN_CUDA(cudaMemcpyAsync(cnt, d_cnt4, sizeof cnt, cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaMemcpyAsync(&pst, d_status, sizeof pst, cudaMemcpyDeviceToHost, st));
     FLN_CUDA(cudaStreamSynchronize(st));
-    ctx.stats.ms_main_kernel += ctx.elapsed(ctx.ev2, ctx.ev3);
     if (pst & 1)
       throw Error(FLN_ERR_STACK_OVERFLOW, "Barnes-Hut traversal stack exceeded its bound (depth " +
                                               std::to_string(maxdepth) + ").");
@@ -3179,6 +3257,11 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
       ctx.stats.bh_leaf_evals = cnt[1];
       ctx.stats.beta_retried = (int64_t)cnt[2];
       ctx.stats.bh_escalated = (int64_t)cnt[3];
+      check_slots<<<np_grid, 256, 0, st>>>(FA);
+      FLN_CUDA(cudaGetLastError());
+      ++launches;
+      read_block();
+      finish_call(block.redo);
       return launches;
     }
     // A bounded wait ran out: redo the stage with budgeted rounds, which
@@ -3186,140 +3269,71 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     ctx.stats.bh_wait_timeouts += 1;
     d_bkt = reinterpret_cast<BucketChunk *>(ctx.d_bh[21].need((size_t)(2 * bkt_cap) * sizeof(BucketChunk)));
     d_status = reinterpret_cast<int32_t *>(d_counts + 2);
-    FLN_CUDA(cudaMemsetAsync(d_counts, 0, 2 * sizeof(double) + sizeof(int32_t), st));
-    FLN_CUDA(cudaMemsetAsync(d_counts + 5, 0, 3 * sizeof(double), st));
+    FLN_CUDA(cudaMemsetAsync(d_block, 0, sizeof(BhBlock), st));
   }
-  std::vector<int32_t> all(np);
-  std::iota(all.begin(), all.end(), 0);
-  std::vector<double> itol(np, b0 * b0);
-  FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-  pass(all, itol, ctx.recording.rec != nullptr, use_front, 0);
-  FLN_CUDA(cudaEventRecord(ctx.ev3, st));
-  finish_sums<<<(int)((np + 255) / 256), 256, 0, st>>>(d_acc, d_acc_err, d_acc_exact, d_slot_pair, np, d_lk_out,
-                                                       d_err_out);
+  if (use_front) FLN_CUDA(cudaMemsetAsync(d_lost, 0, np, st));
+  pass(nullptr, np, ctx.recording.rec != nullptr, use_front, 0);
+  finish_first<<<np_grid, 256, 0, st>>>(FA);
   FLN_CUDA(cudaGetLastError());
   ++launches;
-  // Error estimate and beta retry (lnc.cpp:165-184).
-  std::vector<double> err(np);
-  FLN_CUDA(cudaMemcpyAsync(err.data(), d_err_out, np * sizeof(double), cudaMemcpyDeviceToHost, st));
-  int32_t status = 0;
-  FLN_CUDA(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, st));
-  std::vector<uint8_t> lost;
+  read_block();
+  int32_t status;
+  auto status_of = [&]() { std::memcpy(&status, &block.counts[2], sizeof status); };
+  status_of();
   if (use_front) {
-    lost.resize(np);
-    FLN_CUDA(cudaMemcpyAsync(lost.data(), d_lost, np, cudaMemcpyDeviceToHost, st));
+    front_n = (int64_t)std::min<unsigned long long>(block.front, (unsigned long long)front_cap);
+    ctx.bh_front_hint = std::max<int64_t>(ctx.bh_front_hint, (int64_t)block.front);
+    ctx.stats.bh_front_records = (int64_t)block.front;
   }
-  FLN_CUDA(cudaStreamSynchronize(st));
-  ctx.stats.ms_main_kernel += ctx.elapsed(ctx.ev2, ctx.ev3);
-  std::vector<int32_t> flags(np, 0), retry_slots;
-  std::vector<char> retried(np, 0);
-  for (int64_t s = 0; s < np; ++s) {
-    const int64_t p = order[s];
-    const double e = err[p] * prm.error_est_scale;
-    err[p] = e;
-    // With a positive target, beta* > beta0 needs e > target: below it
-    // (e / target)^(1/4) <= 1 (pow is monotonic and exact at 1), and NaN
-    // compares false either way. The test spares the host most pow calls
-    // while the GPU waits.
-    if (prm.target_error > 0 && !(e > prm.target_error)) continue;
-    const double tb = std::min(std::pow(e / prm.target_error, 0.25) * b0, prm.barnes_hut_beta_limit);
-    if (tb > b0) {
-      retry_slots.push_back((int32_t)s);
-      itol[s] = tb * tb;
-      flags[p] |= FLN_PAIR_BETA_RETRIED;
-      retried[p] = 1;
-    }
-  }
-  ctx.stats.beta_retried = (int64_t)retry_slots.size();
-  std::vector<double> far_leaf(8, 0.0);
-  if (!retry_slots.empty()) {
-    FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-    if (use_front && (status & 1) == 0) {
-      // A node pair opened at beta0 is opened at beta* > beta0 (far at beta*
-      // implies far at beta0), and an exact pair stays exact (the bucket test
-      // does not depend on beta). So the beta* pass is the beta0 pass
-      // continued from its far node pairs: the slot keeps its sums, the
-      // frontier pairs still far keep their values, the ones that open give
-      // theirs back (bh_traverse_cont). Slots whose frontier did not fit start
-      // from the roots.
-      std::vector<uint8_t> skip(np, 1);
-      std::vector<int32_t> cont, from_roots;
-      for (int32_t sl : retry_slots) {
-        if (lost[sl]) {
-          from_roots.push_back(sl);
-        } else {
-          cont.push_back(sl);
-          skip[sl] = 0;
-        }
-      }
-      FLN_CUDA(cudaMemcpyAsync(d_skip, skip.data(), np, cudaMemcpyHostToDevice, st));
-      ctx.stats.bh_retry_from_roots = (int64_t)from_roots.size();
-      pass(from_roots, itol, false, false, cont.empty() ? 0 : front_n);
-    } else {
-      ctx.stats.bh_retry_from_roots = (int64_t)retry_slots.size();
-      pass(retry_slots, itol, false, false, 0);
-    }
-    FLN_CUDA(cudaEventRecord(ctx.ev3, st));
-    finish_sums<<<(int)((np + 255) / 256), 256, 0, st>>>(d_acc, d_acc_err, d_acc_exact, d_slot_pair, np, d_lk_out,
-                                                         d_err_out);
-    FLN_CUDA(cudaGetLastError());
-    ++launches;
-    // The reported estimate is that of the final run, scaled like the first
-    // (the reference stops using it after the retry; the margin check here
-    // needs both on one scale).
-    std::vector<double> e2(np);
-    FLN_CUDA(cudaMemcpyAsync(e2.data(), d_err_out, np * sizeof(double), cudaMemcpyDeviceToHost, st));
-    FLN_CUDA(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, st));
-    FLN_CUDA(cudaStreamSynchronize(st));
-    const double ms = ctx.elapsed(ctx.ev2, ctx.ev3);
-    ctx.stats.ms_main_kernel += ms;
-    ctx.stats.ms_retry += ms;
-    for (int64_t p = 0; p < np; ++p)
-      if (retried[p]) err[p] = e2[p] * prm.error_est_scale;
-  }
-  // Escalation (beyond the reference): a pair whose estimate still exceeds
-  // bh_err_limit is re-run with twice its beta, up to bh_escalations times
-  // (beta <= 4 x beta_limit); what stays above goes to the FP64 direct sum.
+  ctx.stats.beta_retried = block.retry;
   ctx.stats.bh_escalated = 0;
-  for (int esc = 0; esc < prm.bh_escalations; ++esc) {
-    std::vector<int32_t> up;
-    for (int64_t s = 0; s < np; ++s) {
-      const int64_t p = order[s];
-      const double beta = std::sqrt(itol[s]);
-      if (!(err[p] <= prm.bh_err_limit) && beta < 4.0 * prm.barnes_hut_beta_limit) {
-        up.push_back((int32_t)s);
-        const double nb = std::min(2.0 * beta, 4.0 * prm.barnes_hut_beta_limit);
-        itol[s] = nb * nb;
-        flags[p] |= FLN_PAIR_BETA_ESCALATED;
-      }
-    }
-    if (up.empty()) break;
-    ctx.stats.bh_escalated += (int64_t)up.size();
-    FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-    pass(up, itol, false, false, 0);
-    FLN_CUDA(cudaEventRecord(ctx.ev3, st));
-    finish_sums<<<(int)((np + 255) / 256), 256, 0, st>>>(d_acc, d_acc_err, d_acc_exact, d_slot_pair, np, d_lk_out,
-                                                         d_err_out);
+  const bool again = block.retry > 0 || block.escalate > 0;
+  if (block.retry > 0) {
+    // A node pair opened at beta0 is opened at beta* > beta0 (far at beta*
+    // implies far at beta0), and an exact pair stays exact (the bucket test
+    // does not depend on beta). So the beta* pass is the beta0 pass continued
+    // from its far node pairs: the slot keeps its sums, the frontier pairs
+    // still far keep their values, the ones that open give theirs back
+    // (bh_traverse_cont). Slots whose frontier did not fit start from the
+    // roots. The reported estimate is that of the final run, scaled like the
+    // first (the reference stops using it after the retry; the margin check
+    // here needs both on one scale).
+    ctx.stats.bh_retry_from_roots = block.roots;
+    pass(d_lists, block.roots, false, false, block.retry > block.roots ? front_n : 0);
+    finish_again<<<np_grid, 256, 0, st>>>(FA, nullptr, np, FLN_PAIR_BETA_RETRIED);
     FLN_CUDA(cudaGetLastError());
     ++launches;
-    std::vector<double> e3(np);
-    FLN_CUDA(cudaMemcpyAsync(e3.data(), d_err_out, np * sizeof(double), cudaMemcpyDeviceToHost, st));
-    FLN_CUDA(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, st));
-    FLN_CUDA(cudaStreamSynchronize(st));
-    const double ms = ctx.elapsed(ctx.ev2, ctx.ev3);
-    ctx.stats.ms_main_kernel += ms;
-    ctx.stats.ms_retry += ms;
-    for (int32_t s : up) err[order[s]] = e3[order[s]] * prm.error_est_scale;
   }
-  FLN_CUDA(cudaMemcpyAsync(far_leaf.data(), d_counts, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  FLN_CUDA(cudaMemcpyAsync(d_err_out, err.data(), np * sizeof(double), cudaMemcpyHostToDevice, st));
-  if (d_flags_out) FLN_CUDA(cudaMemcpyAsync(d_flags_out, flags.data(), np * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  FLN_CUDA(cudaStreamSynchronize(st));
-  ctx.stats.bh_far_evals = far_leaf[0];
-  ctx.stats.bh_leaf_evals = far_leaf[1];
-  ctx.stats.bh_exact_entries = prm.bh_schedule == 0 ? far_leaf[5] : far_leaf[1];
-  ctx.stats.bh_far_reused = far_leaf[6];
-  ctx.stats.bh_far_subtracted = far_leaf[7];
+  // Escalation: a pair whose estimate still exceeds bh_err_limit is re-run
+  // with twice its beta, up to bh_escalations times; what stays above goes to
+  // the FP64 direct sum.
+  for (int esc = 0; again && esc < prm.bh_escalations; ++esc) {
+    FLN_CUDA(cudaMemsetAsync(&d_block->escalate, 0, sizeof(int32_t), st));
+    escalate_slots<<<np_grid, 256, 0, st>>>(FA, d_lists);
+    FLN_CUDA(cudaGetLastError());
+    ++launches;
+    read_block();
+    if (block.escalate == 0) break;
+    ctx.stats.bh_escalated += block.escalate;
+    const int32_t up = block.escalate;
+    pass(d_lists, up, false, false, 0);
+    finish_again<<<(up + 255) / 256, 256, 0, st>>>(FA, d_lists, up, 0);
+    FLN_CUDA(cudaGetLastError());
+    ++launches;
+  }
+  if (again) {
+    FLN_CUDA(cudaMemsetAsync(&d_block->redo, 0, sizeof(int32_t), st));
+    check_slots<<<np_grid, 256, 0, st>>>(FA);
+    FLN_CUDA(cudaGetLastError());
+    ++launches;
+    read_block();
+    status_of();
+  }
+  ctx.stats.bh_far_evals = block.counts[0];
+  ctx.stats.bh_leaf_evals = block.counts[1];
+  ctx.stats.bh_exact_entries = prm.bh_schedule == 0 ? block.counts[5] : block.counts[1];
+  ctx.stats.bh_far_reused = block.counts[6];
+  ctx.stats.bh_far_subtracted = block.counts[7];
   if (status & 1)
     throw Error(FLN_ERR_STACK_OVERFLOW, "Barnes-Hut traversal stack exceeded its bound (depth " +
                                             std::to_string(maxdepth) + ").");
@@ -3328,6 +3342,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   if (status != 0)
     throw Error(FLN_ERR_INTERNAL, "Barnes-Hut work list exceeded its capacity (status " + std::to_string(status) +
                                       ").");
+  finish_call(block.redo);
   return launches;
 }
 
@@ -3343,11 +3358,30 @@ void learned_collect(Context &ctx, const double *d_xyz, const int64_t *d_off, co
   const int64_t np = (int64_t)h_pairs.size() / 2;
   if (np == 0 || cap <= 0) return;
   cudaStream_t st = ctx.stream;
+  // The pairs by decreasing estimated work: the sample's hash takes a pair's
+  // place in this order.
+  std::vector<int32_t> order(np), sorted(2 * np);
+  std::iota(order.begin(), order.end(), 0);
+  std::vector<double> cost(np);
+  for (int64_t p = 0; p < np; ++p) {
+    const double a = (double)(h_off[h_pairs[2 * p] + 1] - h_off[h_pairs[2 * p]]);
+    const double b = (double)(h_off[h_pairs[2 * p + 1] + 1] - h_off[h_pairs[2 * p + 1]]);
+    cost[p] = (a + b) * std::log2(a + b + 2.0);
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  for (int64_t k = 0; k < np; ++k) {
+    sorted[2 * k] = h_pairs[2 * order[k]];
+    sorted[2 * k + 1] = h_pairs[2 * order[k] + 1];
+  }
+  int32_t *d_slots = ctx.d_learn[7].as<int32_t>(2 * np);
+  FLN_CUDA(cudaMemcpyAsync(d_slots, sorted.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, st));
   int4 *d_rec = ctx.d_learn[0].as<int4>(cap);
   unsigned long long *d_cnt = ctx.d_learn[1].as<unsigned long long>(1);
   fln_params p = prm;
   p.bh_tree = 0;
   p.bh_schedule = 0;
+  p.fp64_margin = -1.0;  // the sums are not used: recompute none
+  p.bh_err_limit = HUGE_VAL;
   double *d_lk = ctx.d_learn[2].as<double>(2 * np);
   const LearnedCfg saved = ctx.learned;
   unsigned long long cnt = 0;
@@ -3363,7 +3397,7 @@ void learned_collect(Context &ctx, const double *d_xyz, const int64_t *d_off, co
     ctx.recording.s_min = s_min;
     ctx.recording.keep = (uint32_t)std::min(4294967295.0, std::max(0.0, keep) * 4294967296.0);
     try {
-      barnes_hut_device(ctx, d_xyz, d_off, h_off, h_pairs, p, d_lk, d_lk + np, nullptr);
+      barnes_hut_device(ctx, d_xyz, d_off, h_off, sorted, d_slots, p, d_lk, d_lk + np, nullptr);
     } catch (...) {
       ctx.learned = saved;
       ctx.recording = Recording{};
@@ -3383,7 +3417,6 @@ void learned_collect(Context &ctx, const double *d_xyz, const int64_t *d_off, co
   const int64_t *d_base = static_cast<const int64_t *>(ctx.d_bh[1].ptr);
   const NodeHdr *d_hdr = static_cast<const NodeHdr *>(ctx.d_bh[9].ptr);
   const NodeMom *d_mom = static_cast<const NodeMom *>(ctx.d_bh[10].ptr);
-  const int32_t *d_slots = static_cast<const int32_t *>(ctx.d_bh[11].ptr);
   float *d_X = ctx.d_learn[3].as<float>(kMlpIn * n);
   double *d_approx = ctx.d_learn[4].as<double>(n);
   float *d_T = ctx.d_learn[5].as<float>(3 * n);

@@ -151,9 +151,6 @@ void copy_d2h(Context &ctx, cudaStream_t stream, void *h_dst, const void *d_src,
   }
 }
 
-// Scatters src[k] into dst[idx[k]] for the FP64 recompute (defined in bh.cu).
-void scatter_doubles(Context &ctx, const double *src, const int32_t *idx, int64_t n, double *dst);
-
 static void clear_stats(Context &ctx) {
   ctx.stats.ms_main_kernel = 0;
   ctx.stats.ms_tree_build = 0;
@@ -189,53 +186,20 @@ static int run_direct(Context &ctx, const double *d_xyz, const int64_t *d_off, i
   return r.launches;
 }
 
-// Barnes–Hut over device-resident loops and pairs, then the margin check and
-// FP64 direct-sum recompute of the pairs that fail it.
+// Barnes–Hut over device-resident loops and pairs, with the margin check and
+// FP64 direct-sum recompute of the pairs that fail it. d_pairs may be null.
 static int run_barnes_hut(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                          const std::vector<int32_t> &h_pairs, const fln_params &prm, double *d_lk, double *d_err,
-                          int32_t *d_flags) {
+                          const std::vector<int32_t> &h_pairs, const int32_t *d_pairs, const fln_params &prm,
+                          double *d_lk, double *d_err, int32_t *d_flags) {
   const int64_t np = (int64_t)h_pairs.size() / 2;
   clear_stats(ctx);
   if (!d_err) d_err = ctx.d_err.as<double>(std::max<int64_t>(np, 1));
-  int launches = barnes_hut_device(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags);
-  if (np > 0) {
-    std::vector<double> lk(np), err(np, 0.0);
-    FLN_CUDA(cudaMemcpyAsync(lk.data(), d_lk, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-    FLN_CUDA(cudaMemcpyAsync(err.data(), d_err, np * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-    FLN_CUDA(cudaStreamSynchronize(ctx.stream));
-    std::vector<int32_t> redo_idx, redo_pairs;
-    for (int64_t p = 0; p < np; ++p) {
-      const double r = std::round(lk[p]);
-      const double margin = 0.5 - std::fabs(lk[p] - r);
-      // Low margin, non-finite, or an error estimate that could reach the
-      // rounding boundary: recompute in FP64 direct sum.
-      if (!(margin >= prm.fp64_margin) || !(err[p] <= prm.bh_err_limit)) {
-        redo_idx.push_back((int32_t)p);
-        redo_pairs.push_back(h_pairs[2 * p]);
-        redo_pairs.push_back(h_pairs[2 * p + 1]);
-      }
-    }
-    if (!redo_idx.empty()) {
-      const int64_t nr = (int64_t)redo_idx.size();
-      double *d_tmp = ctx.d_redo.as<double>(nr + nr / 2 + 2 + nr);
-      int32_t *d_idx = reinterpret_cast<int32_t *>(d_tmp + nr), *d_pr = d_idx + nr + (nr & 1);
-      FLN_CUDA(cudaMemcpyAsync(d_pr, redo_pairs.data(), 2 * nr * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
-      launches += direct_sum_device(ctx, d_xyz, d_off, (int32_t)h_off.size() - 1, d_pr, nr, FLN_PREC_FP64, 0.0, -1.0,
-                                    d_tmp, nullptr, nullptr)
-                      .launches;
-      FLN_CUDA(cudaMemcpyAsync(d_idx, redo_idx.data(), nr * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
-      scatter_doubles(ctx, d_tmp, d_idx, nr, d_lk);
-      ++launches;
-      if (d_flags) {
-        std::vector<int32_t> fl(np, 0);
-        FLN_CUDA(cudaMemcpyAsync(fl.data(), d_flags, np * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx.stream));
-        FLN_CUDA(cudaStreamSynchronize(ctx.stream));
-        for (int32_t p : redo_idx) fl[p] |= FLN_PAIR_FP64_RECOMPUTED;
-        FLN_CUDA(cudaMemcpyAsync(d_flags, fl.data(), np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
-      }
-      ctx.stats.fp64_recomputed = nr;
-    }
+  if (!d_pairs && np > 0) {
+    int32_t *d = ctx.d_pairs.as<int32_t>(2 * np);
+    FLN_CUDA(cudaMemcpyAsync(d, h_pairs.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
+    d_pairs = d;
   }
+  const int launches = barnes_hut_device(ctx, d_xyz, d_off, h_off, h_pairs, d_pairs, prm, d_lk, d_err, d_flags);
   double sp = 0;
   for (int64_t p = 0; p < np; ++p)
     sp += (double)(h_off[h_pairs[2 * p] + 1] - h_off[h_pairs[2 * p]]) *
@@ -400,7 +364,7 @@ void compute_pairs_resident(Context &ctx, const double *d_xyz, const int64_t *d_
   ctx.xyz_pieces = 0;
   int launches;
   if (method == FLN_METHOD_BARNESHUT) {
-    launches = run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags);
+    launches = run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, nullptr, prm, d_lk, d_err, d_flags);
   } else {
     int32_t *d_pairs = ctx.d_pairs.as<int32_t>(2 * np);
     FLN_CUDA(cudaMemcpyAsync(d_pairs, h_pairs.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, ctx.stream));
@@ -476,7 +440,7 @@ void compute_pairs_host(Context &ctx, const double *xyz, const int64_t *loop_off
   if (npairs == 1) tail.known_work = (double)(h_off[h_pairs[0] + 1] - h_off[h_pairs[0]]) *
                                      (double)(h_off[h_pairs[1] + 1] - h_off[h_pairs[1]]);
   try {
-    launches = bh ? run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, prm, d_lk, d_err, d_flags)
+    launches = bh ? run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, d_pairs, prm, d_lk, d_err, d_flags)
                   : run_direct(ctx, d_xyz, d_off, nloops, d_pairs, npairs, prm, d_lk, d_err, d_flags, &tail, &complete);
   } catch (...) {
     wait_xyz_pieces(ctx);
@@ -703,7 +667,8 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz, const i
       check_inputs(h_off, nloops, h_pairs);
       launches = method == FLN_METHOD_DIRECTSUM
                      ? run_direct(c, d_xyz, d_loop_offsets, nloops, d_pairs, 0, prm, d_lk_out, d_err_out, d_flags_out)
-                     : run_barnes_hut(c, d_xyz, d_loop_offsets, h_off, h_pairs, prm, d_lk_out, d_err_out, d_flags_out);
+                     : run_barnes_hut(c, d_xyz, d_loop_offsets, h_off, h_pairs, d_pairs, prm, d_lk_out, d_err_out,
+                                      d_flags_out);
     }
     if (!complete) {
       FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
@@ -1014,11 +979,13 @@ fln_status fln_autotune(fln_ctx *ctx, const double *xyz, const int64_t *loop_off
     const int64_t np = (int64_t)h_pairs.size() / 2;
     double *d_lk = c.d_lk.as<double>(np), *d_err = c.d_err.as<double>(np);
     int32_t *d_fl = c.d_flags.as<int32_t>(np);
+    int32_t *d_pr = c.d_pairs.as<int32_t>(2 * np);
+    FLN_CUDA(cudaMemcpyAsync(d_pr, h_pairs.data(), 2 * np * sizeof(int32_t), cudaMemcpyHostToDevice, c.stream));
     auto time_of = [&](const fln_params &p) {
       double best = 1e300;
       for (int rep = 0; rep < 3; ++rep) {
         FLN_CUDA(cudaEventRecord(c.ev0, c.stream));
-        run_barnes_hut(c, d_xyz, d_off, h_off, h_pairs, p, d_lk, d_err, d_fl);
+        run_barnes_hut(c, d_xyz, d_off, h_off, h_pairs, d_pr, p, d_lk, d_err, d_fl);
         FLN_CUDA(cudaEventRecord(c.ev1, c.stream));
         best = std::min(best, (double)c.elapsed(c.ev0, c.ev1));
       }

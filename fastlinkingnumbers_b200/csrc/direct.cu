@@ -1091,6 +1091,23 @@ void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t m
 
 }  // namespace
 
+int recompute_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops, const int32_t *d_pairs,
+                    const int32_t *d_list, int64_t n, double *d_lk, int32_t *d_flags) {
+  if (n <= 0) return 0;
+  // The list first: the direct sum uses the buffers it may lie in.
+  int32_t *list = ctx.d_redo.as<int32_t>(3 * n + (n & 1) + 2 * n), *pairs = list + n;
+  double *sums = reinterpret_cast<double *>(list + 3 * n + (n & 1));
+  const int grid = (int)((n + 255) / 256);
+  FLN_CUDA(cudaMemcpyAsync(list, d_list, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, ctx.stream));
+  gather_pairs<<<grid, 256, 0, ctx.stream>>>(list, n, d_pairs, pairs);
+  FLN_CUDA(cudaGetLastError());
+  const int launches =
+      direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, n, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr, nullptr).launches;
+  scatter_redo<<<grid, 256, 0, ctx.stream>>>(list, n, sums, d_lk, d_flags);
+  FLN_CUDA(cudaGetLastError());
+  return launches + 2;
+}
+
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
                                const int32_t *d_pairs, int64_t np, int precision, double near_factor, double margin,
                                double *d_lk, double *d_err, int32_t *d_flags, int tile_shape, const DirectTail *tail) {
@@ -1157,21 +1174,8 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   R.work = head.work;
   R.redone = (int64_t)head.redo;
   R.complete = tail && R.redone == 0;
-  if (R.redone > 0) {
-    const int64_t nr = R.redone;
-    int32_t *list = ctx.d_redo.as<int32_t>(3 * nr + (nr & 1) + 2 * nr);  // list, pairs, sums
-    FLN_CUDA(cudaMemcpyAsync(list, d_redo, nr * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    int32_t *pairs = list + nr;
-    double *sums = reinterpret_cast<double *>(list + 3 * nr + (nr & 1));
-    const int grid = (int)((nr + 255) / 256);
-    gather_pairs<<<grid, 256, 0, st>>>(list, nr, d_pairs, pairs);
-    FLN_CUDA(cudaGetLastError());
-    R.launches += 2 + direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, nr, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr,
-                                        nullptr)
-                      .launches;
-    scatter_redo<<<grid, 256, 0, st>>>(list, nr, sums, d_lk, d_flags);
-    FLN_CUDA(cudaGetLastError());
-  }
+  if (R.redone > 0)
+    R.launches += recompute_pairs(ctx, d_xyz, d_off, nloops, d_pairs, d_redo, R.redone, d_lk, d_flags);
   return R;
 }
 

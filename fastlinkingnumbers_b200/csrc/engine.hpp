@@ -216,11 +216,19 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
                                double margin, double *d_lk, double *d_err, int32_t *d_flags, int tile_shape = 0,
                                const DirectTail *tail = nullptr);
 
+// FP64 direct sums of the n pairs in d_list (indices into d_pairs), written
+// back to d_lk; d_flags (may be null) gets FLN_PAIR_FP64_RECOMPUTED there.
+int recompute_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops, const int32_t *d_pairs,
+                    const int32_t *d_list, int64_t n, double *d_lk, int32_t *d_flags);
+
 // Barnes–Hut over the same inputs; err per pair after ERROR_EST_SCALE and the
-// reference's beta retry; flags gets FLN_PAIR_BETA_RETRIED. Returns launches.
+// reference's beta retry; flags (may be null) gets FLN_PAIR_BETA_RETRIED and
+// FLN_PAIR_BETA_ESCALATED. Pairs that fail the margin check (prm.fp64_margin)
+// or whose estimate stays above prm.bh_err_limit are recomputed in FP64 direct
+// sum. d_pairs: the pairs on the device. Returns launches.
 int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, const std::vector<int64_t> &h_off,
-                      const std::vector<int32_t> &h_pairs, const fln_params &prm, double *d_lk_out,
-                      double *d_err_out, int32_t *d_flags_out);
+                      const std::vector<int32_t> &h_pairs, const int32_t *d_pairs, const fln_params &prm,
+                      double *d_lk_out, double *d_err_out, int32_t *d_flags_out);
 
 // Runs the Barnes–Hut stage (curve-order trees, beta0, learned criterion off)
 // while sampling node pairs with separation in [s_min, 1.25 beta0] (opened
