@@ -749,13 +749,17 @@ struct Batch {
 // from them instead of from the roots. Beside each pair, its separation
 // ratio (|dr|^2 + eps^2 - eps^2) / (r1 + r2)^2 in FP32 (front_ratio): a pair
 // whose ratio clears the retry's beta^2 by a margin far above the FP32
-// rounding is far at that beta without loading its headers.
+// rounding is far at that beta without loading its headers. And its value and
+// error estimate: a pair the retry opens gives them back without being
+// evaluated again.
 constexpr int kFrontPairs = 128;
-struct FrontRec {
+struct __align__(32) FrontRec {
   int32_t slot;
   int32_t count;
+  int32_t pad[6];            // every array starts on a 32-byte sector
   int2 pairs[kFrontPairs];
   float ratio[kFrontPairs];
+  double2 value[kFrontPairs];
 };
 // The ratio in FP32 from the FP64 quantities of the far test: three roundings
 // (two conversions, one __fdividef of at most 2 ulp), so it lies within
@@ -1055,7 +1059,7 @@ __device__ __noinline__ void shift_down(int2 *stack, int k, int n, int lane) {
   }
 }
 
-// Appends n (<= 32) far node pairs and their separation ratios (front_ratio),
+// Appends n (<= 32) far node pairs, their separation ratios (front_ratio) and values,
 // one per lane (lanes < n), to the warp's
 // open frontier record of `slot`, reserving records as they fill. The open
 // record is (fr, ffill); fr < 0 means none. A record is closed (its header
@@ -1070,7 +1074,7 @@ __device__ __forceinline__ void front_close(const TravArgs &A, int &fr, int &ffi
   ffill = 0;
 }
 __device__ __forceinline__ void front_put(const TravArgs &A, int &fr, int &ffill, int slot, int2 q, float ratio,
-                                          int n, int lane) {
+                                          double2 value, int n, int lane) {
   const int need = (fr < 0 ? 1 : 0) + (ffill + n > kFrontPairs ? 1 : 0);
   int c = 0;  // record index (clamped: past the capacity only "lost" matters)
   if (lane == 0 && need)
@@ -1083,6 +1087,7 @@ __device__ __forceinline__ void front_put(const TravArgs &A, int &fr, int &ffill
     const int at = pos < kFrontPairs ? pos : pos - kFrontPairs;
     A.front[dst].pairs[at] = q;
     A.front[dst].ratio[at] = ratio;
+    A.front[dst].value[at] = value;
   }
   if (lane == 0 && (cur >= A.front_cap || (ffill + n > kFrontPairs && nxt >= A.front_cap))) A.front_lost[slot] = 1;
   if (ffill + n >= kFrontPairs) {
@@ -1112,12 +1117,12 @@ __device__ __forceinline__ void front_put(const TravArgs &A, int &fr, int &ffill
 // sums of the slot. A node pair's far-field value and estimate do not depend
 // on beta, so a frontier pair that is still far at the slot's beta is left
 // alone: its value is already in the sums. Most such pairs are recognised at
-// intake from the ratio recorded with them (front_clear); the rest go on the
-// stack marked by bit 31 of their first node id and take the full test. A frontier pair that is opened now has its first-pass value and
-// estimate subtracted (queued with a negative squared separation, evaluated
-// at the one far-field call site, so the value is the one the first pass
-// added) and is then exact or split like any pair.
-constexpr int kFrontFlag = int(0x80000000u);
+// intake from the ratio recorded with them (front_clear). The rest give back
+// there what the first pass added, which is recorded with them, and go on the
+// stack like any pair; one in the narrow band that is far after all adds the
+// same value again. (Evaluating the opened pairs a second time to give them
+// back was a fifth of all far-field evaluations of 171 walks of 30,000 steps:
+// 117.4 ms per call, 110.7 with the recorded values.)
 // Sum of a per-lane 32-bit count over the warp, in FP64 (no overflow).
 __device__ __forceinline__ double warp_sum_u32(unsigned v) {
   unsigned long long s = v;
@@ -1129,7 +1134,7 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
   constexpr bool kFront = kMode == 1, kCont = kMode == 2;
   __shared__ int2 s_stack[kWarps][kStack];
   __shared__ int2 s_far[kWarps][64];
-  __shared__ float4 s_farv[kWarps][64];  // separation (x, y, z) and its square (negative: subtract), per queued far pair
+  __shared__ float4 s_farv[kWarps][64];  // separation (x, y, z) and its square, per queued far pair
   __shared__ float2 s_farr[kWarps][64];  // the two Eq. 14 weights (far_weights)
   __shared__ float s_fart[kWarps][kFront ? 64 : 1];  // separation ratios for the frontier (front_ratio)
   __shared__ std::conditional_t<kLearn, MlpFrag, int> s_mlp;
@@ -1235,26 +1240,28 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
     // Threshold of the learned criterion: tau x (beta0 / beta)^4 in later passes.
     const float log10_tau = A.learned.log10_tau + 2.f * (float)log10(A.beta0 * A.beta0 / itolsq);
     int top = cnt0;
+    double sum = 0.0, err = 0.0;
     if (kCont && from_front) {
       // Frontier pairs still clearly far at this slot's beta keep their
-      // first-pass value and need no classification; the others go on the
-      // stack, marked, for the full test.
+      // first-pass value; the others give it back and take the full test.
       const float clear = front_clear(itolsq);
-      const float *ratio = A.in1[b - A.nin].ratio;
+      const FrontRec &r = A.in1[b - A.nin];
       top = 0;
       for (int x0 = 0; x0 < cnt0; x0 += 32) {
         const int x = x0 + lane;
-        int2 v = make_int2(0, 0);
-        bool keep = false;
-        if (x < cnt0) {
-          v = src[x];
-          keep = !(ratio[x] > clear);
+        const bool open = x < cnt0 && !(r.ratio[x] > clear);
+        const unsigned om = __ballot_sync(0xffffffffu, open);
+        if (lane == 0) {
+          s_fcount[w][0] += (unsigned)(min(cnt0 - x0, 32) - __popc(om));
+          s_fcount[w][1] += (unsigned)__popc(om);
         }
-        const unsigned km = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) s_fcount[w][0] += (unsigned)(min(cnt0 - x0, 32) - __popc(km));
-        v.x |= kFrontFlag;
-        if (keep) stack[top + __popc(km & ((1u << lane) - 1))] = v;
-        top += __popc(km);
+        if (open) {
+          const double2 v = r.value[x];
+          sum -= v.x;
+          err -= v.y;
+          stack[top + __popc(om & ((1u << lane) - 1))] = src[x];
+        }
+        top += __popc(om);
       }
     } else {
       for (int x = lane; x < cnt0; x += 32) stack[x] = src[x];
@@ -1263,7 +1270,6 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
     int bc = -1;  // open chunk of the exact list
     int bfill = 0;      // entries in it
     bool overflow = false;
-    double sum = 0.0, err = 0.0;
     __syncwarp();
     for (bool done = false; !done;) {
       if (top == 0 && nspill > 0) {  // refill from the spill buffer
@@ -1312,11 +1318,6 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
         if (act) pr = stack[top - cnt + lane];
         __syncwarp();
         top -= cnt;
-        bool fpair = false;  // a frontier pair of the continued retry
-        if constexpr (kCont) {
-          fpair = pr.x < 0;
-          pr.x &= ~kFrontFlag;
-        }
         int kind = 0;  // 0 none, 1 exact (leaf pair or bucket), 2 far, 3 split
         int4 ex = make_int4(0, 0, 1, 1);
         int2 c0 = make_int2(0, 0), c1 = make_int2(0, 0);
@@ -1392,26 +1393,6 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
             if (cand && y < log10_tau) kind = 2;
           }
         }
-        // Continued retry: a frontier pair still far keeps its first-pass
-        // value; one that opens gives it back (subtract) and goes on.
-        bool sub = false;
-        if constexpr (kCont) {
-          bool kept = false;
-          if (fpair) {
-            if (kind == 2) {
-              kind = 0;
-              kept = true;
-            } else {
-              sub = true;
-              fv.w = -fv.w;
-            }
-          }
-          const unsigned km = __ballot_sync(0xffffffffu, kept), um = __ballot_sync(0xffffffffu, sub);
-          if (lane == 0) {
-            s_fcount[w][0] += (unsigned)__popc(km);
-            s_fcount[w][1] += (unsigned)__popc(um);
-          }
-        }
         const unsigned sm = __ballot_sync(0xffffffffu, kind == 3);
         const int ns = __popc(sm);
         if (top + 2 * ns > kStack) {  // spill the oldest half
@@ -1435,9 +1416,9 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
             stack[top + 2 * rank + 1] = c1;
           }
           top += 2 * ns;
-          const unsigned fm = __ballot_sync(0xffffffffu, kind == 2 || sub);
+          const unsigned fm = __ballot_sync(0xffffffffu, kind == 2);
           const unsigned lm = __ballot_sync(0xffffffffu, kind == 1);
-          if (kind == 2 || sub) {
+          if (kind == 2) {
             const int at = nf + __popc(fm & ((1u << lane) - 1));
             farq[at] = pr;
             farv[at] = fv;
@@ -1445,7 +1426,7 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
             if constexpr (kFront) fart[at] = fratio;
           }
 #if FLN_BH_PREFETCH & 2
-          if (kind == 2 || sub) {
+          if (kind == 2) {
             prefetch_record(M1 + pr.x);
             prefetch_record(M2 + pr.y);
           }
@@ -1481,23 +1462,12 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
         }
       }
       // Far-field evaluation, 32 queued pairs at a time, and what is left
-      // once the batch is done: the one far-field call site of the kernel
-      // (a subtraction then gives back exactly what the first pass added).
+      // once the batch is done.
       const int drain = staged ? kStagePairs : 32;
       while (nf >= drain || (done && nf > 0)) {
         const int m = min(nf, drain);
         int2 q = make_int2(0, 0);
         if (lane < m) q = farq[nf - m + lane];
-        if constexpr (kFront) {
-          int frec = s_fstate[w][0], ffill = s_fstate[w][1];
-          __syncwarp();
-          front_put(A, frec, ffill, slot, q, lane < m ? fart[nf - m + lane] : 0.f, m, lane);
-          if (lane == 0) {
-            s_fstate[w][0] = frec;
-            s_fstate[w][1] = ffill;
-          }
-          __syncwarp();
-        }
         if (staged) {
           if (lane == 0) mbar_expect(mbar, (uint32_t)(m * 2 * sizeof(NodeMom)));
           __syncwarp();
@@ -1513,23 +1483,28 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
           }
           mphase ^= 1u;
         }
+        double fs = 0.0, fe = 0.0;
         if (lane < m) {
           const float4 v = farv[nf - m + lane];
           const float2 rr = farr[nf - m + lane];  // Eq. 14 weights
-          double fs = 0.0, fe = 0.0;
           if (staged)
-            far_eval(stage_read(stage, lane), stage_read(stage, kStagePairs + lane), v.x, v.y, v.z,
-                     (double)fabsf(v.w), rr.x, rr.y, fs, fe);
+            far_eval(stage_read(stage, lane), stage_read(stage, kStagePairs + lane), v.x, v.y, v.z, (double)v.w, rr.x,
+                     rr.y, fs, fe);
           else
-            far_eval(load_mom(M1 + q.x), load_mom(M2 + q.y), v.x, v.y, v.z, (double)fabsf(v.w), rr.x, rr.y, fs, fe);
-          if (v.w < 0.f) {
-            sum -= fs;
-            err -= fe;
-          } else {
-            sum += fs;
-            err += fe;
-            nfar += 1;
+            far_eval(load_mom(M1 + q.x), load_mom(M2 + q.y), v.x, v.y, v.z, (double)v.w, rr.x, rr.y, fs, fe);
+          sum += fs;
+          err += fe;
+          nfar += 1;
+        }
+        if constexpr (kFront) {
+          int frec = s_fstate[w][0], ffill = s_fstate[w][1];
+          __syncwarp();
+          front_put(A, frec, ffill, slot, q, lane < m ? fart[nf - m + lane] : 0.f, make_double2(fs, fe), m, lane);
+          if (lane == 0) {
+            s_fstate[w][0] = frec;
+            s_fstate[w][1] = ffill;
           }
+          __syncwarp();
         }
         nf -= m;
         __syncwarp();
@@ -3015,7 +2990,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     if (want_hint == 0 || want_hint > have) {  // the buffer must grow: ask how much memory is free
       size_t free_b = 0, total_b = 0;
       FLN_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      want = want_hint > 0 ? want_hint : std::min<size_t>((size_t)16 << 30, free_b / 5) / sizeof(FrontRec);
+      want = want_hint > 0 ? want_hint : std::min<size_t>((size_t)32 << 30, free_b / 3) / sizeof(FrontRec);
       want = std::max(want, have);
       if (want > have && (want - have) * sizeof(FrontRec) > free_b / 2) want = have + free_b / 2 / sizeof(FrontRec);
     }
