@@ -279,14 +279,17 @@ __device__ void accumulate_child(BuildNode &P, const BuildNode &C) {
     }
 }
 
-__device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg,
-                                   int32_t kids) {
+__device__ __forceinline__ double box_rsq(const BuildNode &B) {
   const double dx = B.hi[0] - B.lo[0], dy = B.hi[1] - B.lo[1], dz = B.hi[2] - B.lo[2];
+  return 0.25 * (dx * dx + dy * dy + dz * dz);
+}
+__device__ void finish_record_regs(const BuildNode &B, double rsq, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg,
+                                   int32_t kids) {
   H.m[0] = B.mid[0];
   H.m[1] = B.mid[1];
   H.m[2] = B.mid[2];
-  H.rsq = 0.25 * (dx * dx + dy * dy + dz * dz);
-  H.r = sqrt(H.rsq);
+  H.rsq = rsq;
+  H.r = sqrt(rsq);
   H.left = leaf ? -1 - seg : kids;
   H.lo = B.seg_lo;
   H.cnt = B.seg_cnt;
@@ -308,10 +311,10 @@ __device__ void finish_record_regs(const BuildNode &B, NodeHdr &H, NodeMom &M, b
 
 // Traversal records of a node, formed in registers and stored as vectors.
 __device__ __forceinline__ void finish_record(const BuildNode &B, NodeHdr &H, NodeMom &M, bool leaf, int32_t seg,
-                                              int32_t kids) {
+                                              int32_t kids, double rsq) {
   NodeHdr h;
   NodeMom m;
-  finish_record_regs(B, h, m, leaf, seg, kids);
+  finish_record_regs(B, rsq, h, m, leaf, seg, kids);
   put32(&H, h);
   put32(&M, m);
 }
@@ -356,7 +359,7 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
     const int32_t seg = A.leaf_seg[base + node];
     BuildNode B;
     leaf_build(A.xyz, o, n, seg, B);
-    finish_record(B, A.hdr[base + node], A.mom[base + node], true, seg, 0);
+    finish_record(B, A.hdr[base + node], A.mom[base + node], true, seg, 0, box_rsq(B));
   }
   for (int guard = 0; guard < 128; ++guard) {
     const int32_t par = A.parent[base + node];
@@ -383,7 +386,7 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
     P.seg_lo = L.seg_lo;
     P.seg_cnt = L.seg_cnt + R.seg_cnt;
     A.bn[base + par] = P;
-    finish_record(P, A.hdr[base + par], A.mom[base + par], false, 0, kids);
+    finish_record(P, A.hdr[base + par], A.mom[base + par], false, 0, kids, box_rsq(P));
     node = par;
   }
 }
@@ -409,8 +412,8 @@ __global__ void build_moments(TreeArgs A, const int64_t *seg_start2, int64_t tot
 // depend on who arrives last. FP64 throughout; records are rounded to FP32 at
 // the end.
 //
-// What bounds it: 384 B of records are written per segment; measured 4.0 ms for
-// 28M segments of mixed sizes (2.7 TB/s of records) and 2.4 ms for 14.1M,
+// What bounds it: 384 B of records are written per segment; measured 3.89 ms for
+// 28M segments of mixed sizes (2.7 TB/s of records) and 2.34 ms for 14.1M,
 // against 8.6 and 4.66 ms for the build it replaces (topology, leaf,
 // height-bucket, small-node and one launch per height), which read each vertex
 // about 30 times through scattered 8-byte loads and wrote 16-byte pieces. It
@@ -612,6 +615,18 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
           P.mid[a] = 0.5 * (P.hi[a] + P.lo[a]);
           P.t[a] = 0.0;
         }
+        // The box is done with before the sums start: 128 registers hold the
+        // rest with 16 bytes of spills a thread instead of 56 (3.89 ms, 4.01
+        // with the box kept to the end; three CTAs of 168 registers 4.25).
+        const double rsq = box_rsq(P);
+        double *rec = s_rec + (d < 0 ? 2 * x : x) * kRecD;
+        const bool keep = d < 0 || (d == 0 && !(over && parent_is_summed(x)));
+        if (keep)
+          for (int a = 0; a < 3; ++a) {
+            rec[kRLo + a] = P.lo[a];
+            rec[kRHi + a] = P.hi[a];
+            rec[kRMid + a] = P.mid[a];
+          }
         for (int a = 0; a < 9; ++a) P.D[a] = 0.0;
         for (int a = 0; a < 18; ++a) P.Q[a] = 0.0;
         const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
@@ -631,15 +646,9 @@ __global__ void __launch_bounds__(kBuildThreads, 4) build_curve_trees(TreeArgs A
         }
         P.seg_lo = v.lo;
         P.seg_cnt = cnt;
-        finish_record(P, hdr[v.pos], mom[v.pos], false, 0, child_place(v.lo, v.lefts));
-        if (d < 0 || (d == 0 && !(over && parent_is_summed(x)))) {
-          double *rec = s_rec + (d < 0 ? 2 * x : x) * kRecD;
-          for (int a = 0; a < 3; ++a) {
-            rec[kRLo + a] = P.lo[a];
-            rec[kRHi + a] = P.hi[a];
-            rec[kRMid + a] = P.mid[a];
-            rec[kRT + a] = P.t[a];
-          }
+        finish_record(P, hdr[v.pos], mom[v.pos], false, 0, child_place(v.lo, v.lefts), rsq);
+        if (keep) {
+          for (int a = 0; a < 3; ++a) rec[kRT + a] = P.t[a];
           for (int a = 0; a < 9; ++a) rec[kRD + a] = P.D[a];
           for (int a = 0; a < 18; ++a) rec[kRQ + a] = P.Q[a];
         }
