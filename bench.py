@@ -407,8 +407,8 @@ def run_ours(args, rank, world, local_rank):
                          "schedule": ["rounds, fused evaluation", "persistent queue", "rounds, split evaluation"][args.bh_schedule],
                          "exact_bucket_segments": 1 if (args.bh_tree == 1 or args.bh_schedule != 0)
                          else (prm.bh_bucket or 8),
-                         "round_budget": prm.bh_budget or 256,
-                         "traversal_ctas_per_sm": prm.bh_occupancy or 5},
+                         "round_budget": prm.bh_budget or 128,
+                         "traversal_ctas_per_sm": prm.bh_occupancy or 6},
         "certificate_ms": ms,
         "autotune": tune,
         "e2e": {"value": world * units / (e2e_ms * 1e-3) / 1e9, "unit": UNIT, "ms_per_step": e2e_ms,

@@ -73,7 +73,7 @@ constexpr int kWarps = 4;          // warps per traversal CTA
 #ifndef FLN_BH_CARVEOUT
 #define FLN_BH_CARVEOUT 44
 #endif
-// Six and seven CTAs per SM (fln_params.bh_occupancy).
+// The same for six (the default) and seven CTAs per SM.
 #ifndef FLN_BH_CARVEOUT_6
 #define FLN_BH_CARVEOUT_6 58
 #endif
@@ -1877,8 +1877,11 @@ __global__ void __launch_bounds__(32 * kBkWarps, FLN_BUCKET_MIN_CTAS) bh_buckets
 }
 
 // The traversal kernels at N CTAs per SM (fln_params.bh_occupancy): 5 (96
-// registers), 6 (80) or 7 (72, with some spills). The traversal is bound by
-// dependent loads, so more resident warps can pay for the spills. (Without a
+// registers), 6 (80, the default) or 7 (72, more spills). The traversal is
+// bound by the latency of dependent loads: neither half the header loads nor
+// a seventh fewer instructions made it faster, more resident warps do. 171
+// walks of 30,000 steps at 5 / 6 / 7: 110.6 / 109.4 / 117 ms per call, mixed
+// sizes 17.9 / 17.6 / 18.2, 60 walks of 2,000 steps 1.195 / 1.18. (Without a
 // minimum CTA count ptxas assumes one and took up to 138 registers.)
 //   bh_traverse_oN        plain
 //   bh_traverse_front_oN  the first pass, which records its frontier
@@ -2924,7 +2927,7 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   // Counters of a round: [0] queue, [1] next-round count, [2] exact (or far)
   // chunks, [3] leaf chunks; a set per round, cleared kCtrRounds at a time.
   unsigned long long *d_ctr = d_acc + 3 * np;
-  const TraverseSet &TS = kTraverseSets[prm.bh_occupancy == 6 ? 1 : prm.bh_occupancy == 7 ? 2 : 0];
+  const TraverseSet &TS = kTraverseSets[(prm.bh_occupancy > 0 ? prm.bh_occupancy : kDefaultBhCtas) - 5];
   static const bool round_log = std::getenv("FLN_BH_ROUND_LOG") != nullptr;
   // Carveouts and occupancies are set and queried once per context: driver
   // queries on every call cost host time while the GPU waits.

@@ -957,7 +957,7 @@ fln_status fln_autotune_direct(fln_ctx *ctx, const double *xyz, const int64_t *l
     r.best_budget = best.bh_budget > 0 ? best.bh_budget : kDefaultBhBudget;
     r.best_beta = best.barnes_hut_init_beta;
     r.best_bucket = best.bh_bucket > 0 ? best.bh_bucket : 8;
-    r.best_occupancy = best.bh_occupancy > 0 ? best.bh_occupancy : 5;
+    r.best_occupancy = best.bh_occupancy > 0 ? best.bh_occupancy : kDefaultBhCtas;
     *out = best;
     if (result) *result = r;
   });
@@ -1027,7 +1027,8 @@ fln_status fln_autotune(fln_ctx *ctx, const double *xyz, const int64_t *loop_off
       try_budgets(base);  // the caller's own beta
     {  // traversal occupancy at the best setting (the same node pairs)
       const fln_params around = best;
-      for (int occ : {6, 7}) {
+      for (int occ : {5, 6, 7}) {
+        if (occ == (around.bh_occupancy > 0 ? around.bh_occupancy : kDefaultBhCtas)) continue;
         fln_params p = around;
         p.bh_occupancy = occ;
         const double ms = time_of(p);
@@ -1057,7 +1058,7 @@ fln_status fln_autotune(fln_ctx *ctx, const double *xyz, const int64_t *loop_off
     r.best_budget = best.bh_budget;
     r.best_beta = best.barnes_hut_init_beta;
     r.best_bucket = best.bh_bucket > 0 ? best.bh_bucket : 8;
-    r.best_occupancy = best.bh_occupancy > 0 ? best.bh_occupancy : 5;
+    r.best_occupancy = best.bh_occupancy > 0 ? best.bh_occupancy : kDefaultBhCtas;
     *out = best;
     if (result) *result = r;
   });

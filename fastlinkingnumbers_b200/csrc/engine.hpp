@@ -185,6 +185,7 @@ constexpr double kDefaultNearFactor = 4.0;
 // launch) when fln_params.bh_budget is 0: on the polymer step with the exact
 // list, 128 ran the traversal in 48.0 ms against 49.6 ms at 256.
 constexpr int kDefaultBhBudget = 128;
+constexpr int kDefaultBhCtas = 6;  // fln_params.bh_occupancy 0
 
 // Plans (on the device) and runs the direct sum over `npairs` pairs of the
 // loops in device memory; everything but the returned counts stays there.
