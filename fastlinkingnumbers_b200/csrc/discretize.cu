@@ -45,12 +45,20 @@ namespace {
 
 constexpr int kDWarps = 4;
 constexpr int kDStack = 256;  // shared stack entries per warp
-constexpr int kBudget = 256;  // steps per batch and launch
+// Steps per batch and launch. A step is one dependent load after another
+// (1.1 us), so a launch with few batches takes its budget's length whatever
+// they hold, and one curve pair's overlaps stay on one warp: with at most four
+// batches per warp the stacks are handed on after 32 steps. 100 walks of 20,011
+// points, 22 rounds: 30 launches of up to 577 us, 5.67 ms in all, with
+// 256 steps throughout; 63 launches, 2.13 ms by this rule.
+constexpr int kBudget = 256, kShortBudget = 32;
 
-struct DNode {
+struct __align__(32) DNode {
   double lo[3], hi[3];
   int32_t a, b;  // range [a, b) of the curve's live pieces
+  int64_t pad;   // 64 B: two 32-byte loads (load_node)
 };
+static_assert(sizeof(DNode) == 64, "DNode layout");
 
 struct DBatch {
   int32_t slot;
@@ -232,6 +240,7 @@ struct DTravArgs {
   uint8_t *hit;
   unsigned long long *overlaps;
   int32_t *status;
+  int32_t budget;  // steps per batch
 };
 
 // Writes entries [0, n) of stack as batches of slot `slot` to the next
@@ -276,6 +285,19 @@ __device__ __noinline__ void shift_down_d(int2 *stack, int k, int n, int lane) {
   }
 }
 
+// A node by the two loads that hold all of it, issued together. (Six
+// comparisons in turn, each loading what it needs, made a step 2.1 us.)
+__device__ __forceinline__ DNode load_node(const DNode *p) {
+  DNode n;
+  unsigned long long *w = reinterpret_cast<unsigned long long *>(&n);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(w[4 * h]), "=l"(w[4 * h + 1]), "=l"(w[4 * h + 2]), "=l"(w[4 * h + 3])
+        : "l"(reinterpret_cast<const char *>(p) + 32 * h));
+  return n;
+}
+
 __global__ void __launch_bounds__(32 * kDWarps) disc_traverse(DTravArgs A) {
   __shared__ int2 s_stack[kDWarps][kDStack];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -296,7 +318,7 @@ __global__ void __launch_bounds__(32 * kDWarps) disc_traverse(DTravArgs A) {
     int top = cnt0;
     __syncwarp();
     for (int steps = 0; top > 0; ++steps) {
-      if (steps >= kBudget) {  // hand the rest on
+      if (steps >= A.budget) {  // hand the rest on
         hand_on(A, slot, stack, top, lane);
         top = 0;
         __syncwarp();
@@ -311,9 +333,9 @@ __global__ void __launch_bounds__(32 * kDWarps) disc_traverse(DTravArgs A) {
       bool split = false;
       int2 c0 = make_int2(0, 0), c1 = make_int2(0, 0);
       if (act) {
-        const DNode &X = NI[pr.x], &Y = NJ[pr.y];
-        const bool meet = X.lo[0] <= Y.hi[0] && X.lo[1] <= Y.hi[1] && X.lo[2] <= Y.hi[2] && Y.lo[0] <= X.hi[0] &&
-                          Y.lo[1] <= X.hi[1] && Y.lo[2] <= X.hi[2];
+        const DNode X = load_node(NI + pr.x), Y = load_node(NJ + pr.y);
+        const bool meet = (X.lo[0] <= Y.hi[0]) & (X.lo[1] <= Y.hi[1]) & (X.lo[2] <= Y.hi[2]) & (Y.lo[0] <= X.hi[0]) &
+                          (Y.lo[1] <= X.hi[1]) & (Y.lo[2] <= X.hi[2]);
         if (meet) {
           const int32_t sx = X.b - X.a, sy = Y.b - Y.a;
           if (sx == 1 && sy == 1) {
@@ -782,8 +804,8 @@ DiscretizedOnDevice discretize_device(Context &ctx, const std::vector<CurveData>
       }
     const int64_t nslots = (int64_t)sc.size() / 2;
     uint8_t *d_hit = buf<uint8_t>(B[28], n);
-    unsigned long long *d_ctr = buf<unsigned long long>(B[29], 4);  // overlaps, queue, next count
-    int32_t *d_status = buf<int32_t>(B[30], 1);
+    unsigned long long *d_ctr = buf<unsigned long long>(B[29], 4);  // overlaps, queue, next count, status
+    int32_t *d_status = reinterpret_cast<int32_t *>(d_ctr + 3);
     overlaps = 0;
     FLN_CUDA(cudaMemsetAsync(d_hit, 0, (size_t)std::max<int64_t>(n, 1), st));
     if (nslots > 0) {
@@ -796,7 +818,6 @@ DiscretizedOnDevice discretize_device(Context &ctx, const std::vector<CurveData>
         DBatch *bin = d_b, *bout = d_b + out_cap;
         FLN_CUDA(cudaMemsetAsync(d_hit, 0, (size_t)std::max<int64_t>(n, 1), st));
         FLN_CUDA(cudaMemsetAsync(d_ctr, 0, 4 * sizeof(unsigned long long), st));
-        FLN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int32_t), st));
         root_batches_d<<<(int)((nslots + 255) / 256), 256, 0, st>>>(d_sc, nslots, d_loff, bin);
         FLN_CUDA(cudaGetLastError());
         int64_t nin = nslots;
@@ -804,16 +825,17 @@ DiscretizedOnDevice discretize_device(Context &ctx, const std::vector<CurveData>
         for (int r = 0; nin > 0 && r < 1000000; ++r) {
           FLN_CUDA(cudaMemsetAsync(d_ctr + 1, 0, 2 * sizeof(unsigned long long), st));
           DTravArgs A{d_nodes, d_loff, static_cast<const int32_t *>(B[18].ptr), d_sc, bin, nin, bout, out_cap,
-                      d_ctr + 2, d_ctr + 1, d_hit, d_ctr, d_status};
+                      d_ctr + 2, d_ctr + 1, d_hit, d_ctr, d_status,
+                      nin <= 4 * nwarps ? kShortBudget : kBudget};
           const int g = (int)std::max<int64_t>(1, std::min<int64_t>((nin + kDWarps - 1) / kDWarps, grid));
           disc_traverse<<<g, 32 * kDWarps, 0, st>>>(A);
           FLN_CUDA(cudaGetLastError());
-          unsigned long long next = 0;
-          FLN_CUDA(cudaMemcpyAsync(&next, d_ctr + 2, sizeof next, cudaMemcpyDeviceToHost, st));
-          FLN_CUDA(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, st));
+          unsigned long long next[2] = {0, 0};
+          FLN_CUDA(cudaMemcpyAsync(next, d_ctr + 2, sizeof next, cudaMemcpyDeviceToHost, st));
           FLN_CUDA(cudaStreamSynchronize(st));
+          status = (int32_t)next[1];
           if (status) break;
-          nin = (int64_t)next;
+          nin = (int64_t)next[0];
           std::swap(bin, bout);
         }
         if (!status) break;
