@@ -157,64 +157,6 @@ __device__ __forceinline__ NodeMom load_mom(const NodeMom *p) {
   return m;
 }
 
-// Moment records of far pairs staged in shared memory by bulk copies (1) or
-// loaded by the lanes (0). A scattered 32-byte load costs the L1 data pipe
-// one wavefront per lane, and the moment records are about half of the
-// traversal's loads; a bulk copy of a record (cp.async.bulk, 128 bytes,
-// completion counted on an mbarrier) is done by the copy engine instead, and
-// the lanes then read the staged records from shared memory at 128 bytes per
-// wavefront. Slots are 144 bytes apart (16-byte aligned, as bulk copies
-// require), so chunk k of slot s sits in bank group (s + k) mod 8 and 8 lanes
-// reading the same chunk of 8 consecutive slots do not conflict.
-#ifndef FLN_BH_TMA_MOM
-#define FLN_BH_TMA_MOM 0
-#endif
-constexpr int kStagePairs = 16;            // far pairs per staged drain
-constexpr int kSlotF4 = 9;                 // slot stride in float4 (144 bytes)
-constexpr int kStageWaitPolls = 1 << 20;   // bounded wait on the staging barrier
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// Waits for the barrier's phase of the given parity; false if it did not
-// complete within kStageWaitPolls tries.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-  const uint32_t a = smem_u32(bar);
-  for (int i = 0; i < kStageWaitPolls; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-// One 128-byte moment record into a shared-memory slot (both 16-byte aligned).
-__device__ __forceinline__ void bulk_record(void *dst, const NodeMom *src, uint64_t *bar) {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"((uint32_t)sizeof(NodeMom)), "r"(smem_u32(bar))
-               : "memory");
-}
-// The record staged in slot s.
-__device__ __forceinline__ NodeMom stage_read(const float4 *stage, int s) {
-  NodeMom m;
-  float4 *d = reinterpret_cast<float4 *>(&m);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) d[k] = stage[kSlotF4 * s + k];
-  return m;
-}
-
-
 struct TreeArgs {
   const double *xyz;
   const int64_t *off;        // loop vertex offsets
@@ -1033,24 +975,15 @@ __device__ __forceinline__ void load3(const double *xyz, int64_t v, double *p) {
 #ifndef FLN_BH_BUDGET
 #define FLN_BH_BUDGET kDefaultBhBudget
 #endif
-// Software prefetch of node records (generic addresses; the records are
-// valid device memory). Bit 0: the next step's headers into L1; bit 1: the
-// moment records of queued far-field and leaf pairs into L1. Same step:
-// none 207.4 ms, bit 1 206.5 ms, bit 0 211.7 ms, both 212.2 ms.
 // Node pairs (neither far nor split further) of at most this many segments
 // a side are summed exactly, segment pair by segment pair.
 #ifndef FLN_BH_BUCKET
 #define FLN_BH_BUCKET 8
 #endif
-#ifndef FLN_BH_PREFETCH
-#define FLN_BH_PREFETCH 2
-#endif
-__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.L1 [%0];" ::"l"(p)); }
-template <class T>
-__device__ __forceinline__ void prefetch_record(const T *p) {
-  prefetch_l1(p);
-  if constexpr (sizeof(T) > 128) prefetch_l1(reinterpret_cast<const char *>(p) + sizeof(T) - 1);
-}
+// The moment record of a queued far pair, into L1 before the drain loads it
+// (206.5 ms against 207.4 without; the next step's headers too: 212.2; an
+// earlier form of the polymer step).
+__device__ __forceinline__ void prefetch_record(const NodeMom *p) { asm volatile("prefetch.L1 [%0];" ::"l"(p)); }
 
 // stack[0, n) = stack[k, k + n), warp-wide, in passes of 32 that read before
 // they write: the lanes of a warp need not run the passes in step
@@ -1130,7 +1063,7 @@ __device__ __forceinline__ void front_put(const TravArgs &A, int &fr, int &ffill
 // there what the first pass added, which is recorded with them, and go on the
 // stack like any pair; one in the narrow band that is far after all adds the
 // same value again. (Evaluating the opened pairs a second time to give them
-// back was a fifth of all far-field evaluations of 171 walks of 30,000 steps:
+// back was a fifth of all far-field evaluations of 200 walks of 50,000 steps:
 // 117.4 ms per call, 110.7 with the recorded values.)
 // Sum of a per-lane 32-bit count over the warp, in FP64 (no overflow).
 __device__ __forceinline__ double warp_sum_u32(unsigned v) {
@@ -1147,21 +1080,8 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
   __shared__ float2 s_farr[kWarps][64];  // the two Eq. 14 weights (far_weights)
   __shared__ float s_fart[kWarps][kFront ? 64 : 1];  // separation ratios for the frontier (front_ratio)
   __shared__ std::conditional_t<kLearn, MlpFrag, int> s_mlp;
-  // Staged moment records (FLN_BH_TMA_MOM): node 1's in slots [0, 16), node
-  // 2's in [16, 32), one barrier per warp.
-  __shared__ __align__(128) float4 s_stage[kWarps][FLN_BH_TMA_MOM ? 2 * kStagePairs * kSlotF4 : 1];
-  __shared__ __align__(8) uint64_t s_mbar[kWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int gw = blockIdx.x * kWarps + w;
-  float4 *stage = s_stage[w];
-  uint64_t *mbar = &s_mbar[w];
-  uint32_t mphase = 0;
-  const bool staged = FLN_BH_TMA_MOM != 0;
-  bool sfail = false;  // a staging wait ran out (status 16)
-  if (staged) {
-    if (lane == 0) mbar_init(mbar, 1);
-    __syncwarp();
-  }
   int2 *stack = s_stack[w];
   int2 *farq = s_far[w];
   float4 *farv = s_farv[w];
@@ -1201,7 +1121,6 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
   }
   const long long total = A.nin + A.nin1;
   for (;;) {
-    if (sfail) break;
     long long b = 0;
     if (lane == 0) {
       // Past the soft limit of the exact list this round takes no new batch
@@ -1434,12 +1353,10 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
             farr[at] = fr;
             if constexpr (kFront) fart[at] = fratio;
           }
-#if FLN_BH_PREFETCH & 2
           if (kind == 2) {
             prefetch_record(M1 + pr.x);
             prefetch_record(M2 + pr.y);
           }
-#endif
           nf += __popc(fm);
           if (lm) {  // append the exact pairs to the list, 32 entries per chunk
             const int ne = __popc(lm), pos = bfill + __popc(lm & ((1u << lane) - 1));
@@ -1472,35 +1389,15 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
       }
       // Far-field evaluation, 32 queued pairs at a time, and what is left
       // once the batch is done.
-      const int drain = staged ? kStagePairs : 32;
-      while (nf >= drain || (done && nf > 0)) {
-        const int m = min(nf, drain);
+      while (nf >= 32 || (done && nf > 0)) {
+        const int m = min(nf, 32);
         int2 q = make_int2(0, 0);
         if (lane < m) q = farq[nf - m + lane];
-        if (staged) {
-          if (lane == 0) mbar_expect(mbar, (uint32_t)(m * 2 * sizeof(NodeMom)));
-          __syncwarp();
-          if (lane < m) {
-            bulk_record(stage + kSlotF4 * lane, M1 + q.x, mbar);
-            bulk_record(stage + kSlotF4 * (kStagePairs + lane), M2 + q.y, mbar);
-          }
-          if (!__all_sync(0xffffffffu, mbar_wait(mbar, mphase))) {
-            sfail = true;
-            if (lane == 0) atomicOr(A.status, 16);
-            done = true;
-            break;
-          }
-          mphase ^= 1u;
-        }
         double fs = 0.0, fe = 0.0;
         if (lane < m) {
           const float4 v = farv[nf - m + lane];
           const float2 rr = farr[nf - m + lane];  // Eq. 14 weights
-          if (staged)
-            far_eval(stage_read(stage, lane), stage_read(stage, kStagePairs + lane), v.x, v.y, v.z, (double)v.w, rr.x,
-                     rr.y, fs, fe);
-          else
-            far_eval(load_mom(M1 + q.x), load_mom(M2 + q.y), v.x, v.y, v.z, (double)v.w, rr.x, rr.y, fs, fe);
+          far_eval(load_mom(M1 + q.x), load_mom(M2 + q.y), v.x, v.y, v.z, (double)v.w, rr.x, rr.y, fs, fe);
           sum += fs;
           err += fe;
           nfar += 1;
@@ -1539,9 +1436,6 @@ __device__ __forceinline__ void traverse(const TravArgs &A) {
     __syncwarp();
     front_close(A, frec, ffill, fslot, lane);
   }
-  // A staging wait that ran out leaves copies in flight: give them another
-  // bounded wait before the CTA's shared memory is released.
-  if (sfail) mbar_wait(mbar, mphase);
   const double wfar = warp_sum_u32(nfar);
   if (lane == 0) {
     atomicAdd(A.counts, wfar);
@@ -1879,8 +1773,8 @@ __global__ void __launch_bounds__(32 * kBkWarps, FLN_BUCKET_MIN_CTAS) bh_buckets
 // The traversal kernels at N CTAs per SM (fln_params.bh_occupancy): 5 (96
 // registers), 6 (80, the default) or 7 (72, more spills). The traversal is
 // bound by the latency of dependent loads: neither half the header loads nor
-// a seventh fewer instructions made it faster, more resident warps do. 171
-// walks of 30,000 steps at 5 / 6 / 7: 110.6 / 109.4 / 117 ms per call, mixed
+// a seventh fewer instructions made it faster, more resident warps do. 200
+// walks of 50,000 steps at 5 / 6 / 7: 110.6 / 109.4 / 117 ms per call, mixed
 // sizes 17.9 / 17.6 / 18.2, 60 walks of 2,000 steps 1.195 / 1.18. (Without a
 // minimum CTA count ptxas assumes one and took up to 138 registers.)
 //   bh_traverse_oN        plain
@@ -3324,8 +3218,6 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   if (status & 1)
     throw Error(FLN_ERR_STACK_OVERFLOW, "Barnes-Hut traversal stack exceeded its bound (depth " +
                                             std::to_string(maxdepth) + ").");
-  if (status & 16)
-    throw Error(FLN_ERR_INTERNAL, "Barnes-Hut moment staging did not complete within its bounded wait.");
   if (status != 0)
     throw Error(FLN_ERR_INTERNAL, "Barnes-Hut work list exceeded its capacity (status " + std::to_string(status) +
                                       ").");

@@ -214,7 +214,7 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz,
  * framework owns the device's memory pool, latency-critical loops that must
  * not take allocator locks, or paths where an allocation failure cannot be
  * handled. Every array is the caller's device memory; the only other memory
- * used is one fixed device array inside libfln.so (about 9.3 MB per GPU,
+ * used is one fixed device array inside libfln.so (about 8.9 MB per GPU,
  * held until the process exits). Limits: npairs <= 65536 and at most 2^20
  * work items (one item = 128 segments of the longer loop of a pair, summed
  * over pairs); larger calls return FLN_ERR_INVALID_ARGUMENT. precision is
