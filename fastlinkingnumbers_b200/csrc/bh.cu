@@ -4,37 +4,37 @@
 // segments. Default ("curve-order"): node = contiguous segment range
 // [lo, hi), split at lo + (hi - lo) / 2; a polyline is continuous, so these
 // ranges are spatially compact and the tree needs no sort. Its topology is
-// implicit: the internal node splitting at s has local id s - 1, found by a
-// root-to-node descent per node. Optionally the reference's kd-median tree
+// implicit: a node's range and place follow from its path. Optionally the reference's kd-median tree
 // (ModifiedKdBVH.h:207-237) is built on the host and uploaded (bh_tree = 1).
 // Storage: the two children of a node lie side by side, at an even position
-// of the loop's record arrays (node_place), so that the headers of a pair of
+// of the loop's record arrays (child_place), so that the headers of a pair of
 // siblings share one 128-byte line; the root is at position 1, and position 0
 // is unused. A node's id in the traversal is its position.
 //
 // Moments (compute_link.h:95-114, compute_link.cpp:333-389) are built in
-// FP64 bottom-up: each leaf thread walks to the root; at every parent the
-// second arriving child computes the parent (box union, centre, the Eq. 21-23
-// shift of monopole c_M, dipole C_D, quadrupole C_Q) and continues. They are
+// FP64 bottom-up: every parent gets the box union, the centre and the Eq.
+// 21-23 shift of monopole c_M, dipole C_D and quadrupole C_Q of its children,
+// block by block in shared memory (build_curve_trees). They are
 // then stored for traversal in FP32 relative to the node centre; the centre
 // itself stays FP64 so node separations are formed in FP64. Each C_Q[k] is
 // symmetric in its last two indices (leaf c_k c c^T / 12; the shift adds
 // c_k r r^T + (r D_k) + (r D_k)^T), so 6 of its 9 entries are stored.
 //
-// Traversal (compute_link.cpp:547-666, :695-841). One warp per loop pair,
-// pairs taken from a device queue. The warp keeps a LIFO of node pairs in
+// Traversal (compute_link.cpp:547-666, :695-841). One warp per batch of node
+// pairs of a loop pair, batches taken from a device queue. The warp keeps a LIFO of node pairs in
 // shared memory (spilling its oldest half to a global buffer when full) and
 // classifies up to 32 pairs per step, one per lane:
-//   leaf-leaf        -> exact one-arctan term (compute_link.cpp:576-606);
+//   leaf-leaf, or few segments a side
+//                    -> exact terms (compute_link.cpp:576-606), in a kernel of
+//                       their own (bh_buckets);
 //   far (|dr|^2 + eps^2 > (r1 + r2)^2 beta^2 + eps^2)
 //                    -> monopole + dipole + quadrupole (Eq. 29-30) and the
 //                       Eq. 14 error estimate (compute_link.cpp:411-524);
 //   otherwise        -> push the two children of the larger node (the
 //                       internal one if the other is a leaf).
-// Far and leaf pairs go to two per-warp queues and are evaluated 32 at a
-// time, so the expensive branches run with full warps. Leaf-leaf pairs
-// closer than one segment length are evaluated in FP64 from the vertices.
-// Sums are FP64 per lane, reduced per pair in a fixed order.
+// Far pairs go to a per-warp queue and are evaluated 32 at a time, so the
+// expensive branch runs with full warps. Sums are FP64 per lane and batch,
+// added per loop pair in fixed point, so their order does not matter.
 #include <cuda/atomic>
 #include <cuda_runtime.h>
 
@@ -58,11 +58,10 @@ constexpr double kInvTwoPi = 0.15915494309189533576888376337251436;
 constexpr double kInvFourPi = 0.079577471545947667884441881686257181;
 constexpr double kInvRt3 = 0.57735026918962576450914878050195746;
 constexpr int kWarps = 4;          // warps per traversal CTA
-// Shared-memory stack entries per warp (> 128). 224 keeps a traversal CTA at
-// 11 KB of shared memory, so five CTAs fit a 64 KB carveout and leave the
-// rest of the SM's 256 KB to L1, which holds the node records the warps
-// re-read: 182.9 ms against 188.8 ms with 512 entries (14M-segment polymer
-// step, B200).
+// Shared-memory stack entries per warp (> 128). Few, because the rest of the
+// SM's 256 KB is L1, which holds the node records the warps re-read: 182.9 ms
+// against 188.8 ms with 512 entries (14M-segment polymer step, an earlier
+// form, B200).
 #ifndef FLN_BH_STACK
 #define FLN_BH_STACK 224
 #endif
@@ -73,7 +72,8 @@ constexpr int kWarps = 4;          // warps per traversal CTA
 #ifndef FLN_BH_CARVEOUT
 #define FLN_BH_CARVEOUT 44
 #endif
-// The same for six (the default) and seven CTAs per SM.
+// The same for six (the default) and seven CTAs per SM. 48 / 52 / 58 / 66: 109.9
+// / 109.9 / 109.4 / 109.3 ms per call of 200 walks of 50,000 steps.
 #ifndef FLN_BH_CARVEOUT_6
 #define FLN_BH_CARVEOUT_6 58
 #endif
@@ -2933,6 +2933,12 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     };
     if (prm.bh_schedule != 2 && !ctx.exact_stream)
       FLN_CUDA(cudaStreamCreateWithFlags(&ctx.exact_stream, cudaStreamNonBlocking));
+    // Which input a round leaves to the next when its exact list reaches the
+    // soft limit follows the warps' timing, and so does the next round's
+    // amount of work. A batch must be cut at the same steps in every run (its
+    // far sum is added once), so from the first round whose list passes the
+    // limit, taken in part or not, the pass keeps the full budget.
+    bool limited = false;
     try {
       for (int round = 0; (nin > 0 || pos < nstream) && round < 65536; ++round) {
         const int par = round & 1;
@@ -2996,7 +3002,11 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         }
         const int gmax = (A.learned.frag && !A.rec) ? grid_l : (front ? grid_f : grid);
         const int64_t work = nin + (nstream - pos);
-        A.budget = round_budget(budget, tot_leaf, work, (int64_t)gmax * kWarps);
+        if (!limited) A.budget = round_budget(budget, tot_leaf, work, (int64_t)gmax * kWarps);
+        // A round of a short budget takes all its input: its list cannot fill
+        // (at most budget + 1 chunks a batch).
+        if (A.budget < budget && work * (A.budget + 1) > bkt_cap) A.budget = budget;
+        if (A.budget < budget) A.bkt_soft = bkt_cap;
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>((work + kWarps - 1) / kWarps, gmax));
         const cudaEvent_t trav0 = mark(st);
         if (A.rec)
@@ -3022,10 +3032,11 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
         }
         launches += 2;
         ++ctx.stats.bh_rounds;
-        FLN_CUDA(cudaMemcpyAsync(const_cast<unsigned long long *>(h_ctr), c, 2 * sizeof(unsigned long long),
+        FLN_CUDA(cudaMemcpyAsync(const_cast<unsigned long long *>(h_ctr), c, 3 * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, st));
         FLN_CUDA(cudaStreamSynchronize(st));
         const unsigned long long c2[2] = {h_ctr[0], h_ctr[1]};
+        limited = limited || (int64_t)h_ctr[2] > bkt_soft;
         if (round_log) {  // FLN_BH_ROUND_LOG: cumulative counts after each round, for profiling
           FLN_CUDA(cudaStreamSynchronize(ctx.exact_stream));
           double cnt[8];
