@@ -155,10 +155,10 @@ typedef struct fln_stats {
                                    the first pass for the retry to continue from */
   int64_t bh_retry_from_roots;  /* Barnes–Hut: retried pairs that restarted from the roots (frontier not
                                    kept for them, or bh_retry_from_roots set) */
-  double bh_far_reused;         /* Barnes–Hut: frontier node pairs still far at the retry's beta, whose
-                                   first-pass values were kept (not evaluated again) */
-  double bh_far_subtracted;     /* Barnes–Hut: frontier node pairs opened by the retry, whose first-pass
-                                   values were given back */
+  double bh_far_reused;         /* Barnes–Hut: frontier node pairs far at the retry's beta (by a margin of
+                                   1e-5), whose first-pass values were kept (not evaluated again) */
+  double bh_far_subtracted;     /* Barnes–Hut: the other frontier node pairs, whose first-pass values were
+                                   given back before the full test */
   double ms_traverse;           /* Barnes–Hut bh_schedule 0: device time of the traversal launches (CUDA
                                    events on the launching stream; the exact-list launches run beside them
                                    on a second stream, so ms_traverse + ms_exact can exceed
