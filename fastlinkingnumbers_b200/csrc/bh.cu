@@ -2697,9 +2697,11 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   std::vector<int64_t> node_base(nl_all, 0), seg_all(1, 0), blk_start(1, 0);
   int64_t nodes = 0;
   int maxdepth = 0;
+  int64_t longest = 0;
   for (int l = 0; l < nl_all; ++l) {
     if (!need[l]) continue;
     const int64_t n = h_off[l + 1] - h_off[l];
+    longest = std::max(longest, n);
     loops.push_back(l);
     node_base[l] = nodes;
     nodes += 2 * n;  // position 0 is unused; even, so that sibling headers share a line
@@ -2892,12 +2894,19 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
   if (use_front) {
     const size_t have = ctx.d_bh[23].bytes / sizeof(FrontRec);
     const size_t want_hint = ctx.bh_front_hint > 0 ? (size_t)(1.25 * (double)ctx.bh_front_hint) + 1024 : 0;
+    // A call larger than those before it: a record for every 16 segments of
+    // each pair of loops as long as the longest (60 walks of 2,000 steps write
+    // one for every 110 of theirs, 200 walks of 50,000 one for every 440), so
+    // that small calls do not take the memory of large ones.
+    const size_t guess = (size_t)np * (size_t)(4 + longest / 8);
     size_t want = have;
-    if (want_hint == 0 || want_hint > have) {  // the buffer must grow: ask how much memory is free
+    if (guess > ctx.bh_front_guess || want_hint > have) {  // the buffer may have to grow: ask how much memory is free
       size_t free_b = 0, total_b = 0;
       FLN_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      want = want_hint > 0 ? want_hint : std::min<size_t>((size_t)32 << 30, free_b / 3) / sizeof(FrontRec);
-      want = std::max(want, have);
+      const size_t room = std::min<size_t>((size_t)32 << 30, free_b / 3) / sizeof(FrontRec);
+      if (guess > ctx.bh_front_guess) want = std::max(want, std::min(guess, room));
+      want = std::max(want, want_hint);
+      ctx.bh_front_guess = std::max(ctx.bh_front_guess, guess);
       if (want > have && (want - have) * sizeof(FrontRec) > free_b / 2) want = have + free_b / 2 / sizeof(FrontRec);
     }
     front_cap = (int64_t)std::max<size_t>(want, 1024);

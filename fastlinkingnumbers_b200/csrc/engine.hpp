@@ -108,6 +108,7 @@ struct Context {
   // Device buffers.
   DevBuf d_xyz, d_off, d_pairs, d_loops, d_items, d_partial, d_counter, d_lk, d_err, d_flags, d_near, d_redo;
   DevBuf d_bh[28];
+  size_t bh_front_guess = 0;  // the most records a call's size has asked for
   int64_t bh_front_hint = 0;  // frontier records of the largest Barnes–Hut first pass so far
   // CTAs per SM of the traversal kernels (per occupancy set), of the learned
   // traversal and of bh_classify; 0 until first queried.
