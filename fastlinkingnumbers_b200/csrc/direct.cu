@@ -75,6 +75,7 @@ struct DirectArgs {
   int64_t target;             // items a call should have at least (plan_span)
   double least;               // calls of less work (PlanHead::work) take the whole of curve 2 per item
   int block;                  // curve-1 segments per item
+  bool few;                   // mixed: calls of at most kFewItems items go to direct_mixed_few_kernel
   bool lone;                  // one pair in FP64: direct_fp64_lone_kernel below kLoneWork
   PlanHead *head;
   double *partial;            // per item
@@ -148,6 +149,16 @@ __device__ __forceinline__ Item item_of(const DirectArgs &A, int64_t item, int b
 __device__ __forceinline__ int64_t plan_ready(const DirectArgs &A) {
   const int64_t n = (int64_t)A.head->items;
   return A.head->status == 0 && n <= A.cap ? n : 0;
+}
+// A mixed plan of few items (direct_mixed_few_kernel): at most six CTAs of 128
+// threads per SM, the point where two packed segments per thread begin to pay
+// (below), and curve 2 longer than the loops whose runs the packed kernel gives
+// to several groups of threads (64 rings of 32 segments: 84 us packed, 103 not).
+constexpr int64_t kFewItems = 888;
+constexpr double kFewWork = 128 * 128;  // segment pairs per item, at least
+__device__ __forceinline__ bool plan_few(const DirectArgs &A) {
+  return A.few && (int64_t)A.head->items <= kFewItems && A.head->work < kMixedSpans &&
+         A.head->work >= kFewWork * (double)A.head->items;
 }
 
 __device__ __forceinline__ double3 load_v(const double *xyz, int64_t v) {
@@ -716,7 +727,7 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   const unsigned below = (1u << lane) - 1;
   int2 *queue = s_near[threadIdx.x >> 5];
   double *term = s_term[threadIdx.x >> 5];
-  const int64_t items = plan_ready(A), span = plan_span(A, A.head->work);
+  const int64_t items = plan_few(A) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
   unsigned long long near_count = 0;
   for (;;) {
     __syncthreads();
@@ -915,6 +926,150 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   if (near_count) atomicAdd(&A.head->near, near_count);
 }
 
+// arctan(t) for |t| <= 1/4, the series of atan_small2.
+__device__ __forceinline__ float atan_small(float t) {
+  const float u = t * t;
+  float p = fmaf(u, 1.0f / 9.0f, -1.0f / 7.0f);
+  p = fmaf(p, u, 1.0f / 5.0f);
+  p = fmaf(p, u, -1.0f / 3.0f);
+  p = fmaf(p, u, 1.0f);
+  return p * t;
+}
+
+// The mixed sum of few items, one segment per thread: with at most a few CTAs
+// per SM a call lasts as long as one thread's walk, and a walk of two packed
+// segments takes longer than a walk of one. Terms, runs and sums are those of
+// direct_mixed_kernel, bit for bit. A CTA takes the item of its number: taken
+// from the queue, two items often met on one SM while others had none (5 walks
+// of 998 steps: 900 us). Whole calls, packed / this: 4 walks of 500 steps (30
+// items) 901 / 490 us, 5 of 998 (94) 1,104 / 764, 6 of 2,000 (290) 1,938 / 1,504,
+// 8 of 2,000 (609) 2,234 / 1,792; at 1,060 items 2,539 / 2,795.
+template <int kB, int kT>
+__global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
+  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = length of segment t
+  __shared__ double s_red[kB / 32];
+  __shared__ float s_box[kB / 32][14];
+  const float INF = __int_as_float(0x7f800000);
+  const int64_t item = blockIdx.x;
+  if (!plan_few(A) || item >= plan_ready(A)) return;
+  const Item it = item_of(A, item, kB, int64_t(1) << 62);
+  const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
+  const int64_t i = it.first + threadIdx.x;
+  const bool active = i < n1;
+  double3 p0 = make_double3(0, 0, 0), p1 = p0;
+  if (active) {
+    p0 = load_v(A.xyz, o1 + i);
+    p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
+  }
+  const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
+  const float len1 = sqrtf(ex * ex + ey * ey + ez * ez);
+  double acc = 0.0, near_turns = 0.0;
+  int turns = 0;
+  unsigned near_count = 0;
+  for (int64_t k0 = 0; k0 < n2; k0 += kT) {
+    const int kt = (int)min(n2 - k0, (int64_t)kT);
+    const double3 O = load_v(A.xyz, o2 + k0);
+    __syncthreads();
+    for (int t = threadIdx.x; t <= kt; t += kB) {
+      const int64_t kk = k0 + t;
+      const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
+      sq[t] = make_float4((float)(v.x - O.x), (float)(v.y - O.y), (float)(v.z - O.z), 0.f);
+    }
+    __syncthreads();
+    const float r0x = (float)(p0.x - O.x), r0y = (float)(p0.y - O.y), r0z = (float)(p0.z - O.z);
+    const float r1x = (float)(p1.x - O.x), r1y = (float)(p1.y - O.y), r1z = (float)(p1.z - O.z);
+    // Boxes of this thread's curve-1 segment (slots 0-2, length 3) and of
+    // its curve-2 tile vertices (slots 4-6, length 3 of the max).
+    float lo[7], hi[7];
+    for (int v = 0; v < 7; ++v) {
+      lo[v] = INF;
+      hi[v] = -INF;
+    }
+    if (active) {
+      lo[0] = fminf(r0x, r1x); hi[0] = fmaxf(r0x, r1x);
+      lo[1] = fminf(r0y, r1y); hi[1] = fmaxf(r0y, r1y);
+      lo[2] = fminf(r0z, r1z); hi[2] = fmaxf(r0z, r1z);
+      hi[3] = len1;
+    }
+    for (int t = threadIdx.x; t < kt; t += kB) {
+      const float4 a = sq[t], b = sq[t + 1];
+      const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
+      const float len = sqrtf(fx * fx + fy * fy + fz * fz);
+      sq[t].w = len;
+      lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
+      lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
+      lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
+      hi[3] = fmaxf(hi[3], len);
+    }
+    float bx[14];
+    block_minmax7<kB>(lo, hi, s_box, bx);
+    __syncthreads();
+    // Box gap between the CTA's curve-1 segments and this tile: no segment
+    // pair can be near-singular when it exceeds near_factor x (longest segment).
+    const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
+    const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
+    const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
+    const float lim = A.near_factor * bx[10];
+    const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
+    if (!active) continue;
+    float4 q = sq[0];
+    float ax = q.x - r0x, ay = q.y - r0y, az = q.z - r0z;
+    float bx_ = q.x - r1x, by = q.y - r1y, bz = q.z - r1z;
+    const float aa = ax * ax + ay * ay + az * az, bb = bx_ * bx_ + by * by + bz * bz;
+    float la = sqrtf(aa), lb = sqrtf(bb);
+    float ab = ax * bx_ + ay * by + az * bz;
+    float accf = 0.f;
+    for (int k = 0; k < kt; ++k) {
+      const float4 qn = sq[k + 1];
+      const float cx = qn.x - r1x, cy = qn.y - r1y, cz = qn.z - r1z;
+      const float dx = qn.x - r0x, dy = qn.y - r0y, dz = qn.z - r0z;
+      const float cc = cx * cx + cy * cy + cz * cz, dd = dx * dx + dy * dy + dz * dz;
+      const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
+      const float cd = cx * dx + cy * dy + cz * dz;
+      bool near = false;
+      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
+      if (near) {
+        const int64_t kk = k0 + k, kn = kk + 1;
+        near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
+        ++near_count;
+      } else {
+        const float ca = cx * ax + cy * ay + cz * az;
+        const float cb = cx * bx_ + cy * by + cz * bz;
+        const float ad = ax * dx + ay * dy + az * dz;
+        const float fx = qn.x - q.x, fy = qn.y - q.y, fz = qn.z - q.z;
+        const float det = ax * (fy * ez - fz * ey) + ay * (fz * ex - fx * ez) + az * (fx * ey - fy * ex);
+        const float t = la * lc;
+        const float div1 = t * lb + ab * lc + ca * lb + cb * la;
+        const float div2 = t * ld + ad * lc + ca * ld + cd * la;
+        const float sdiv = div1 + div2;
+        const float xp = div1 * div2 - det * det;
+        const float yp = det * sdiv;
+        float term;
+        if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
+          term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
+        } else {
+          term = atan2f(yp, xp);
+          if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;
+        }
+        accf += term;
+      }
+      if ((k & 31) == 31) {
+        acc += (double)accf;
+        accf = 0.f;
+      }
+      q = qn;
+      ax = dx; ay = dy; az = dz;
+      bx_ = cx; by = cy; bz = cz;
+      la = ld; lb = lc; ab = cd;
+    }
+    acc += (double)accf;
+  }
+  const double v = active ? acc * kInvTwoPi + (double)turns + near_turns : 0.0;
+  const double s = block_sum<kB>(v, s_red);
+  if (threadIdx.x == 0) A.partial[item] = s;
+  if (near_count) atomicAdd(&A.head->near, (unsigned long long)near_count);
+}
+
 // Sums the item partials of each pair, a warp per pair, in item order, and
 // checks the sum's margin to the rounding boundary (margin < 0: no check):
 // pairs that fail it, or are not finite, go to the list `redo`. The estimate
@@ -1073,6 +1228,8 @@ void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, doub
     direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
     if (known_work >= 0 && known_work < kLoneWork) return;
   }
+  // The plan fits one of the two.
+  if (A.few) direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, kFewItems), kB, 0, st>>>(A);
   const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, threads);
   kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), threads, 0, st>>>(A);
 }
@@ -1127,12 +1284,13 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   // a kernel of its own.
   const double least = precision == FLN_PREC_MIXED ? kMixedSpans : 0.0;
   const bool lone = precision == FLN_PREC_FP64 && np == 1 && tile_shape == 0;
+  const bool few = precision == FLN_PREC_MIXED && np <= kFewItems;  // (a pair has at least one item)
   // Room for the items: of the largest call so far, or a guess; a plan that
   // does not fit runs no kernel and is made again with room.
   ctx.direct_items = std::max<int64_t>(ctx.direct_items, std::max<int64_t>(4 * target, 2 * np));
   for (int attempt = 0;; ++attempt) {
     const int64_t cap = ctx.direct_items;
-    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, kB, lone,
+    DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, kB, few, lone,
                  d_head, ctx.d_partial.as<double>(cap), (float)near_factor};
     if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
       plan_small<<<1, 1024, 0, st>>>(A, nloops);
@@ -1357,7 +1515,8 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The default tile shape (the planning kernel cuts items of kBlockSegs).
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, false, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs,
+                     precision == FLN_PREC_MIXED && (int64_t)h.items <= kFewItems, false, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
   launch_direct(0, s, sms, precision, (int64_t)h.items, -1.0, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
