@@ -568,10 +568,10 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   return r;
 }
 // 1 / sqrt(x) and y / x by the hardware's approximations, as rsqrtf and
-// __fdividef but for subnormal x (treated as 0): a subnormal squared distance
-// is far below any segment length, so its pair is a near one, and a
-// subnormal x of a term (64 |q - p|^6, coordinates of 1e-7 and less) has lost
-// the term's digits already.
+// __fdividef but for subnormal numbers (treated as 0): of a squared distance
+// (below 1e-19: the pair's other distances are about a segment's length, and
+// it is a near one), and of a term's y beside an x of 2^-88 and more (kSmallX),
+// where the flushed y changes the angle by less than 2^-38.
 __device__ __forceinline__ float rsqrt_normal(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -588,6 +588,15 @@ struct F2x3 {
 __device__ __forceinline__ F2 dot2(const F2x3 &a, const F2x3 &b) {
   return fma2(a.z, b.z, fma2(a.x, b.x, mul2(a.y, b.y)));
 }
+// Small terms. A term (x, y) is 64 d^6 at a distance d. The series for small
+// angles takes x above 4 kSmallX (d of about 2e-5), where a flushed y does no
+// harm; the comparison has that bound in the addend of x / 4, which changes
+// nothing for larger x. Below, a term takes the full arctangent, and one whose x
+// and y are both below kTinyTerm (subnormal, d of about 2e-7), too short of
+// digits for an angle, is evaluated in FP64 like a near one.
+constexpr float kSmallX = 0x1p-90f, kTinyTerm = 0x1p-126f;
+__device__ __forceinline__ bool tiny_term(float x, float y) { return fabsf(x) < kTinyTerm && fabsf(y) < kTinyTerm; }
+
 __device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, float by, float bz) {
   return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
 }
@@ -660,8 +669,20 @@ __device__ __forceinline__ void mix_at(const MixSegs &S, const MixVertex &v, Mix
   w.ab = dot2(w.b, w.a);
 }
 
-// Terms of one step that are not both on the fast path: near pairs get 0 and
-// their bit, the others the full arctangent with the branch turn.
+// One term that is neither near nor on the packed path: a tiny one gets 0 and
+// its bit, the others the full arctangent with the branch turn.
+__device__ __forceinline__ void mix_slow1(float xp, float yp, float sdiv, float det, unsigned bit, float &t,
+                                          unsigned &mask, int &turns) {
+  if (tiny_term(xp, yp)) {
+    t = 0.f;
+    mask |= bit;
+  } else {
+    t = atan2f(yp, xp);
+    if (sdiv < 0.f && det != 0.f) turns += det > 0.f ? 1 : -1;
+  }
+}
+// Terms of one step that are not both on the packed path: near ones get 0 and
+// their bit.
 __device__ __forceinline__ void mix_slow(F2 xp, F2 yp, F2 sdiv, F2 det, bool near0, bool near1, bool fast0, bool fast1,
                                          unsigned bit, float &t0, float &t1, unsigned &mask0, unsigned &mask1,
                                          int &turns0, int &turns1) {
@@ -669,15 +690,13 @@ __device__ __forceinline__ void mix_slow(F2 xp, F2 yp, F2 sdiv, F2 det, bool nea
     t0 = 0.f;
     mask0 |= bit;
   } else if (!fast0) {
-    t0 = atan2f(lo2(yp), lo2(xp));
-    if (lo2(sdiv) < 0.f && lo2(det) != 0.f) turns0 += lo2(det) > 0.f ? 1 : -1;
+    mix_slow1(lo2(xp), lo2(yp), lo2(sdiv), lo2(det), bit, t0, mask0, turns0);
   }
   if (near1) {
     t1 = 0.f;
     mask1 |= bit;
   } else if (!fast1) {
-    t1 = atan2f(hi2(yp), hi2(xp));
-    if (hi2(sdiv) < 0.f && hi2(det) != 0.f) turns1 += hi2(det) > 0.f ? 1 : -1;
+    mix_slow1(hi2(xp), hi2(yp), hi2(sdiv), hi2(det), bit, t1, mask1, turns1);
   }
 }
 
@@ -705,7 +724,7 @@ __device__ __forceinline__ void mix_step(const MixSegs &S, const MixWalk &a, Mix
   const F2 sdiv = add2(div1, div2);
   const F2 xp = fma2(div1, div2, mul2(det, neg2(det)));
   const F2 yp = mul2(det, sdiv);
-  const F2 quarter = mul2(xp, pack2(0.25f, 0.25f));
+  const F2 quarter = fma2(xp, pack2(0.25f, 0.25f), pack2(-kSmallX, -kSmallX));
   const bool fast0 = lo2(sdiv) > 0.f && fabsf(lo2(yp)) < lo2(quarter);
   const bool fast1 = hi2(sdiv) > 0.f && fabsf(hi2(yp)) < hi2(quarter);
   // (fz.z: near_factor x the length of this curve-2 segment)
@@ -1073,8 +1092,13 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
         const float xp = div1 * div2 - det * det;
         const float yp = det * sdiv;
         float term;
-        if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
+        if (sdiv > 0.f && fabsf(yp) < __fmaf_rn(xp, 0.25f, -kSmallX)) {
           term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
+        } else if (tiny_term(xp, yp)) {
+          const int64_t kk = k0 + k, kn = kk + 1;
+          near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
+          ++near_count;
+          term = 0.f;
         } else {
           term = atan2f(yp, xp);
           if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;

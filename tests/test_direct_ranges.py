@@ -48,3 +48,11 @@ def test_fp64_sums_at_every_scale(sizes, scale):
     for npairs in (1, 3):  # the lone pair's kernel and the batched one
         # A term's rounding is a few 1e-16 and the 40,000 terms add up to one turn: below 1e-11 in all.
         np.testing.assert_allclose(sums(off, xyz, npairs, N.PREC_FP64), -1.0, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("sizes", [(64, 60), (300, 200)])  # two segments per thread, and one
+@pytest.mark.parametrize("scale", [1e-17, 1e-12, 1e-9, 1e-8, 1e-7, 3e-7, 1e-6, 3e-6, 1e-5, 3e-5, 1e-4, 1e5])
+def test_mixed_sums_at_small_scales(sizes, scale):
+    """Terms of 64 d^6 that are subnormal in FP32, or 0, or small enough that their parts are."""
+    off, xyz = hopf(*sizes, scale)
+    np.testing.assert_allclose(sums(off, xyz, 3, N.PREC_MIXED), -1.0, rtol=0, atol=1e-5)
