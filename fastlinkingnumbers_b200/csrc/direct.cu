@@ -157,9 +157,11 @@ __device__ __forceinline__ int64_t plan_ready(const DirectArgs &A) {
 // to several groups of threads (64 rings of 32 segments: 84 us packed, 103 not).
 constexpr int64_t kFewItems = 888;
 constexpr double kFewWork = 128 * 128;  // segment pairs per item, at least
+__host__ __device__ __forceinline__ bool few_items(int64_t items, double work) {
+  return items <= kFewItems && work < kMixedSpans && work >= kFewWork * (double)items;
+}
 __device__ __forceinline__ bool plan_few(const DirectArgs &A) {
-  return A.few && (int64_t)A.head->items <= kFewItems && A.head->work < kMixedSpans &&
-         A.head->work >= kFewWork * (double)A.head->items;
+  return A.few && few_items((int64_t)A.head->items, A.head->work);
 }
 
 __device__ __forceinline__ double3 load_v(const double *xyz, int64_t v) {
@@ -1271,30 +1273,32 @@ constexpr TileShape kShapes[kDirectTileShapes] = {{128, 256}, {128, 128}, {128, 
                                                   {256, 256}, {256, 512}, {64, 256}};
 static_assert(kShapes[0].block == kBlockSegs && kShapes[0].tile == kTile, "the default shape comes first");
 
+// The sum kernel that a plan needs, where the host knows it; otherwise those it
+// may need are all launched, and the plan fits one of them.
+enum class SumKernel { kUnknown, kLone, kFew, kMany };
+
 template <int kB, int kT>
-void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, double known_work, const DirectArgs &A) {
+void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, SumKernel which, const DirectArgs &A) {
+  if (A.lone && which != SumKernel::kMany)
+    direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
+  if (A.few && which != SumKernel::kMany)
+    direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, kFewItems), kB, 0, st>>>(A);
+  if (which == SumKernel::kLone || which == SumKernel::kFew) return;
   auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
   const int threads = precision == FLN_PREC_FP64 ? kB : kB / 2;
-  if (A.lone) {
-    // Where the host does not know the work, the plan fits one of the two.
-    direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
-    if (known_work >= 0 && known_work < kLoneWork) return;
-  }
-  // The plan fits one of the two.
-  if (A.few) direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, kFewItems), kB, 0, st>>>(A);
   const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, threads);
   kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), threads, 0, st>>>(A);
 }
 
-void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, double known_work,
+void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t most, SumKernel which,
                    const DirectArgs &A) {
   switch (shape) {
-    case 1: launch_direct_t<128, 128>(st, sms, precision, most, known_work, A); break;
-    case 2: launch_direct_t<128, 512>(st, sms, precision, most, known_work, A); break;
-    case 3: launch_direct_t<256, 256>(st, sms, precision, most, known_work, A); break;
-    case 4: launch_direct_t<256, 512>(st, sms, precision, most, known_work, A); break;
-    case 5: launch_direct_t<64, 256>(st, sms, precision, most, known_work, A); break;
-    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, known_work, A); break;
+    case 1: launch_direct_t<128, 128>(st, sms, precision, most, which, A); break;
+    case 2: launch_direct_t<128, 512>(st, sms, precision, most, which, A); break;
+    case 3: launch_direct_t<256, 256>(st, sms, precision, most, which, A); break;
+    case 4: launch_direct_t<256, 512>(st, sms, precision, most, which, A); break;
+    case 5: launch_direct_t<64, 256>(st, sms, precision, most, which, A); break;
+    default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, which, A); break;
   }
 }
 
@@ -1355,7 +1359,8 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
     }
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, tail ? tail->known_work : -1.0, A);
+    const bool is_lone = lone && tail && tail->known_work >= 0 && tail->known_work < kLoneWork;
+    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, is_lone ? SumKernel::kLone : SumKernel::kUnknown, A);
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev3, st));
     reduce_items_kernel<<<(int)((np + 7) / 8), 256, 0, st>>>(A, margin, d_lk, d_err, d_flags, d_redo);
@@ -1445,6 +1450,7 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
   int64_t *start = reinterpret_cast<int64_t *>(scratch + kNaStart);
   __shared__ long long s_warp[32];
   __shared__ long long s_carry;
+  __shared__ double s_work[32];
   __shared__ int s_status;
   if (threadIdx.x == 0) {
     s_carry = 0;
@@ -1452,6 +1458,7 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double work = 0.0;
   for (int64_t base = 0; base < npairs; base += 1024) {
     const int64_t p = base + threadIdx.x;
     long long items = 0;
@@ -1465,6 +1472,7 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
           atomicOr(&s_status, 2);
         } else {
           items = (max(na, nb) + kBlockSegs - 1) / kBlockSegs;
+          work += (double)na * (double)nb;
         }
       }
     }
@@ -1491,9 +1499,14 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
     if (threadIdx.x == 0) s_carry += s_warp[31];
     __syncthreads();
   }
+  for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
+  if (lane == 0) s_work[warp] = work;
+  __syncthreads();
   if (threadIdx.x == 0) {
+    work = 0.0;
+    for (int w = 0; w < 32; ++w) work += s_work[w];
     start[npairs] = s_carry;
-    *h = PlanHead{0, 0, (unsigned long long)s_carry, 0, 0.0, s_status, 0};
+    *h = PlanHead{0, 0, (unsigned long long)s_carry, 0, work, s_status, 0};
   }
 }
 
@@ -1565,12 +1578,13 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // The default tile shape (the planning kernel cuts items of kBlockSegs).
+  // The default tile shape (the planning kernel cuts items of kBlockSegs), whole
+  // walks of curve 2 at any amount of work.
+  const bool few = precision == FLN_PREC_MIXED && few_items((int64_t)h.items, h.work);
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs,
-                     precision == FLN_PREC_MIXED && (int64_t)h.items <= kFewItems, false, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few, false, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
-  launch_direct(0, s, sms, precision, (int64_t)h.items, -1.0, A);
+  launch_direct(0, s, sms, precision, (int64_t)h.items, few ? SumKernel::kFew : SumKernel::kMany, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FLN_ERR_CUDA, std::string("fln_linking_numbers_direct_noalloc: ") + cudaGetErrorString(e));

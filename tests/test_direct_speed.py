@@ -1,0 +1,68 @@
+"""Which kernel a direct sum runs, seen from its time: each call against another of
+the same sums, so that the device's clock drops out. The bounds lie halfway between
+the ratio with the right kernel and with the wrong one."""
+import ctypes as C
+import time
+
+import numpy as np
+import pytest
+
+from fastlinkingnumbers_b200 import Engine
+from fastlinkingnumbers_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+
+def walks(sizes, seed, spread):
+    """Closed Gaussian walks about centres in a cube of side `spread`."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in sizes:
+        s = rng.normal(size=(n, 3))
+        p = np.cumsum(s - s.mean(axis=0), axis=0)
+        out.append(p - p.mean(axis=0) + spread * rng.uniform(size=3))
+    return np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64), np.concatenate(out)
+
+
+def all_pairs(n):
+    return np.stack(np.triu_indices(n, 1), axis=1).astype(np.int32)
+
+
+class Calls:
+    """Device-array calls of one set of loops and pairs; time() is the best of many."""
+
+    def __init__(self, off, xyz, pairs):
+        import torch
+        self.torch, self.engine, self.lib = torch, Engine(0), N.load()
+        self.n, self.nloops = len(pairs), len(off) - 1
+        self.d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (xyz, off, pairs)]
+        self.lk = torch.zeros(self.n, dtype=torch.float64, device="cuda")
+
+    def allocating(self, precision, **params):
+        self.engine.linking_numbers_device(self.d[0].data_ptr(), self.d[1].data_ptr(), self.nloops,
+                                           self.d[2].data_ptr(), self.n, self.lk.data_ptr(), method="directsum",
+                                           precision=precision, **params)
+
+    def noalloc(self, precision):
+        st = self.lib.fln_linking_numbers_direct_noalloc(
+            C.c_void_p(self.d[0].data_ptr()), C.c_void_p(self.d[1].data_ptr()), self.nloops,
+            C.c_void_p(self.d[2].data_ptr()), self.n, precision, C.c_void_p(self.lk.data_ptr()), None)
+        assert st == 0, self.lib.fln_last_error()
+
+    def time(self, call, *args, **params):
+        best = 1e9
+        for _ in range(25):
+            self.torch.cuda.synchronize()
+            t = time.perf_counter()
+            call(*args, **params)
+            self.torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        return best
+
+
+@pytest.mark.parametrize("loops,steps", [(5, 998), (8, 2000)])
+def test_allocation_free_call_of_few_items(loops, steps):
+    """The allocation-free mixed call runs the kernel of few items as the allocating one does (times
+    of 0.95 of its; with the kernel of many 2.4 and 1.4)."""
+    c = Calls(*walks([steps] * loops, 3, 10.0), all_pairs(loops))
+    assert c.time(c.noalloc, N.PREC_MIXED) < 1.2 * c.time(c.allocating, N.PREC_MIXED)
