@@ -590,14 +590,14 @@ struct F2x3 {
 __device__ __forceinline__ F2 dot2(const F2x3 &a, const F2x3 &b) {
   return fma2(a.z, b.z, fma2(a.x, b.x, mul2(a.y, b.y)));
 }
-// Small terms. A term (x, y) is 64 d^6 at a distance d. The series for small
-// angles takes x above 4 kSmallX (d of about 2e-5), where a flushed y does no
-// harm; the comparison has that bound in the addend of x / 4, which changes
-// nothing for larger x. Below, a term takes the full arctangent, and one whose x
-// and y are both below kTinyTerm (subnormal, d of about 2e-7), too short of
-// digits for an angle, is evaluated in FP64 like a near one.
-constexpr float kSmallX = 0x1p-90f, kTinyTerm = 0x1p-126f;
-__device__ __forceinline__ bool tiny_term(float x, float y) { return fabsf(x) < kTinyTerm && fabsf(y) < kTinyTerm; }
+// Small terms. A term (x, y) is 64 d^6 at a distance d. A pair with an endpoint
+// distance below kNearLeast counts as near whatever its segments' lengths: its x
+// and y would be subnormal, too short of digits for an angle (d of 2e-7), or 0
+// (1e-8). The series for small angles takes x above 4 kSmallX (d of about 2e-5),
+// where a flushed y does no harm; the comparison has that bound in the addend
+// of x / 4, which changes nothing for larger x. Between the two a term takes the
+// full arctangent. (Tests of x and y themselves cost 1 to 3 %.)
+constexpr float kSmallX = 0x1p-90f, kNearLeast = 1e-6f;
 
 __device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, float by, float bz) {
   return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
@@ -656,7 +656,7 @@ struct MixWalk {
 struct MixSegs {
   F2x3 ra, rb;  // p_j, p_{j+1} relative to the tile's origin
   F2x3 e, ne;   // e = p_{j+1} - p_j and -e
-  float near0, near1;  // near_factor x their lengths
+  float near0, near1;  // near_factor x their lengths, kNearLeast at least
 };
 
 // Vectors and norms of the walk at vertex v. The products of the shared
@@ -671,20 +671,8 @@ __device__ __forceinline__ void mix_at(const MixSegs &S, const MixVertex &v, Mix
   w.ab = dot2(w.b, w.a);
 }
 
-// One term that is neither near nor on the packed path: a tiny one gets 0 and
-// its bit, the others the full arctangent with the branch turn.
-__device__ __forceinline__ void mix_slow1(float xp, float yp, float sdiv, float det, unsigned bit, float &t,
-                                          unsigned &mask, int &turns) {
-  if (tiny_term(xp, yp)) {
-    t = 0.f;
-    mask |= bit;
-  } else {
-    t = atan2f(yp, xp);
-    if (sdiv < 0.f && det != 0.f) turns += det > 0.f ? 1 : -1;
-  }
-}
-// Terms of one step that are not both on the packed path: near ones get 0 and
-// their bit.
+// Terms of one step that are not both on the packed path: near pairs get 0 and
+// their bit, the others the full arctangent with the branch turn.
 __device__ __forceinline__ void mix_slow(F2 xp, F2 yp, F2 sdiv, F2 det, bool near0, bool near1, bool fast0, bool fast1,
                                          unsigned bit, float &t0, float &t1, unsigned &mask0, unsigned &mask1,
                                          int &turns0, int &turns1) {
@@ -692,13 +680,15 @@ __device__ __forceinline__ void mix_slow(F2 xp, F2 yp, F2 sdiv, F2 det, bool nea
     t0 = 0.f;
     mask0 |= bit;
   } else if (!fast0) {
-    mix_slow1(lo2(xp), lo2(yp), lo2(sdiv), lo2(det), bit, t0, mask0, turns0);
+    t0 = atan2f(lo2(yp), lo2(xp));
+    if (lo2(sdiv) < 0.f && lo2(det) != 0.f) turns0 += lo2(det) > 0.f ? 1 : -1;
   }
   if (near1) {
     t1 = 0.f;
     mask1 |= bit;
   } else if (!fast1) {
-    mix_slow1(hi2(xp), hi2(yp), hi2(sdiv), hi2(det), bit, t1, mask1, turns1);
+    t1 = atan2f(hi2(yp), hi2(xp));
+    if (hi2(sdiv) < 0.f && hi2(det) != 0.f) turns1 += hi2(det) > 0.f ? 1 : -1;
   }
 }
 
@@ -803,8 +793,8 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
       S.ne = F2x3{neg2(S.e.x), neg2(S.e.y), neg2(S.e.z)};
       len0 = sqrtf(dot_f(x0, y0, z0, x0, y0, z0));
       len1 = sqrtf(dot_f(x1, y1, z1, x1, y1, z1));
-      S.near0 = A.near_factor * len0;
-      S.near1 = A.near_factor * len1;
+      S.near0 = fmaxf(A.near_factor * len0, kNearLeast);
+      S.near1 = fmaxf(A.near_factor * len1, kNearLeast);
     }
     double acc0 = 0.0, acc1 = 0.0, near0 = 0.0, near1 = 0.0;
     int turns0 = 0, turns1 = 0, queued = 0;
@@ -886,11 +876,11 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
       block_minmax7<kThreads>(lo, hi, s_box, bx);
       __syncthreads();
       // Box gap between the CTA's curve-1 segments and this tile: no segment
-      // pair can be near-singular when it exceeds near_factor x (longest segment).
+      // pair can be near when it exceeds near_factor x (longest segment) and kNearLeast.
       const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
       const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
       const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
-      const float lim = A.near_factor * bx[10];
+      const float lim = fmaxf(A.near_factor * bx[10], kNearLeast);
       const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
       // The runs of 32 steps of this thread's group.
       const int runs = (kt + 31) / 32, ra = runs * grp / groups, rb = runs * (grp + 1) / groups;
@@ -995,7 +985,7 @@ __device__ __forceinline__ float atan_small(float t) {
 // 8 of 2,000 (609) 2,234 / 1,792; at 1,060 items 2,539 / 2,795.
 template <int kB, int kT>
 __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
-  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = length of segment t
+  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = near_factor x length of segment t
   __shared__ double s_red[kB / 32];
   __shared__ float s_box[kB / 32][14];
   const float INF = __int_as_float(0x7f800000);
@@ -1011,7 +1001,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
     p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
   }
   const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
-  const float len1 = sqrtf(ex * ex + ey * ey + ez * ez);
+  const float len1 = sqrtf(ex * ex + ey * ey + ez * ez), near1 = fmaxf(A.near_factor * len1, kNearLeast);
   double acc = 0.0, near_turns = 0.0;
   int turns = 0;
   unsigned near_count = 0;
@@ -1044,7 +1034,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
       const float4 a = sq[t], b = sq[t + 1];
       const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
       const float len = sqrtf(fx * fx + fy * fy + fz * fz);
-      sq[t].w = len;
+      sq[t].w = A.near_factor * len;
       lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
       lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
       lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
@@ -1054,11 +1044,11 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
     block_minmax7<kB>(lo, hi, s_box, bx);
     __syncthreads();
     // Box gap between the CTA's curve-1 segments and this tile: no segment
-    // pair can be near-singular when it exceeds near_factor x (longest segment).
+    // pair can be near when it exceeds near_factor x (longest segment) and kNearLeast.
     const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
     const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
     const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
-    const float lim = A.near_factor * bx[10];
+    const float lim = fmaxf(A.near_factor * bx[10], kNearLeast);
     const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
     if (!active) continue;
     float4 q = sq[0];
@@ -1076,7 +1066,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
       const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
       const float cd = cx * dx + cy * dy + cz * dz;
       bool near = false;
-      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
+      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < fmaxf(near1, q.w);
       if (near) {
         const int64_t kk = k0 + k, kn = kk + 1;
         near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
@@ -1096,11 +1086,6 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
         float term;
         if (sdiv > 0.f && fabsf(yp) < __fmaf_rn(xp, 0.25f, -kSmallX)) {
           term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
-        } else if (tiny_term(xp, yp)) {
-          const int64_t kk = k0 + k, kn = kk + 1;
-          near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
-          ++near_count;
-          term = 0.f;
         } else {
           term = atan2f(yp, xp);
           if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;
