@@ -76,7 +76,7 @@ struct DirectArgs {
   int64_t target;             // items a call should have at least (plan_span)
   double least;               // calls of less work (PlanHead::work) take the whole of curve 2 per item
   int block;                  // curve-1 segments per item
-  bool few;                   // mixed: calls of at most kFewItems items go to direct_mixed_few_kernel
+  int64_t few;                // mixed: most items of a call for direct_mixed_few_kernel (few_items); 0: none
   bool lone;                  // one pair in FP64: direct_fp64_lone_kernel below kLoneWork
   PlanHead *head;
   double *partial;            // per item
@@ -151,17 +151,19 @@ __device__ __forceinline__ int64_t plan_ready(const DirectArgs &A) {
   const int64_t n = (int64_t)A.head->items;
   return A.head->status == 0 && n <= A.cap ? n : 0;
 }
-// A mixed plan of few items (direct_mixed_few_kernel): at most six CTAs of 128
-// threads per SM, the point where two packed segments per thread begin to pay
-// (below), and curve 2 longer than the loops whose runs the packed kernel gives
-// to several groups of threads (64 rings of 32 segments: 84 us packed, 103 not).
-constexpr int64_t kFewItems = 888;
-constexpr double kFewWork = 128 * 128;  // segment pairs per item, at least
-__host__ __device__ __forceinline__ bool few_items(int64_t items, double work) {
-  return items <= kFewItems && work < kMixedSpans && work >= kFewWork * (double)items;
+// A mixed plan of few items (direct_mixed_few_kernel): at most `most`, the CTAs
+// of that kernel that fit the chip at once (beyond, it needs a second wave: 9
+// walks of 2,000 steps, 576 items of 592: 1.91 ms packed, 1.83 by this kernel;
+// 10 of 2,000, 720 items: 1.64 and 1.95), and loops longer than those of which
+// the packed kernel gives the runs to two groups of threads (15 x 15 linked rings
+// of 64 segments: 114 us packed, 123 by this kernel; 20 walks of 72 steps, all
+// pairs near: 256 and 141).
+constexpr double kFewWork = 64 * 64;  // segment pairs per item, more than
+__host__ __device__ __forceinline__ bool few_items(int64_t items, double work, int64_t most) {
+  return items <= most && work < kMixedSpans && work > kFewWork * (double)items;
 }
 __device__ __forceinline__ bool plan_few(const DirectArgs &A) {
-  return A.few && few_items((int64_t)A.head->items, A.head->work);
+  return A.few > 0 && few_items((int64_t)A.head->items, A.head->work, A.few);
 }
 
 __device__ __forceinline__ double3 load_v(const double *xyz, int64_t v) {
@@ -638,6 +640,11 @@ __device__ __forceinline__ void block_minmax7(float *lo, float *hi, float (*s_bo
   }
 }
 
+// Lanes of a warp with a near pair from which each evaluates its own (24 / 30 /
+// 32 / never: 100 walks of 60 steps on one spot 501 / 511 / 523 / 560 us a call,
+// 100 x 100 linked rings 824 / 823 / 812 / 801).
+constexpr int kDenseNear = 24;
+
 // A tile vertex: q relative to the tile's origin and the segment f to the next
 // vertex, every value twice (the two halves of a packed operand), and
 // near_factor x the segment's length.
@@ -739,8 +746,13 @@ __device__ __forceinline__ void mix_step(const MixSegs &S, const MixWalk &a, Mix
 // an item takes the whole of curve 2 (but for large calls, kMixedSpans), and
 // only loops of at most kB / 2 segments make several groups of threads, a run
 // of 32 steps each.
-// Near pairs are noted in a bit mask per run, queued per warp, evaluated 32 at
-// a time in FP64 and added to their segment's sum in order.
+// Near pairs are noted in a bit mask per run and evaluated in FP64 by the warp
+// together, 32 of a queue at a time, or by their own lanes where nearly all have
+// one (kDenseNear), and added to their segment's sum in order. (A lane finds the
+// queued pairs of its segments by one match of the 32 owners; looking through
+// all 32 cost as much as the terms: 100 x 100 linked rings 954 us a call, 824
+// now; 100 walks of 60 steps on one spot, nearly all pairs near, 856 -> 501, 794
+// by one scalar segment per thread with near pairs as a divergent call.)
 //
 // Bound: issue and the FMA pipe together. A step of 64 segment pairs needs 50
 // packed and 8 scalar FMA-pipe operations (108 cycles of a scheduler's pipe, 709
@@ -757,6 +769,7 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   __shared__ MixVertex tile[kT + 1];
   __shared__ int2 s_near[kThreads / 32][64];  // (curve-1 segment of the item x 32 + lane, curve-2 segment) left to FP64
   __shared__ double s_term[kThreads / 32][32];
+  __shared__ unsigned s_mine[kThreads / 32][32];  // per lane: the flushed pairs of its segments
   __shared__ double s_red[kB / 32];
   __shared__ double s_seg[kB];  // per segment of the item
   __shared__ float s_box[kThreads / 32][14];
@@ -766,6 +779,7 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   const unsigned below = (1u << lane) - 1;
   int2 *queue = s_near[threadIdx.x >> 5];
   double *term = s_term[threadIdx.x >> 5];
+  unsigned *mine = s_mine[threadIdx.x >> 5];
   const int64_t items = plan_few(A) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
   unsigned long long near_count = 0;
   for (;;) {
@@ -798,31 +812,6 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
     }
     double acc0 = 0.0, acc1 = 0.0, near0 = 0.0, near1 = 0.0;
     int turns0 = 0, turns1 = 0, queued = 0;
-    // Evaluates the oldest n queued pairs (n <= 32); every lane adds those of
-    // its segments, oldest first.
-    auto flush = [&](int n) {
-      int2 q = make_int2(0, 0);
-      if (lane < n) {
-        q = queue[lane];
-        int64_t seg = it.first + (q.x >> 5);
-        if (seg >= n1) seg -= n1;
-        term[lane] = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)seg, q.y));
-      }
-      __syncwarp();
-      for (int x = 0; x < n; ++x) {
-        const int who = queue[x].x;
-        const double v = term[x];
-        if ((who & 31) == lane) {
-          if (who >> 5 == at) near0 += v;
-          else near1 += v;
-        }
-      }
-      __syncwarp();
-      q = queue[32 + lane];
-      __syncwarp();
-      queue[lane] = q;
-      __syncwarp();
-    };
     for (int64_t k0 = it.k0; k0 < it.k1; k0 += kT) {  // a span is a multiple of kT (kMixedSpans)
       const int kt = (int)min(it.k1 - k0, (int64_t)kT);
       const double3 O = load_v(A.xyz, o2 + k0);
@@ -918,28 +907,67 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
           acc1 += (double)sum1;
           if (!second) near_mask1 = 0;
         }
-        // Queue this run's near pairs, one per lane at a time; evaluate 32 at a time.
-        while (__any_sync(0xffffffffu, (near_mask0 | near_mask1) != 0)) {
+        // The run's near pairs, one per lane at a time: evaluated at once when
+        // most lanes have one, else queued, and 32 of the queue evaluated
+        // together, oldest first (what is left, before lanes evaluate their own
+        // and at the item's end). A lane adds the pairs of its segments in order.
+#pragma unroll 1
+        for (;;) {
           const bool has = (near_mask0 | near_mask1) != 0;
           const unsigned m = __ballot_sync(0xffffffffu, has);
-          if (has) {
-            const bool first = near_mask0 != 0;
-            const int k = __ffs(first ? near_mask0 : near_mask1) - 1;
-            if (first) near_mask0 &= near_mask0 - 1;
-            else near_mask1 &= near_mask1 - 1;
-            queue[queued + __popc(m & below)] = make_int2((first ? at : at + 1) << 5 | lane, (int)(k0 + j0 + k));
+          const bool dense = __popc(m) >= kDenseNear, own = dense && queued == 0;
+          if (m == 0 && !(queued > 0 && k0 + kT >= it.k1 && r + 1 == rounds)) break;
+          int2 q = make_int2(0, 0);  // (segment of the item x 32 + lane, curve-2 segment)
+          bool valid = false;
+          if (own || (m && !dense)) {
+            if (has) {
+              const bool first = near_mask0 != 0;
+              const int k = __ffs(first ? near_mask0 : near_mask1) - 1;
+              if (first) near_mask0 &= near_mask0 - 1;
+              else near_mask1 &= near_mask1 - 1;
+              q = make_int2((first ? at : at + 1) << 5 | lane, (int)(k0 + j0 + k));
+              if (!own) queue[queued + __popc(m & below)] = q;
+            }
+            near_count += lane == 0 ? __popc(m) : 0;
+            valid = own && has;
+            if (!own) {
+              queued += __popc(m);
+              __syncwarp();
+              if (queued < 32) continue;
+            }
           }
-          queued += __popc(m);
-          near_count += lane == 0 ? __popc(m) : 0;
+          const int n = min(queued, 32);
+          if (!own) {
+            valid = lane < n;
+            q = queue[lane];
+          }
+          double v = 0.0;
+          if (valid) v = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)it.first + (q.x >> 5), q.y));
+          if (own) {
+            if (q.x >> 5 == at) near0 += v;
+            else near1 += v;
+            continue;
+          }
+          if (valid) term[lane] = v;
+          mine[lane] = 0;
           __syncwarp();
-          if (queued >= 32) {
-            flush(32);
-            queued -= 32;
+          const unsigned of = __match_any_sync(0xffffffffu, valid ? q.x & 31 : 32 + lane);
+          if (valid) mine[q.x & 31] = of;
+          __syncwarp();
+          for (unsigned b = mine[lane]; b; b &= b - 1) {
+            const int x = __ffs(b) - 1;
+            if (queue[x].x >> 5 == at) near0 += term[x];
+            else near1 += term[x];
           }
+          __syncwarp();
+          q = queue[32 + lane];
+          __syncwarp();
+          queue[lane] = q;
+          __syncwarp();
+          queued -= n;
         }
       }
     }
-    if (queued > 0) flush(queued);
     // The item's sum: 32 segments at a time by a butterfly, those sums in order.
     for (int g = 0; g < groups; ++g) {
       if (grp == g) {
@@ -980,9 +1008,9 @@ __device__ __forceinline__ float atan_small(float t) {
 // segments takes longer than a walk of one. Terms, runs and sums are those of
 // direct_mixed_kernel, bit for bit. A CTA takes the item of its number: taken
 // from the queue, two items often met on one SM while others had none (5 walks
-// of 998 steps: 900 us). Whole calls, packed / this: 4 walks of 500 steps (30
-// items) 901 / 490 us, 5 of 998 (94) 1,104 / 764, 6 of 2,000 (290) 1,938 / 1,504,
-// 8 of 2,000 (609) 2,234 / 1,792; at 1,060 items 2,539 / 2,795.
+// of 998 steps: 900 us). Whole calls, packed / this: 4 walks of 500 steps (24
+// items) 797 / 492 us, 5 of 998 (80) 1,268 / 880, 8 of 2,000 (448) 1,495 / 1,363,
+// 12 of 2,000 (1,056) 2,144 / 2,766.
 template <int kB, int kT>
 __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
   __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = near_factor x length of segment t
@@ -1266,8 +1294,8 @@ template <int kB, int kT>
 void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, SumKernel which, const DirectArgs &A) {
   if (A.lone && which != SumKernel::kMany)
     direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
-  if (A.few && which != SumKernel::kMany)
-    direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, kFewItems), kB, 0, st>>>(A);
+  if (A.few > 0 && which != SumKernel::kMany)
+    direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, A.few), kB, 0, st>>>(A);
   if (which == SumKernel::kLone || which == SumKernel::kFew) return;
   auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
   const int threads = precision == FLN_PREC_FP64 ? kB : kB / 2;
@@ -1285,6 +1313,15 @@ void launch_direct(int shape, cudaStream_t st, int sms, int precision, int64_t m
     case 5: launch_direct_t<64, 256>(st, sms, precision, most, which, A); break;
     default: launch_direct_t<kBlockSegs, kTile>(st, sms, precision, most, which, A); break;
   }
+}
+
+// Most items of a plan for direct_mixed_few_kernel: its resident CTAs.
+int64_t few_most(int shape, int sms) {
+  const void *k[kDirectTileShapes] = {
+      (const void *)direct_mixed_few_kernel<128, 256>, (const void *)direct_mixed_few_kernel<128, 128>,
+      (const void *)direct_mixed_few_kernel<128, 512>, (const void *)direct_mixed_few_kernel<256, 256>,
+      (const void *)direct_mixed_few_kernel<256, 512>, (const void *)direct_mixed_few_kernel<64, 256>};
+  return (int64_t)sms * occupancy_of(k[shape], kShapes[shape].block);
 }
 
 }  // namespace
@@ -1325,7 +1362,8 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   // a kernel of its own.
   const double least = precision == FLN_PREC_MIXED ? kMixedSpans : 0.0;
   const bool lone = precision == FLN_PREC_FP64 && np == 1 && tile_shape == 0;
-  const bool few = precision == FLN_PREC_MIXED && np <= kFewItems;  // (a pair has at least one item)
+  int64_t few = precision == FLN_PREC_MIXED ? few_most(tile_shape, ctx.num_sms) : 0;
+  if (np > few) few = 0;  // (a pair has at least one item)
   // Room for the items: of the largest call so far, or a guess; a plan that
   // does not fit runs no kernel and is made again with room.
   ctx.direct_items = std::max<int64_t>(ctx.direct_items, std::max<int64_t>(4 * target, 2 * np));
@@ -1565,9 +1603,10 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The default tile shape (the planning kernel cuts items of kBlockSegs), whole
   // walks of curve 2 at any amount of work.
-  const bool few = precision == FLN_PREC_MIXED && few_items((int64_t)h.items, h.work);
+  const int64_t most = precision == FLN_PREC_MIXED ? few_most(0, sms) : 0;
+  const bool few = few_items((int64_t)h.items, h.work, most);
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few, false, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, false, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
   launch_direct(0, s, sms, precision, (int64_t)h.items, few ? SumKernel::kFew : SumKernel::kMany, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
