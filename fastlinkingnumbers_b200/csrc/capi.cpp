@@ -437,8 +437,8 @@ void compute_pairs_host(Context &ctx, const double *xyz, const int64_t *loop_off
     tail.d_src = d_lk;
     tail.bytes = 2 * np1 * sizeof(double) + np1 * sizeof(int32_t);
   }
-  if (npairs == 1) tail.known_work = (double)(h_off[h_pairs[0] + 1] - h_off[h_pairs[0]]) *
-                                     (double)(h_off[h_pairs[1] + 1] - h_off[h_pairs[1]]);
+  if (npairs == 1)
+    tail.known_longest = std::max(h_off[h_pairs[0] + 1] - h_off[h_pairs[0]], h_off[h_pairs[1] + 1] - h_off[h_pairs[1]]);
   try {
     launches = bh ? run_barnes_hut(ctx, d_xyz, d_off, h_off, h_pairs, d_pairs, prm, d_lk, d_err, d_flags)
                   : run_direct(ctx, d_xyz, d_off, nloops, d_pairs, npairs, prm, d_lk, d_err, d_flags, &tail, &complete);

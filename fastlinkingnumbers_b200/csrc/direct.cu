@@ -59,6 +59,7 @@ struct PlanHead {
   unsigned long long near;   // mixed: segment pairs evaluated in FP64
   unsigned long long items;
   unsigned long long redo;   // pairs that failed the margin check
+  unsigned long long longest;  // segments of the longest loop of a pair
   double work;               // sum over pairs of n_i n_j
   int32_t status;            // kBad* bits
   int32_t pad;
@@ -77,7 +78,7 @@ struct DirectArgs {
   double least;               // calls of less work (PlanHead::work) take the whole of curve 2 per item
   int block;                  // curve-1 segments per item
   int64_t few;                // mixed: most items of a call for direct_mixed_few_kernel (few_items); 0: none
-  bool lone;                  // one pair in FP64: direct_fp64_lone_kernel below kLoneWork
+  int64_t lone;               // one pair in FP64: the longest loop for direct_fp64_lone_kernel; 0: none
   PlanHead *head;
   double *partial;            // per item
   float near_factor;
@@ -91,16 +92,21 @@ struct DirectArgs {
 // regroups its FP64 sum, and below that the sums stay bit for bit those of one
 // walk per segment (all there is to see when no loops are linked).
 constexpr double kMixedSpans = 1 << 30;
-// A lone pair of less work than this goes to direct_fp64_lone_kernel, 32
-// curve-1 segments an item.
-constexpr double kLoneWork = 1 << 30;
+// A lone pair goes to direct_fp64_lone_kernel, 32 curve-1 segments an item, when
+// its items are resident at once, two CTAs per SM. The kernel is for loops that
+// fill few CTAs; longer ones it takes a wave at a time. Calls by this kernel /
+// the general one (one thread per segment before both): 300 x 211 segments 79 /
+// 70 us (135), 5,000 x 4,286 397 / 258 (1,285), 10,000 x 8,572 1,112 / 454
+// (2,487), 30,000 x 20 115 / 77 (89), 200,000 x 300 845 / 416 (536), 200,000 x 2,000
+// 3,572 / 1,645 (2,914). (Below the line it stays for its sums, see there.)
 constexpr int kLoneSegs = 32;
-__device__ __forceinline__ bool plan_lone(const DirectArgs &A, double work) { return A.lone && work < kLoneWork; }
-__device__ __forceinline__ int plan_block(const DirectArgs &A, double work) {
-  return plan_lone(A, work) ? kLoneSegs : A.block;
+constexpr int64_t kLonePerSm = 2;
+__device__ __forceinline__ bool plan_lone(const DirectArgs &A) {
+  return A.lone > 0 && (int64_t)A.head->longest <= A.lone;
 }
+__device__ __forceinline__ int plan_block(const DirectArgs &A) { return plan_lone(A) ? kLoneSegs : A.block; }
 __device__ __forceinline__ int64_t plan_span(const DirectArgs &A, double work) {
-  if (work < A.least || plan_lone(A, work)) return int64_t(1) << 62;
+  if (work < A.least || plan_lone(A)) return int64_t(1) << 62;
   const double want = work / ((double)A.block * (double)A.target);
   int64_t span = 32;
   while ((double)span < want) span *= 2;
@@ -364,7 +370,7 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
   __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
   __shared__ long long s_item;
-  const int64_t items = plan_lone(A, A.head->work) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
+  const int64_t items = plan_lone(A) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
@@ -454,7 +460,7 @@ __global__ void __launch_bounds__(256) direct_fp64_lone_kernel(DirectArgs A) {
   __shared__ int s_turns[7][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double work = A.head->work;
-  const int64_t items = plan_lone(A, work) ? plan_ready(A) : 0;
+  const int64_t items = plan_lone(A) ? plan_ready(A) : 0;
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
     const Item it = item_of(A, item, kLoneSegs, plan_span(A, work));
     const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
@@ -1146,8 +1152,8 @@ __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double 
   const int lane = threadIdx.x & 31;
   if (p >= A.npairs || (plan_ready(A) == 0)) return;
   const double work = A.head->work;
-  const int64_t span = plan_span(A, work), block = plan_block(A, work);
-  const int per = plan_lone(A, work) ? kBlockSegs / kLoneSegs : 1;  // a lone pair's items count in fours
+  const int64_t span = plan_span(A, work), block = plan_block(A);
+  const int per = plan_lone(A) ? kBlockSegs / kLoneSegs : 1;  // a lone pair's items count in fours
   const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
   const int64_t na = A.off[a + 1] - A.off[a], nb = A.off[b + 1] - A.off[b];
   const int64_t n = (max(na, nb) + block - 1) / block * ((min(na, nb) + span - 1) / span), s = A.start[p];
@@ -1155,6 +1161,11 @@ __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double 
   for (int64_t x0 = 0; x0 < n; x0 += 32) {  // 32 loads at once, added one after another
     const double v = x0 + lane < n ? A.partial[s + x0 + lane] : 0.0;
     const int m = (int)min(n - x0, (int64_t)32);
+    if (per == 1) {
+#pragma unroll 8
+      for (int j = 0; j < m; ++j) acc += __shfl_sync(0xffffffffu, v, j);
+      continue;
+    }
     for (int j = 0; j < m; ++j) {
       part += __shfl_sync(0xffffffffu, v, j);
       if ((j + 1) % per == 0 || j + 1 == m) {
@@ -1170,10 +1181,11 @@ __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double 
   if (margin >= 0.0 && !(0.5 - fabs(acc - round(acc)) >= margin)) redo[atomicAdd(&A.head->redo, 1ULL)] = (int32_t)p;
 }
 
-// Checks the offsets and pairs and sums n_i n_j (a whole number: exact in any
-// order below 2^53), for the thread's share of them.
+// Checks the offsets and pairs, sums n_i n_j (a whole number: exact in any order
+// below 2^53) and finds the longest loop, for the thread's share of them.
 __device__ __forceinline__ void plan_check(const int64_t *off, int32_t nloops, const int32_t *pairs, int64_t npairs,
-                                           int64_t t, int64_t nt, int &status, double &work) {
+                                           int64_t t, int64_t nt, int &status, double &work,
+                                           unsigned long long &longest) {
   if (t == 0 && off[0] != 0) status |= kBadStart;
   for (int64_t l = t; l < nloops; l += nt)
     if (off[l + 1] < off[l]) status |= kBadOrder;
@@ -1187,13 +1199,14 @@ __device__ __forceinline__ void plan_check(const int64_t *off, int32_t nloops, c
     if (na < 2 || nb < 2) status |= kBadSize;
     if (a == b) status |= kBadSame;
     work += (double)na * (double)nb;
+    longest = max(longest, (unsigned long long)max(max(na, nb), int64_t(0)));
   }
 }
 
 // Items of the pairs [p0 + 32 w, ...) of a warp: reserved with one atomic,
 // pairs in order, and written to the item list.
 __device__ __forceinline__ void plan_warp(const DirectArgs &A, int64_t p, double work, int lane) {
-  const int64_t span = plan_span(A, work), block = plan_block(A, work);
+  const int64_t span = plan_span(A, work), block = plan_block(A);
   int64_t n = 0;
   if (p < A.npairs) {
     const int a = A.pairs[2 * p], b = A.pairs[2 * p + 1];
@@ -1220,8 +1233,10 @@ __device__ __forceinline__ void plan_warp(const DirectArgs &A, int64_t p, double
 __global__ void __launch_bounds__(256) plan_work(DirectArgs A, int32_t nloops) {
   int status = 0;
   double work = 0.0;
+  unsigned long long longest = 0;
   plan_check(A.off, nloops, A.pairs, A.npairs, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
-             (int64_t)gridDim.x * blockDim.x, status, work);
+             (int64_t)gridDim.x * blockDim.x, status, work, longest);
+  if (A.lone > 0 && longest > 0) A.head->longest = longest;  // one pair: one thread has it
   status = __reduce_or_sync(0xffffffffu, status);
   for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
   if ((threadIdx.x & 31) == 0) {
@@ -1246,7 +1261,8 @@ __global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops)
   __syncthreads();
   int status = 0;
   double work = 0.0;
-  plan_check(A.off, nloops, A.pairs, A.npairs, threadIdx.x, 1024, status, work);
+  unsigned long long longest = 0;
+  plan_check(A.off, nloops, A.pairs, A.npairs, threadIdx.x, 1024, status, work, longest);
   status = __reduce_or_sync(0xffffffffu, status);
   for (int o = 16; o; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
   if (lane == 0) {
@@ -1256,7 +1272,8 @@ __global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops)
   __syncthreads();
   work = 0.0;
   for (int x = 0; x < 32; ++x) work += s_work[x];
-  if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, work, s_status, 0};
+  // (A lone pair is thread 0's.)
+  if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, A.lone > 0 ? longest : 0, work, s_status, 0};
   __syncthreads();
   if (s_status) return;
   for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, p, work, lane);
@@ -1292,8 +1309,8 @@ enum class SumKernel { kUnknown, kLone, kFew, kMany };
 
 template <int kB, int kT>
 void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, SumKernel which, const DirectArgs &A) {
-  if (A.lone && which != SumKernel::kMany)
-    direct_fp64_lone_kernel<<<(int)std::min<int64_t>(most, 2 * sms), 256, 0, st>>>(A);
+  if (A.lone > 0 && which != SumKernel::kMany)
+    direct_fp64_lone_kernel<<<(int)std::min(most, kLonePerSm * sms), 256, 0, st>>>(A);
   if (A.few > 0 && which != SumKernel::kMany)
     direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, A.few), kB, 0, st>>>(A);
   if (which == SumKernel::kLone || which == SumKernel::kFew) return;
@@ -1361,7 +1378,7 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   // FP64 sums and large mixed ones are cut along curve 2; a lone FP64 pair has
   // a kernel of its own.
   const double least = precision == FLN_PREC_MIXED ? kMixedSpans : 0.0;
-  const bool lone = precision == FLN_PREC_FP64 && np == 1 && tile_shape == 0;
+  const int64_t lone = precision == FLN_PREC_FP64 && np == 1 && tile_shape == 0 ? kLonePerSm * ctx.num_sms * kLoneSegs : 0;
   int64_t few = precision == FLN_PREC_MIXED ? few_most(tile_shape, ctx.num_sms) : 0;
   if (np > few) few = 0;  // (a pair has at least one item)
   // Room for the items: of the largest call so far, or a guess; a plan that
@@ -1382,8 +1399,10 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
     }
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev2, st));
-    const bool is_lone = lone && tail && tail->known_work >= 0 && tail->known_work < kLoneWork;
-    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, is_lone ? SumKernel::kLone : SumKernel::kUnknown, A);
+    SumKernel which = SumKernel::kUnknown;
+    if (lone > 0 && tail && tail->known_longest > 0)
+      which = tail->known_longest <= lone ? SumKernel::kLone : SumKernel::kMany;
+    launch_direct(tile_shape, st, ctx.num_sms, precision, cap, which, A);
     FLN_CUDA(cudaGetLastError());
     FLN_CUDA(cudaEventRecord(ctx.ev3, st));
     reduce_items_kernel<<<(int)((np + 7) / 8), 256, 0, st>>>(A, margin, d_lk, d_err, d_flags, d_redo);
@@ -1529,7 +1548,7 @@ __global__ void __launch_bounds__(1024) noalloc_plan(const int64_t *off, int32_t
     work = 0.0;
     for (int w = 0; w < 32; ++w) work += s_work[w];
     start[npairs] = s_carry;
-    *h = PlanHead{0, 0, (unsigned long long)s_carry, 0, work, s_status, 0};
+    *h = PlanHead{0, 0, (unsigned long long)s_carry, 0, 0, work, s_status, 0};
   }
 }
 
@@ -1606,7 +1625,7 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   const int64_t most = precision == FLN_PREC_MIXED ? few_most(0, sms) : 0;
   const bool few = few_items((int64_t)h.items, h.work, most);
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, false, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, 0, reinterpret_cast<PlanHead *>(scratch),
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
   launch_direct(0, s, sms, precision, (int64_t)h.items, few ? SumKernel::kFew : SumKernel::kMany, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);

@@ -210,7 +210,7 @@ struct DirectTail {
   void *h_dst = nullptr;  // pinned
   const void *d_src = nullptr;
   size_t bytes = 0;
-  double known_work = -1.0;  // sum of n_i n_j where the host knows it
+  int64_t known_longest = 0;  // of one pair: segments of its longer loop where the host knows it
 };
 constexpr int kDirectTileShapes = 6;
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,

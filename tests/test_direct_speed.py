@@ -75,3 +75,12 @@ def test_mixed_sum_of_near_loops(loops, steps, most):
     and 4.3 when a warp looked for every pair's owner in turn)."""
     c = Calls(*walks([steps] * loops, 5, 1.0), all_pairs(loops))
     assert c.time(c.allocating, N.PREC_MIXED) < most * c.time(c.allocating, N.PREC_FP64)
+
+
+@pytest.mark.parametrize("sizes", [(200000, 20), (200000, 300), (10000, 8572)])
+def test_long_lone_pair(sizes):
+    """A lone FP64 pair with a long loop runs the general kernel: the times of another tile shape,
+    which always does (with the lone pairs' kernel 2.8, 1.8 and 2.3 times as long)."""
+    c = Calls(*walks(sizes, 7, 5.0), all_pairs(2))
+    general = c.time(c.allocating, N.PREC_FP64, direct_tile=1)
+    assert c.time(c.allocating, N.PREC_FP64) < 1.4 * general
