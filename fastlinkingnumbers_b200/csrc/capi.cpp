@@ -508,7 +508,8 @@ void upload_loops(Context &ctx, const double *xyz, const int64_t *loop_offsets, 
 // The polylines of a Discretize on their way to the model, on the context's
 // copy stream from a thread of its own (started only when they are on the
 // device). finish() waits for them and passes their failure on; the destructor
-// waits too, so that nothing outlives a call that throws.
+// waits too, so that nothing outlives a call that throws. Either way a model
+// whose polylines have arrived is prepared.
 class PolylineCopy {
  public:
   PolylineCopy(Context &ctx, Model &m, const DiscretizedOnDevice &d) : ctx_(ctx), m_(m), d_(d) {
@@ -527,20 +528,19 @@ class PolylineCopy {
   }
   PolylineCopy(const PolylineCopy &) = delete;
   PolylineCopy &operator=(const PolylineCopy &) = delete;
-  ~PolylineCopy() {
-    if (!thread_.joinable()) return;
-    thread_.join();
-    release_discretized(ctx_);
-  }
+  ~PolylineCopy() { join(); }
   void finish() {
-    if (!thread_.joinable()) return;
-    thread_.join();
+    join();
     if (failure_) std::rethrow_exception(failure_);
-    m_.prepared = true;
-    release_discretized(ctx_);
   }
 
  private:
+  void join() {
+    if (!thread_.joinable()) return;
+    thread_.join();
+    if (!failure_) m_.prepared = true;
+    release_discretized(ctx_);
+  }
   Context &ctx_;
   Model &m_;
   DiscretizedOnDevice d_;
