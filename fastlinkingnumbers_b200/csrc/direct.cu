@@ -45,6 +45,7 @@
 #include <string>
 
 #include "engine.hpp"
+#include "root.cuh"
 
 namespace fln {
 namespace {
@@ -223,18 +224,6 @@ __device__ __forceinline__ int renorm(double &x, double &y) {
   x *= s;
   y *= s;
   return e;
-}
-
-// sqrt(x) for x > 0, within an ulp: the hardware's approximate reciprocal
-// root y (relative error below 2^-19) and one Householder step of third order
-// on h = x y with e = 1 - h y: sqrt(x) = h (1 + e/2 + 3/8 e^2 + O(e^3)). Five
-// FP64 operations and no branch.
-__device__ __forceinline__ double root(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = x * y;
-  const double e = fma(-h, y, 1.0);
-  return fma(fma(0.375, e, 0.5), e * h, h);
 }
 
 // A sum of angles as a complex product (x, y) and a count of full turns (the
