@@ -2897,13 +2897,17 @@ int barnes_hut_device(Context &ctx, const double *d_xyz, const int64_t *d_off, c
     // A call larger than those before it: a record for every 16 segments of
     // each pair of loops as long as the longest (60 walks of 2,000 steps write
     // one for every 110 of theirs, 200 walks of 50,000 one for every 440), so
-    // that small calls do not take the memory of large ones.
+    // that small calls do not take the memory of large ones; and a fifth of the
+    // free memory at most, which other programs may want too. (Pairs whose
+    // records do not fit are retried from the roots: 400 walks of 50,000 steps
+    // write 9.75M of the 9.5M that 32 GB hold, 218 ms for the first call and 202
+    // once the buffer has grown.)
     const size_t guess = (size_t)np * (size_t)(4 + longest / 8);
     size_t want = have;
     if (guess > ctx.bh_front_guess || want_hint > have) {  // the buffer may have to grow: ask how much memory is free
       size_t free_b = 0, total_b = 0;
       FLN_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      const size_t room = std::min<size_t>((size_t)32 << 30, free_b / 3) / sizeof(FrontRec);
+      const size_t room = std::min<size_t>((size_t)32 << 30, free_b / 5) / sizeof(FrontRec);
       if (guess > ctx.bh_front_guess) want = std::max(want, std::min(guess, room));
       want = std::max(want, want_hint);
       ctx.bh_front_guess = std::max(ctx.bh_front_guess, guess);
