@@ -595,6 +595,9 @@ __device__ __forceinline__ F2 dot2(const F2x3 &a, const F2x3 &b) {
 // of x / 4, which changes nothing for larger x. Between the two a term takes the
 // full arctangent. (Tests of x and y themselves cost 1 to 3 %.)
 constexpr float kSmallX = 0x1p-90f, kNearLeast = 1e-6f;
+// The segment length whose near distance is kNearLeast, taken in place of
+// shorter ones (near_factor 0: not a number, and no pair is near).
+__device__ __forceinline__ float least_length(float near_factor) { return kNearLeast / near_factor; }
 
 __device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, float by, float bz) {
   return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
@@ -658,7 +661,7 @@ struct MixWalk {
 struct MixSegs {
   F2x3 ra, rb;  // p_j, p_{j+1} relative to the tile's origin
   F2x3 e, ne;   // e = p_{j+1} - p_j and -e
-  float near0, near1;  // near_factor x their lengths, kNearLeast at least
+  float near0, near1;  // near_factor x their lengths
 };
 
 // Vectors and norms of the walk at vertex v. The products of the shared
@@ -800,10 +803,10 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
       const float x1 = (float)(p2.x - p1.x), y1 = (float)(p2.y - p1.y), z1 = (float)(p2.z - p1.z);
       S.e = F2x3{pack2(x0, x1), pack2(y0, y1), pack2(z0, z1)};
       S.ne = F2x3{neg2(S.e.x), neg2(S.e.y), neg2(S.e.z)};
-      len0 = sqrtf(dot_f(x0, y0, z0, x0, y0, z0));
-      len1 = sqrtf(dot_f(x1, y1, z1, x1, y1, z1));
-      S.near0 = fmaxf(A.near_factor * len0, kNearLeast);
-      S.near1 = fmaxf(A.near_factor * len1, kNearLeast);
+      len0 = fmaxf(sqrtf(dot_f(x0, y0, z0, x0, y0, z0)), least_length(A.near_factor));
+      len1 = fmaxf(sqrtf(dot_f(x1, y1, z1, x1, y1, z1)), least_length(A.near_factor));
+      S.near0 = A.near_factor * len0;
+      S.near1 = A.near_factor * len1;
     }
     double acc0 = 0.0, acc1 = 0.0, near0 = 0.0, near1 = 0.0;
     int turns0 = 0, turns1 = 0, queued = 0;
@@ -860,11 +863,11 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
       block_minmax7<kThreads>(lo, hi, s_box, bx);
       __syncthreads();
       // Box gap between the CTA's curve-1 segments and this tile: no segment
-      // pair can be near when it exceeds near_factor x (longest segment) and kNearLeast.
+      // pair can be near when it exceeds near_factor x (longest segment).
       const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
       const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
       const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
-      const float lim = fmaxf(A.near_factor * bx[10], kNearLeast);
+      const float lim = A.near_factor * bx[10];
       const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
       // The runs of 32 steps of this thread's group.
       const int runs = (kt + 31) / 32, ra = runs * grp / groups, rb = runs * (grp + 1) / groups;
@@ -1008,7 +1011,7 @@ __device__ __forceinline__ float atan_small(float t) {
 // 12 of 2,000 (1,056) 2,144 / 2,766.
 template <int kB, int kT>
 __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
-  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = near_factor x length of segment t
+  __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = length of segment t
   __shared__ double s_red[kB / 32];
   __shared__ float s_box[kB / 32][14];
   const float INF = __int_as_float(0x7f800000);
@@ -1024,7 +1027,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
     p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
   }
   const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
-  const float len1 = sqrtf(ex * ex + ey * ey + ez * ez), near1 = fmaxf(A.near_factor * len1, kNearLeast);
+  const float len1 = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez), least_length(A.near_factor));
   double acc = 0.0, near_turns = 0.0;
   int turns = 0;
   unsigned near_count = 0;
@@ -1057,7 +1060,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
       const float4 a = sq[t], b = sq[t + 1];
       const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
       const float len = sqrtf(fx * fx + fy * fy + fz * fz);
-      sq[t].w = A.near_factor * len;
+      sq[t].w = len;
       lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
       lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
       lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
@@ -1067,11 +1070,11 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
     block_minmax7<kB>(lo, hi, s_box, bx);
     __syncthreads();
     // Box gap between the CTA's curve-1 segments and this tile: no segment
-    // pair can be near when it exceeds near_factor x (longest segment) and kNearLeast.
+    // pair can be near when it exceeds near_factor x (longest segment).
     const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
     const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
     const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
-    const float lim = fmaxf(A.near_factor * bx[10], kNearLeast);
+    const float lim = A.near_factor * bx[10];
     const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
     if (!active) continue;
     float4 q = sq[0];
@@ -1089,7 +1092,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
       const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
       const float cd = cx * dx + cy * dy + cz * dz;
       bool near = false;
-      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < fmaxf(near1, q.w);
+      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
       if (near) {
         const int64_t kk = k0 + k, kn = kk + 1;
         near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
@@ -1107,7 +1110,7 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
         const float xp = div1 * div2 - det * det;
         const float yp = det * sdiv;
         float term;
-        if (sdiv > 0.f && fabsf(yp) < __fmaf_rn(xp, 0.25f, -kSmallX)) {
+        if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
           term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
         } else {
           term = atan2f(yp, xp);
