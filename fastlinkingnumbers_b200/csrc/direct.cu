@@ -65,6 +65,7 @@ struct PlanHead {
   int32_t status;            // kBad* bits
   int32_t pad;
 };
+constexpr int kSmRanks = 256;  // sm_turn: CTAs per SM that asked, and one counter for all, behind the head
 constexpr int kBadStart = 1, kBadOrder = 2, kBadPair = 4, kBadSize = 8, kBadSame = 16;
 
 struct DirectArgs {
@@ -81,6 +82,8 @@ struct DirectArgs {
   int64_t few;                // mixed: most items of a call for direct_mixed_few_kernel (few_items); 0: none
   int64_t lone;               // one pair in FP64: the longest loop for direct_fp64_lone_kernel; 0: none
   PlanHead *head;
+  unsigned *sm_rank;          // kSmRanks + 1 counters, 0 at first; null: the grid has no more CTAs than items
+  int sms;
   double *partial;            // per item
   float near_factor;
 };
@@ -158,19 +161,40 @@ __device__ __forceinline__ int64_t plan_ready(const DirectArgs &A) {
   const int64_t n = (int64_t)A.head->items;
   return A.head->status == 0 && n <= A.cap ? n : 0;
 }
-// A mixed plan of few items (direct_mixed_few_kernel): at most `most`, the CTAs
-// of that kernel that fit the chip at once (beyond, it needs a second wave: 9
-// walks of 2,000 steps, 576 items of 592: 1.91 ms packed, 1.83 by this kernel;
-// 10 of 2,000, 720 items: 1.64 and 1.95), and loops longer than those of which
-// the packed kernel gives the runs to two groups of threads (15 x 15 linked rings
-// of 64 segments: 114 us packed, 123 by this kernel; 20 walks of 72 steps, all
-// pairs near: 256 and 141).
+// A mixed plan of few items (direct_mixed_few_kernel). Calls by the packed kernel
+// / by this one:
+//  - at most `most` items, the CTAs of this kernel that fit the chip at once; it
+//    needs a second wave beyond (9 walks of 2,000 steps, 576 items of 592: 1.97 /
+//    1.74 ms; 10 of 2,000, 720 items: 1.57 / 1.95);
+//  - loops longer than those of which the packed kernel gives the runs to two
+//    groups of threads (200 linked rings of 64 segments: 79 / 91 us, but 20 walks
+//    of 30 steps, all pairs near: 120 / 92; 20 of 72 steps: 228 / 139);
+//  - walks of curve 2 of at most 3,500 segments: longer ones meet enough near
+//    pairs for the packed kernel's warps to evaluate them together (4 of 500
+//    steps 0.80 / 0.49 ms; 2 of 3,000 1.15 to 1.97 / 1.42 to 1.69;
+//    6 of 4,000 1.57 to 2.35 / 1.78 to 2.27; 10,000 2.08 to 2.21 / 2.48 to 2.73; two
+//    stretches of 10,000 of one walk 4.26 / 8.69).
 constexpr double kFewWork = 64 * 64;  // segment pairs per item, more than
+constexpr double kFewMost = 128 * 3500.0;
 __host__ __device__ __forceinline__ bool few_items(int64_t items, double work, int64_t most) {
-  return items <= most && work < kMixedSpans && work > kFewWork * (double)items;
+  return items <= most && work < kMixedSpans && work > kFewWork * (double)items && work < kFewMost * (double)items;
 }
 __device__ __forceinline__ bool plan_few(const DirectArgs &A) {
   return A.few > 0 && few_items((int64_t)A.head->items, A.head->work, A.few);
+}
+
+// Whether this CTA takes items of a plan with fewer items than CTAs (thread 0
+// asks): items / SMs CTAs on each SM do, and one more on as many as the
+// remainder. All CTAs at the queue at once, two items often met on one SM while
+// others had none (3 walks of 5,000 steps far apart, 120 items: 1.19 ms by CTA
+// number, 1.01 this way). The queue hands out every item as long as one CTA takes
+// part, and the first to ask does.
+__device__ __forceinline__ bool sm_turn(const DirectArgs &A, int64_t items) {
+  if (!A.sm_rank || items >= (int64_t)gridDim.x) return true;
+  unsigned sm;
+  asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+  const int64_t each = items / A.sms, rank = atomicAdd(&A.sm_rank[sm % kSmRanks], 1u);
+  return rank < each || (rank == each && atomicAdd(&A.sm_rank[kSmRanks], 1u) < items % A.sms);
 }
 
 __device__ __forceinline__ double3 load_v(const double *xyz, int64_t v) {
@@ -780,9 +804,9 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
   unsigned *mine = s_mine[threadIdx.x >> 5];
   const int64_t items = plan_few(A) ? 0 : plan_ready(A), span = plan_span(A, A.head->work);
   unsigned long long near_count = 0;
+  if (threadIdx.x == 0) s_item = items > 0 && sm_turn(A, items) ? 0 : INT64_MAX;
   for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
+    if (threadIdx.x == 0 && s_item < INT64_MAX) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
     __syncthreads();
     const int64_t item = s_item;
     if (item >= items) break;
@@ -1004,134 +1028,139 @@ __device__ __forceinline__ float atan_small(float t) {
 // The mixed sum of few items, one segment per thread: with at most a few CTAs
 // per SM a call lasts as long as one thread's walk, and a walk of two packed
 // segments takes longer than a walk of one. Terms, runs and sums are those of
-// direct_mixed_kernel, bit for bit. A CTA takes the item of its number: taken
-// from the queue, two items often met on one SM while others had none (5 walks
-// of 998 steps: 900 us). Whole calls, packed / this: 4 walks of 500 steps (24
-// items) 797 / 492 us, 5 of 998 (80) 1,268 / 880, 8 of 2,000 (448) 1,495 / 1,363,
-// 12 of 2,000 (1,056) 2,144 / 2,766.
+// direct_mixed_kernel, bit for bit (down to distances of 2e-5, see kSmallX).
+// The times of both stand at few_items.
 template <int kB, int kT>
 __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
   __shared__ float4 sq[kT + 1];  // xyz relative to the tile origin; w = length of segment t
   __shared__ double s_red[kB / 32];
   __shared__ float s_box[kB / 32][14];
   const float INF = __int_as_float(0x7f800000);
-  const int64_t item = blockIdx.x;
-  if (!plan_few(A) || item >= plan_ready(A)) return;
-  const Item it = item_of(A, item, kB, int64_t(1) << 62);
-  const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
-  const int64_t i = it.first + threadIdx.x;
-  const bool active = i < n1;
-  double3 p0 = make_double3(0, 0, 0), p1 = p0;
-  if (active) {
-    p0 = load_v(A.xyz, o1 + i);
-    p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
-  }
-  const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
-  const float len1 = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez), least_length(A.near_factor));
-  double acc = 0.0, near_turns = 0.0;
-  int turns = 0;
+  __shared__ long long s_item;
+  const int64_t items = plan_few(A) ? plan_ready(A) : 0;
+  if (items == 0) return;
+  if (threadIdx.x == 0) s_item = sm_turn(A, items) ? 0 : INT64_MAX;
   unsigned near_count = 0;
-  for (int64_t k0 = 0; k0 < n2; k0 += kT) {
-    const int kt = (int)min(n2 - k0, (int64_t)kT);
-    const double3 O = load_v(A.xyz, o2 + k0);
+  for (;;) {
+    if (threadIdx.x == 0 && s_item < INT64_MAX) s_item = (long long)atomicAdd(&A.head->queue, 1ULL);
     __syncthreads();
-    for (int t = threadIdx.x; t <= kt; t += kB) {
-      const int64_t kk = k0 + t;
-      const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
-      sq[t] = make_float4((float)(v.x - O.x), (float)(v.y - O.y), (float)(v.z - O.z), 0.f);
-    }
-    __syncthreads();
-    const float r0x = (float)(p0.x - O.x), r0y = (float)(p0.y - O.y), r0z = (float)(p0.z - O.z);
-    const float r1x = (float)(p1.x - O.x), r1y = (float)(p1.y - O.y), r1z = (float)(p1.z - O.z);
-    // Boxes of this thread's curve-1 segment (slots 0-2, length 3) and of
-    // its curve-2 tile vertices (slots 4-6, length 3 of the max).
-    float lo[7], hi[7];
-    for (int v = 0; v < 7; ++v) {
-      lo[v] = INF;
-      hi[v] = -INF;
-    }
+    const int64_t item = s_item;
+    if (item >= items) break;
+    const Item it = item_of(A, item, kB, int64_t(1) << 62);
+    const int64_t o1 = it.o1, n1 = it.n1, o2 = it.o2, n2 = it.n2;
+    const int64_t i = it.first + threadIdx.x;
+    const bool active = i < n1;
+    double3 p0 = make_double3(0, 0, 0), p1 = p0;
     if (active) {
-      lo[0] = fminf(r0x, r1x); hi[0] = fmaxf(r0x, r1x);
-      lo[1] = fminf(r0y, r1y); hi[1] = fmaxf(r0y, r1y);
-      lo[2] = fminf(r0z, r1z); hi[2] = fmaxf(r0z, r1z);
-      hi[3] = len1;
+      p0 = load_v(A.xyz, o1 + i);
+      p1 = load_v(A.xyz, o1 + (i + 1 == n1 ? 0 : i + 1));
     }
-    for (int t = threadIdx.x; t < kt; t += kB) {
-      const float4 a = sq[t], b = sq[t + 1];
-      const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
-      const float len = sqrtf(fx * fx + fy * fy + fz * fz);
-      sq[t].w = len;
-      lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
-      lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
-      lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
-      hi[3] = fmaxf(hi[3], len);
-    }
-    float bx[14];
-    block_minmax7<kB>(lo, hi, s_box, bx);
-    __syncthreads();
-    // Box gap between the CTA's curve-1 segments and this tile: no segment
-    // pair can be near when it exceeds near_factor x (longest segment).
-    const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
-    const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
-    const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
-    const float lim = A.near_factor * bx[10];
-    const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
-    if (!active) continue;
-    float4 q = sq[0];
-    float ax = q.x - r0x, ay = q.y - r0y, az = q.z - r0z;
-    float bx_ = q.x - r1x, by = q.y - r1y, bz = q.z - r1z;
-    const float aa = ax * ax + ay * ay + az * az, bb = bx_ * bx_ + by * by + bz * bz;
-    float la = sqrtf(aa), lb = sqrtf(bb);
-    float ab = ax * bx_ + ay * by + az * bz;
-    float accf = 0.f;
-    for (int k = 0; k < kt; ++k) {
-      const float4 qn = sq[k + 1];
-      const float cx = qn.x - r1x, cy = qn.y - r1y, cz = qn.z - r1z;
-      const float dx = qn.x - r0x, dy = qn.y - r0y, dz = qn.z - r0z;
-      const float cc = cx * cx + cy * cy + cz * cz, dd = dx * dx + dy * dy + dz * dz;
-      const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
-      const float cd = cx * dx + cy * dy + cz * dz;
-      bool near = false;
-      if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
-      if (near) {
-        const int64_t kk = k0 + k, kn = kk + 1;
-        near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
-        ++near_count;
-      } else {
-        const float ca = cx * ax + cy * ay + cz * az;
-        const float cb = cx * bx_ + cy * by + cz * bz;
-        const float ad = ax * dx + ay * dy + az * dz;
-        const float fx = qn.x - q.x, fy = qn.y - q.y, fz = qn.z - q.z;
-        const float det = ax * (fy * ez - fz * ey) + ay * (fz * ex - fx * ez) + az * (fx * ey - fy * ex);
-        const float t = la * lc;
-        const float div1 = t * lb + ab * lc + ca * lb + cb * la;
-        const float div2 = t * ld + ad * lc + ca * ld + cd * la;
-        const float sdiv = div1 + div2;
-        const float xp = div1 * div2 - det * det;
-        const float yp = det * sdiv;
-        float term;
-        if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
-          term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
+    const float ex = (float)(p1.x - p0.x), ey = (float)(p1.y - p0.y), ez = (float)(p1.z - p0.z);
+    const float len1 = fmaxf(sqrtf(ex * ex + ey * ey + ez * ez), least_length(A.near_factor));
+    double acc = 0.0, near_turns = 0.0;
+    int turns = 0;
+    for (int64_t k0 = 0; k0 < n2; k0 += kT) {
+      const int kt = (int)min(n2 - k0, (int64_t)kT);
+      const double3 O = load_v(A.xyz, o2 + k0);
+      __syncthreads();
+      for (int t = threadIdx.x; t <= kt; t += kB) {
+        const int64_t kk = k0 + t;
+        const double3 v = load_v(A.xyz, o2 + (kk == n2 ? 0 : kk));
+        sq[t] = make_float4((float)(v.x - O.x), (float)(v.y - O.y), (float)(v.z - O.z), 0.f);
+      }
+      __syncthreads();
+      const float r0x = (float)(p0.x - O.x), r0y = (float)(p0.y - O.y), r0z = (float)(p0.z - O.z);
+      const float r1x = (float)(p1.x - O.x), r1y = (float)(p1.y - O.y), r1z = (float)(p1.z - O.z);
+      // Boxes of this thread's curve-1 segment (slots 0-2, length 3) and of
+      // its curve-2 tile vertices (slots 4-6, length 3 of the max).
+      float lo[7], hi[7];
+      for (int v = 0; v < 7; ++v) {
+        lo[v] = INF;
+        hi[v] = -INF;
+      }
+      if (active) {
+        lo[0] = fminf(r0x, r1x); hi[0] = fmaxf(r0x, r1x);
+        lo[1] = fminf(r0y, r1y); hi[1] = fmaxf(r0y, r1y);
+        lo[2] = fminf(r0z, r1z); hi[2] = fmaxf(r0z, r1z);
+        hi[3] = len1;
+      }
+      for (int t = threadIdx.x; t < kt; t += kB) {
+        const float4 a = sq[t], b = sq[t + 1];
+        const float fx = b.x - a.x, fy = b.y - a.y, fz = b.z - a.z;
+        const float len = sqrtf(fx * fx + fy * fy + fz * fz);
+        sq[t].w = len;
+        lo[4] = fminf(lo[4], fminf(a.x, b.x)); hi[4] = fmaxf(hi[4], fmaxf(a.x, b.x));
+        lo[5] = fminf(lo[5], fminf(a.y, b.y)); hi[5] = fmaxf(hi[5], fmaxf(a.y, b.y));
+        lo[6] = fminf(lo[6], fminf(a.z, b.z)); hi[6] = fmaxf(hi[6], fmaxf(a.z, b.z));
+        hi[3] = fmaxf(hi[3], len);
+      }
+      float bx[14];
+      block_minmax7<kB>(lo, hi, s_box, bx);
+      __syncthreads();
+      // Box gap between the CTA's curve-1 segments and this tile: no segment
+      // pair can be near when it exceeds near_factor x (longest segment).
+      const float gx = fmaxf(0.f, fmaxf(bx[4] - bx[7], bx[0] - bx[11]));
+      const float gy = fmaxf(0.f, fmaxf(bx[5] - bx[8], bx[1] - bx[12]));
+      const float gz = fmaxf(0.f, fmaxf(bx[6] - bx[9], bx[2] - bx[13]));
+      const float lim = A.near_factor * bx[10];
+      const bool far_tile = gx * gx + gy * gy + gz * gz > 1.0001f * lim * lim;
+      if (!active) continue;
+      float4 q = sq[0];
+      float ax = q.x - r0x, ay = q.y - r0y, az = q.z - r0z;
+      float bx_ = q.x - r1x, by = q.y - r1y, bz = q.z - r1z;
+      const float aa = ax * ax + ay * ay + az * az, bb = bx_ * bx_ + by * by + bz * bz;
+      float la = sqrtf(aa), lb = sqrtf(bb);
+      float ab = ax * bx_ + ay * by + az * bz;
+      float accf = 0.f;
+      for (int k = 0; k < kt; ++k) {
+        const float4 qn = sq[k + 1];
+        const float cx = qn.x - r1x, cy = qn.y - r1y, cz = qn.z - r1z;
+        const float dx = qn.x - r0x, dy = qn.y - r0y, dz = qn.z - r0z;
+        const float cc = cx * cx + cy * cy + cz * cz, dd = dx * dx + dy * dy + dz * dz;
+        const float lc = cc * rsqrtf(cc), ld = dd * rsqrtf(dd);
+        const float cd = cx * dx + cy * dy + cz * dz;
+        bool near = false;
+        if (!far_tile) near = fminf(fminf(la, lb), fminf(lc, ld)) < A.near_factor * fmaxf(len1, q.w);
+        if (near) {
+          const int64_t kk = k0 + k, kn = kk + 1;
+          near_turns += term_fp64(p0, p1, load_v(A.xyz, o2 + kk), load_v(A.xyz, o2 + (kn == n2 ? 0 : kn)));
+          ++near_count;
         } else {
-          term = atan2f(yp, xp);
-          if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;
+          const float ca = cx * ax + cy * ay + cz * az;
+          const float cb = cx * bx_ + cy * by + cz * bz;
+          const float ad = ax * dx + ay * dy + az * dz;
+          const float fx = qn.x - q.x, fy = qn.y - q.y, fz = qn.z - q.z;
+          const float det = ax * (fy * ez - fz * ey) + ay * (fz * ex - fx * ez) + az * (fx * ey - fy * ex);
+          const float t = la * lc;
+          const float div1 = t * lb + ab * lc + ca * lb + cb * la;
+          const float div2 = t * ld + ad * lc + ca * ld + cd * la;
+          const float sdiv = div1 + div2;
+          const float xp = div1 * div2 - det * det;
+          const float yp = det * sdiv;
+          float term;
+          if (sdiv > 0.f && fabsf(yp) < 0.25f * xp) {
+            term = atan_small(__fdividef(yp, xp));  // principal branch, |angle| < 0.245
+          } else {
+            term = atan2f(yp, xp);
+            if (sdiv < 0.f && det != 0.f) turns += (det > 0.f) ? 1 : -1;
+          }
+          accf += term;
         }
-        accf += term;
+        if ((k & 31) == 31) {
+          acc += (double)accf;
+          accf = 0.f;
+        }
+        q = qn;
+        ax = dx; ay = dy; az = dz;
+        bx_ = cx; by = cy; bz = cz;
+        la = ld; lb = lc; ab = cd;
       }
-      if ((k & 31) == 31) {
-        acc += (double)accf;
-        accf = 0.f;
-      }
-      q = qn;
-      ax = dx; ay = dy; az = dz;
-      bx_ = cx; by = cy; bz = cz;
-      la = ld; lb = lc; ab = cd;
+      acc += (double)accf;
     }
-    acc += (double)accf;
+    const double v = active ? acc * kInvTwoPi + (double)turns + near_turns : 0.0;
+    const double s = block_sum<kB>(v, s_red);
+    if (threadIdx.x == 0) A.partial[item] = s;
   }
-  const double v = active ? acc * kInvTwoPi + (double)turns + near_turns : 0.0;
-  const double s = block_sum<kB>(v, s_red);
-  if (threadIdx.x == 0) A.partial[item] = s;
   if (near_count) atomicAdd(&A.head->near, (unsigned long long)near_count);
 }
 
@@ -1266,6 +1295,7 @@ __global__ void __launch_bounds__(1024) plan_small(DirectArgs A, int32_t nloops)
   for (int x = 0; x < 32; ++x) work += s_work[x];
   // (A lone pair is thread 0's.)
   if (threadIdx.x == 0) *A.head = PlanHead{0, 0, 0, 0, A.lone > 0 ? longest : 0, work, s_status, 0};
+  if (threadIdx.x <= kSmRanks) A.sm_rank[threadIdx.x] = 0;
   __syncthreads();
   if (s_status) return;
   for (int64_t p = threadIdx.x; p - lane < A.npairs; p += 1024) plan_warp(A, p, work, lane);
@@ -1362,7 +1392,9 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   if (np > INT32_MAX) throw Error(FLN_ERR_INVALID_ARGUMENT, "more than 2^31 - 1 pairs");
   const int kB = kShapes[tile_shape].block;
   cudaStream_t st = ctx.stream;
-  PlanHead *d_head = ctx.d_counter.as<PlanHead>(1);
+  constexpr size_t kHeadBytes = sizeof(PlanHead) + (kSmRanks + 1) * sizeof(unsigned);
+  PlanHead *d_head = static_cast<PlanHead *>(ctx.d_counter.need(kHeadBytes));
+  unsigned *d_rank = reinterpret_cast<unsigned *>(d_head + 1);
   int64_t *d_start = ctx.d_items.as<int64_t>(np);
   int32_t *d_redo = margin >= 0 ? ctx.d_near.as<int32_t>(np) : nullptr;
   PlanHead &head = *static_cast<PlanHead *>(ctx.h_head.need(sizeof(PlanHead)));
@@ -1379,11 +1411,11 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   for (int attempt = 0;; ++attempt) {
     const int64_t cap = ctx.direct_items;
     DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, kB, few, lone,
-                 d_head, ctx.d_partial.as<double>(cap), (float)near_factor};
+                 d_head, d_rank, ctx.num_sms, ctx.d_partial.as<double>(cap), (float)near_factor};
     if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
       plan_small<<<1, 1024, 0, st>>>(A, nloops);
     } else {
-      FLN_CUDA(cudaMemsetAsync(d_head, 0, sizeof(PlanHead), st));
+      FLN_CUDA(cudaMemsetAsync(d_head, 0, kHeadBytes, st));
       const int64_t most = std::max<int64_t>(np, nloops);
       plan_work<<<(int)std::min<int64_t>((most + 255) / 256, 8 * ctx.num_sms), 256, 0, st>>>(A, nloops);
       plan_items<<<(int)((np + 255) / 256), 256, 0, st>>>(A);
@@ -1617,7 +1649,7 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   const int64_t most = precision == FLN_PREC_MIXED ? few_most(0, sms) : 0;
   const bool few = few_items((int64_t)h.items, h.work, most);
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
-                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, 0, reinterpret_cast<PlanHead *>(scratch),
+                     (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, 0, reinterpret_cast<PlanHead *>(scratch), nullptr, sms,
                      reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
   launch_direct(0, s, sms, precision, (int64_t)h.items, few ? SumKernel::kFew : SumKernel::kMany, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
