@@ -34,3 +34,20 @@ def test_large_mixed_sum(sizes):
     np.testing.assert_allclose(c.lk.cpu().numpy(), whole, rtol=0, atol=1e-9)
     c.allocating(N.PREC_FP64)
     np.testing.assert_allclose(c.lk.cpu().numpy(), whole, rtol=0, atol=1e-5)
+
+
+# Mixed plans with fewer items than CTAs: around the numbers of SMs (148) and of the few-items
+# kernel's CTAs (592), by it (curve 2 of 300 segments) and by the packed one (30).
+@pytest.mark.parametrize("other", [30, 300])
+@pytest.mark.parametrize("items", [1, 2, 147, 148, 149, 296, 591, 592, 593, 1183, 1184, 1185])
+def test_few_items(items, other):
+    c = Calls(*walks((128 * items - 5, other), items, 5.0), all_pairs(2))
+    c.noalloc(N.PREC_MIXED)  # a grid of as many CTAs as items
+    ref = c.lk.cpu().numpy().copy()
+    for _ in range(3):
+        c.lk.fill_(7.0)
+        c.torch.cuda.synchronize()
+        c.allocating(N.PREC_MIXED, fp64_margin=-1.0)
+        assert c.lk.cpu().numpy()[0] == ref[0]
+    c.allocating(N.PREC_FP64)
+    np.testing.assert_allclose(c.lk.cpu().numpy(), ref, rtol=0, atol=1e-5)
