@@ -86,6 +86,7 @@ struct DirectArgs {
   int sms;
   double *partial;            // per item
   float near_factor;
+  bool wide;                  // FP64: the kernel that forms shares out of range again (host)
 };
 
 // Curve-2 segments per item. A call whose pairs give few items of kBlockSegs
@@ -374,11 +375,14 @@ __device__ __noinline__ double sum_terms(const double *xyz, int64_t o1, int64_t 
 // between rescalings, so the product overflows above d = 1e25 and loses digits
 // below 1e-23 (a single term below 1e-50), or when two vertices meet. The
 // smallest product before a rescaling is kept (one integer minimum per two
-// steps and segment); a thread that saw one below kLeastScale, or whose product
-// is not finite, forms its share again term by term (sum_terms). The 12 walks:
-// 6.04 ms a call without this, 6.16 with it.
+// steps and segment); the share of a thread that saw one below kLeastScale, or
+// whose product is not finite, is not a number, which its pair's sum shows to
+// the reduction. kWide forms such a share again term by term (sum_terms); that
+// code costs the others 1.5 %, so a call runs the kernel without it and has the
+// pairs concerned summed again. The 12 walks: 6.01 ms a call without any of
+// this, 6.02 with the check, 6.13 with kWide.
 constexpr int kLeastScale = (1023 - 900) << 20;  // exponent bits of 2^-900: two terms at d = 1e-23
-template <int kB, int kT>
+template <int kB, int kT, bool kWide = false>
 __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_kernel(DirectArgs A) {
   __shared__ TileVertex tile[kT + 1];
   __shared__ double s_red[kB / 32];
@@ -442,7 +446,10 @@ __global__ void __launch_bounds__(kB, 384 / kB > 0 ? 384 / kB : 1) direct_fp64_k
     }
     double v = 0.0;
     if (active && (least < kLeastScale || !(fabs(s0.x) + fabs(s0.y) + fabs(s1.x) + fabs(s1.y) < 1e300))) {
-      v = sum_terms(A.xyz, o1, n1, it.first + at, second ? 2 : 1, o2, n2, it.k0, it.k1, kT, grp, groups);
+      if constexpr (kWide)
+        v = sum_terms(A.xyz, o1, n1, it.first + at, second ? 2 : 1, o2, n2, it.k0, it.k1, kT, grp, groups);
+      else
+        v = __longlong_as_double(0x7ff8000000000000ll);
     } else if (active) {
       if (second) {
         s0.add(s1.x, s1.y, 0.0, 0.0);
@@ -1165,9 +1172,9 @@ __global__ void __launch_bounds__(kB) direct_mixed_few_kernel(DirectArgs A) {
 }
 
 // Sums the item partials of each pair, a warp per pair, in item order, and
-// checks the sum's margin to the rounding boundary (margin < 0: no check):
-// pairs that fail it, or are not finite, go to the list `redo`. The estimate
-// and the flags of a direct sum are 0.
+// checks it if there is a list `redo`: sums that are not numbers go there and,
+// with a margin >= 0, those nearer than that to the rounding boundary. The
+// estimate and the flags of a direct sum are 0.
 __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double margin, double *lk, double *err, int32_t *flags, int32_t *redo) {
   const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1199,7 +1206,7 @@ __global__ void __launch_bounds__(256) reduce_items_kernel(DirectArgs A, double 
   lk[p] = acc;
   if (err) err[p] = 0.0;
   if (flags) flags[p] = 0;
-  if (margin >= 0.0 && !(0.5 - fabs(acc - round(acc)) >= margin)) redo[atomicAdd(&A.head->redo, 1ULL)] = (int32_t)p;
+  if (redo && !(0.5 - fabs(acc - round(acc)) >= margin)) redo[atomicAdd(&A.head->redo, 1ULL)] = (int32_t)p;
 }
 
 // Checks the offsets and pairs, sums n_i n_j (a whole number: exact in any order
@@ -1336,7 +1343,9 @@ void launch_direct_t(cudaStream_t st, int sms, int precision, int64_t most, SumK
   if (A.few > 0 && which != SumKernel::kMany)
     direct_mixed_few_kernel<kB, kT><<<(int)std::min(most, A.few), kB, 0, st>>>(A);
   if (which == SumKernel::kLone || which == SumKernel::kFew) return;
-  auto kernel = precision == FLN_PREC_FP64 ? direct_fp64_kernel<kB, kT> : direct_mixed_kernel<kB, kT>;
+  auto kernel = precision != FLN_PREC_FP64 ? direct_mixed_kernel<kB, kT> : direct_fp64_kernel<kB, kT>;
+  if constexpr (kB == kBlockSegs && kT == kTile)
+    if (precision == FLN_PREC_FP64 && A.wide) kernel = direct_fp64_kernel<kB, kT, true>;
   const int threads = precision == FLN_PREC_FP64 ? kB : kB / 2;
   const int64_t resident = (int64_t)sms * occupancy_of((const void *)kernel, threads);
   kernel<<<(int)std::max<int64_t>(1, std::min(most, resident)), threads, 0, st>>>(A);
@@ -1376,7 +1385,8 @@ int recompute_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, int
   gather_pairs<<<grid, 256, 0, ctx.stream>>>(list, n, d_pairs, pairs);
   FLN_CUDA(cudaGetLastError());
   const int launches =
-      direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, n, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr, nullptr).launches;
+      direct_sum_device(ctx, d_xyz, d_off, nloops, pairs, n, FLN_PREC_FP64, 0.0, -1.0, sums, nullptr, nullptr, 0, nullptr,
+                        true).launches;
   scatter_redo<<<grid, 256, 0, ctx.stream>>>(list, n, sums, d_lk, d_flags);
   FLN_CUDA(cudaGetLastError());
   return launches + 2;
@@ -1384,7 +1394,8 @@ int recompute_pairs(Context &ctx, const double *d_xyz, const int64_t *d_off, int
 
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
                                const int32_t *d_pairs, int64_t np, int precision, double near_factor, double margin,
-                               double *d_lk, double *d_err, int32_t *d_flags, int tile_shape, const DirectTail *tail) {
+                               double *d_lk, double *d_err, int32_t *d_flags, int tile_shape, const DirectTail *tail,
+                               bool wide) {
   if (tile_shape < 0 || tile_shape >= kDirectTileShapes)
     throw Error(FLN_ERR_INVALID_ARGUMENT, "direct_tile in [0, " + std::to_string(kDirectTileShapes - 1) + "]");
   DirectResult R;
@@ -1396,7 +1407,7 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   PlanHead *d_head = static_cast<PlanHead *>(ctx.d_counter.need(kHeadBytes));
   unsigned *d_rank = reinterpret_cast<unsigned *>(d_head + 1);
   int64_t *d_start = ctx.d_items.as<int64_t>(np);
-  int32_t *d_redo = margin >= 0 ? ctx.d_near.as<int32_t>(np) : nullptr;
+  int32_t *d_redo = wide ? nullptr : ctx.d_near.as<int32_t>(np);
   PlanHead &head = *static_cast<PlanHead *>(ctx.h_head.need(sizeof(PlanHead)));
   const int64_t target = (int64_t)ctx.num_sms * 8 * (512 / kB);
   // FP64 sums and large mixed ones are cut along curve 2; a lone FP64 pair has
@@ -1411,7 +1422,7 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   for (int attempt = 0;; ++attempt) {
     const int64_t cap = ctx.direct_items;
     DirectArgs A{d_xyz, d_off, d_pairs, d_start, ctx.d_loops.as<int32_t>(cap), (int32_t)np, cap, target, least, kB, few, lone,
-                 d_head, d_rank, ctx.num_sms, ctx.d_partial.as<double>(cap), (float)near_factor};
+                 d_head, d_rank, ctx.num_sms, ctx.d_partial.as<double>(cap), (float)near_factor, wide};
     if (np <= kPlanSmall && nloops <= 16 * kPlanSmall) {
       plan_small<<<1, 1024, 0, st>>>(A, nloops);
     } else {
@@ -1453,10 +1464,12 @@ DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t 
   ctx.stats.ms_main_kernel += ms;
   R.near_terms = (double)head.near;
   R.work = head.work;
-  R.redone = (int64_t)head.redo;
-  R.complete = tail && R.redone == 0;
-  if (R.redone > 0)
-    R.launches += recompute_pairs(ctx, d_xyz, d_off, nloops, d_pairs, d_redo, R.redone, d_lk, d_flags);
+  const int64_t redo = (int64_t)head.redo;
+  const bool mixed = precision == FLN_PREC_MIXED;
+  if (mixed) R.redone = redo;
+  R.complete = tail && redo == 0;
+  if (redo > 0)
+    R.launches += recompute_pairs(ctx, d_xyz, d_off, nloops, d_pairs, d_redo, redo, d_lk, mixed ? d_flags : nullptr);
   return R;
 }
 
@@ -1650,7 +1663,7 @@ extern "C" fln_status fln_linking_numbers_direct_noalloc(const double *d_xyz, co
   const bool few = few_items((int64_t)h.items, h.work, most);
   const DirectArgs A{d_xyz, d_loop_offsets, d_pairs, reinterpret_cast<int64_t *>(scratch + kNaStart), nullptr,
                      (int32_t)npairs, (int64_t)h.items, 1, 1e300, kBlockSegs, few ? most : 0, 0, reinterpret_cast<PlanHead *>(scratch), nullptr, sms,
-                     reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor};
+                     reinterpret_cast<double *>(scratch + kNaPartial), (float)kDefaultNearFactor, true};
   launch_direct(0, s, sms, precision, (int64_t)h.items, few ? SumKernel::kFew : SumKernel::kMany, A);
   reduce_items_kernel<<<(int)((npairs + 7) / 8), 256, 0, s>>>(A, -1.0, d_lk_out, nullptr, nullptr, nullptr);
   e = cudaGetLastError();

@@ -193,7 +193,9 @@ constexpr int kDefaultBhCtas = 6;  // fln_params.bh_occupancy 0
 // Checks the offsets and pairs; throws FLN_ERR_INVALID_ARGUMENT before any sum
 // is written when they are bad. margin >= 0: pairs whose distance to the
 // rounding boundary is below it, or which are not finite, are recomputed in
-// FP64 (FLN_PAIR_FP64_RECOMPUTED). d_err and d_flags may be null; they get 0
+// FP64 (FLN_PAIR_FP64_RECOMPUTED). Of an FP64 sum, pairs whose products leave
+// the kernel's range are summed again by the wide kernel (wide: all pairs are,
+// at once). d_err and d_flags may be null; they get 0
 // otherwise. tile_shape: index into the direct sum's tile shapes
 // (fln_params.direct_tile).
 struct DirectResult {
@@ -216,7 +218,7 @@ constexpr int kDirectTileShapes = 6;
 DirectResult direct_sum_device(Context &ctx, const double *d_xyz, const int64_t *d_off, int32_t nloops,
                                const int32_t *d_pairs, int64_t npairs, int precision, double near_factor,
                                double margin, double *d_lk, double *d_err, int32_t *d_flags, int tile_shape = 0,
-                               const DirectTail *tail = nullptr);
+                               const DirectTail *tail = nullptr, bool wide = false);
 
 // FP64 direct sums of the n pairs in d_list (indices into d_pairs), written
 // back to d_lk; d_flags (may be null) gets FLN_PAIR_FP64_RECOMPUTED there.
