@@ -367,7 +367,7 @@ def run_ours(args, rank, world, local_rank):
                 "algorithmic_bytes_per_launch": alg, "far_node_pairs_per_step": far,
                 "exact_node_pairs_per_step": ent, "ms_per_launch": trav_ms,
                 "dram_gbs": dram_gbs, "dram_frac": dram_gbs / peaks["hbm_gbs"] if dram_gbs else None,
-                "limiter": "L1 wavefronts and dependent-load latency (node records are re-read from L1/L2); "
+                "limiter": "latency of dependent loads (node records are re-read from L1/L2); "
                            "DRAM runs at dram_frac of the copy peak",
                 "alone": None if alone is None else {
                     "note": "one untimed step with each exact list after its traversal on one stream",
@@ -562,8 +562,9 @@ def main():
     ap.add_argument("--loop-steps", type=int, default=50000)
     ap.add_argument("--cpu-seconds", type=float, default=15.0)
     ap.add_argument("--direct-sample", type=int, default=64)
-    ap.add_argument("--traffic-bytes-per-node-pair", type=float, default=66.4,
-                    help="DRAM bytes per node pair measured by ncu on the polymer workload (0: none)")
+    ap.add_argument("--traffic-bytes-per-node-pair", type=float, default=67.3,
+                    help="DRAM bytes per node pair measured by ncu on the polymer workload: 69 in the first pass, 65 in "
+                         "the retry, weighted by their time (0: none)")
     ap.add_argument("--cli-leg", type=int, default=1,
                     help="also time the verifycurves CLI end to end on the workload written as BCC")
     ap.add_argument("--bh-bucket", type=int, default=0,

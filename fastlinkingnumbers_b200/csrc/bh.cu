@@ -949,7 +949,8 @@ __device__ __noinline__ double seg_term_fp64(const double *xyz, int64_t p0i, int
 // left to FP64 (seg_term_fp64).
 
 // arctan(t) for |t| <= 1/4 from its Maclaurin series t - t^3/3 + t^5/5 - t^7/7
-// + t^9/9; the first omitted term is below 2.2e-8 |t|, under FP32 rounding.
+// + t^9/9; the first omitted term, t^11/11, is below 8.7e-8 |t| (2.2e-8 at 1/4),
+// about one rounding of FP32 there and less for smaller angles.
 __device__ __forceinline__ float atan_quarter(float t) {
   const float u = t * t;
   float p = fmaf(u, 1.0f / 9.0f, -1.0f / 7.0f);
@@ -1797,14 +1798,17 @@ FLN_TRAVERSE_KERNELS(7)
 // rounds of a small call, the last heavy loop pairs of a large one) a step
 // costs its load latency and most warps have nothing to do, so the stacks are
 // handed on early; with several batches per warp the longer budget saves
-// rounds and hand-overs. B200, whole calls, one budget throughout: 60 walks of
-// 2,000 steps 2.05 ms at 128 and 1.46 at 16; mixed sizes (28M segments) 25.8 ms
-// at 128, 23.8 at 16, 23.4 at 32; 200 walks of 50,000 steps 121.9 ms at 128,
-// 124.6 at 32 and 135 at 16. By this rule: 1.45, 23.2 and 120.4 ms.
-// Calls of fewer than kShortRounds segments keep the full budget: they end
-// after a round or two either way, and the sums of unlinked loops, which are
-// nothing but errors of 1e-3 and less, show in their ninth digit how the
-// partial sums were grouped when each is rounded to 2^-40.
+// rounds and hand-overs. B200, whole calls, one budget throughout, when the rule
+// was made: 60 walks of 2,000 steps 2.05 ms at 128 and 1.46 at 16; mixed sizes
+// (28M segments) 25.8 ms at 128, 23.8 at 16, 23.4 at 32; 200 walks of 50,000 steps
+// 121.9 ms at 128, 124.6 at 32 and 135 at 16; by the rule 1.45, 23.2 and 120.4 ms.
+// Calls of fewer than kShortRounds segments keep the full budget, for their
+// digits and not for their time: the sums of unlinked loops, which are nothing
+// but errors of 1e-3 and less, show in their ninth digit how the partial sums
+// were grouped when each is rounded to 2^-40. They take four to seven rounds,
+// and short ones would be faster: 50 walks of 1,500 steps (107,000 segments) 1.79
+// ms at 128, 1.09 at 32, 0.98 at 16; 60 of 500 (46,000) 1.06, 0.74, 0.64; 10 of 1,000
+// (13,000) 1.36, 0.75, 0.66. (fln_params.bh_budget gives them short rounds.)
 constexpr int64_t kShortRounds = int64_t(1) << 17;
 int round_budget(int budget, int64_t segments, int64_t work, int64_t warps) {
   if (segments < kShortRounds) return budget;

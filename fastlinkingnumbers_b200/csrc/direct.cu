@@ -2,12 +2,12 @@
 //
 // Work: every potential loop pair (i, j) is split into items: kBlockSegs
 // consecutive segments of its longer loop ("curve 1") against a span of the
-// other; one CTA of kBlockSegs threads takes items from a device work queue
-// (an atomic counter) until it runs dry, so all pairs — 16-segment rings to
-// 2^18-segment loops — run in one persistent launch. The items are planned on
-// the device (plan_items), so that a call has one host wait. Each thread owns
-// one or two curve-1 segments and walks curve-2 segments, which the CTA stages
-// tile by tile in shared memory (coalesced loads, broadcast reads). Per segment pair it evaluates the
+// other; a CTA takes items from a device work queue (an atomic counter) until it
+// runs dry, so all pairs — 16-segment rings to 2^18-segment loops — run in one
+// persistent launch. The items are planned on the device (plan_items), so that a
+// call has one host wait. Each thread owns one or two curve-1 segments and walks
+// curve-2 segments, which the CTA stages tile by tile in shared memory (coalesced
+// loads, broadcast reads). Per segment pair it evaluates the
 // closed-form solid-angle term of Arai 2013 as the reference does
 // (src/compute_link.cpp:126-178, :200-280): with a = q_k - p_i,
 // b = q_k - p_{i+1}, c = q_{k+1} - p_{i+1}, d = q_{k+1} - p_i,
@@ -25,14 +25,16 @@
 //    ComputeLinkingNumberDirectFast (Bertolazzi et al. 2019) — a running
 //    complex product with a count of negative-x-axis crossings — and one
 //    atan2 per thread per item. The product is rescaled by an exact power of
-//    two each step instead of the reference's division.
-//  * MIXED: coordinates relative to the tile's first vertex in FP32, one
-//    FP32 atan2 per segment pair, FP32 sums over one tile of kTile terms and
-//    FP64 sums above that. det uses the identity det = a . (f x e) with
-//    e = p_{i+1} - p_i and f = q_{k+1} - q_k, which keeps its relative
-//    accuracy for distant pairs. A segment pair whose closest endpoint
-//    distance is below near_factor x (longer segment length) is recomputed
-//    in FP64 (near-singular terms).
+//    two every second step instead of the reference's division (range: see
+//    kLeastScale).
+//  * MIXED: coordinates relative to the tile's first vertex in FP32, one FP32
+//    arctangent per segment pair (a series for small angles, else atan2f), FP32
+//    sums over runs of 32 terms and FP64 sums above that. det uses the identity
+//    det = a . (f x e) with e = p_{i+1} - p_i and f = q_{k+1} - q_k, which keeps
+//    its relative accuracy for distant pairs. A segment pair whose closest
+//    endpoint distance is below near_factor x (longer segment length), or below
+//    kNearLeast, is evaluated in FP64 (near-singular and too small terms). FP32
+//    holds a term, 64 d^6, up to distances d of 9e5 from the tile's segments.
 // Item results go to one FP64 partial per item; a second kernel sums them
 // per pair in a fixed order, so results are deterministic.
 #include <cuda_runtime.h>
@@ -93,9 +95,10 @@ struct DirectArgs {
 // segments is cut along curve 2 as well, so that it fills the chip and ends
 // evenly: `target` items (eight per resident CTA) of about the same work, down
 // to 32 segments, below which a CTA's start costs more than its terms. The
-// mixed precision does so only from kMixedSpans segment pairs: cutting a walk
-// regroups its FP64 sum, and below that the sums stay bit for bit those of one
-// walk per segment (all there is to see when no loops are linked).
+// mixed precision does so only from kMixedSpans segment pairs. That line is no
+// measured one: cutting a walk regroups its FP64 sum, and below it the sums stay
+// bit for bit those of one walk per segment (all there is to see when no loops
+// are linked).
 constexpr double kMixedSpans = 1 << 30;
 // A lone pair goes to direct_fp64_lone_kernel, 32 curve-1 segments an item, when
 // its items are resident at once, two CTAs per SM. The kernel is for loops that
@@ -367,9 +370,9 @@ __device__ __noinline__ double sum_terms(const double *xyz, int64_t o1, int64_t 
 // plus one for every other instruction; hence the sign tests in a rare branch,
 // the tile in 16-byte loads, the rescaling once per two steps and the
 // two-state walk. 12 walks of 4,001 steps (1.84e9 segment pairs), B200: 12.6 ms
-// with one segment per thread, 8.0 with two, 7.6 with the two-state walk, 6.9
-// with the rest (267 G segment pairs/s; 372 G at 200 cycles a step). Twelve
-// warps of 144 registers per SM; sixteen of 128 took 7.1 ms.
+// with one segment per thread, 8.0 with two, 7.6 with the two-state walk, 6.8
+// with the rest (269 G segment pairs/s; 372 G at 200 cycles a step). Twelve
+// warps of 152 registers per SM; sixteen of 128 took 7.1 ms.
 //
 // Range: a term is at most 64 d^6 at a distance d, and two terms are multiplied
 // between rescalings, so the product overflows above d = 1e25 and loses digits
@@ -635,7 +638,8 @@ __device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, f
 }
 
 // arctan(t) for |t| <= 1/4 from its Maclaurin series t - t^3/3 + t^5/5 - t^7/7
-// + t^9/9; the first omitted term is below 2.2e-8 |t|, under FP32 rounding.
+// + t^9/9; the first omitted term, t^11/11, is below 8.7e-8 |t| (2.2e-8 at 1/4),
+// about one rounding of FP32 there and less for smaller angles.
 __device__ __forceinline__ F2 atan_small2(F2 t) {
   auto c = [](float v) { return pack2(v, v); };
   const F2 u = mul2(t, t);
@@ -790,7 +794,7 @@ __device__ __forceinline__ void mix_step(const MixSegs &S, const MixWalk &a, Mix
 // B200, whole call: 22.6 ms with one scalar segment per thread and near pairs
 // as a divergent call; 16.7 packed with the near queue; 14.7 with the near and
 // slow terms in one branch, subnormals flushed in the reciprocal and root, and
-// cuts along curve 2. 10,000 linked rings: 1.49 -> 0.87 ms of kernel. Sixteen
+// cuts along curve 2. 10,000 linked rings: 1.49 -> 0.75 ms of kernel. Sixteen
 // warps of 128 registers per SM: 12 of 162 take 14.9 ms, 20 of 96 16.0.
 template <int kB, int kT>
 __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectArgs A) {

@@ -76,7 +76,8 @@ typedef struct fln_params {
   int32_t precision;            /* fln_precision; default FLN_PREC_MIXED */
   double fp64_margin;           /* recompute in FP64 when 0.5 - |lk - round(lk)| < this; default 0.25 */
   double near_factor;           /* mixed direct sum: a segment pair whose closest endpoint distance is
-                                   below near_factor * (longer segment length) is evaluated in FP64; 4.0 */
+                                   below near_factor * (longer segment length) is evaluated in FP64; 4.0.
+                                   One nearer than 1e-6 is as well (unless near_factor is 0) */
   int32_t bh_tree;              /* Barnes–Hut tree: 0 = curve-order tree (default), 1 = the reference's
                                    kd-median tree (ModifiedKdBVH.h:207-237) */
   int32_t bh_escalations;       /* after the reference's retry, a pair whose scaled error estimate is still
@@ -89,9 +90,10 @@ typedef struct fln_params {
   int32_t host_prepare;         /* fln_certificate_compute: 0 = Discretize and the potential-link searches
                                    on the context's GPU (default), 1 = on the host; same output bit for bit */
   int32_t bh_budget;            /* most traversal steps a warp spends on a batch per launch before handing
-                                   the rest on; 0 = 128. Launches with few batches hand on after 16 or 32
-                                   steps, so that idle warps get work. The node pairs stay the same; only the grouping of
-                                   the FP64 partial sums changes (last-bit differences). */
+                                   the rest on; 0 = 128. In calls of 2^17 segments and more, launches with
+                                   few batches hand on after 16 or 32 steps, so that idle warps get work.
+                                   The node pairs stay the same; only the grouping of the FP64 partial sums
+                                   changes (last-bit differences). */
   int32_t bh_bucket;            /* curve-order trees, bh_schedule 0: a node pair that is neither far nor a
                                    leaf pair and has at most this many segments a side is summed exactly,
                                    segment pair by segment pair; 0 = 8, 1 = leaf pairs only (the
@@ -180,7 +182,15 @@ void fln_default_params(fln_params *p);
  * (as an opaque pointer) is used and not destroyed. The context also keeps
  * two internal streams (the pieces of a pinned vertex copy; the Barnes-Hut
  * exact-list launches), joined back to `stream` by events before a call's
- * results are read, so work queued on `stream` after a call sees them. */
+ * results are read, so work queued on `stream` after a call sees them.
+ *
+ * Device memory: a context keeps its buffers from call to call, sized for the
+ * largest so far, and gives them back when it is destroyed. The largest are a
+ * Barnes-Hut call's trees (384 bytes per segment), its frontier (3,616 bytes
+ * per 128 far node pairs; the first buffer up to a fifth of the free memory,
+ * 32 GB at most, later ones up to half of it if a call has written more; none
+ * with bh_retry_from_roots), its work lists (about 3 GB), and up to 4 GB of
+ * Discretize's buffers. */
 fln_status fln_ctx_create(int device, void *stream, fln_ctx **out);
 void fln_ctx_destroy(fln_ctx *ctx);
 fln_status fln_ctx_stats(const fln_ctx *ctx, fln_stats *out);
@@ -220,8 +230,9 @@ fln_status fln_linking_numbers_device(fln_ctx *ctx, const double *d_xyz,
  * over pairs); larger calls return FLN_ERR_INVALID_ARGUMENT. precision is
  * FLN_PREC_FP64 or FLN_PREC_MIXED; the results are the raw sums of that
  * precision (no margin recompute), the mixed one with the default
- * near_factor, 4.0, so they equal those of fln_linking_numbers_device with
- * the same precision and fp64_margin = 0. Work is queued on `stream` (a
+ * near_factor, 4.0, so they are those of fln_linking_numbers_device with the
+ * same precision and fp64_margin = 0 but for the order of FP64 additions (the
+ * other call cuts long walks into spans). Work is queued on `stream` (a
  * cudaStream_t, NULL = default stream) of the current device. Every call
  * reads the plan's size and status back to the host, so it blocks the
  * calling thread until the work queued earlier on `stream` and a small
