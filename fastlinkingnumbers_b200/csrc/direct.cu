@@ -673,9 +673,9 @@ __device__ __forceinline__ void block_minmax7(float *lo, float *hi, float (*s_bo
   }
 }
 
-// Lanes of a warp with a near pair from which each evaluates its own (24 / 30 /
-// 32 / never: 100 walks of 60 steps on one spot 501 / 511 / 523 / 560 us a call,
-// 100 x 100 linked rings 824 / 823 / 812 / 801).
+// Lanes of a warp with a near pair from which each evaluates its own (24 / never:
+// 100 walks of 60 steps on one spot 480 / 543 us a call, 12 walks of 20,000 76.1 /
+// 80.2 ms, 100 x 100 linked rings 857 / 816 us).
 constexpr int kDenseNear = 24;
 
 // A tile vertex: q relative to the tile's origin and the segment f to the next
@@ -783,9 +783,12 @@ __device__ __forceinline__ void mix_step(const MixSegs &S, const MixWalk &a, Mix
 // together, 32 of a queue at a time, or by their own lanes where nearly all have
 // one (kDenseNear), and added to their segment's sum in order. (A lane finds the
 // queued pairs of its segments by one match of the 32 owners; looking through
-// all 32 cost as much as the terms: 100 x 100 linked rings 954 us a call, 824
-// now; 100 walks of 60 steps on one spot, nearly all pairs near, 856 -> 501, 794
-// by one scalar segment per thread with near pairs as a divergent call.)
+// all 32 cost as much as the terms: 100 x 100 linked rings 954 us a call, 857
+// now; 100 walks of 60 steps on one spot, nearly all pairs near, 849 -> 480, 786
+// by one scalar segment per thread with near pairs as a divergent call. The walk
+// of far pairs pays for the registers of this code, by 0 to 8 % for one form or
+// another of it: one loop with a single place of evaluation took 4 % more on 12
+// walks of 20,000 steps, 4 % less on the rings.)
 //
 // Bound: issue and the FMA pipe together. A step of 64 segment pairs needs 50
 // packed and 8 scalar FMA-pipe operations (108 cycles of a scheduler's pipe, 709
@@ -845,6 +848,30 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
     }
     double acc0 = 0.0, acc1 = 0.0, near0 = 0.0, near1 = 0.0;
     int turns0 = 0, turns1 = 0, queued = 0;
+    // Evaluates the oldest n queued pairs (n <= 32); every lane adds those of its
+    // segments, oldest first.
+    auto flush = [&](int n) {
+      int2 q = make_int2(32 + lane, 0);  // (of no lane's segments)
+      if (lane < n) {
+        q = queue[lane];
+        term[lane] = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)(it.first + (q.x >> 5)), q.y));
+      }
+      mine[lane] = 0;
+      __syncwarp();
+      const unsigned of = __match_any_sync(0xffffffffu, lane < n ? q.x & 31 : q.x);
+      if (lane < n) mine[q.x & 31] = of;
+      __syncwarp();
+      for (unsigned m = mine[lane]; m; m &= m - 1) {
+        const int x = __ffs(m) - 1;
+        if (queue[x].x >> 5 == at) near0 += term[x];
+        else near1 += term[x];
+      }
+      __syncwarp();
+      q = queue[32 + lane];
+      __syncwarp();
+      queue[lane] = q;
+      __syncwarp();
+    };
     for (int64_t k0 = it.k0; k0 < it.k1; k0 += kT) {  // a span is a multiple of kT (kMixedSpans)
       const int kt = (int)min(it.k1 - k0, (int64_t)kT);
       const double3 O = load_v(A.xyz, o2 + k0);
@@ -940,67 +967,43 @@ __global__ void __launch_bounds__(kB / 2, 1024 / kB) direct_mixed_kernel(DirectA
           acc1 += (double)sum1;
           if (!second) near_mask1 = 0;
         }
-        // The run's near pairs, one per lane at a time: evaluated at once when
-        // most lanes have one, else queued, and 32 of the queue evaluated
-        // together, oldest first (what is left, before lanes evaluate their own
-        // and at the item's end). A lane adds the pairs of its segments in order.
-#pragma unroll 1
-        for (;;) {
+        // This run's near pairs, one per lane at a time: evaluated at once when
+        // most lanes have one (after what is queued: a lane adds its segments'
+        // pairs in order), else queued, and 32 of the queue evaluated together.
+        while (__any_sync(0xffffffffu, (near_mask0 | near_mask1) != 0)) {
           const bool has = (near_mask0 | near_mask1) != 0;
           const unsigned m = __ballot_sync(0xffffffffu, has);
-          const bool dense = __popc(m) >= kDenseNear, own = dense && queued == 0;
-          if (m == 0 && !(queued > 0 && k0 + kT >= it.k1 && r + 1 == rounds)) break;
-          int2 q = make_int2(0, 0);  // (segment of the item x 32 + lane, curve-2 segment)
-          bool valid = false;
-          if (own || (m && !dense)) {
-            if (has) {
-              const bool first = near_mask0 != 0;
-              const int k = __ffs(first ? near_mask0 : near_mask1) - 1;
-              if (first) near_mask0 &= near_mask0 - 1;
-              else near_mask1 &= near_mask1 - 1;
-              q = make_int2((first ? at : at + 1) << 5 | lane, (int)(k0 + j0 + k));
-              if (!own) queue[queued + __popc(m & below)] = q;
+          near_count += lane == 0 ? __popc(m) : 0;
+          const bool dense = __popc(m) >= kDenseNear;
+          if (dense && queued > 0) {
+            flush(queued);
+            queued = 0;
+          }
+          if (has) {
+            const bool first = near_mask0 != 0;
+            const int k = __ffs(first ? near_mask0 : near_mask1) - 1;
+            if (first) near_mask0 &= near_mask0 - 1;
+            else near_mask1 &= near_mask1 - 1;
+            const int seg = first ? at : at + 1, step = (int)(k0 + j0 + k);
+            if (dense) {
+              const double v = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)it.first + seg, step));
+              if (first) near0 += v;
+              else near1 += v;
+            } else {
+              queue[queued + __popc(m & below)] = make_int2(seg << 5 | lane, step);
             }
-            near_count += lane == 0 ? __popc(m) : 0;
-            valid = own && has;
-            if (!own) {
-              queued += __popc(m);
-              __syncwarp();
-              if (queued < 32) continue;
-            }
           }
-          const int n = min(queued, 32);
-          if (!own) {
-            valid = lane < n;
-            q = queue[lane];
+          if (dense) continue;
+          queued += __popc(m);
+          __syncwarp();
+          if (queued >= 32) {
+            flush(32);
+            queued -= 32;
           }
-          double v = 0.0;
-          if (valid) v = near_term(A.xyz, o1, n1, o2, n2, make_int2((int)it.first + (q.x >> 5), q.y));
-          if (own) {
-            if (q.x >> 5 == at) near0 += v;
-            else near1 += v;
-            continue;
-          }
-          if (valid) term[lane] = v;
-          mine[lane] = 0;
-          __syncwarp();
-          const unsigned of = __match_any_sync(0xffffffffu, valid ? q.x & 31 : 32 + lane);
-          if (valid) mine[q.x & 31] = of;
-          __syncwarp();
-          for (unsigned b = mine[lane]; b; b &= b - 1) {
-            const int x = __ffs(b) - 1;
-            if (queue[x].x >> 5 == at) near0 += term[x];
-            else near1 += term[x];
-          }
-          __syncwarp();
-          q = queue[32 + lane];
-          __syncwarp();
-          queue[lane] = q;
-          __syncwarp();
-          queued -= n;
         }
       }
     }
+    if (queued > 0) flush(queued);
     // The item's sum: 32 segments at a time by a butterfly, those sums in order.
     for (int g = 0; g < groups; ++g) {
       if (grp == g) {
