@@ -390,7 +390,7 @@ def run_ours(args, rank, world, local_rank):
                          "radius) per node pair handed to the exact list; traffic = DRAM read+write per "
                          "node pair from the small-case ncu captures in "
                          "profiles/bh_traverse_bh_buckets_polymer_6M.md x node pairs; node records are "
-                         "mostly re-read from L1/L2: the kernel is bound by L1 wavefronts and latency, not "
+                         "mostly re-read from L1/L2: the kernel is bound by the latency of dependent loads, not "
                          "by HBM. In the timed steps each round's exact list runs beside the next "
                          "traversal on a second stream, so a traversal launch's events include the time "
                          "the two kernels share the SMs; 'alone' times them one after the other")}

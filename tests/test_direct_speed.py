@@ -71,7 +71,7 @@ def test_allocation_free_call_of_few_items(loops, steps):
 @pytest.mark.parametrize("loops,steps,most", [(10, 60, 2.6), (20, 100, 4.4), (20, 130, 4.8), (100, 60, 3.4)])
 def test_mixed_sum_of_near_loops(loops, steps, most):
     """Loops on one spot, nearly all segment pairs near ones: the mixed sum evaluates them in FP64
-    about as fast as lanes can (2.2, 2.2, 2.8 and 2.6 times the FP64 sum; it was 3.2, 6.8, 7.0
+    about as fast as lanes can (2.0, 2.1, 2.3 and 2.4 times the FP64 sum; it was 3.2, 6.8, 7.0
     and 4.3 when a warp looked for every pair's owner in turn)."""
     c = Calls(*walks([steps] * loops, 5, 1.0), all_pairs(loops))
     assert c.time(c.allocating, N.PREC_MIXED) < most * c.time(c.allocating, N.PREC_FP64)
