@@ -73,7 +73,9 @@ typedef struct fln_params {
   double epssq;                 /* 1e-24 CERTIFICATE_EPSSQ (lnc.cpp:24) */
   double target_error;          /* 0.1   TARGET_ERROR (lnc.cpp:25) */
   double error_est_scale;       /* 0.05  ERROR_EST_SCALE (lnc.cpp:26) */
-  int32_t precision;            /* fln_precision; default FLN_PREC_MIXED */
+  int32_t precision;            /* fln_precision; default FLN_PREC_MIXED. Direct sums: the mixed precision holds
+                                   distances between the curves of 1e-17 to 9e5 (its terms are products of
+                                   six in FP32), FP64 1e-50 to 1e50; linking numbers do not depend on the unit */
   double fp64_margin;           /* recompute in FP64 when 0.5 - |lk - round(lk)| < this; default 0.25 */
   double near_factor;           /* mixed direct sum: a segment pair whose closest endpoint distance is
                                    below near_factor * (longer segment length) is evaluated in FP64; 4.0.
